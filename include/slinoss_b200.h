@@ -209,6 +209,39 @@ int slx_v2x2ssd_bwd_finish(const slx_scan_shape *s, const void *U, const float *
                            float *dB_prev /*[opt]*/, float *dU_prev /*[opt]*/,
                            void *workspace, size_t workspace_bytes, void *stream);
 
+/* The whole op with the streaming tensors in the dtypes their owners hold them (an slx_dtype
+ * code beside each pointer) and with everything a carried stream needs written by the op's own
+ * kernels: no conversion or copy launches around the call.  Every pointer is optional. */
+typedef struct {
+  const void *initial_states; /* (BH,P,2N)                                              */
+  const void *B_prev, *U_prev; /* (BH,2N), (BH,P), both or neither, both as prev_dtype:
+                                * SLX_F32 or the activation dtype                      */
+  void *final_copy;            /* (BH,P,2N): the final state once more, as final_dtype   */
+  void *B_last, *U_last;       /* (BH,2N), (BH,P): row T-1 of B and U, activation dtype  */
+  int32_t initial_dtype, prev_dtype, final_dtype;
+} slx_scan_ends;
+/* As slx_v2x2ssd_fwd; e and final_state (fp32) may be NULL, and so may Y: then only the chunk
+ * states are computed. */
+int slx_v2x2ssd_fwd_stream(const slx_scan_shape *s, const void *U, const float *M,
+                           const float *K, const void *B, const void *C,
+                           const slx_scan_ends *e /*[opt]*/, void *Y /*[opt]*/,
+                           float *final_state /*[opt]*/, void *chunk_starts,
+                           float *m_chunk, void *increments /*[opt]*/, void *stream);
+typedef struct {
+  const void *B_prev, *U_prev; /* as in the forward                                      */
+  const void *d_final;         /* (BH,P,2N) as d_final_dtype                             */
+  void *d_initial;             /* (BH,P,2N) as d_initial_dtype                           */
+  void *dB_prev, *dU_prev;     /* (BH,2N), (BH,P) as d_prev_dtype                        */
+  int32_t prev_dtype, d_final_dtype, d_initial_dtype, d_prev_dtype;
+} slx_scan_grad_ends;
+/* As slx_v2x2ssd_bwd; e may be NULL.  Same workspace. */
+int slx_v2x2ssd_bwd_stream(const slx_scan_shape *s, const void *U, const float *M,
+                           const float *K, const void *B, const void *C,
+                           const slx_scan_grad_ends *e /*[opt]*/, const void *chunk_starts,
+                           const float *m_chunk, const float *final_state, const void *dY,
+                           void *dU, float *dM, float *dK, void *dB, void *dC,
+                           void *workspace, size_t workspace_bytes, void *stream);
+
 /* ---- segment chaining across devices (no counterpart in the reference) ------ */
 
 /* A segment of a sequence acts on the incoming scan state as z_out = m_seg * z_in + f
@@ -267,6 +300,28 @@ int slx_scanprep_bwd(const slx_prep_shape *s, const void *params, const void *bc
                      float *d_bias, float *d_scale, void *workspace,
                      size_t workspace_bytes, void *stream);
 
+/* The layer's learnable parameters as they lie: seven per-head biases (dt, gamma, omega,
+ * mix_r, mix_theta, mix_k_prev, mix_k_curr; H values each) and the RMS-norm scales
+ * (H,2,N) of B and C [needed iff normalize_bc], all in one dtype. */
+typedef struct {
+  const void *bias[7];
+  const void *b_scale, *c_scale;
+  int32_t dtype;
+} slx_prep_params;
+
+/* slx_scanprep_fwd / _bwd on the parameters themselves: nothing is gathered or converted
+ * around the call.  The parameter gradients are written in the parameters' dtype: d_bias
+ * (7,H), d_b_scale and d_c_scale (H,2,N). */
+int slx_scanprep_fwd_params(const slx_prep_shape *s, const void *value, const void *params,
+                            const void *bc, const slx_prep_params *p, void *U, float *M,
+                            float *K, void *B, void *C, void *stream);
+int slx_scanprep_bwd_params(const slx_prep_shape *s, const void *params, const void *bc,
+                            const slx_prep_params *p, const void *dU, const float *dM,
+                            const float *dK, const void *dB, const void *dC, void *d_value,
+                            void *d_params, void *d_bc, void *d_bias, void *d_b_scale,
+                            void *d_c_scale, void *workspace, size_t workspace_bytes,
+                            void *stream);
+
 /* ---- one-token decode step ------------------------------------------------- */
 
 typedef struct {
@@ -293,6 +348,16 @@ int slx_decode_step(const slx_decode_shape *s, const void *value, const void *pa
                     const void *b_prev /*[opt]*/, const void *u_prev /*[opt]*/, void *out,
                     float *state_out, void *b_last /*[opt]*/, void *u_last /*[opt]*/,
                     void *stream);
+
+/* slx_decode_step on the layer's own parameters, with value, params, bc and gate as column
+ * slices of one projection row: batch_strides = elements between the batches of value, params,
+ * bc and gate [NULL = contiguous]; skip (heads, P) in any dtype. */
+int slx_decode_step_params(const slx_decode_shape *s, const void *value, const void *params,
+                           const void *bc, const void *gate, const int64_t *batch_strides /*[opt]*/,
+                           const void *skip, int32_t skip_dtype, const slx_prep_params *p,
+                           const float *state_in /*[opt]*/, const void *b_prev /*[opt]*/,
+                           const void *u_prev /*[opt]*/, void *out, float *state_out,
+                           void *b_last /*[opt]*/, void *u_last /*[opt]*/, void *stream);
 
 /* ---- depthwise causal conv1d --------------------------------------------- */
 
@@ -333,6 +398,13 @@ int slx_cconv1d_bwd(const slx_conv_shape *s, const void *x, const void *weight,
                     const void *d_next_state, void *dx, float *dweight,
                     float *dbias, float *dstate, void *workspace,
                     size_t workspace_bytes, void *stream);
+
+/* slx_cconv1d_bwd with dweight, dbias and dstate written as grad_dtype (the fp32 sums rounded once). */
+int slx_cconv1d_bwd_as(const slx_conv_shape *s, const void *x, const void *weight,
+                       const void *bias, const void *state, const void *dy,
+                       const void *d_next_state, void *dx, void *dweight, void *dbias,
+                       void *dstate, int32_t grad_dtype, void *workspace,
+                       size_t workspace_bytes, void *stream);
 
 /* Same computation and results as slx_cconv1d_bwd, for callers that cannot hand
  * over a workspace because they cannot allocate device memory at call time: a
@@ -380,6 +452,15 @@ int slx_gate_skip_bwd(const slx_glue_shape *s, const void *y, const void *u,
                       const void *gate, const float *skip, const void *d_out, void *dy,
                       void *du, void *d_gate, float *d_skip, void *workspace,
                       size_t workspace_bytes, void *stream);
+
+/* The two calls with skip (and its gradient) in any dtype. */
+int slx_gate_skip_fwd_as(const slx_glue_shape *s, const void *y, const void *u,
+                         const void *gate, const void *skip, int32_t skip_dtype, void *out,
+                         void *stream);
+int slx_gate_skip_bwd_as(const slx_glue_shape *s, const void *y, const void *u,
+                         const void *gate, const void *skip, int32_t skip_dtype,
+                         const void *d_out, void *dy, void *du, void *d_gate, void *d_skip,
+                         void *workspace, size_t workspace_bytes, void *stream);
 
 /* ---- diagnostics ----------------------------------------------------------- */
 

@@ -1,4 +1,5 @@
-"""ctypes binding of ``libslinoss_b200.so`` (the C ABI in ``include/slinoss_b200.h``).
+"""Binding of ``libslinoss_b200.so`` (the C ABI in ``include/slinoss_b200.h``): ``host()`` is the native
+extension the ops run through, ``lib()`` the ctypes view of every entry point (stages, tests, benchmark).
 
 The library is the only compute path of this package: if it is missing or a
 symbol is absent, the import of any op fails loudly -- there is no CPU or
@@ -8,6 +9,7 @@ framework fallback.
 from __future__ import annotations
 
 import ctypes
+import importlib.util
 import os
 from ctypes import POINTER, Structure, c_char_p, c_float, c_int32, c_int64, c_size_t, c_void_p
 from pathlib import Path
@@ -62,6 +64,8 @@ SIGNATURES = {
     "slx_state_passing_fwd": (c_int32, [c_int32] * 4 + [_P, c_int32] + [_P] * 3 + [c_int32] + [_P] * 2),
     "slx_chunk_scan_fwd": (c_int32, [POINTER(ScanShape)] + [_P] * 10),
     "slx_v2x2ssd_fwd": (c_int32, [POINTER(ScanShape)] + [_P] * 14),
+    "slx_v2x2ssd_fwd_stream": (c_int32, [POINTER(ScanShape)] + [_P] * 12),
+    "slx_v2x2ssd_bwd_stream": (c_int32, [POINTER(ScanShape)] + [_P] * 16 + [c_size_t, _P]),
     "slx_v2x2ssd_bwd_workspace_bytes": (c_size_t, [POINTER(ScanShape)]),
     "slx_chunk_scan_bwd_dz0": (c_int32, [POINTER(ScanShape)] + [_P] * 4 + [c_int32, _P]),
     "slx_state_passing_bwd_partials_bytes": (c_size_t, [c_int32] * 4),
@@ -73,6 +77,12 @@ SIGNATURES = {
     "slx_scanprep_fwd": (c_int32, [POINTER(PrepShape)] + [_P] * 11),
     "slx_scanprep_bwd_workspace_bytes": (c_size_t, [POINTER(PrepShape)]),
     "slx_scanprep_bwd": (c_int32, [POINTER(PrepShape)] + [_P] * 15 + [c_size_t, _P]),
+    "slx_scanprep_fwd_params": (c_int32, [POINTER(PrepShape)] + [_P] * 10),
+    "slx_scanprep_bwd_params": (c_int32, [POINTER(PrepShape)] + [_P] * 15 + [c_size_t, _P]),
+    "slx_decode_step_params": (c_int32, [POINTER(DecodeShape)] + [_P] * 6 + [c_int32] + [_P] * 9),
+    "slx_gate_skip_fwd_as": (c_int32, [POINTER(GlueShape)] + [_P] * 4 + [c_int32] + [_P] * 2),
+    "slx_gate_skip_bwd_as": (c_int32, [POINTER(GlueShape)] + [_P] * 4 + [c_int32] + [_P] * 6 + [c_size_t, _P]),
+    "slx_cconv1d_bwd_as": (c_int32, [POINTER(ConvShape)] + [_P] * 10 + [c_int32, _P, c_size_t, _P]),
     "slx_cconv1d_bwd_noalloc": (c_int32, [POINTER(ConvShape)] + [_P] * 11),
     "slx_gate_skip_fwd": (c_int32, [POINTER(GlueShape)] + [_P] * 6),
     "slx_gate_skip_bwd_workspace_bytes": (c_size_t, [POINTER(GlueShape)]),
@@ -90,6 +100,25 @@ SIGNATURES = {
     "slx_cconv1d_bwd_workspace_bytes": (c_size_t, [POINTER(ConvShape)]),
     "slx_cconv1d_bwd": (c_int32, [POINTER(ConvShape)] + [_P] * 11 + [c_size_t, _P]),
 }
+
+_host = None
+
+
+def host():
+    """The native host extension (``csrc/host``), loaded once."""
+    global _host
+    if _host is None:
+        lib()  # the product library first, with its own error when it is missing
+        path = LIB_PATH.with_name("_host.so")
+        if not path.exists():
+            raise RuntimeError(f"{path} is missing: build it first (python -m slinoss_b200.build). There is no "
+                               "fallback path.")
+        spec = importlib.util.spec_from_file_location("_host", path)
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+        _host = module
+    return _host
+
 
 SELFTEST_LIB_PATH = LIB_PATH.with_name("libslinoss_b200_selftest.so")
 SELFTEST_SIGNATURES = {

@@ -19,6 +19,7 @@ from typing import Optional, Tuple, Union
 
 import torch
 
+from . import _lib
 from .ops.cconv1d import cconv1d_b200, cconv1d_update_b200
 from .ops.decode import mixer_decode_step_b200
 from .ops.glue import gate_skip_b200
@@ -105,26 +106,37 @@ class B200MixerDecodeBackend:
 
     def __call__(self, owner, inputs, state):
         sp = owner.scanprep
-        v = inputs.value
+        v, params, bc, gate, skip = inputs.value, inputs.params, inputs.bc, inputs.gate, inputs.skip
+        normalize = bool(getattr(sp, "normalize_bc", True))
+        hyper = (sp.dt_min, sp.dt_max, sp.r_min, sp.r_max, sp.theta_bound, sp.k_max, sp.eps)
+        pars = (sp.dt_bias, sp.gamma_bias, sp.omega_bias, sp.mix_r_bias, sp.mix_theta_bias, sp.mix_k_prev_bias,
+                sp.mix_k_curr_bias)
+        if normalize:
+            pars += (sp.b_scale, sp.c_scale)
+        if state.state is not None and state.b_prev is not None and state.u_prev is not None:
+            # the common token: rows are column slices of the projection's output, read where they are, and the
+            # carried tensors are updated in place; anything else answers None
+            out = _lib.host().decode_step(v, params, bc, gate, skip, state.state, state.b_prev, state.u_prev, normalize,
+                                          hyper, pars, state.state, state.b_prev, state.u_prev)
+            if out is not None:
+                return out[0], self.state_cls(state=out[1], b_prev=out[2], u_prev=out[3])
         b, H, P = map(int, v.shape)
-        N = int(inputs.bc.shape[-1])
+        N = int(bc.shape[-1])
 
         def reuse(t, shape, dtype):
             ok = (t is not None and tuple(t.shape) == shape and t.dtype == dtype and t.is_contiguous()
                   and t.device == v.device)
             return t if ok else None
 
+        biases = dict(zip(("dt_bias", "gamma_bias", "omega_bias", "mix_r_bias", "mix_theta_bias", "mix_k_prev_bias",
+                           "mix_k_curr_bias", "b_scale", "c_scale"), pars))
         gated, fin, b_last, u_last = mixer_decode_step_b200(
-            v.contiguous(), inputs.params.contiguous(), inputs.bc.contiguous(), inputs.gate.contiguous(),
-            inputs.skip, initial_states=state.state, B_prev=state.b_prev, U_prev=state.u_prev,
-            dt_min=sp.dt_min, dt_max=sp.dt_max, r_min=sp.r_min, r_max=sp.r_max, theta_bound=sp.theta_bound,
-            k_max=sp.k_max, eps=sp.eps, dt_bias=sp.dt_bias, gamma_bias=sp.gamma_bias, omega_bias=sp.omega_bias,
-            mix_r_bias=sp.mix_r_bias, mix_theta_bias=sp.mix_theta_bias, mix_k_prev_bias=sp.mix_k_prev_bias,
-            mix_k_curr_bias=sp.mix_k_curr_bias, b_scale=getattr(sp, "b_scale", None),
-            c_scale=getattr(sp, "c_scale", None), normalize_bc=bool(getattr(sp, "normalize_bc", True)),
+            v.contiguous(), params.contiguous(), bc.contiguous(), gate.contiguous(), skip, initial_states=state.state,
+            B_prev=state.b_prev, U_prev=state.u_prev, dt_min=sp.dt_min, dt_max=sp.dt_max, r_min=sp.r_min,
+            r_max=sp.r_max, theta_bound=sp.theta_bound, k_max=sp.k_max, eps=sp.eps, normalize_bc=normalize,
             final_state_out=reuse(state.state, (b, H, P, 2 * N), torch.float32),
             b_last_out=reuse(state.b_prev, (b, H, 2 * N), v.dtype),
-            u_last_out=reuse(state.u_prev, (b, H, P), v.dtype))
+            u_last_out=reuse(state.u_prev, (b, H, P), v.dtype), **biases)
         return gated, self.state_cls(state=fin, b_prev=b_last, u_prev=u_last)
 
 

@@ -3,8 +3,9 @@
 ``python -m slinoss_b200.build`` (or ``build()``) compiles every ``csrc/*.cu``
 with nvcc for ``sm_100a`` and links one C-ABI shared library,
 ``_C/libslinoss_b200.so``, whose exports are declared in
-``include/slinoss_b200.h``.  There is no JIT and no fallback: importing the ops
-without this library raises.  ``build_selftest()`` builds ``csrc/selftest/*.cu`` into a
+``include/slinoss_b200.h``, then the host extension ``_C/_host.so`` (g++, ``csrc/host``)
+that the Python ops call it through.  There is no JIT and no fallback: calling the ops
+without these libraries raises.  ``build_selftest()`` builds ``csrc/selftest/*.cu`` into a
 second, test-only library (``include/slinoss_b200_selftest.h``) that the product never loads.
 """
 
@@ -20,6 +21,7 @@ PKG = Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 OUT_DIR = PKG / "_C"
 LIB = OUT_DIR / "libslinoss_b200.so"
+HOST_LIB = OUT_DIR / "_host.so"
 SELFTEST_LIB = OUT_DIR / "libslinoss_b200_selftest.so"
 
 NVCC_FLAGS = [
@@ -76,9 +78,37 @@ def _compile_and_link(sources, lib: Path, force: bool, verbose: bool) -> Path:
     return lib
 
 
+def build_host(force: bool = False) -> Path:
+    """The native host path (``csrc/host/*.cpp``): a Python extension module over libtorch and the product library,
+    which it finds beside itself."""
+    import sysconfig
+
+    from torch.utils import cpp_extension
+
+    sources = sorted((CSRC / "host").glob("*.cpp"))
+    newest = max(f.stat().st_mtime for f in sources + list((PKG.parent / "include").glob("*.h")))
+    if not force and HOST_LIB.exists() and HOST_LIB.stat().st_mtime >= newest:
+        return HOST_LIB
+    cuda = Path(_nvcc()).resolve().parents[1]
+    includes = [*cpp_extension.include_paths(), sysconfig.get_paths()["include"], str(cuda / "include")]
+    tmp = OUT_DIR / f"_host.{os.getpid()}.tmp.so"
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-DTORCH_EXTENSION_NAME=_host",
+           *(f"-isystem{p}" for p in includes), *map(str, sources), "-o", str(tmp),
+           *(f"-L{p}" for p in cpp_extension.library_paths()), f"-L{OUT_DIR}", f"-L{cuda / 'lib64'}",
+           "-ltorch_python", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda", "-lslinoss_b200",
+           "-Wl,-rpath,$ORIGIN"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"g++ failed for the host extension:\n{r.stdout}\n{r.stderr}")
+    os.replace(tmp, HOST_LIB)
+    return HOST_LIB
+
+
 def build(force: bool = False, verbose: bool = False) -> Path:
-    """The product library: every ``csrc/*.cu``."""
-    return _compile_and_link(sorted(CSRC.glob("*.cu")), LIB, force, verbose)
+    """The product library (every ``csrc/*.cu``) and the host extension over it."""
+    lib = _compile_and_link(sorted(CSRC.glob("*.cu")), LIB, force, verbose)
+    build_host(force)
+    return lib
 
 
 def build_selftest(force: bool = False, verbose: bool = False) -> Path:

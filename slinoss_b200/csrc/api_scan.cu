@@ -48,6 +48,12 @@ static int check_shape(const slx_scan_shape *s, ScanDims *d) {
   return SLX_OK;
 }
 
+// the token in front of the sequence: (BH, D) and (BH, P) rows in one dtype, both NULL when there is none
+struct PrevRow {
+  const void *B, *U;
+  int dtype;
+};
+
 template <typename K>
 static int set_smem(K kernel, size_t bytes) {
   return ensure_dyn_smem(kernel, bytes);
@@ -71,8 +77,8 @@ static int set_smem(K kernel, size_t bytes) {
 // ---- stage launchers ----------------------------------------------------------
 template <typename T, int L, int MODE>
 static int launch_outer(const ScanDims &d, const void *A, const void *X, const float *M, const float *K,
-                        const float *Bprev, const float *Uprev, float *out, float *m_chunk, cudaStream_t st) {
-  OuterArgs<T> a{(const T *)A, (const T *)X, M, K, Bprev, Uprev, out, m_chunk, d};
+                        const PrevRow &pv, float *out, float *m_chunk, cudaStream_t st) {
+  OuterArgs<T> a{(const T *)A, (const T *)X, M, K, pv.B, pv.U, pv.dtype, out, m_chunk, d};
   auto kern = chunk_outer_kernel<T, L, MODE>;
   size_t smem = outer_smem_bytes<L>();
   int rc = set_smem(kern, smem);
@@ -83,9 +89,9 @@ static int launch_outer(const ScanDims &d, const void *A, const void *X, const f
 
 template <typename T, int L>
 static int launch_scan_fwd(const ScanDims &d, const void *U, const float *M, const float *K, const void *B,
-                           const void *C, const float *starts, const float *Bprev, const float *Uprev, void *Y,
+                           const void *C, const float *starts, const PrevRow &pv, void *Y,
                            cudaStream_t st) {
-  ScanFwdArgs<T> a{(const T *)U, (const T *)B, (const T *)C, M, K, starts, Bprev, Uprev, (T *)Y, nullptr, d};
+  ScanFwdArgs<T> a{(const T *)U, (const T *)B, (const T *)C, M, K, starts, pv.B, pv.U, pv.dtype, (T *)Y, nullptr, d};
   auto kern = chunk_scan_fwd_kernel<T, L>;
   size_t smem = scan_fwd_smem_bytes<L>();
   int rc = set_smem(kern, smem);
@@ -157,9 +163,9 @@ static int make_tile_map(CUtensorMap *map, const void *base, int BH, int T_, int
 
 template <typename T>
 static int launch_scan_fwd_tc(const ScanDims &d, const void *U, const float *M, const float *K, const void *B,
-                              const void *C, const float *starts, const float *Bprev, const float *Uprev, void *Y,
+                              const void *C, const float *starts, const PrevRow &pv, void *Y,
                               cudaStream_t st) {
-  ScanFwdArgs<T> a{(const T *)U, (const T *)B, (const T *)C, M, K, starts, Bprev, Uprev, (T *)Y, nullptr, d};
+  ScanFwdArgs<T> a{(const T *)U, (const T *)B, (const T *)C, M, K, starts, pv.B, pv.U, pv.dtype, (T *)Y, nullptr, d};
   auto kern = chunk_scan_fwd_tc_kernel<T>;
   size_t smem = scan_fwd_tc_smem_bytes();
   int rc = set_smem(kern, smem);
@@ -194,9 +200,10 @@ static int persistent_grid(int total) {
 // Forward chunk scan, persistent warp-specialised kernel (scan_ws_fwd.cuh)
 template <typename T>
 static int launch_scan_fwd_ws(const ScanDims &d, const void *U, const float *M, const float *K, const void *B,
-                              const void *C, const void *starts, const float *Bprev, const float *Uprev, void *Y,
+                              const void *C, const void *starts, const PrevRow &pv, void *Y,
                               cudaStream_t st) {
-  ScanFwdArgs<T> a{(const T *)U, (const T *)B, (const T *)C, M, K, (const float *)starts, Bprev, Uprev, (T *)Y, nullptr, d};
+  ScanFwdArgs<T> a{(const T *)U, (const T *)B, (const T *)C, M, K, (const float *)starts, pv.B, pv.U, pv.dtype,
+                   (T *)Y, nullptr, d};
   auto kern = chunk_scan_fwd_ws_kernel<T>;
   const size_t smem = scan_ws_fwd_smem_bytes();
   int rc = set_smem(kern, smem);
@@ -214,8 +221,8 @@ static int launch_scan_fwd_ws(const ScanDims &d, const void *U, const float *M, 
 
 template <typename T, int MODE, typename OT>
 static int launch_outer_tc_t(const ScanDims &d, const void *A, const void *X, const float *M, const float *K,
-                             const float *Bprev, const float *Uprev, void *out, float *m_chunk, cudaStream_t st) {
-  OuterArgs<T> a{(const T *)A, (const T *)X, M, K, Bprev, Uprev, (float *)out, m_chunk, d};
+                             const PrevRow &pv, void *out, float *m_chunk, cudaStream_t st) {
+  OuterArgs<T> a{(const T *)A, (const T *)X, M, K, pv.B, pv.U, pv.dtype, (float *)out, m_chunk, d};
   auto kern = chunk_outer_tc_kernel<T, MODE, OT>;
   size_t smem = outer_tc_smem_bytes();
   int rc = set_smem(kern, smem);
@@ -226,10 +233,10 @@ static int launch_outer_tc_t(const ScanDims &d, const void *A, const void *X, co
 // `out` holds fp32 values, or (half_out) values of the activation dtype T
 template <typename T, int MODE>
 static int launch_outer_tc(const ScanDims &d, const void *A, const void *X, const float *M, const float *K,
-                           const float *Bprev, const float *Uprev, void *out, bool half_out, float *m_chunk,
+                           const PrevRow &pv, void *out, bool half_out, float *m_chunk,
                            cudaStream_t st) {
-  if (half_out) return launch_outer_tc_t<T, MODE, T>(d, A, X, M, K, Bprev, Uprev, out, m_chunk, st);
-  return launch_outer_tc_t<T, MODE, float>(d, A, X, M, K, Bprev, Uprev, out, m_chunk, st);
+  if (half_out) return launch_outer_tc_t<T, MODE, T>(d, A, X, M, K, pv, out, m_chunk, st);
+  return launch_outer_tc_t<T, MODE, float>(d, A, X, M, K, pv, out, m_chunk, st);
 }
 
 template <typename T>
@@ -269,38 +276,43 @@ static int launch_scan_bwd_ws(const ScanDims &d, const ScanBwdArgs<T> &a, cudaSt
 }
 
 template <typename ST, typename IT>
-static int launch_state_fwd_t(int BH, int NC, int P, int N, const IT *inc, const float *m_chunk, const float *init,
-                              ST *starts, float *final_state, cudaStream_t st) {
+static int launch_state_fwd_t(int BH, int NC, int P, int N, const IT *inc, const float *m_chunk, const StateEnds &ends,
+                              ST *starts, cudaStream_t st) {
   const int elems = P * 2 * N;
   // (eight values per thread, as the reverse pass uses for all-half storage, measured 0.100 against 0.095 ms here)
   if (elems % 4 == 0) {
     int nv = elems / 4;
-    state_passing_fwd_kernel<4, ST, IT><<<dim3((nv + 255) / 256, BH), 256, 0, st>>>(inc, m_chunk, init, starts,
-                                                                                  final_state, NC, nv);
+    state_passing_fwd_kernel<4, ST, IT><<<dim3((nv + 255) / 256, BH), 256, 0, st>>>(inc, m_chunk, ends, starts, NC, nv);
   } else {
     int nv = elems / 2;
-    state_passing_fwd_kernel<2, ST, IT><<<dim3((nv + 255) / 256, BH), 256, 0, st>>>(inc, m_chunk, init, starts,
-                                                                                  final_state, NC, nv);
+    state_passing_fwd_kernel<2, ST, IT><<<dim3((nv + 255) / 256, BH), 256, 0, st>>>(inc, m_chunk, ends, starts, NC, nv);
   }
   return check_launch("state_passing_fwd");
 }
 // inc_dtype is fp32 or starts_dtype (checked by the callers)
 static int launch_state_fwd(int BH, int NC, int P, int N, const void *inc, int inc_dtype, const float *m_chunk,
-                            const float *init, void *starts, int starts_dtype, float *final_state, cudaStream_t st) {
+                            const StateEnds &ends, void *starts, int starts_dtype, cudaStream_t st) {
   const bool half_inc = inc_dtype != SLX_F32;
   if (starts_dtype == SLX_BF16) {
     using H = __nv_bfloat16;
-    if (half_inc) return launch_state_fwd_t<H, H>(BH, NC, P, N, (const H *)inc, m_chunk, init, (H *)starts, final_state, st);
-    return launch_state_fwd_t<H, float>(BH, NC, P, N, (const float *)inc, m_chunk, init, (H *)starts, final_state, st);
+    if (half_inc) return launch_state_fwd_t<H, H>(BH, NC, P, N, (const H *)inc, m_chunk, ends, (H *)starts, st);
+    return launch_state_fwd_t<H, float>(BH, NC, P, N, (const float *)inc, m_chunk, ends, (H *)starts, st);
   }
   if (starts_dtype == SLX_F16) {
     using H = __half;
-    if (half_inc) return launch_state_fwd_t<H, H>(BH, NC, P, N, (const H *)inc, m_chunk, init, (H *)starts, final_state, st);
-    return launch_state_fwd_t<H, float>(BH, NC, P, N, (const float *)inc, m_chunk, init, (H *)starts, final_state, st);
+    if (half_inc) return launch_state_fwd_t<H, H>(BH, NC, P, N, (const H *)inc, m_chunk, ends, (H *)starts, st);
+    return launch_state_fwd_t<H, float>(BH, NC, P, N, (const float *)inc, m_chunk, ends, (H *)starts, st);
   }
-  return launch_state_fwd_t<float, float>(BH, NC, P, N, (const float *)inc, m_chunk, init, (float *)starts, final_state,
-                                          st);
+  return launch_state_fwd_t<float, float>(BH, NC, P, N, (const float *)inc, m_chunk, ends, (float *)starts, st);
 }
+
+// gradients at either end of the reverse pass, in the caller's dtypes (both optional)
+struct StateGradEnds {
+  const void *d_final;
+  int d_final_dtype;
+  void *d_initial;
+  int d_initial_dtype;
+};
 
 static int state_bwd_vec(int P, int N, bool all_half) {
   const int elems = P * 2 * N;
@@ -316,21 +328,24 @@ static int state_bwd_parts(int P, int N) {
 
 template <typename ST, typename IT>
 static int launch_state_bwd_t(int BH, int NC, int P, int N, const IT *dZ0, const float *m_chunk, const ST *starts,
-                              const float *final_state, const float *d_final, ST *d_inc, float *d_initial,
+                              const float *final_state, const StateGradEnds &ge, ST *d_inc,
                               float *zdot, float *partials, cudaStream_t st) {
   const int elems = P * 2 * N;
   const int vec = state_bwd_vec(P, N, sizeof(ST) == 2 && sizeof(IT) == 2);
   const int nblk = (elems / vec + 255) / 256;
   if (vec == 8) {
     if constexpr (sizeof(ST) == 2 && sizeof(IT) == 2)
-      state_passing_bwd_kernel<8, ST, IT><<<dim3(nblk, BH), 256, 0, st>>>(dZ0, m_chunk, starts, final_state, d_final,
-                                                                         d_inc, d_initial, partials, NC, elems / 8);
+      state_passing_bwd_kernel<8, ST, IT><<<dim3(nblk, BH), 256, 0, st>>>(dZ0, m_chunk, starts, final_state, ge.d_final,
+                                                                         ge.d_final_dtype, d_inc, ge.d_initial,
+                                                                         ge.d_initial_dtype, partials, NC, elems / 8);
   } else if (vec == 4) {
-    state_passing_bwd_kernel<4, ST, IT><<<dim3(nblk, BH), 256, 0, st>>>(dZ0, m_chunk, starts, final_state, d_final,
-                                                                       d_inc, d_initial, partials, NC, elems / 4);
+    state_passing_bwd_kernel<4, ST, IT><<<dim3(nblk, BH), 256, 0, st>>>(dZ0, m_chunk, starts, final_state, ge.d_final,
+                                                                       ge.d_final_dtype, d_inc, ge.d_initial,
+                                                                       ge.d_initial_dtype, partials, NC, elems / 4);
   } else {
-    state_passing_bwd_kernel<2, ST, IT><<<dim3(nblk, BH), 256, 0, st>>>(dZ0, m_chunk, starts, final_state, d_final,
-                                                                       d_inc, d_initial, partials, NC, elems / 2);
+    state_passing_bwd_kernel<2, ST, IT><<<dim3(nblk, BH), 256, 0, st>>>(dZ0, m_chunk, starts, final_state, ge.d_final,
+                                                                       ge.d_final_dtype, d_inc, ge.d_initial,
+                                                                       ge.d_initial_dtype, partials, NC, elems / 2);
   }
   int rc = check_launch("state_passing_bwd");
   if (rc || partials == nullptr) return rc;
@@ -340,27 +355,27 @@ static int launch_state_bwd_t(int BH, int NC, int P, int N, const IT *dZ0, const
 }
 // dz0_dtype is fp32 or starts_dtype (checked by the callers)
 static int launch_state_bwd(int BH, int NC, int P, int N, const void *dZ0, int dz0_dtype, const float *m_chunk,
-                            const void *starts, int starts_dtype, const float *final_state, const float *d_final,
-                            void *d_inc, float *d_initial, float *zdot, float *partials, cudaStream_t st) {
+                            const void *starts, int starts_dtype, const float *final_state, const StateGradEnds &ge,
+                            void *d_inc, float *zdot, float *partials, cudaStream_t st) {
   const bool half_dz = dz0_dtype != SLX_F32;
   if (starts_dtype == SLX_BF16) {
     using H = __nv_bfloat16;
     if (half_dz)
-      return launch_state_bwd_t<H, H>(BH, NC, P, N, (const H *)dZ0, m_chunk, (const H *)starts, final_state, d_final,
-                                      (H *)d_inc, d_initial, zdot, partials, st);
+      return launch_state_bwd_t<H, H>(BH, NC, P, N, (const H *)dZ0, m_chunk, (const H *)starts, final_state, ge,
+                                      (H *)d_inc, zdot, partials, st);
     return launch_state_bwd_t<H, float>(BH, NC, P, N, (const float *)dZ0, m_chunk, (const H *)starts, final_state,
-                                        d_final, (H *)d_inc, d_initial, zdot, partials, st);
+                                        ge, (H *)d_inc, zdot, partials, st);
   }
   if (starts_dtype == SLX_F16) {
     using H = __half;
     if (half_dz)
-      return launch_state_bwd_t<H, H>(BH, NC, P, N, (const H *)dZ0, m_chunk, (const H *)starts, final_state, d_final,
-                                      (H *)d_inc, d_initial, zdot, partials, st);
+      return launch_state_bwd_t<H, H>(BH, NC, P, N, (const H *)dZ0, m_chunk, (const H *)starts, final_state, ge,
+                                      (H *)d_inc, zdot, partials, st);
     return launch_state_bwd_t<H, float>(BH, NC, P, N, (const float *)dZ0, m_chunk, (const H *)starts, final_state,
-                                        d_final, (H *)d_inc, d_initial, zdot, partials, st);
+                                        ge, (H *)d_inc, zdot, partials, st);
   }
   return launch_state_bwd_t<float, float>(BH, NC, P, N, (const float *)dZ0, m_chunk, (const float *)starts, final_state,
-                                          d_final, (float *)d_inc, d_initial, zdot, partials, st);
+                                          ge, (float *)d_inc, zdot, partials, st);
 }
 
 // workspace layout of the backward (256-byte aligned sections; dZ0 and d_inc as starts_dtype, the rest fp32)
@@ -412,6 +427,84 @@ static int exchange_status(int which, int *host_out, const char *what) {
   return SLX_OK;
 }
 
+// ---- stages with the streaming rows in the caller's dtype ----------------------------------------
+static int chunk_increment_impl(const slx_scan_shape *s, const void *U, const float *M, const float *K, const void *B,
+                                const PrevRow &pv, void *inc, int inc_dtype, float *m_chunk, void *stream) {
+  ScanDims d;
+  int rc = check_shape(s, &d);
+  if (rc) return rc;
+  SLX_REQUIRE(U && M && K && B && inc && m_chunk, SLX_E_NULL, "chunk_increment_fwd: NULL tensor");
+  SLX_REQUIRE(inc_dtype == SLX_F32 || (use_tc(s) && inc_dtype == s->dtype), SLX_E_DTYPE,
+              "chunk_increment_fwd: inc_dtype %d must be fp32, or the activation dtype on the tensor-core path",
+              inc_dtype);
+  SLX_REQUIRE_ALIGNED("chunk_increment_fwd", U, M, K, B, inc, m_chunk);
+  SLX_REQUIRE(pv.B == nullptr || pv.dtype == SLX_F32 || pv.dtype == s->dtype, SLX_E_DTYPE,
+              "B_prev and U_prev must be fp32 or of the activation dtype");
+  SLX_REQUIRE((pv.B == nullptr) == (pv.U == nullptr), SLX_E_NULL, "B_prev and U_prev must be passed together");
+  if (use_tc(s)) {
+    if (s->dtype == SLX_BF16)
+      return launch_outer_tc<__nv_bfloat16, 0>(d, U, B, M, K, pv, inc, inc_dtype != SLX_F32, m_chunk,
+                                               as_stream(stream));
+    return launch_outer_tc<__half, 0>(d, U, B, M, K, pv, inc, inc_dtype != SLX_F32, m_chunk, as_stream(stream));
+  }
+  SLX_DISPATCH_T(s->dtype, SLX_DISPATCH_L(d.L, rc = (launch_outer<T_, L_, 0>(d, U, B, M, K, pv, (float *)inc, m_chunk,
+                                                                              as_stream(stream)))));
+  return rc;
+}
+
+static int chunk_scan_impl(const slx_scan_shape *s, const void *U, const float *M, const float *K, const void *B,
+                           const void *C, const void *chunk_starts, const PrevRow &pv, void *Y, void *stream) {
+  ScanDims d;
+  int rc = check_shape(s, &d);
+  if (rc) return rc;
+  SLX_REQUIRE(U && M && K && B && C && chunk_starts && Y, SLX_E_NULL, "chunk_scan_fwd: NULL tensor");
+  SLX_REQUIRE_ALIGNED("chunk_scan_fwd", U, M, K, B, C, chunk_starts, Y);
+  SLX_REQUIRE(pv.B == nullptr || pv.dtype == SLX_F32 || pv.dtype == s->dtype, SLX_E_DTYPE,
+              "B_prev and U_prev must be fp32 or of the activation dtype");
+  SLX_REQUIRE((pv.B == nullptr) == (pv.U == nullptr), SLX_E_NULL, "B_prev and U_prev must be passed together");
+  if (use_tc(s) && g_use_tc == 2) {
+    if (s->dtype == SLX_BF16)
+      return launch_scan_fwd_ws<__nv_bfloat16>(d, U, M, K, B, C, chunk_starts, pv, Y, as_stream(stream));
+    return launch_scan_fwd_ws<__half>(d, U, M, K, B, C, chunk_starts, pv, Y, as_stream(stream));
+  }
+  if (use_tc(s)) {
+    if (s->dtype == SLX_BF16)
+      return launch_scan_fwd_tc<__nv_bfloat16>(d, U, M, K, B, C, (const float *)chunk_starts, pv, Y, as_stream(stream));
+    return launch_scan_fwd_tc<__half>(d, U, M, K, B, C, (const float *)chunk_starts, pv, Y, as_stream(stream));
+  }
+  SLX_DISPATCH_T(s->dtype, SLX_DISPATCH_L(d.L, rc = (launch_scan_fwd<T_, L_>(d, U, M, K, B, C, (const float *)chunk_starts,
+                                                                             pv, Y, as_stream(stream)))));
+  return rc;
+}
+
+static int chunk_scan_bwd_impl(const slx_scan_shape *s, const void *U, const float *M, const float *K, const void *B,
+                               const void *C, const PrevRow &pv, const void *chunk_starts, const void *d_inc,
+                               const float *zdot, const void *dY, void *dU, float *dM, float *dK, void *dB, void *dC,
+                               float *carryB, float *carryU, void *stream) {
+  ScanDims d;
+  int rc = check_shape(s, &d);
+  if (rc) return rc;
+  SLX_REQUIRE(U && M && K && B && C && chunk_starts && d_inc && zdot && dY && dU && dM && dK && dB && dC && carryB &&
+                  carryU,
+              SLX_E_NULL, "chunk_scan_bwd: NULL tensor");
+  SLX_REQUIRE_ALIGNED("chunk_scan_bwd", U, M, K, B, C, chunk_starts, d_inc, dY, dU, dM, dK, dB, dC, carryB, carryU);
+  SLX_REQUIRE(pv.B == nullptr || pv.dtype == SLX_F32 || pv.dtype == s->dtype, SLX_E_DTYPE,
+              "B_prev and U_prev must be fp32 or of the activation dtype");
+  SLX_REQUIRE((pv.B == nullptr) == (pv.U == nullptr), SLX_E_NULL, "B_prev and U_prev must be passed together");
+  const bool tc = use_tc(s);
+  SLX_DISPATCH_T(s->dtype, {
+    ScanBwdArgs<T_> a{(const T_ *)U, (const T_ *)B, (const T_ *)C, (const T_ *)dY, M, K, (const float *)chunk_starts,
+                      (const float *)d_inc, zdot,
+                      pv.B, pv.U, pv.dtype, (T_ *)dU, (T_ *)dB, (T_ *)dC, dM, dK, carryB, carryU, d};
+    if constexpr (!std::is_same<T_, float>::value) {
+      if (tc && g_use_tc == 2) return launch_scan_bwd_ws<T_>(d, a, as_stream(stream));
+      if (tc) return launch_scan_bwd_tc<T_>(d, a, as_stream(stream));
+    }
+    SLX_DISPATCH_L(d.L, rc = (launch_scan_bwd<T_, L_>(d, a, as_stream(stream))));
+  });
+  return rc;
+}
+
 }  // namespace slx
 
 using namespace slx;
@@ -457,25 +550,7 @@ const char *slx_last_error_string(void) { return g_err; }
 int slx_chunk_increment_fwd(const slx_scan_shape *s, const void *U, const float *M, const float *K, const void *B,
                             const float *B_prev, const float *U_prev, void *inc, int32_t inc_dtype, float *m_chunk,
                             void *stream) {
-  ScanDims d;
-  int rc = check_shape(s, &d);
-  if (rc) return rc;
-  SLX_REQUIRE(U && M && K && B && inc && m_chunk, SLX_E_NULL, "chunk_increment_fwd: NULL tensor");
-  SLX_REQUIRE(inc_dtype == SLX_F32 || (use_tc(s) && inc_dtype == s->dtype), SLX_E_DTYPE,
-              "chunk_increment_fwd: inc_dtype %d must be fp32, or the activation dtype on the tensor-core path",
-              inc_dtype);
-  SLX_REQUIRE_ALIGNED("chunk_increment_fwd", U, M, K, B, B_prev, U_prev, inc, m_chunk);
-  SLX_REQUIRE((B_prev == nullptr) == (U_prev == nullptr), SLX_E_NULL, "B_prev and U_prev must be passed together");
-  if (use_tc(s)) {
-    if (s->dtype == SLX_BF16)
-      return launch_outer_tc<__nv_bfloat16, 0>(d, U, B, M, K, B_prev, U_prev, inc, inc_dtype != SLX_F32, m_chunk,
-                                               as_stream(stream));
-    return launch_outer_tc<__half, 0>(d, U, B, M, K, B_prev, U_prev, inc, inc_dtype != SLX_F32, m_chunk,
-                                      as_stream(stream));
-  }
-  SLX_DISPATCH_T(s->dtype, SLX_DISPATCH_L(d.L, rc = (launch_outer<T_, L_, 0>(d, U, B, M, K, B_prev, U_prev, (float *)inc,
-                                                                              m_chunk, as_stream(stream)))));
-  return rc;
+  return chunk_increment_impl(s, U, M, K, B, PrevRow{B_prev, U_prev, SLX_F32}, inc, inc_dtype, m_chunk, stream);
 }
 
 int slx_state_passing_fwd(int32_t BH, int32_t NC, int32_t P, int32_t N, const void *inc, int32_t inc_dtype,
@@ -494,56 +569,67 @@ int slx_state_passing_fwd(int32_t BH, int32_t NC, int32_t P, int32_t N, const vo
   if (chunk_starts == nullptr && inc_dtype != SLX_F32) starts_dtype = inc_dtype;  // nothing is stored as starts_dtype
   SLX_REQUIRE(inc_dtype == SLX_F32 || inc_dtype == starts_dtype, SLX_E_DTYPE,
               "state_passing_fwd: inc_dtype %d must be fp32 or starts_dtype %d", inc_dtype, starts_dtype);
-  return launch_state_fwd(BH, NC, P, N, inc, inc_dtype, m_chunk, initial_states, chunk_starts, starts_dtype,
-                          final_state, as_stream(stream));
+  StateEnds ends{};
+  ends.init = initial_states;
+  ends.final_state = final_state;
+  return launch_state_fwd(BH, NC, P, N, inc, inc_dtype, m_chunk, ends, chunk_starts, starts_dtype, as_stream(stream));
 }
 
 int slx_chunk_scan_fwd(const slx_scan_shape *s, const void *U, const float *M, const float *K, const void *B,
                        const void *C, const void *chunk_starts, const float *B_prev, const float *U_prev, void *Y,
                        void *stream) {
+  return chunk_scan_impl(s, U, M, K, B, C, chunk_starts, PrevRow{B_prev, U_prev, SLX_F32}, Y, stream);
+}
+
+int slx_v2x2ssd_fwd_stream(const slx_scan_shape *s, const void *U, const float *M, const float *K, const void *B,
+                           const void *C, const slx_scan_ends *e, void *Y, float *final_state, void *chunk_starts,
+                           float *m_chunk, void *increments, void *stream) {
   ScanDims d;
   int rc = check_shape(s, &d);
   if (rc) return rc;
-  SLX_REQUIRE(U && M && K && B && C && chunk_starts && Y, SLX_E_NULL, "chunk_scan_fwd: NULL tensor");
-  SLX_REQUIRE_ALIGNED("chunk_scan_fwd", U, M, K, B, C, chunk_starts, B_prev, U_prev, Y);
-  SLX_REQUIRE((B_prev == nullptr) == (U_prev == nullptr), SLX_E_NULL, "B_prev and U_prev must be passed together");
-  if (use_tc(s) && g_use_tc == 2) {
-    if (s->dtype == SLX_BF16)
-      return launch_scan_fwd_ws<__nv_bfloat16>(d, U, M, K, B, C, chunk_starts, B_prev, U_prev, Y, as_stream(stream));
-    return launch_scan_fwd_ws<__half>(d, U, M, K, B, C, chunk_starts, B_prev, U_prev, Y, as_stream(stream));
+  const int sdt = s->starts_dtype;
+  SLX_REQUIRE(increments != nullptr || sdt == SLX_F32, SLX_E_NULL,
+              "v2x2ssd_fwd: this shape keeps chunk_starts in the activation dtype and needs the increments buffer");
+  const slx_scan_ends none{};
+  if (e == nullptr) e = &none;
+  SLX_REQUIRE((e->B_last == nullptr) == (e->U_last == nullptr), SLX_E_NULL, "B_last and U_last must be passed together");
+  SLX_REQUIRE_ALIGNED("v2x2ssd_fwd", e->initial_states, e->final_copy, final_state, chunk_starts, increments);
+  SLX_REQUIRE(chunk_starts != nullptr && m_chunk != nullptr, SLX_E_NULL, "v2x2ssd_fwd: NULL tensor");
+  const PrevRow pv{e->B_prev, e->U_prev, e->prev_dtype};
+  void *inc = increments ? increments : chunk_starts;  // increments are stored as starts_dtype, like the states
+  rc = chunk_increment_impl(s, U, M, K, B, pv, inc, sdt, m_chunk, stream);
+  if (rc) return rc;
+  StateEnds ends{};
+  ends.init = e->initial_states;
+  ends.init_dtype = e->initial_dtype;
+  ends.final_state = final_state;
+  ends.final_copy = e->final_copy;
+  ends.final_dtype = e->final_dtype;
+  if (e->B_last) {
+    const int units = s->dtype == SLX_F32 ? 2 : 1;
+    ends.B = B;
+    ends.U = U;
+    ends.B_last = e->B_last;
+    ends.U_last = e->U_last;
+    ends.b_units = d.D * units;
+    ends.u_units = d.P * units;
+    ends.T = d.T;
   }
-  if (use_tc(s)) {
-    if (s->dtype == SLX_BF16)
-      return launch_scan_fwd_tc<__nv_bfloat16>(d, U, M, K, B, C, (const float *)chunk_starts, B_prev, U_prev, Y,
-                                               as_stream(stream));
-    return launch_scan_fwd_tc<__half>(d, U, M, K, B, C, (const float *)chunk_starts, B_prev, U_prev, Y,
-                                      as_stream(stream));
-  }
-  SLX_DISPATCH_T(s->dtype, SLX_DISPATCH_L(d.L, rc = (launch_scan_fwd<T_, L_>(d, U, M, K, B, C, (const float *)chunk_starts, B_prev,
-                                                                             U_prev, Y, as_stream(stream)))));
-  return rc;
+  rc = launch_state_fwd(d.BH, d.NC, d.P, d.N, inc, sdt, m_chunk, ends, chunk_starts, sdt, as_stream(stream));
+  if (rc) return rc;
+  if (Y == nullptr) return SLX_OK;  // only the chunk states were asked for
+  return chunk_scan_impl(s, U, M, K, B, C, chunk_starts, pv, Y, stream);
 }
 
 int slx_v2x2ssd_fwd(const slx_scan_shape *s, const void *U, const float *M, const float *K, const void *B,
                     const void *C, const float *initial_states, const float *B_prev, const float *U_prev, void *Y,
                     float *final_state, void *chunk_starts, float *m_chunk, void *increments, void *stream) {
-  ScanDims d0;
-  {
-    int rc0 = check_shape(s, &d0);
-    if (rc0) return rc0;
-  }
-  const int sdt = s->starts_dtype;
-  SLX_REQUIRE(increments != nullptr || sdt == SLX_F32, SLX_E_NULL,
-              "v2x2ssd_fwd: this shape keeps chunk_starts in the activation dtype and needs the increments buffer");
-  void *inc = increments ? increments : chunk_starts;  // increments are stored as starts_dtype, like the states
-  int rc = slx_chunk_increment_fwd(s, U, M, K, B, B_prev, U_prev, inc, sdt, m_chunk, stream);
-  if (rc) return rc;
-  SLX_REQUIRE(final_state != nullptr, SLX_E_NULL, "v2x2ssd_fwd: final_state is NULL");
-  const int NC = (s->T + s->chunk - 1) / s->chunk;
-  rc = slx_state_passing_fwd(s->batch_heads, NC, s->P, s->N, inc, sdt, m_chunk, initial_states, chunk_starts, sdt,
-                             final_state, stream);
-  if (rc) return rc;
-  return slx_chunk_scan_fwd(s, U, M, K, B, C, chunk_starts, B_prev, U_prev, Y, stream);
+  SLX_REQUIRE(final_state != nullptr && Y != nullptr, SLX_E_NULL, "v2x2ssd_fwd: NULL tensor");
+  slx_scan_ends e{};
+  e.initial_states = initial_states;
+  e.B_prev = B_prev;
+  e.U_prev = U_prev;
+  return slx_v2x2ssd_fwd_stream(s, U, M, K, B, C, &e, Y, final_state, chunk_starts, m_chunk, increments, stream);
 }
 
 size_t slx_state_passing_bwd_partials_bytes(int32_t BH, int32_t NC, int32_t P, int32_t N) {
@@ -567,15 +653,16 @@ int slx_chunk_scan_bwd_dz0(const slx_scan_shape *s, const float *M, const void *
               "chunk_scan_bwd_dz0: dz0_dtype %d must be fp32, or the activation dtype on the tensor-core path",
               dz0_dtype);
   SLX_REQUIRE_ALIGNED("chunk_scan_bwd_dz0", M, C, dY, dZ0);
+  const PrevRow none{nullptr, nullptr, SLX_F32};
   if (use_tc(s)) {
     if (s->dtype == SLX_BF16)
-      return launch_outer_tc<__nv_bfloat16, 1>(d, dY, C, M, nullptr, nullptr, nullptr, dZ0, dz0_dtype != SLX_F32,
-                                               nullptr, as_stream(stream));
-    return launch_outer_tc<__half, 1>(d, dY, C, M, nullptr, nullptr, nullptr, dZ0, dz0_dtype != SLX_F32, nullptr,
+      return launch_outer_tc<__nv_bfloat16, 1>(d, dY, C, M, nullptr, none, dZ0, dz0_dtype != SLX_F32, nullptr,
+                                               as_stream(stream));
+    return launch_outer_tc<__half, 1>(d, dY, C, M, nullptr, none, dZ0, dz0_dtype != SLX_F32, nullptr,
                                       as_stream(stream));
   }
-  SLX_DISPATCH_T(s->dtype, SLX_DISPATCH_L(d.L, rc = (launch_outer<T_, L_, 1>(d, dY, C, M, nullptr, nullptr, nullptr,
-                                                                              (float *)dZ0, nullptr, as_stream(stream)))));
+  SLX_DISPATCH_T(s->dtype, SLX_DISPATCH_L(d.L, rc = (launch_outer<T_, L_, 1>(d, dY, C, M, nullptr, none, (float *)dZ0,
+                                                                              nullptr, as_stream(stream)))));
   return rc;
 }
 
@@ -603,49 +690,33 @@ int slx_state_passing_bwd(int32_t BH, int32_t NC, int32_t P, int32_t N, const vo
   if (d_inc == nullptr && zdot == nullptr && dz0_dtype != SLX_F32) starts_dtype = dz0_dtype;
   SLX_REQUIRE(dz0_dtype == SLX_F32 || dz0_dtype == starts_dtype, SLX_E_DTYPE,
               "state_passing_bwd: dz0_dtype %d must be fp32 or starts_dtype %d", dz0_dtype, starts_dtype);
-  return launch_state_bwd(BH, NC, P, N, dZ0, dz0_dtype, m_chunk, chunk_starts, starts_dtype, final_state, d_final,
-                          d_inc, d_initial, zdot, zdot_partials, as_stream(stream));
+  return launch_state_bwd(BH, NC, P, N, dZ0, dz0_dtype, m_chunk, chunk_starts, starts_dtype, final_state,
+                          StateGradEnds{d_final, SLX_F32, d_initial, SLX_F32}, d_inc, zdot, zdot_partials,
+                          as_stream(stream));
 }
 
 int slx_chunk_scan_bwd(const slx_scan_shape *s, const void *U, const float *M, const float *K, const void *B,
                        const void *C, const float *B_prev, const float *U_prev, const void *chunk_starts,
                        const void *d_inc, const float *zdot, const void *dY, void *dU, float *dM, float *dK,
                        void *dB, void *dC, float *carryB, float *carryU, void *stream) {
-  ScanDims d;
-  int rc = check_shape(s, &d);
-  if (rc) return rc;
-  SLX_REQUIRE(U && M && K && B && C && chunk_starts && d_inc && zdot && dY && dU && dM && dK && dB && dC && carryB &&
-                  carryU,
-              SLX_E_NULL, "chunk_scan_bwd: NULL tensor");
-  SLX_REQUIRE_ALIGNED("chunk_scan_bwd", U, M, K, B, C, B_prev, U_prev, chunk_starts, d_inc, dY, dU, dM, dK, dB, dC,
-                      carryB, carryU);
-  SLX_REQUIRE((B_prev == nullptr) == (U_prev == nullptr), SLX_E_NULL, "B_prev and U_prev must be passed together");
-  const bool tc = use_tc(s);
-  SLX_DISPATCH_T(s->dtype, {
-    ScanBwdArgs<T_> a{(const T_ *)U, (const T_ *)B, (const T_ *)C, (const T_ *)dY, M, K, (const float *)chunk_starts,
-                      (const float *)d_inc, zdot,
-                      B_prev, U_prev, (T_ *)dU, (T_ *)dB, (T_ *)dC, dM, dK, carryB, carryU, d};
-    if constexpr (!std::is_same<T_, float>::value) {
-      if (tc && g_use_tc == 2) return launch_scan_bwd_ws<T_>(d, a, as_stream(stream));
-      if (tc) return launch_scan_bwd_tc<T_>(d, a, as_stream(stream));
-    }
-    SLX_DISPATCH_L(d.L, rc = (launch_scan_bwd<T_, L_>(d, a, as_stream(stream))));
-  });
-  return rc;
+  return chunk_scan_bwd_impl(s, U, M, K, B, C, PrevRow{B_prev, U_prev, SLX_F32}, chunk_starts, d_inc, zdot, dY, dU, dM,
+                             dK, dB, dC, carryB, carryU, stream);
 }
 
 static int v2x2ssd_bwd_impl(const slx_scan_shape *s, const void *U, const float *M, const float *K, const void *B,
-                            const void *C, const float *B_prev, const float *U_prev, const void *chunk_starts,
-                            const float *m_chunk, const float *final_state, const void *dY, const float *d_final,
-                            void *dU, float *dM, float *dK, void *dB, void *dC, float *d_initial, float *dB_prev,
-                            float *dU_prev, void *workspace, size_t workspace_bytes, void *stream, bool dz0_ready) {
+                            const void *C, const slx_scan_grad_ends *e, const void *chunk_starts,
+                            const float *m_chunk, const float *final_state, const void *dY, void *dU, float *dM,
+                            float *dK, void *dB, void *dC, void *workspace, size_t workspace_bytes, void *stream,
+                            bool dz0_ready) {
   ScanDims d;
   int rc = check_shape(s, &d);
   if (rc) return rc;
+  const slx_scan_grad_ends none{};
+  if (e == nullptr) e = &none;
   SLX_REQUIRE(U && M && K && B && C && chunk_starts && m_chunk && final_state && dY && dU && dM && dK && dB && dC,
               SLX_E_NULL, "v2x2ssd_bwd: NULL tensor");
-  SLX_REQUIRE_ALIGNED("v2x2ssd_bwd", final_state, d_final, d_initial, dB_prev, dU_prev);
-  SLX_REQUIRE((B_prev == nullptr) == (U_prev == nullptr), SLX_E_NULL, "B_prev and U_prev must be passed together");
+  SLX_REQUIRE_ALIGNED("v2x2ssd_bwd", final_state, e->d_final, e->d_initial);
+  SLX_REQUIRE((e->B_prev == nullptr) == (e->U_prev == nullptr), SLX_E_NULL, "B_prev and U_prev must be passed together");
   const BwdWs w = bwd_ws(d, s->starts_dtype);
   SLX_REQUIRE(workspace != nullptr && workspace_bytes >= w.total, SLX_E_WORKSPACE,
               "v2x2ssd_bwd: workspace of %zu bytes needed, %zu given", w.total, workspace_bytes);
@@ -665,17 +736,38 @@ static int v2x2ssd_bwd_impl(const slx_scan_shape *s, const void *U, const float 
     if (rc) return rc;
   }
   rc = launch_state_bwd(d.BH, d.NC, d.P, d.N, dz0, s->starts_dtype, m_chunk, chunk_starts, s->starts_dtype,
-                        final_state, d_final, d_inc, d_initial, zdot, partials, st);
+                        final_state, StateGradEnds{e->d_final, e->d_final_dtype, e->d_initial, e->d_initial_dtype},
+                        d_inc, zdot, partials, st);
   if (rc) return rc;
-  rc = slx_chunk_scan_bwd(s, U, M, K, B, C, B_prev, U_prev, chunk_starts, d_inc, zdot, dY, dU, dM, dK, dB, dC, carryB,
-                          carryU, stream);
+  rc = chunk_scan_bwd_impl(s, U, M, K, B, C, PrevRow{e->B_prev, e->U_prev, e->prev_dtype}, chunk_starts, d_inc, zdot,
+                           dY, dU, dM, dK, dB, dC, carryB, carryU, stream);
   if (rc) return rc;
   SLX_DISPATCH_T(s->dtype, {
-    carry_fixup_kernel<T_><<<dim3(d.NC, d.BH), 128, 0, st>>>(carryB, carryU, (T_ *)dB, (T_ *)dU, dB_prev, dU_prev,
-                                                              d.T, d.P, d.D, d.L, d.NC);
+    carry_fixup_kernel<T_><<<dim3(d.NC, d.BH), 128, 0, st>>>(carryB, carryU, (T_ *)dB, (T_ *)dU, e->dB_prev,
+                                                              e->dU_prev, e->d_prev_dtype, d.T, d.P, d.D, d.L, d.NC);
     rc = check_launch("carry_fixup");
   });
   return rc;
+}
+
+static slx_scan_grad_ends f32_grad_ends(const float *B_prev, const float *U_prev, const float *d_final,
+                                        float *d_initial, float *dB_prev, float *dU_prev) {
+  slx_scan_grad_ends e{};
+  e.B_prev = B_prev;
+  e.U_prev = U_prev;
+  e.d_final = d_final;
+  e.d_initial = d_initial;
+  e.dB_prev = dB_prev;
+  e.dU_prev = dU_prev;
+  return e;
+}
+
+int slx_v2x2ssd_bwd_stream(const slx_scan_shape *s, const void *U, const float *M, const float *K, const void *B,
+                           const void *C, const slx_scan_grad_ends *e, const void *chunk_starts, const float *m_chunk,
+                           const float *final_state, const void *dY, void *dU, float *dM, float *dK, void *dB, void *dC,
+                           void *workspace, size_t workspace_bytes, void *stream) {
+  return v2x2ssd_bwd_impl(s, U, M, K, B, C, e, chunk_starts, m_chunk, final_state, dY, dU, dM, dK, dB, dC, workspace,
+                          workspace_bytes, stream, false);
 }
 
 int slx_v2x2ssd_bwd(const slx_scan_shape *s, const void *U, const float *M, const float *K, const void *B,
@@ -683,8 +775,9 @@ int slx_v2x2ssd_bwd(const slx_scan_shape *s, const void *U, const float *M, cons
                     const float *m_chunk, const float *final_state, const void *dY, const float *d_final, void *dU,
                     float *dM, float *dK, void *dB, void *dC, float *d_initial, float *dB_prev, float *dU_prev,
                     void *workspace, size_t workspace_bytes, void *stream) {
-  return v2x2ssd_bwd_impl(s, U, M, K, B, C, B_prev, U_prev, chunk_starts, m_chunk, final_state, dY, d_final, dU, dM,
-                          dK, dB, dC, d_initial, dB_prev, dU_prev, workspace, workspace_bytes, stream, false);
+  const slx_scan_grad_ends e = f32_grad_ends(B_prev, U_prev, d_final, d_initial, dB_prev, dU_prev);
+  return v2x2ssd_bwd_impl(s, U, M, K, B, C, &e, chunk_starts, m_chunk, final_state, dY, dU, dM, dK, dB, dC, workspace,
+                          workspace_bytes, stream, false);
 }
 
 int slx_v2x2ssd_bwd_begin(const slx_scan_shape *s, const float *M, const void *C, const float *m_chunk,
@@ -703,7 +796,8 @@ int slx_v2x2ssd_bwd_begin(const slx_scan_shape *s, const float *M, const void *C
   rc = slx_chunk_scan_bwd_dz0(s, M, C, dY, dz0, s->starts_dtype, stream);
   if (rc) return rc;
   return launch_state_bwd(d.BH, d.NC, d.P, d.N, dz0, s->starts_dtype, m_chunk, nullptr, s->starts_dtype, nullptr,
-                          nullptr, nullptr, d_initial_zero_final, nullptr, nullptr, as_stream(stream));
+                          StateGradEnds{nullptr, SLX_F32, d_initial_zero_final, SLX_F32}, nullptr, nullptr, nullptr,
+                          as_stream(stream));
 }
 
 int slx_v2x2ssd_bwd_finish(const slx_scan_shape *s, const void *U, const float *M, const float *K, const void *B,
@@ -711,8 +805,9 @@ int slx_v2x2ssd_bwd_finish(const slx_scan_shape *s, const void *U, const float *
                            const float *m_chunk, const float *final_state, const void *dY, const float *d_final,
                            void *dU, float *dM, float *dK, void *dB, void *dC, float *d_initial, float *dB_prev,
                            float *dU_prev, void *workspace, size_t workspace_bytes, void *stream) {
-  return v2x2ssd_bwd_impl(s, U, M, K, B, C, B_prev, U_prev, chunk_starts, m_chunk, final_state, dY, d_final, dU, dM,
-                          dK, dB, dC, d_initial, dB_prev, dU_prev, workspace, workspace_bytes, stream, true);
+  const slx_scan_grad_ends e = f32_grad_ends(B_prev, U_prev, d_final, d_initial, dB_prev, dU_prev);
+  return v2x2ssd_bwd_impl(s, U, M, K, B, C, &e, chunk_starts, m_chunk, final_state, dY, dU, dM, dK, dB, dC, workspace,
+                          workspace_bytes, stream, true);
 }
 
 }  // extern "C"

@@ -109,6 +109,21 @@ template <> __device__ __forceinline__ float from_f<float>(float v) { return v; 
 template <> __device__ __forceinline__ __nv_bfloat16 from_f<__nv_bfloat16>(float v) { return __float2bfloat16_rn(v); }
 template <> __device__ __forceinline__ __half from_f<__half>(float v) { return __float2half_rn(v); }
 
+// ---- small tensors in whatever dtype their owner holds them (slx_dtype code; the branch is uniform) ------
+__device__ __forceinline__ float load_as_f(const void *p, int dtype, size_t i) {
+  if (dtype == SLX_BF16) return __bfloat162float(static_cast<const __nv_bfloat16 *>(p)[i]);
+  if (dtype == SLX_F16) return __half2float(static_cast<const __half *>(p)[i]);
+  return static_cast<const float *>(p)[i];
+}
+__device__ __forceinline__ float2 load_as_f2(const void *p, int dtype, size_t i) {
+  return make_float2(load_as_f(p, dtype, i), load_as_f(p, dtype, i + 1));
+}
+__device__ __forceinline__ void store_as(void *p, int dtype, size_t i, float v) {
+  if (dtype == SLX_BF16) static_cast<__nv_bfloat16 *>(p)[i] = __float2bfloat16_rn(v);
+  else if (dtype == SLX_F16) static_cast<__half *>(p)[i] = __float2half_rn(v);
+  else static_cast<float *>(p)[i] = v;
+}
+
 // ---- complex numbers as float2 ------------------------------------------------
 __device__ __forceinline__ float2 cmul(float2 a, float2 b) {
   return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);

@@ -230,7 +230,7 @@ __device__ __forceinline__ void apply_dyact(const ConvDims &d, int t, const floa
 template <typename T, int VEC>
 __global__ void __launch_bounds__(kConvThreads) cconv1d_bwd_dstate_kernel(
     const T *__restrict__ x, const T *__restrict__ weight, const T *__restrict__ bias, const T *__restrict__ state,
-    const T *__restrict__ dy, const T *__restrict__ d_next, float *__restrict__ dstate, ConvDims d) {
+    const T *__restrict__ dy, const T *__restrict__ d_next, void *__restrict__ dstate, int grad_dtype, ConvDims d) {
   const int c0 = (blockIdx.x * kConvThreads + threadIdx.x) * VEC;
   if (c0 >= d.C) return;
   const int b = blockIdx.z;
@@ -264,7 +264,7 @@ __global__ void __launch_bounds__(kConvThreads) cconv1d_bwd_dstate_kernel(
       }
       int in = i - d.T;  // next_state index that aliases this state slot when T < W-1
       if (d_next && in >= 0) acc += to_f(d_next[((long long)b * d.C + c0 + e) * (d.W - 1) + in]);
-      dstate[((long long)b * d.C + c0 + e) * (d.W - 1) + i] = acc;
+      store_as(dstate, grad_dtype, ((size_t)b * d.C + c0 + e) * (d.W - 1) + i, acc);
     }
   }
 }
@@ -683,9 +683,9 @@ __global__ void __launch_bounds__(kConvThreads) cconv1d_fwd_staged_kernel(const 
 // the eight shares.  The order of every sum is fixed, so the result does not vary from run to run.
 constexpr int kConvReduceRows = 8;
 __global__ void __launch_bounds__(32 * kConvReduceRows) cconv1d_reduce_kernel(const float *__restrict__ part,
-                                                                              float *__restrict__ dweight,
-                                                                              float *__restrict__ dbias, int n_parts,
-                                                                              int C, int W) {
+                                                                              void *__restrict__ dweight,
+                                                                              void *__restrict__ dbias, int grad_dtype,
+                                                                              int n_parts, int C, int W) {
   __shared__ float share[kConvReduceRows][32];
   const int e = blockIdx.x * 32 + threadIdx.x, row = threadIdx.y;
   const size_t stride = (size_t)C * 5;
@@ -710,10 +710,10 @@ __global__ void __launch_bounds__(32 * kConvReduceRows) cconv1d_reduce_kernel(co
   for (int r = 1; r < kConvReduceRows; ++r) acc += share[r][threadIdx.x];
   const int c = e / 5, k = e % 5;
   if (k == 4) {
-    if (dbias) dbias[c] = acc;
+    if (dbias) store_as(dbias, grad_dtype, c, acc);
   } else {
     const int j = k - (4 - W);
-    if (j >= 0) dweight[(long long)c * W + j] = acc;
+    if (j >= 0) store_as(dweight, grad_dtype, (size_t)c * W + j, acc);
   }
 }
 
@@ -868,9 +868,9 @@ size_t slx_cconv1d_bwd_workspace_bytes(const slx_conv_shape *s) {
   return sizeof(float) * (size_t)d.batch * n_tiles * d.C * 5;
 }
 
-int slx_cconv1d_bwd(const slx_conv_shape *s, const void *x, const void *weight, const void *bias, const void *state,
-                    const void *dy, const void *d_next_state, void *dx, float *dweight, float *dbias, float *dstate,
-                    void *workspace, size_t workspace_bytes, void *stream) {
+int slx_cconv1d_bwd_as(const slx_conv_shape *s, const void *x, const void *weight, const void *bias, const void *state,
+                       const void *dy, const void *d_next_state, void *dx, void *dweight, void *dbias, void *dstate,
+                       int32_t grad_dtype, void *workspace, size_t workspace_bytes, void *stream) {
   ConvDims d;
   int rc = check_conv(s, &d);
   if (rc) return rc;
@@ -896,7 +896,7 @@ int slx_cconv1d_bwd(const slx_conv_shape *s, const void *x, const void *weight, 
       kern<<<dim3(nblk, n_tiles, d.batch), kConvThreads, ring, st>>>(xp, wp, bp, sp, gp, np, (T_ *)dx, part, d, tile);
       if (dstate)
         cconv1d_bwd_dstate_kernel<T_, VFULL><<<dim3(nblk, 1, d.batch), kConvThreads, 0, st>>>(xp, wp, bp, sp, gp, np,
-                                                                                            dstate, d);
+                                                                                            dstate, grad_dtype, d);
     } else {
       const int nblk = (d.C + kConvThreads - 1) / kConvThreads;
       const int tile = conv_tile(d.T, true);
@@ -905,14 +905,21 @@ int slx_cconv1d_bwd(const slx_conv_shape *s, const void *x, const void *weight, 
                                                                                      (T_ *)dx, part, d, tile);
       if (dstate)
         cconv1d_bwd_dstate_kernel<T_, 1><<<dim3(nblk, 1, d.batch), kConvThreads, 0, st>>>(xp, wp, bp, sp, gp, np,
-                                                                                        dstate, d);
+                                                                                        dstate, grad_dtype, d);
     }
   });
   rc = check_launch("cconv1d_bwd");
   if (rc) return rc;
-  cconv1d_reduce_kernel<<<(d.C * 5 + 31) / 32, dim3(32, kConvReduceRows), 0, st>>>(part, dweight, dbias,
+  cconv1d_reduce_kernel<<<(d.C * 5 + 31) / 32, dim3(32, kConvReduceRows), 0, st>>>(part, dweight, dbias, grad_dtype,
                                                                                    d.batch * n_tiles, d.C, d.W);
   return check_launch("cconv1d_reduce");
+}
+
+int slx_cconv1d_bwd(const slx_conv_shape *s, const void *x, const void *weight, const void *bias, const void *state,
+                    const void *dy, const void *d_next_state, void *dx, float *dweight, float *dbias, float *dstate,
+                    void *workspace, size_t workspace_bytes, void *stream) {
+  return slx_cconv1d_bwd_as(s, x, weight, bias, state, dy, d_next_state, dx, dweight, dbias, dstate, SLX_F32, workspace,
+                            workspace_bytes, stream);
 }
 
 }  // extern "C"

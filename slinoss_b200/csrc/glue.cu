@@ -21,6 +21,7 @@ struct GlueDims {
   int batch, T, H, P;
   long long gate_stride;  // elements between tokens of gate (it may be a column slice of a wider row)
   long long gate_batch_stride;
+  int skip_dtype;
 };
 
 template <typename T>
@@ -52,7 +53,7 @@ __device__ __forceinline__ void st8(T *p, const float (&v)[8]) {
 // thread index -> (head, first channel); C8 = H*P/8 threads carry data
 template <typename T>
 __global__ void __launch_bounds__(256) gate_skip_fwd_kernel(const T *__restrict__ y, const T *__restrict__ u,
-                                                            const T *__restrict__ gate, const float *__restrict__ skip,
+                                                            const T *__restrict__ gate, const void *__restrict__ skip,
                                                             T *__restrict__ out, GlueDims d) {
   const int v = blockIdx.x * blockDim.x + threadIdx.x;
   const int C8 = d.H * d.P / 8;
@@ -62,7 +63,7 @@ __global__ void __launch_bounds__(256) gate_skip_fwd_kernel(const T *__restrict_
   const int t1 = min(t0 + kGlueTile, d.T);
   float sk[8];
 #pragma unroll
-  for (int i = 0; i < 8; ++i) sk[i] = skip[ch + i];
+  for (int i = 0; i < 8; ++i) sk[i] = load_as_f(skip, d.skip_dtype, ch + i);
   const size_t yrow = (((size_t)b * d.H + h) * d.T) * d.P + p;
   for (int t = t0; t < t1; ++t) {
     float yv[8], uv[8], gv[8], o[8];
@@ -84,7 +85,7 @@ __global__ void __launch_bounds__(256) gate_skip_fwd_kernel(const T *__restrict_
 // d_out (b,T,H*P) -> dy, du (b,H,T,P), d_gate (b,T,H*P) contiguous, per-tile partials of d_skip
 template <typename T>
 __global__ void __launch_bounds__(256) gate_skip_bwd_kernel(const T *__restrict__ y, const T *__restrict__ u,
-                                                            const T *__restrict__ gate, const float *__restrict__ skip,
+                                                            const T *__restrict__ gate, const void *__restrict__ skip,
                                                             const T *__restrict__ d_out, T *__restrict__ dy,
                                                             T *__restrict__ du, T *__restrict__ d_gate,
                                                             float *__restrict__ part, GlueDims d) {
@@ -97,7 +98,7 @@ __global__ void __launch_bounds__(256) gate_skip_bwd_kernel(const T *__restrict_
   float sk[8], acc[8];
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
-    sk[i] = to_f(from_f<T>(skip[ch + i]));
+    sk[i] = to_f(from_f<T>(load_as_f(skip, d.skip_dtype, ch + i)));
     acc[i] = 0.f;
   }
   const size_t yrow = (((size_t)b * d.H + h) * d.T) * d.P + p;
@@ -129,8 +130,8 @@ __global__ void __launch_bounds__(256) gate_skip_bwd_kernel(const T *__restrict_
 
 // d_skip[c] = sum over the partial rows, in a fixed order: 32 channels x 16 row groups per CTA, every
 // thread adds the rows of its group (i = g, g + 16, ...), then the 16 group sums are added in order.
-__global__ void __launch_bounds__(512) gate_skip_reduce_kernel(const float *__restrict__ part, float *__restrict__ d_skip,
-                                                               int n_part, int C) {
+__global__ void __launch_bounds__(512) gate_skip_reduce_kernel(const float *__restrict__ part, void *__restrict__ d_skip,
+                                                               int skip_dtype, int n_part, int C) {
   __shared__ float red[16][33];
   const int cx = threadIdx.x & 31, g = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + cx;
@@ -143,7 +144,7 @@ __global__ void __launch_bounds__(512) gate_skip_reduce_kernel(const float *__re
     float tot = 0.f;
 #pragma unroll
     for (int k = 0; k < 16; ++k) tot += red[k][cx];
-    d_skip[c] = tot;
+    store_as(d_skip, skip_dtype, c, tot);
   }
 }
 
@@ -179,13 +180,14 @@ using namespace slx;
 
 extern "C" {
 
-int slx_gate_skip_fwd(const slx_glue_shape *s, const void *y, const void *u, const void *gate, const float *skip,
-                      void *out, void *stream) {
+int slx_gate_skip_fwd_as(const slx_glue_shape *s, const void *y, const void *u, const void *gate, const void *skip,
+                         int32_t skip_dtype, void *out, void *stream) {
   GlueDims d;
   int rc = check_glue(s, &d);
   if (rc) return rc;
   SLX_REQUIRE(y && u && gate && skip && out, SLX_E_NULL, "gate_skip_fwd: NULL tensor");
-  SLX_REQUIRE(glue_aligned({y, u, gate, skip, out}), SLX_E_UNSUPPORTED, "gate_skip_fwd: pointers must be 16-byte aligned");
+  d.skip_dtype = skip_dtype;
+  SLX_REQUIRE(glue_aligned({y, u, gate, out}), SLX_E_UNSUPPORTED, "gate_skip_fwd: pointers must be 16-byte aligned");
   const int C8 = d.H * d.P / 8;
   const int threads = C8 >= 256 ? 256 : ((C8 + 31) / 32) * 32;
   const dim3 grid((C8 + threads - 1) / threads, (d.T + kGlueTile - 1) / kGlueTile, d.batch);
@@ -195,6 +197,10 @@ int slx_gate_skip_fwd(const slx_glue_shape *s, const void *y, const void *u, con
   });
   return check_launch("gate_skip_fwd");
 }
+int slx_gate_skip_fwd(const slx_glue_shape *s, const void *y, const void *u, const void *gate, const float *skip,
+                      void *out, void *stream) {
+  return slx_gate_skip_fwd_as(s, y, u, gate, skip, SLX_F32, out, stream);
+}
 
 size_t slx_gate_skip_bwd_workspace_bytes(const slx_glue_shape *s) {
   GlueDims d;
@@ -202,14 +208,15 @@ size_t slx_gate_skip_bwd_workspace_bytes(const slx_glue_shape *s) {
   return sizeof(float) * (size_t)d.batch * ((d.T + kGlueTile - 1) / kGlueTile) * d.H * d.P;
 }
 
-int slx_gate_skip_bwd(const slx_glue_shape *s, const void *y, const void *u, const void *gate, const float *skip,
-                      const void *d_out, void *dy, void *du, void *d_gate, float *d_skip, void *workspace,
-                      size_t workspace_bytes, void *stream) {
+int slx_gate_skip_bwd_as(const slx_glue_shape *s, const void *y, const void *u, const void *gate, const void *skip,
+                         int32_t skip_dtype, const void *d_out, void *dy, void *du, void *d_gate, void *d_skip,
+                         void *workspace, size_t workspace_bytes, void *stream) {
   GlueDims d;
   int rc = check_glue(s, &d);
   if (rc) return rc;
   SLX_REQUIRE(y && u && gate && skip && d_out && dy && du && d_gate && d_skip, SLX_E_NULL, "gate_skip_bwd: NULL tensor");
-  SLX_REQUIRE(glue_aligned({y, u, gate, skip, d_out, dy, du, d_gate, d_skip, workspace}), SLX_E_UNSUPPORTED,
+  d.skip_dtype = skip_dtype;
+  SLX_REQUIRE(glue_aligned({y, u, gate, d_out, dy, du, d_gate, workspace}), SLX_E_UNSUPPORTED,
               "gate_skip_bwd: pointers must be 16-byte aligned");
   const size_t need = slx_gate_skip_bwd_workspace_bytes(s);
   SLX_REQUIRE(workspace && workspace_bytes >= need, SLX_E_WORKSPACE, "gate_skip_bwd: workspace of %zu bytes needed",
@@ -227,8 +234,15 @@ int slx_gate_skip_bwd(const slx_glue_shape *s, const void *y, const void *u, con
   rc = check_launch("gate_skip_bwd");
   if (rc) return rc;
   const int C = d.H * d.P;
-  gate_skip_reduce_kernel<<<(C + 31) / 32, 512, 0, as_stream(stream)>>>(part, d_skip, d.batch * n_tiles, C);
+  gate_skip_reduce_kernel<<<(C + 31) / 32, 512, 0, as_stream(stream)>>>(part, d_skip, skip_dtype, d.batch * n_tiles,
+                                                                         C);
   return check_launch("gate_skip_reduce");
+}
+int slx_gate_skip_bwd(const slx_glue_shape *s, const void *y, const void *u, const void *gate, const float *skip,
+                      const void *d_out, void *dy, void *du, void *d_gate, float *d_skip, void *workspace,
+                      size_t workspace_bytes, void *stream) {
+  return slx_gate_skip_bwd_as(s, y, u, gate, skip, SLX_F32, d_out, dy, du, d_gate, d_skip, workspace, workspace_bytes,
+                              stream);
 }
 
 }  // extern "C"

@@ -1,0 +1,845 @@
+// Native host path of the ops: argument checks of the common case, output and workspace allocation, the
+// autograd nodes and the calls into the C ABI (include/slinoss_b200.h).
+//
+// What bounds the small calls is the host: a Python autograd.Function, ctypes argument conversion and torch's
+// operator dispatch together took 110-260 us per scan or layer call, several times the kernels of a short
+// sequence (one token of decode: 213 us for 8 us of kernels).  Here a call costs the allocations and the launches.
+//
+// Every entry point takes the form in which programs normally call the op (one device, contiguous, 16-byte aligned,
+// matching shapes and dtypes) and returns None for anything else; the Python function above it then raises the
+// error, or converts the arguments and calls again.
+#include <ATen/ATen.h>
+#include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/autograd/function.h>
+#include <torch/csrc/autograd/functions/utils.h>
+#include <torch/csrc/autograd/saved_variable.h>
+#include <torch/csrc/utils/pybind.h>
+
+#include <optional>
+#include <tuple>
+#include <vector>
+
+#include "../../../include/slinoss_b200.h"
+
+namespace py = pybind11;
+using at::Tensor;
+using torch::autograd::Node;
+using torch::autograd::SavedVariable;
+using torch::autograd::variable_list;
+using OptTensor = std::optional<Tensor>;
+
+namespace {
+
+int code_of(at::ScalarType t) {
+  switch (t) {
+    case at::kFloat: return SLX_F32;
+    case at::kBFloat16: return SLX_BF16;
+    case at::kHalf: return SLX_F16;
+    default: return -1;
+  }
+}
+at::ScalarType type_of(int code) { return code == SLX_BF16 ? at::kBFloat16 : code == SLX_F16 ? at::kHalf : at::kFloat; }
+
+// A non-zero status as the exception the reference would raise.
+void check(int status, const char *what) {
+  if (status == SLX_OK) return;
+  const char *msg = slx_last_error_string();
+  if (status == SLX_E_DTYPE) TORCH_CHECK_TYPE(false, what, ": ", msg);
+  if (status < 0) TORCH_CHECK_VALUE(false, what, ": ", msg);
+  TORCH_CHECK(false, what, ": CUDA error ", status, ": ", msg);
+}
+
+Tensor empty(at::IntArrayRef sizes, at::ScalarType t, const at::Device &dev) {
+  return Tensor(at::detail::empty_cuda(sizes, t, dev, std::nullopt));
+}
+void *ptr(const Tensor &t) { return t.defined() ? t.data_ptr() : nullptr; }
+const void *cptr(const OptTensor &t) { return t ? t->data_ptr() : nullptr; }
+float *fptr(const Tensor &t) { return t.defined() ? static_cast<float *>(t.data_ptr()) : nullptr; }
+bool aligned(const Tensor &t) { return (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0; }
+void *stream_of(const at::Device &dev) { return c10::cuda::getCurrentCUDAStream(dev.index()).stream(); }
+bool is(const Tensor &t, const at::Device &dev) { return t.defined() && t.device() == dev; }
+bool shaped(const Tensor &t, at::IntArrayRef sizes) { return t.sizes() == sizes; }
+
+// an incoming gradient in the dtype and layout the kernels read
+Tensor grad_in(const Tensor &g, at::ScalarType t) {
+  Tensor r = g.scalar_type() == t ? g : g.to(t);
+  r = r.contiguous();
+  return aligned(r) ? r : r.clone();
+}
+Tensor saved(SavedVariable &v) { return v.unpack(); }
+SavedVariable keep(const Tensor &t) { return t.defined() ? SavedVariable(t, false) : SavedVariable(); }
+
+template <typename N>
+std::shared_ptr<N> make_node(torch::autograd::edge_list edges) {
+  std::shared_ptr<N> node(new N(), torch::autograd::deleteNode);
+  node->set_next_edges(std::move(edges));
+  return node;
+}
+
+// ------------------------------------------------------------------------------------------------------------
+// chunked scan
+// ------------------------------------------------------------------------------------------------------------
+struct ScanDims {
+  int64_t b, h, T, P, D, L, NC;
+  slx_scan_shape s;
+  at::Device dev = at::kCUDA;
+  at::ScalarType act;
+};
+
+ScanDims scan_dims(const Tensor &U, const Tensor &B, int64_t L) {
+  ScanDims d;
+  d.b = U.size(0);
+  d.h = U.size(1);
+  d.T = U.size(2);
+  d.P = U.size(3);
+  d.D = B.size(3);
+  d.L = L;
+  d.NC = (d.T + L - 1) / L;
+  d.dev = U.device();
+  d.act = U.scalar_type();
+  d.s = slx_scan_shape{(int32_t)(d.b * d.h), (int32_t)d.T, (int32_t)d.P, (int32_t)(d.D / 2), (int32_t)L,
+                       code_of(d.act), SLX_F32};
+  d.s.starts_dtype = slx_scan_starts_dtype(&d.s);
+  return d;
+}
+
+struct ScanForward {
+  Tensor Y, final32, final_copy, B_last, U_last, starts, mch;
+};
+
+ScanForward scan_forward(const ScanDims &d, const Tensor &U, const Tensor &M, const Tensor &K, const Tensor &B,
+                         const Tensor &C, const OptTensor &init, const OptTensor &Bp, const OptTensor &Up,
+                         bool want_final32, bool want_state, at::ScalarType final_type) {
+  ScanForward r;
+  const at::ScalarType st = type_of(d.s.starts_dtype);
+  const int64_t chunk_sizes[5] = {d.b, d.h, d.NC, d.P, d.D};
+  const int64_t state_sizes[4] = {d.b, d.h, d.P, d.D};
+  r.Y = empty(U.sizes(), d.act, d.dev);
+  r.starts = empty(chunk_sizes, st, d.dev);
+  r.mch = empty({d.b, d.h, d.NC, 2}, at::kFloat, d.dev);
+  // separate increment buffer (stored like the chunk starts): the two-buffer state pass is about 2.5x faster than
+  // the in-place one
+  Tensor inc = empty(chunk_sizes, st, d.dev);
+  slx_scan_ends e{};
+  if (want_state && final_type == at::kFloat) want_final32 = true;
+  if (want_final32) r.final32 = empty(state_sizes, at::kFloat, d.dev);
+  if (want_state) {
+    if (final_type == at::kFloat) {
+      r.final_copy = r.final32;
+    } else {
+      r.final_copy = empty(state_sizes, final_type, d.dev);
+      e.final_copy = ptr(r.final_copy);
+      e.final_dtype = code_of(final_type);
+    }
+    r.B_last = empty({d.b, d.h, d.D}, d.act, d.dev);
+    r.U_last = empty({d.b, d.h, d.P}, d.act, d.dev);
+    e.B_last = ptr(r.B_last);
+    e.U_last = ptr(r.U_last);
+  }
+  if (init) {
+    e.initial_states = init->data_ptr();
+    e.initial_dtype = code_of(init->scalar_type());
+  }
+  if (Bp) {
+    e.B_prev = Bp->data_ptr();
+    e.U_prev = Up->data_ptr();
+    e.prev_dtype = code_of(Bp->scalar_type());
+  }
+  c10::cuda::CUDAGuard guard(d.dev);
+  check(slx_v2x2ssd_fwd_stream(&d.s, ptr(U), fptr(M), fptr(K), ptr(B), ptr(C), &e, ptr(r.Y), fptr(r.final32),
+                               ptr(r.starts), fptr(r.mch), ptr(inc), stream_of(d.dev)),
+        "v2x2ssd forward");
+  return r;
+}
+
+struct ScanGrads {
+  Tensor dU, dM, dK, dB, dC, d_init, dBp, dUp;
+};
+
+ScanGrads scan_backward(const ScanDims &d, const Tensor &U, const Tensor &M, const Tensor &K, const Tensor &B,
+                        const Tensor &C, const Tensor &Bp, const Tensor &Up, const Tensor &starts, const Tensor &mch,
+                        const Tensor &final32, const Tensor &dY, const Tensor &d_final, std::optional<at::ScalarType> init_type,
+                        bool want_prev, const OptTensor &workspace) {
+  ScanGrads g;
+  g.dU = empty(U.sizes(), d.act, d.dev);
+  g.dB = empty(B.sizes(), d.act, d.dev);
+  g.dC = empty(C.sizes(), d.act, d.dev);
+  g.dM = empty(M.sizes(), at::kFloat, d.dev);
+  g.dK = empty(K.sizes(), at::kFloat, d.dev);
+  slx_scan_grad_ends e{};
+  if (Bp.defined()) {
+    e.B_prev = ptr(Bp);
+    e.U_prev = ptr(Up);
+    e.prev_dtype = code_of(Bp.scalar_type());
+  }
+  if (d_final.defined()) {
+    e.d_final = ptr(d_final);
+    e.d_final_dtype = code_of(d_final.scalar_type());
+  }
+  if (init_type) {
+    g.d_init = empty({d.b, d.h, d.P, d.D}, *init_type, d.dev);
+    e.d_initial = ptr(g.d_init);
+    e.d_initial_dtype = code_of(*init_type);
+  }
+  if (want_prev) {
+    const at::ScalarType t = Bp.scalar_type();
+    g.dBp = empty({d.b, d.h, d.D}, t, d.dev);
+    g.dUp = empty({d.b, d.h, d.P}, t, d.dev);
+    e.dB_prev = ptr(g.dBp);
+    e.dU_prev = ptr(g.dUp);
+    e.d_prev_dtype = code_of(t);
+  }
+  const size_t nbytes = slx_v2x2ssd_bwd_workspace_bytes(&d.s);
+  Tensor ws = workspace ? *workspace : empty({(int64_t)nbytes}, at::kByte, d.dev);
+  c10::cuda::CUDAGuard guard(d.dev);
+  if (!workspace) {
+    check(slx_v2x2ssd_bwd_stream(&d.s, ptr(U), fptr(M), fptr(K), ptr(B), ptr(C), &e, ptr(starts), fptr(mch),
+                                 fptr(final32), ptr(dY), ptr(g.dU), fptr(g.dM), fptr(g.dK), ptr(g.dB), ptr(g.dC),
+                                 ptr(ws), nbytes, stream_of(d.dev)),
+          "v2x2ssd backward");
+  } else {  // dZ0 is already in the workspace; this form takes fp32 streaming tensors
+    check(slx_v2x2ssd_bwd_finish(&d.s, ptr(U), fptr(M), fptr(K), ptr(B), ptr(C), fptr(Bp), fptr(Up), ptr(starts),
+                                 fptr(mch), fptr(final32), ptr(dY), fptr(d_final), ptr(g.dU), fptr(g.dM), fptr(g.dK),
+                                 ptr(g.dB), ptr(g.dC), fptr(g.d_init), fptr(g.dBp), fptr(g.dUp), ptr(ws), nbytes,
+                                 stream_of(d.dev)),
+          "v2x2ssd backward");
+  }
+  return g;
+}
+
+struct ScanBackward : public Node {
+  int64_t L = 0;
+  bool recompute = false;
+  SavedVariable U_, M_, K_, B_, C_, mch_, starts_, final_, init_, Bp_, Up_;
+  bool has_init = false, has_prev = false;
+  std::string name() const override { return "V2x2ssdBackward"; }
+
+  void release_variables() override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    for (SavedVariable *v : {&U_, &M_, &K_, &B_, &C_, &mch_, &starts_, &final_, &init_, &Bp_, &Up_}) v->reset_data();
+  }
+
+  variable_list apply(variable_list &&grads) override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    variable_list out(8);
+    const Tensor dY_in = grads[0];
+    const Tensor d_fin_in = grads.size() > 1 ? grads[1] : Tensor();
+    Tensor U = saved(U_), B = saved(B_);
+    if (dY_in.defined() || d_fin_in.defined()) {
+      Tensor M = saved(M_), K = saved(K_), C = saved(C_), mch = saved(mch_), final32 = saved(final_);
+      Tensor Bp, Up;
+      if (has_prev) {
+        Bp = saved(Bp_);
+        Up = saved(Up_);
+      }
+      const ScanDims d = scan_dims(U, B, L);
+      Tensor dY = dY_in.defined() ? grad_in(dY_in, d.act) : at::zeros_like(U);
+      Tensor d_fin;
+      if (d_fin_in.defined())
+        d_fin = grad_in(d_fin_in, code_of(d_fin_in.scalar_type()) < 0 ? at::kFloat : d_fin_in.scalar_type());
+      Tensor starts;
+      std::optional<at::ScalarType> init_type;
+      OptTensor init;
+      if (has_init) {
+        init = saved(init_);
+        init_type = init->scalar_type();
+      }
+      if (recompute) {
+        const at::ScalarType st = type_of(d.s.starts_dtype);
+        const int64_t sizes[5] = {d.b, d.h, d.NC, d.P, d.D};
+        starts = empty(sizes, st, d.dev);
+        Tensor inc = empty(sizes, st, d.dev), m2 = empty({d.b, d.h, d.NC, 2}, at::kFloat, d.dev);
+        slx_scan_ends e{};
+        if (init) {
+          e.initial_states = init->data_ptr();
+          e.initial_dtype = code_of(*init_type);
+        }
+        if (has_prev) {
+          e.B_prev = ptr(Bp);
+          e.U_prev = ptr(Up);
+          e.prev_dtype = code_of(Bp.scalar_type());
+        }
+        c10::cuda::CUDAGuard guard(d.dev);
+        check(slx_v2x2ssd_fwd_stream(&d.s, ptr(U), fptr(M), fptr(K), ptr(B), ptr(C), &e, nullptr, nullptr, ptr(starts),
+                                     fptr(m2), ptr(inc), stream_of(d.dev)),
+              "v2x2ssd chunk starts");
+      } else {
+        starts = saved(starts_);
+      }
+      ScanGrads g = scan_backward(d, U, M, K, B, C, Bp, Up, starts, mch, final32, dY, d_fin, init_type, has_prev,
+                                  std::nullopt);
+      out = {g.dU, g.dM, g.dK, g.dB, g.dC, g.d_init, g.dBp, g.dUp};
+    }
+    // cotangents of the carried-on rows (they are copies of row T-1 of B and U)
+    auto add_last = [](Tensor &acc, const Tensor &like, const Tensor &g) {
+      if (!g.defined()) return;
+      if (!acc.defined()) acc = at::zeros_like(like);
+      acc.select(2, -1).add_(g.to(acc.scalar_type()));
+    };
+    if (grads.size() > 2) add_last(out[3], B, grads[2]);
+    if (grads.size() > 3) add_last(out[0], U, grads[3]);
+    return out;
+  }
+};
+
+bool scan_inputs_plain(const Tensor &U, const Tensor &M, const Tensor &K, const Tensor &B, const Tensor &C,
+                       const OptTensor &init, const OptTensor &Bp, const OptTensor &Up) {
+  if (!U.is_cuda() || U.dim() != 4 || B.dim() != 4) return false;
+  const at::Device dev = U.device();
+  const at::ScalarType act = U.scalar_type();
+  const int64_t b = U.size(0), h = U.size(1), T = U.size(2), P = U.size(3), D = B.size(3);
+  if (code_of(act) < 0 || b == 0 || h == 0 || T == 0 || P == 0 || D == 0 || D % 2 != 0) return false;
+  const int64_t bsz[4] = {b, h, T, D}, msz[4] = {b, h, T, 2}, ksz[5] = {b, h, T, 2, 2};
+  if (!shaped(B, bsz) || !shaped(C, bsz) || !shaped(M, msz) || !shaped(K, ksz)) return false;
+  if (B.scalar_type() != act || C.scalar_type() != act || M.scalar_type() != at::kFloat || K.scalar_type() != at::kFloat)
+    return false;
+  for (const Tensor *t : {&U, &M, &K, &B, &C})
+    if (t->device() != dev || !t->is_contiguous() || !aligned(*t)) return false;
+  if (init) {
+    const int64_t sz[4] = {b, h, P, D};
+    if (!is(*init, dev) || !shaped(*init, sz) || !init->is_contiguous() || !aligned(*init) ||
+        code_of(init->scalar_type()) < 0)
+      return false;
+  }
+  if (Bp.has_value() != Up.has_value()) return false;
+  if (Bp) {
+    const int64_t sb[3] = {b, h, D}, su[3] = {b, h, P};
+    if (!is(*Bp, dev) || !is(*Up, dev) || !shaped(*Bp, sb) || !shaped(*Up, su) || !Bp->is_contiguous() ||
+        !Up->is_contiguous() || (Bp->scalar_type() != act && Bp->scalar_type() != at::kFloat) ||
+        Bp->scalar_type() != Up->scalar_type())
+      return false;
+  }
+  return true;
+}
+
+// (U, M, K, B, C) -> Y or (Y, final, B_last, U_last) in the activation dtype, with autograd.  None: not the
+// plain case.
+py::object v2x2ssd(const Tensor &U, const Tensor &M, const Tensor &K, const Tensor &B, const Tensor &C, int64_t L,
+                   const OptTensor &init, const OptTensor &Bp, const OptTensor &Up, bool return_state, bool retile,
+                   bool recompute, std::optional<at::ScalarType> final_type_in) {
+  if (!scan_inputs_plain(U, M, K, B, C, init, Bp, Up)) return py::none();
+  const int64_t P = U.size(3), D = B.size(3);
+  // chunk_size only says how the sequence is tiled; the tcgen05 kernels tile in 128 tokens
+  if (L > 0 && retile && U.scalar_type() != at::kFloat && P == 64 && D % 64 == 0 && D <= 256) L = 128;
+  if (L != 16 && L != 32 && L != 64 && L != 128) return py::none();
+  const at::ScalarType final_type = final_type_in.value_or(U.scalar_type());
+  if (code_of(final_type) < 0) return py::none();
+  const ScanDims d = scan_dims(U, B, L);
+  const bool grad = torch::autograd::compute_requires_grad(U, M, K, B, C, init.value_or(Tensor()),
+                                                           Bp.value_or(Tensor()), Up.value_or(Tensor()));
+  ScanForward r = scan_forward(d, U, M, K, B, C, init, Bp, Up, grad, return_state, final_type);
+  if (grad) {
+    auto node = make_node<ScanBackward>(torch::autograd::collect_next_edges(
+        U, M, K, B, C, init.value_or(Tensor()), Bp.value_or(Tensor()), Up.value_or(Tensor())));
+    node->L = L;
+    node->recompute = recompute;
+    node->U_ = keep(U);
+    node->M_ = keep(M);
+    node->K_ = keep(K);
+    node->B_ = keep(B);
+    node->C_ = keep(C);
+    node->mch_ = keep(r.mch);
+    node->final_ = keep(r.final32.is_same(r.final_copy) ? r.final32.detach() : r.final32);
+    // What is kept of the chunk-start states, the largest residual: as the kernels exchange them, or (recompute)
+    // nothing: the backward rebuilds them with one more chunk-increment and state pass.
+    if (!recompute) node->starts_ = keep(r.starts);
+    node->has_init = init.has_value();
+    node->has_prev = Bp.has_value();
+    if (init) node->init_ = keep(*init);
+    if (Bp) {
+      node->Bp_ = keep(*Bp);
+      node->Up_ = keep(*Up);
+    }
+    torch::autograd::set_history(r.Y, node);
+    if (return_state)
+      for (Tensor *t : {&r.final_copy, &r.B_last, &r.U_last}) torch::autograd::set_history(*t, node);
+  }
+  if (!return_state) return py::cast(r.Y);
+  return py::make_tuple(r.Y, r.final_copy, r.B_last, r.U_last);
+}
+
+// building blocks of the context-parallel mode: fp32 streaming tensors, no autograd
+py::tuple scan_fwd_parts(const Tensor &U, const Tensor &M, const Tensor &K, const Tensor &B, const Tensor &C,
+                         const OptTensor &init, const OptTensor &Bp, const OptTensor &Up, int64_t L) {
+  ScanForward r = scan_forward(scan_dims(U, B, L), U, M, K, B, C, init, Bp, Up, true, false, at::kFloat);
+  return py::make_tuple(r.Y, r.final32, r.starts, r.mch);
+}
+py::tuple scan_bwd_parts(const Tensor &U, const Tensor &M, const Tensor &K, const Tensor &B, const Tensor &C,
+                         const OptTensor &Bp, const OptTensor &Up, const Tensor &starts, const Tensor &mch,
+                         const Tensor &final32, const Tensor &dY, const OptTensor &d_final, int64_t L,
+                         bool want_initial, bool want_prev, const OptTensor &workspace) {
+  std::optional<at::ScalarType> it;
+  if (want_initial) it = at::kFloat;
+  ScanGrads g = scan_backward(scan_dims(U, B, L), U, M, K, B, C, Bp.value_or(Tensor()), Up.value_or(Tensor()), starts,
+                              mch, final32, dY, d_final.value_or(Tensor()), it, want_prev && Bp.has_value(), workspace);
+  auto opt = [](const Tensor &t) -> py::object { return t.defined() ? py::cast(t) : py::none(); };
+  return py::make_tuple(g.dU, g.dM, g.dK, g.dB, g.dC, opt(g.d_init), opt(g.dBp), opt(g.dUp));
+}
+
+// ------------------------------------------------------------------------------------------------------------
+// scan preparation
+// ------------------------------------------------------------------------------------------------------------
+constexpr int kParamDim = 13;
+
+// (b, T, width) with dense rows equally spaced over (b, T)
+bool dense_rows(const Tensor &x, int64_t width) {
+  return x.dim() >= 3 && x.stride(-1) == 1 && x.stride(1) >= width && (x.size(0) == 1 || x.stride(0) == x.size(1) * x.stride(1));
+}
+
+struct PrepConfig {
+  int64_t H, N, P;
+  bool normalize;
+  float dt_min, dt_max, r_min, r_max, theta_bound, k_max, eps;
+};
+using Hyper = std::tuple<double, double, double, double, double, double, double>;
+
+PrepConfig prep_config(int64_t H, int64_t N, int64_t P, bool normalize, const Hyper &hp) {
+  return PrepConfig{H, N, P, normalize, (float)std::get<0>(hp), (float)std::get<1>(hp), (float)std::get<2>(hp),
+                    (float)std::get<3>(hp), (float)std::get<4>(hp), (float)std::get<5>(hp), (float)std::get<6>(hp)};
+}
+slx_prep_shape prep_shape(const PrepConfig &c, int64_t b, int64_t T, int dtype, int64_t vs, int64_t ps, int64_t bs) {
+  return slx_prep_shape{(int32_t)b, (int32_t)T, (int32_t)c.H, (int32_t)c.P, (int32_t)c.N, dtype, c.normalize ? 1 : 0,
+                        c.dt_min, c.dt_max, c.r_min, c.r_max, c.theta_bound, c.k_max, c.eps, vs, ps, bs};
+}
+
+// The nine parameter tensors in one dtype: as they are where they agree, as fp32 copies otherwise.
+bool prep_params_plain(const std::vector<Tensor> &pars, bool normalize, const at::Device &dev, int64_t H, int64_t N) {
+  const size_t n = normalize ? 9 : 7;
+  if (pars.size() < n) return false;
+  for (size_t i = 0; i < n; ++i) {
+    const Tensor &t = pars[i];
+    if (!t.defined() || t.device() != dev || code_of(t.scalar_type()) < 0 || t.numel() != (i < 7 ? H : 2 * H * N))
+      return false;
+  }
+  return true;
+}
+std::vector<Tensor> uniform_params(const std::vector<Tensor> &pars, bool normalize) {
+  const size_t n = normalize ? 9 : 7;
+  const at::ScalarType t0 = pars[0].scalar_type();
+  bool same = true;
+  for (size_t i = 0; i < n; ++i)
+    same = same && pars[i].scalar_type() == t0 && pars[i].is_contiguous() && (i < 7 || aligned(pars[i]));
+  if (same) return pars;
+  std::vector<Tensor> r(pars.size());
+  for (size_t i = 0; i < n; ++i) {
+    r[i] = pars[i].detach().to(at::kFloat).contiguous();
+    if (!aligned(r[i])) r[i] = r[i].clone();
+  }
+  return r;
+}
+slx_prep_params params_struct(const std::vector<Tensor> &p, bool normalize) {
+  slx_prep_params s{};
+  for (int i = 0; i < 7; ++i) s.bias[i] = ptr(p[i]);
+  if (normalize) {
+    s.b_scale = ptr(p[7]);
+    s.c_scale = ptr(p[8]);
+  }
+  s.dtype = code_of(p[0].scalar_type());
+  return s;
+}
+
+struct PrepBackward : public Node {
+  PrepConfig cfg{};
+  int64_t b = 0, T = 0, ps = 0, bs = 0;
+  std::vector<int64_t> bc_sizes;
+  SavedVariable params_, bc_;
+  std::vector<SavedVariable> pars_;
+  std::vector<at::ScalarType> par_types;
+  std::string name() const override { return "ScanPrepBackward"; }
+  void release_variables() override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    params_.reset_data();
+    bc_.reset_data();
+    for (auto &v : pars_) v.reset_data();
+  }
+  variable_list apply(variable_list &&grads) override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    Tensor params = saved(params_), bc = saved(bc_);
+    std::vector<Tensor> pars(9);
+    const size_t n = cfg.normalize ? 9 : 7;
+    for (size_t i = 0; i < n; ++i) pars[i] = saved(pars_[i]);
+    pars = uniform_params(pars, cfg.normalize);
+    const at::ScalarType act = params.scalar_type(), pt = pars[0].scalar_type();
+    const at::Device dev = params.device();
+    auto in = [&](size_t i, at::IntArrayRef sizes, at::ScalarType t) {
+      return grads[i].defined() ? grad_in(grads[i], t) : at::zeros(sizes, at::TensorOptions().dtype(t).device(dev));
+    };
+    const int64_t H = cfg.H, N = cfg.N, P = cfg.P;
+    Tensor dU = in(0, {b, H, T, P}, act), dM = in(1, {b, H, T, 2}, at::kFloat), dK = in(2, {b, H, T, 2, 2}, at::kFloat),
+           dB = in(3, {b, H, T, 2 * N}, act), dC = in(4, {b, H, T, 2 * N}, act);
+    Tensor d_value = empty({b, T, H * P}, act, dev), d_params = empty({b, T, H * kParamDim}, act, dev);
+    Tensor d_bc = empty(bc_sizes, act, dev), d_bias = empty({7, H}, pt, dev), d_bs, d_cs;
+    if (cfg.normalize) {
+      d_bs = empty({H, 2, N}, pt, dev);
+      d_cs = empty({H, 2, N}, pt, dev);
+    }
+    const slx_prep_shape s = prep_shape(cfg, b, T, code_of(act), H * P, ps, bs);
+    const slx_prep_params pp = params_struct(pars, cfg.normalize);
+    const size_t nbytes = slx_scanprep_bwd_workspace_bytes(&s);
+    Tensor ws = empty({(int64_t)nbytes}, at::kByte, dev);
+    {
+      c10::cuda::CUDAGuard guard(dev);
+      check(slx_scanprep_bwd_params(&s, ptr(params), ptr(bc), &pp, ptr(dU), fptr(dM), fptr(dK), ptr(dB), ptr(dC),
+                                    ptr(d_value), ptr(d_params), ptr(d_bc), ptr(d_bias), ptr(d_bs), ptr(d_cs), ptr(ws),
+                                    nbytes, stream_of(dev)),
+            "scanprep backward");
+    }
+    variable_list out(12);
+    out[0] = d_value;
+    out[1] = d_params;
+    out[2] = d_bc;
+    for (int i = 0; i < 7; ++i) {
+      if (!task_should_compute_output(3 + i)) continue;
+      Tensor g = d_bias.select(0, i);
+      out[3 + i] = par_types[i] == pt ? g : g.to(par_types[i]);
+    }
+    if (cfg.normalize) {
+      out[10] = par_types[7] == pt ? d_bs : d_bs.to(par_types[7]);
+      out[11] = par_types[8] == pt ? d_cs : d_cs.to(par_types[8]);
+    }
+    return out;
+  }
+};
+
+// value (b,T,H*P), params (b,T,H*13), bc (b,T,H,4,N); pars = the seven biases, then b_scale, c_scale
+py::object scanprep(const Tensor &value, const Tensor &params, const Tensor &bc, int64_t H, int64_t N, int64_t P,
+                    bool normalize, const Hyper &hp, const std::vector<Tensor> &pars) {
+  if (!value.is_cuda() || value.dim() != 3 || params.dim() != 3 || bc.dim() != 5) return py::none();
+  const at::Device dev = value.device();
+  const at::ScalarType act = value.scalar_type();
+  const int64_t b = value.size(0), T = value.size(1);
+  if (b == 0 || T == 0 || H <= 0 || N <= 0 || P <= 0 || code_of(act) < 0) return py::none();
+  const int64_t vsz[3] = {b, T, H * P}, psz[3] = {b, T, H * kParamDim}, bsz[5] = {b, T, H, 4, N};
+  if (!shaped(value, vsz) || !shaped(params, psz) || !shaped(bc, bsz)) return py::none();
+  if (params.scalar_type() != act || bc.scalar_type() != act || params.device() != dev || bc.device() != dev)
+    return py::none();
+  if (!prep_params_plain(pars, normalize, dev, H, N)) return py::none();
+  auto rows = [](const Tensor &x, int64_t w) { return dense_rows(x, w) ? x : x.detach().contiguous(); };
+  Tensor v = rows(value, H * P), p = rows(params, H * kParamDim), c = bc;
+  const bool bc_ok = bc.stride(4) == 1 && bc.stride(3) == N && (H == 1 || bc.stride(2) == 4 * N) && bc.stride(1) >= H * 4 * N &&
+                     (b == 1 || bc.stride(0) == T * bc.stride(1));
+  if (!bc_ok) c = bc.detach().contiguous();
+  const PrepConfig cfg = prep_config(H, N, P, normalize, hp);
+  Tensor U = empty({b, H, T, P}, act, dev), M = empty({b, H, T, 2}, at::kFloat, dev),
+         K = empty({b, H, T, 2, 2}, at::kFloat, dev), B = empty({b, H, T, 2 * N}, act, dev),
+         C = empty({b, H, T, 2 * N}, act, dev);
+  const slx_prep_shape s = prep_shape(cfg, b, T, code_of(act), v.stride(1), p.stride(1), c.stride(1));
+  const std::vector<Tensor> up = uniform_params(pars, normalize);
+  const slx_prep_params pp = params_struct(up, normalize);
+  {
+    c10::cuda::CUDAGuard guard(dev);
+    check(slx_scanprep_fwd_params(&s, ptr(v), ptr(p), ptr(c), &pp, ptr(U), fptr(M), fptr(K), ptr(B), ptr(C),
+                                  stream_of(dev)),
+          "scanprep forward");
+  }
+  bool grad = torch::autograd::compute_requires_grad(value, params, bc);
+  if (!grad && at::GradMode::is_enabled())
+    for (const Tensor &t : pars) grad = grad || (t.defined() && t.requires_grad());
+  if (grad) {
+    torch::autograd::edge_list edges = torch::autograd::collect_next_edges(value, params, bc);
+    for (size_t i = 0; i < 9; ++i)
+      edges.push_back(i < pars.size() && pars[i].defined() ? torch::autograd::impl::gradient_edge(pars[i])
+                                                           : torch::autograd::Edge());
+    auto node = make_node<PrepBackward>(std::move(edges));
+    node->cfg = cfg;
+    node->b = b;
+    node->T = T;
+    node->ps = p.stride(1);
+    node->bs = c.stride(1);
+    node->bc_sizes.assign(bsz, bsz + 5);
+    node->params_ = keep(p);
+    node->bc_ = keep(c);
+    const size_t n = normalize ? 9 : 7;
+    node->pars_.reserve(n);
+    for (size_t i = 0; i < n; ++i) {
+      node->pars_.push_back(keep(pars[i]));
+      node->par_types.push_back(pars[i].scalar_type());
+    }
+    for (Tensor *t : {&U, &M, &K, &B, &C}) torch::autograd::set_history(*t, node);
+  }
+  return py::make_tuple(U, M, K, B, C);
+}
+
+// ------------------------------------------------------------------------------------------------------------
+// one-token decode step
+// ------------------------------------------------------------------------------------------------------------
+// value, gate (b,H,P), params (b,H,13), bc (b,H,4,N): rows dense inside a batch, any batch stride.
+bool dense_batch(const Tensor &x, int64_t inner) {
+  int64_t want = 1;
+  for (int64_t i = x.dim() - 1; i >= 1; --i) {
+    if (x.size(i) != 1 && x.stride(i) != want) return false;
+    want *= x.size(i);
+  }
+  return x.size(0) == 1 || x.stride(0) >= inner;
+}
+py::object decode_step(const Tensor &value, const Tensor &params, const Tensor &bc, const Tensor &gate,
+                       const Tensor &skip, const OptTensor &state_in, const OptTensor &Bp, const OptTensor &Up,
+                       bool normalize, const Hyper &hp, const std::vector<Tensor> &pars, const OptTensor &state_out_in,
+                       const OptTensor &b_last_in, const OptTensor &u_last_in) {
+  if (!value.is_cuda() || value.dim() != 3 || bc.dim() != 4) return py::none();
+  const at::Device dev = value.device();
+  const at::ScalarType act = value.scalar_type();
+  const int64_t b = value.size(0), H = value.size(1), P = value.size(2), N = bc.size(3);
+  if (code_of(act) < 0 || b == 0 || H == 0 || P == 0 || N == 0) return py::none();
+  const int64_t vsz[3] = {b, H, P}, psz[3] = {b, H, kParamDim}, bsz[4] = {b, H, 4, N}, ssz[4] = {b, H, P, 2 * N},
+                lsz[3] = {b, H, 2 * N};
+  if (!shaped(params, psz) || !shaped(bc, bsz) || !shaped(gate, vsz) || skip.numel() != H * P) return py::none();
+  for (const Tensor *t : {&params, &bc, &gate, &skip})
+    if (t->device() != dev) return py::none();
+  for (const Tensor *t : {&params, &bc, &gate})
+    if (t->scalar_type() != act) return py::none();
+  if (code_of(skip.scalar_type()) < 0 || !skip.is_contiguous()) return py::none();
+  if (!dense_batch(value, H * P) || !dense_batch(params, H * kParamDim) || !dense_batch(bc, H * 4 * N) ||
+      !dense_batch(gate, H * P))
+    return py::none();
+  if (!prep_params_plain(pars, normalize, dev, H, N)) return py::none();
+  auto fits = [&](const OptTensor &t, at::IntArrayRef sz, at::ScalarType ty) {
+    return !t || (is(*t, dev) && shaped(*t, sz) && t->is_contiguous() && t->scalar_type() == ty);
+  };
+  if (Bp.has_value() != Up.has_value()) return py::none();
+  if (!fits(state_in, ssz, at::kFloat) || !fits(Bp, lsz, act) || !fits(Up, vsz, act) ||
+      !fits(state_out_in, ssz, at::kFloat) || !fits(b_last_in, lsz, act) || !fits(u_last_in, vsz, act))
+    return py::none();
+  Tensor out = empty({b, H * P}, act, dev);
+  Tensor state_out = state_out_in ? *state_out_in : empty(ssz, at::kFloat, dev);
+  Tensor b_last = b_last_in ? *b_last_in : empty(lsz, act, dev);
+  Tensor u_last = u_last_in ? *u_last_in : empty(vsz, act, dev);
+  const PrepConfig c = prep_config(H, N, P, normalize, hp);
+  const slx_decode_shape s{(int32_t)b, (int32_t)H, (int32_t)P, (int32_t)N, code_of(act), normalize ? 1 : 0,
+                           c.dt_min, c.dt_max, c.r_min, c.r_max, c.theta_bound, c.k_max, c.eps};
+  const std::vector<Tensor> up = uniform_params(pars, normalize);
+  const slx_prep_params pp = params_struct(up, normalize);
+  const int64_t strides[4] = {value.stride(0), params.stride(0), bc.stride(0), gate.stride(0)};
+  c10::cuda::CUDAGuard guard(dev);
+  check(slx_decode_step_params(&s, ptr(value), ptr(params), ptr(bc), ptr(gate), strides, ptr(skip),
+                               code_of(skip.scalar_type()), &pp, static_cast<const float *>(cptr(state_in)), cptr(Bp),
+                               cptr(Up), ptr(out), fptr(state_out), ptr(b_last), ptr(u_last), stream_of(dev)),
+        "decode step");
+  return py::make_tuple(out, state_out, b_last, u_last);
+}
+
+// ------------------------------------------------------------------------------------------------------------
+// causal conv
+// ------------------------------------------------------------------------------------------------------------
+Tensor as_type(const Tensor &t, at::ScalarType ty) {
+  return (t.scalar_type() == ty ? t : t.detach().to(ty)).contiguous();
+}
+
+struct ConvBackward : public Node {
+  bool silu = false, has_bias = false, has_state = false;
+  at::ScalarType w_type, b_type, s_type;
+  SavedVariable x_, w_, bias_, state_;
+  std::string name() const override { return "CConv1dBackward"; }
+  void release_variables() override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    for (SavedVariable *v : {&x_, &w_, &bias_, &state_}) v->reset_data();
+  }
+  variable_list apply(variable_list &&grads) override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    Tensor x = saved(x_);
+    const at::ScalarType act = x.scalar_type();
+    const at::Device dev = x.device();
+    Tensor w = as_type(saved(w_), act), bias, state;
+    if (has_bias) bias = as_type(saved(bias_), act);
+    if (has_state) state = as_type(saved(state_), act);
+    const int64_t b = x.size(0), T = x.size(1), C = x.size(2), W = w.size(1);
+    Tensor dy = grads[0].defined() ? grad_in(grads[0], act)
+                                   : at::zeros({b, T, C}, at::TensorOptions().dtype(act).device(dev));
+    Tensor dn;
+    if (grads[1].defined()) dn = as_type(grads[1], act);
+    // the fp32 sums are rounded once, to the dtype of the parameter they belong to
+    const bool one_type = (!has_bias || b_type == w_type) && (!has_state || s_type == w_type) && code_of(w_type) >= 0;
+    const at::ScalarType gt = one_type ? w_type : at::kFloat;
+    Tensor dx = empty({b, T, C}, act, dev), dw = empty({C, W}, gt, dev), db, ds;
+    if (has_bias) db = empty({C}, gt, dev);
+    if (has_state) ds = empty({b, C, W - 1}, gt, dev);
+    const slx_conv_shape s{(int32_t)b, (int32_t)T, (int32_t)C, (int32_t)W, code_of(act), silu ? 1 : 0,
+                           std::max<int64_t>(x.stride(1), C), x.stride(0)};
+    const size_t nbytes = slx_cconv1d_bwd_workspace_bytes(&s);
+    Tensor ws = empty({(int64_t)nbytes}, at::kByte, dev);
+    {
+      c10::cuda::CUDAGuard guard(dev);
+      check(slx_cconv1d_bwd_as(&s, ptr(x), ptr(w), ptr(bias), ptr(state), ptr(dy), ptr(dn), ptr(dx), ptr(dw), ptr(db),
+                               ptr(ds), code_of(gt), ptr(ws), nbytes, stream_of(dev)),
+            "cconv1d backward");
+    }
+    auto back = [&](const Tensor &t, at::ScalarType ty) { return t.defined() && ty != gt ? t.to(ty) : t; };
+    return {dx, back(dw, w_type), back(db, b_type), back(ds, s_type)};
+  }
+};
+
+py::object cconv1d(const Tensor &x_in, const Tensor &weight, const OptTensor &bias, const OptTensor &state, bool silu) {
+  if (!x_in.is_cuda() || x_in.dim() != 3 || weight.dim() != 2) return py::none();
+  const at::Device dev = x_in.device();
+  const at::ScalarType act = x_in.scalar_type();
+  const int64_t b = x_in.size(0), T = x_in.size(1), C = x_in.size(2), W = weight.size(1);
+  if (code_of(act) < 0 || b == 0 || T == 0 || C == 0 || W < 2 || W > 4 || weight.size(0) != C || weight.device() != dev)
+    return py::none();
+  if (bias && (!is(*bias, dev) || bias->numel() != C)) return py::none();
+  const int64_t ssz[3] = {b, C, W - 1};
+  if (state && (!is(*state, dev) || !shaped(*state, ssz))) return py::none();
+  // a column slice of a wider matrix is read where it is; anything else is copied
+  const bool rows = x_in.stride(2) == 1 && (T == 1 || x_in.stride(1) >= C);
+  const Tensor x = rows ? x_in : x_in.detach().contiguous();
+  const Tensor w = as_type(weight, act), bs = bias ? as_type(*bias, act) : Tensor(),
+               st = state ? as_type(*state, act) : Tensor();
+  Tensor y = empty({b, T, C}, act, dev), nxt = empty(ssz, act, dev);
+  const slx_conv_shape s{(int32_t)b, (int32_t)T, (int32_t)C, (int32_t)W, code_of(act), silu ? 1 : 0,
+                         std::max<int64_t>(x.stride(1), C), x.stride(0)};
+  {
+    c10::cuda::CUDAGuard guard(dev);
+    check(slx_cconv1d_fwd(&s, ptr(x), ptr(w), ptr(bs), ptr(st), ptr(y), ptr(nxt), stream_of(dev)), "cconv1d forward");
+  }
+  if (torch::autograd::compute_requires_grad(x_in, weight, bias.value_or(Tensor()), state.value_or(Tensor()))) {
+    auto node = make_node<ConvBackward>(torch::autograd::collect_next_edges(x_in, weight, bias.value_or(Tensor()),
+                                                                            state.value_or(Tensor())));
+    node->silu = silu;
+    node->has_bias = bias.has_value();
+    node->has_state = state.has_value();
+    node->w_type = weight.scalar_type();
+    if (bias) node->b_type = bias->scalar_type();
+    if (state) node->s_type = state->scalar_type();
+    node->x_ = keep(x);
+    node->w_ = keep(weight);
+    if (bias) node->bias_ = keep(*bias);
+    if (state) node->state_ = keep(*state);
+    torch::autograd::set_history(y, node);
+    torch::autograd::set_history(nxt, node);
+  }
+  return py::make_tuple(y, nxt);
+}
+
+// x (b,C), rolling state (b,C,W-1) -> (y, next state); `inplace`: the state tensor itself is rolled
+py::object cconv1d_update(const Tensor &x_in, const Tensor &weight, const OptTensor &bias, const OptTensor &state,
+                          bool silu, bool inplace) {
+  if (!x_in.is_cuda() || x_in.dim() != 2 || weight.dim() != 2) return py::none();
+  const at::Device dev = x_in.device();
+  const at::ScalarType act = x_in.scalar_type();
+  const int64_t b = x_in.size(0), C = x_in.size(1), W = weight.size(1);
+  if (code_of(act) < 0 || b == 0 || C == 0 || W < 2 || W > 4 || weight.size(0) != C || weight.device() != dev)
+    return py::none();
+  if (bias && (!is(*bias, dev) || bias->numel() != C)) return py::none();
+  const int64_t ssz[3] = {b, C, W - 1};
+  if (state && (!is(*state, dev) || !shaped(*state, ssz))) return py::none();
+  if (inplace && (!state || state->scalar_type() != act || !state->is_contiguous())) return py::none();
+  const Tensor x = x_in.stride(1) == 1 ? x_in : x_in.contiguous();
+  const Tensor w = as_type(weight, act), bs = bias ? as_type(*bias, act) : Tensor(),
+               st = state ? as_type(*state, act) : Tensor();
+  Tensor y = empty({b, C}, act, dev), nxt = inplace ? *state : empty(ssz, act, dev);
+  const slx_conv_shape s{(int32_t)b, 1, (int32_t)C, (int32_t)W, code_of(act), silu ? 1 : 0, C, x.stride(0)};
+  c10::cuda::CUDAGuard guard(dev);
+  check(slx_cconv1d_update(&s, ptr(x), ptr(w), ptr(bs), ptr(st), ptr(y), ptr(nxt), stream_of(dev)), "cconv1d update");
+  return py::make_tuple(y, nxt);
+}
+
+// ------------------------------------------------------------------------------------------------------------
+// skip and gate
+// ------------------------------------------------------------------------------------------------------------
+struct GateBackward : public Node {
+  SavedVariable y_, u_, gate_, skip_;
+  at::ScalarType u_type, g_type, s_type;
+  std::vector<int64_t> skip_sizes;
+  std::string name() const override { return "GateSkipBackward"; }
+  void release_variables() override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    for (SavedVariable *v : {&y_, &u_, &gate_, &skip_}) v->reset_data();
+  }
+  variable_list apply(variable_list &&grads) override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    if (!grads[0].defined()) return variable_list(4);
+    Tensor y = saved(y_), u = saved(u_), gate = saved(gate_), skip = saved(skip_);
+    const int64_t b = y.size(0), H = y.size(1), T = y.size(2), P = y.size(3);
+    const at::ScalarType act = y.scalar_type();
+    const at::Device dev = y.device();
+    Tensor go = grad_in(grads[0], act);
+    const at::ScalarType kt = code_of(s_type) >= 0 ? s_type : at::kFloat;
+    Tensor dy = empty(y.sizes(), act, dev), du = empty(y.sizes(), act, dev), dg = empty({b, T, H * P}, act, dev),
+           dsk = empty(skip_sizes, kt, dev);
+    const slx_glue_shape s{(int32_t)b, (int32_t)T, (int32_t)H, (int32_t)P, code_of(act), gate.stride(1), gate.stride(0)};
+    const size_t nbytes = slx_gate_skip_bwd_workspace_bytes(&s);
+    Tensor ws = empty({(int64_t)nbytes}, at::kByte, dev);
+    {
+      c10::cuda::CUDAGuard guard(dev);
+      check(slx_gate_skip_bwd_as(&s, ptr(y), ptr(u), ptr(gate), ptr(skip), code_of(skip.scalar_type()), ptr(go), ptr(dy),
+                                 ptr(du), ptr(dg), ptr(dsk), ptr(ws), nbytes, stream_of(dev)),
+            "gate_skip backward");
+    }
+    auto back = [](const Tensor &t, at::ScalarType ty) { return t.scalar_type() == ty ? t : t.to(ty); };
+    return {dy, back(du, u_type), back(dg, g_type), back(dsk, s_type)};
+  }
+};
+
+py::object gate_skip(const Tensor &y_in, const Tensor &u_in, const Tensor &gate_in, const Tensor &skip_in) {
+  if (!y_in.is_cuda() || y_in.dim() != 4 || gate_in.dim() != 3) return py::none();
+  const at::Device dev = y_in.device();
+  const at::ScalarType act = y_in.scalar_type();
+  const int64_t b = y_in.size(0), H = y_in.size(1), T = y_in.size(2), P = y_in.size(3);
+  const int64_t gsz[3] = {b, T, H * P};
+  if (code_of(act) < 0 || b == 0 || T == 0 || H == 0 || P == 0 || P % 8 != 0 || !shaped(u_in, y_in.sizes()) ||
+      !shaped(gate_in, gsz) || skip_in.numel() != H * P)
+    return py::none();
+  for (const Tensor *t : {&u_in, &gate_in, &skip_in})
+    if (t->device() != dev) return py::none();
+  auto plain = [&](const Tensor &t) {
+    Tensor r = as_type(t, act);
+    return aligned(r) ? r : r.clone();
+  };
+  const Tensor y = plain(y_in), u = plain(u_in);
+  // the gate may be a column slice of a wider row with 16-byte aligned rows
+  Tensor gate = gate_in.scalar_type() == act ? gate_in : gate_in.detach().to(act);
+  if (gate.stride(2) != 1 || gate.stride(1) % 8 != 0 || gate.stride(0) % 8 != 0 || gate.stride(1) < H * P || !aligned(gate))
+    gate = gate.detach().contiguous();
+  Tensor skip = skip_in;
+  if (code_of(skip.scalar_type()) < 0) skip = skip.detach().to(at::kFloat);
+  if (!skip.is_contiguous()) skip = skip.detach().contiguous();
+  Tensor out = empty(gsz, act, dev);
+  const slx_glue_shape s{(int32_t)b, (int32_t)T, (int32_t)H, (int32_t)P, code_of(act), gate.stride(1), gate.stride(0)};
+  {
+    c10::cuda::CUDAGuard guard(dev);
+    check(slx_gate_skip_fwd_as(&s, ptr(y), ptr(u), ptr(gate), ptr(skip), code_of(skip.scalar_type()), ptr(out),
+                               stream_of(dev)),
+          "gate_skip forward");
+  }
+  if (torch::autograd::compute_requires_grad(y_in, u_in, gate_in, skip_in)) {
+    auto node = make_node<GateBackward>(torch::autograd::collect_next_edges(y_in, u_in, gate_in, skip_in));
+    node->y_ = keep(y);
+    node->u_ = keep(u);
+    node->gate_ = keep(gate);
+    node->skip_ = keep(skip);
+    node->u_type = u_in.scalar_type();
+    node->g_type = gate_in.scalar_type();
+    node->s_type = skip_in.scalar_type();
+    node->skip_sizes = skip_in.sizes().vec();
+    torch::autograd::set_history(out, node);
+  }
+  return py::cast(out);
+}
+
+// argument errors that the C ABI reports reach Python as the exceptions the ops document
+template <typename R, typename... A>
+auto python(R (*fn)(A...)) {
+  return [fn](A... args) -> R {
+    try {
+      return fn(args...);
+    } catch (const c10::ValueError &e) {
+      throw py::value_error(e.what_without_backtrace());
+    } catch (const c10::TypeError &e) {
+      throw py::type_error(e.what_without_backtrace());
+    }
+  };
+}
+
+}  // namespace
+
+PYBIND11_MODULE(_host, m) {
+  m.def("v2x2ssd", python(&v2x2ssd));
+  m.def("scan_fwd_parts", python(&scan_fwd_parts));
+  m.def("scan_bwd_parts", python(&scan_bwd_parts));
+  m.def("scanprep", python(&scanprep));
+  m.def("decode_step", python(&decode_step));
+  m.def("cconv1d", python(&cconv1d));
+  m.def("cconv1d_update", python(&cconv1d_update));
+  m.def("gate_skip", python(&gate_skip));
+}

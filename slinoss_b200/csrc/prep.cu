@@ -100,6 +100,16 @@ __device__ __forceinline__ void store_vec(T *p, const float (&v)[VEC]) {
   }
 }
 
+// VEC adjacent RMS-norm scales of plane j, head h
+template <int VEC>
+__device__ __forceinline__ void load_scale(const PrepParams &pp, int h, int j, int N, int n0, float (&v)[VEC]) {
+  const void *base = scale_plane(pp, j);
+  const size_t e = scale_index(pp, h, j, N, n0);
+  if (pp.dtype == SLX_BF16) load_vec<__nv_bfloat16, VEC>(static_cast<const __nv_bfloat16 *>(base) + e, v);
+  else if (pp.dtype == SLX_F16) load_vec<__half, VEC>(static_cast<const __half *>(base) + e, v);
+  else load_vec<float, VEC>(static_cast<const float *>(base) + e, v);
+}
+
 // ---- the 13-value parameter row of one (batch, head, token) ---------------------------------
 // Half types: the row is 26 bytes at an arbitrary 2-byte offset.  `wide` loads the two or three
 // aligned 16-byte vectors that cover it and picks the 13 values out by the (per-thread) offset;
@@ -187,8 +197,7 @@ struct PrepDims {
 // state lanes n in [VEC*(q + G*k), VEC*(q + G*k) + VEC).
 template <typename T, int VEC, int G>
 __global__ void __launch_bounds__(256) scanprep_fwd_kernel(const T *__restrict__ value, const T *__restrict__ params,
-                                                           const T *__restrict__ bc, const float *__restrict__ bias,
-                                                           const float *__restrict__ scale, T *__restrict__ U,
+                                                           const T *__restrict__ bc, PrepParams pp, T *__restrict__ U,
                                                            float *__restrict__ M, float *__restrict__ K,
                                                            T *__restrict__ Bo, T *__restrict__ Co, PrepDims d,
                                                            PrepHyper hp) {
@@ -211,8 +220,7 @@ __global__ void __launch_bounds__(256) scanprep_fwd_kernel(const T *__restrict__
         float p[13];
         const T *pr = params + ((long long)b * d.T + t) * d.ps + (long long)h * 13;
         load_row13<T>(pr, d.wide_params != 0, p);
-#pragma unroll
-        for (int i = 0; i < 13; ++i) p[i] += bias[h * 13 + i];
+        add_bias13(pp, h, p);
         CoefOut o = coef_forward(p, hp, nullptr);
         *reinterpret_cast<float2 *>(M + row * 2) = o.rho;
         *reinterpret_cast<float4 *>(K + row * 4) = make_float4(o.kp.x, o.kp.y, o.kc.x, o.kc.y);
@@ -291,7 +299,7 @@ __global__ void __launch_bounds__(256) scanprep_fwd_kernel(const T *__restrict__
               ss[j] = rsqrtf(group_sum_f<G>(ss[j]) / (float)d.N + 1e-5f);
               if (mine) {
                 float sc[VEC];
-                load_vec<float, VEC>(scale + ((long long)h * 4 + j) * d.N + n0, sc);
+                load_scale<VEC>(pp, h, j, d.N, n0, sc);
 #pragma unroll
                 for (int i = 0; i < VEC; ++i) y[j][i] = (y[j][i] * ss[j]) * sc[i];
               }
@@ -349,7 +357,7 @@ __global__ void __launch_bounds__(256) scanprep_fwd_kernel(const T *__restrict__
             ss[j] = rsqrtf(group_sum_f<G>(ss[j]) / (float)d.N + 1e-5f);
             if (mine) {
               float sc[VEC];
-              load_vec<float, VEC>(scale + ((long long)h * 4 + j) * d.N + n0, sc);
+              load_scale<VEC>(pp, h, j, d.N, n0, sc);
 #pragma unroll
               for (int i = 0; i < VEC; ++i) y[j][i] = (y[j][i] * ss[j]) * sc[i];
             }
@@ -394,7 +402,8 @@ __global__ void __launch_bounds__(256) scanprep_fwd_kernel(const T *__restrict__
             for (int j = 0; j < 4; ++j) {
               load_vec<T, VEC>(bcr + j * d.N + n0, y[j]);
               if (d.normalize) {
-                const float *sc = scale + ((long long)h * 4 + j) * d.N + n0;
+                float sc[VEC];
+                load_scale<VEC>(pp, h, j, d.N, n0, sc);
 #pragma unroll
                 for (int i = 0; i < VEC; ++i) y[j][i] = (y[j][i] * ss[j]) * sc[i];
               }
@@ -420,7 +429,7 @@ __global__ void __launch_bounds__(256) scanprep_fwd_kernel(const T *__restrict__
 }
 
 template <typename T>
-__device__ __forceinline__ void scanprep_bwd_coef_tile(const T *__restrict__ params, const float *__restrict__ bias,
+__device__ __forceinline__ void scanprep_bwd_coef_tile(const T *__restrict__ params, const PrepParams &pp,
                                                        const float *__restrict__ dM, const float *__restrict__ dK,
                                                        T *__restrict__ d_params, float *__restrict__ part,
                                                        const PrepDims &d, const PrepHyper &hp, int rows_per_tile,
@@ -435,15 +444,14 @@ __device__ __forceinline__ void scanprep_bwd_coef_tile(const T *__restrict__ par
 // Partial layout: part[(bh * n_tiles + tile)][4*N + 13].
 template <typename T, int VEC, int G, int KMAX>
 __global__ void __launch_bounds__(256, KMAX == 1 ? 2 : 1) scanprep_bwd_kernel(const T *__restrict__ params, const T *__restrict__ bc,
-                                                           const float *__restrict__ bias,
-                                                           const float *__restrict__ scale, const T *__restrict__ dU,
+                                                           PrepParams pp, const T *__restrict__ dU,
                                                            const float *__restrict__ dM, const float *__restrict__ dK,
                                                            const T *__restrict__ dB, const T *__restrict__ dC,
                                                            T *__restrict__ d_value, T *__restrict__ d_params,
                                                            T *__restrict__ d_bc, float *__restrict__ part, PrepDims d,
                                                            PrepHyper hp, int rows_per_tile, int n_tiles) {
   if ((int)blockIdx.x >= n_tiles) {
-    scanprep_bwd_coef_tile<T>(params, bias, dM, dK, d_params, part, d, hp, rows_per_tile, (int)blockIdx.x - n_tiles,
+    scanprep_bwd_coef_tile<T>(params, pp, dM, dK, d_params, part, d, hp, rows_per_tile, (int)blockIdx.x - n_tiles,
                               n_tiles);
     return;
   }
@@ -469,7 +477,10 @@ __global__ void __launch_bounds__(256, KMAX == 1 ? 2 : 1) scanprep_bwd_kernel(co
   constexpr bool kPacked = (KMAX == 1) && (VEC > 1) && (VEC * sizeof(T) == 16);
   float *sscale = red + (size_t)GPB * W;
   if (kPacked && d.normalize) {
-    for (int e = threadIdx.x; e < 4 * d.N; e += 256) sscale[e] = scale[(long long)h * 4 * d.N + e];
+    for (int e = threadIdx.x; e < 4 * d.N; e += 256) {
+      const int j = e / d.N, n = e - j * d.N;
+      sscale[e] = load_as_f(scale_plane(pp, j), pp.dtype, scale_index(pp, h, j, d.N, n));
+    }
     __syncthreads();
   }
   if constexpr (kPacked) {
@@ -625,7 +636,7 @@ __global__ void __launch_bounds__(256, KMAX == 1 ? 2 : 1) scanprep_bwd_kernel(co
             if (live) dy = (j < 2) ? ib[o / VEC][o % VEC] : ic[o / VEC][o % VEC];
             if (d.normalize) {
               float xv = live ? x[i] * ss[j] : 0.f;
-              float g = dy * scale[((long long)h * 4 + j) * d.N + n0 + i];
+              float g = dy * load_as_f(scale_plane(pp, j), pp.dtype, scale_index(pp, h, j, d.N, n0 + i));
               xh[k][j][i] = xv;
               gg[k][j][i] = g;
               dsc[k][j][i] = fmaf(dy, xv, dsc[k][j][i]);
@@ -686,7 +697,7 @@ __global__ void __launch_bounds__(256, KMAX == 1 ? 2 : 1) scanprep_bwd_kernel(co
 // (part[(bh * n_tiles + tile)][4N .. 4N+13)).  Little traffic, long scalar chains: run by CTAs of
 // their own inside the backward launch.
 template <typename T>
-__device__ __forceinline__ void scanprep_bwd_coef_tile(const T *__restrict__ params, const float *__restrict__ bias,
+__device__ __forceinline__ void scanprep_bwd_coef_tile(const T *__restrict__ params, const PrepParams &pp,
                                                        const float *__restrict__ dM, const float *__restrict__ dK,
                                                        T *__restrict__ d_params, float *__restrict__ part,
                                                        const PrepDims &d, const PrepHyper &hp, int rows_per_tile,
@@ -706,8 +717,7 @@ __device__ __forceinline__ void scanprep_bwd_coef_tile(const T *__restrict__ par
       float p[13], dp[13];
       const T *pr = params + in_row * d.ps + (long long)h * 13;
       load_row13<T>(pr, d.wide_params != 0, p);
-#pragma unroll
-      for (int i = 0; i < 13; ++i) p[i] += bias[h * 13 + i];
+      add_bias13(pp, h, p);
       CoefCtx ctx;
       coef_forward(p, hp, &ctx);
       float2 dm = *reinterpret_cast<const float2 *>(dM + orow * 2);
@@ -735,8 +745,15 @@ __device__ __forceinline__ void scanprep_bwd_coef_tile(const T *__restrict__ par
 }
 
 // d_scale[h][e], d_bias[h][i] = sum over batch and tiles of the partials, fixed order
-__global__ void scanprep_reduce_kernel(const float *__restrict__ part, float *__restrict__ d_bias,
-                                       float *__restrict__ d_scale, int batch, int H, int n_tiles, int N) {
+struct PrepParamGrads {
+  float *bias13;                // [opt] (H,13) fp32, every slot
+  void *bias[7];                // [opt] the seven biases' gradients, H values each, as dtype
+  void *b_scale, *c_scale;      // [opt] as dtype, laid out like the parameters (scale_stride per head)
+  int dtype;
+  long long scale_stride;
+};
+__global__ void scanprep_reduce_kernel(const float *__restrict__ part, PrepParamGrads g, int batch, int H, int n_tiles,
+                                       int N) {
   const int W = 4 * N + 13;
   const int h = blockIdx.y;
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
@@ -755,9 +772,14 @@ __global__ void scanprep_reduce_kernel(const float *__restrict__ part, float *__
     for (; tile < n_tiles; ++tile) acc += pb[(size_t)tile * W];
   }
   if (e < 4 * N) {
-    if (d_scale) d_scale[(size_t)h * 4 * N + e] = acc;
+    const int j = e / N, n = e - j * N;
+    void *base = j < 2 ? g.b_scale : g.c_scale;
+    if (base) store_as(base, g.dtype, (size_t)h * g.scale_stride + (size_t)(j & 1) * N + n, acc);
   } else {
-    d_bias[h * 13 + (e - 4 * N)] = acc;
+    const int slot = e - 4 * N;
+    if (g.bias13) g.bias13[h * 13 + slot] = acc;
+    const int k = slot < 3 ? slot : (slot >= 5 && slot < 9 ? slot - 2 : -1);
+    if (k >= 0 && g.bias[k]) store_as(g.bias[k], g.dtype, h, acc);
   }
 }
 
@@ -818,7 +840,7 @@ constexpr int prep_group() { return VEC == 1 ? 32 : 16; }
 
 template <typename T, int VEC>
 static int launch_prep_fwd(const slx_prep_shape *s, const PrepDims &d, const void *value, const void *params,
-                           const void *bc, const float *bias, const float *scale, void *U, float *M, float *K,
+                           const void *bc, const PrepParams &pp, void *U, float *M, float *K,
                            void *B, void *C, cudaStream_t st) {
   PrepHyper hp = make_hyper(s);
   constexpr int G = prep_group<VEC>();
@@ -826,7 +848,7 @@ static int launch_prep_fwd(const slx_prep_shape *s, const PrepDims &d, const voi
   long long blocks = (n_rows + 255) / 256;
   if (blocks > 148LL * 32) blocks = 148LL * 32;
   scanprep_fwd_kernel<T, VEC, G><<<(unsigned)blocks, 256, 0, st>>>(
-      (const T *)value, (const T *)params, (const T *)bc, bias, scale, (T *)U, M, K, (T *)B, (T *)C, d, hp);
+      (const T *)value, (const T *)params, (const T *)bc, pp, (T *)U, M, K, (T *)B, (T *)C, d, hp);
   return check_launch("scanprep_fwd");
 }
 
@@ -849,9 +871,9 @@ static PrepBwdPlan prep_bwd_plan(const slx_prep_shape *s, int VEC) {
 
 template <typename T, int VEC>
 static int launch_prep_bwd(const slx_prep_shape *s, const PrepDims &d, const void *params, const void *bc,
-                           const float *bias, const float *scale, const void *dU, const float *dM, const float *dK,
-                           const void *dB, const void *dC, void *d_value, void *d_params, void *d_bc, float *d_bias,
-                           float *d_scale, float *part, cudaStream_t st) {
+                           const PrepParams &pp, const void *dU, const float *dM, const float *dK,
+                           const void *dB, const void *dC, void *d_value, void *d_params, void *d_bc,
+                           const PrepParamGrads &pg, float *part, cudaStream_t st) {
   PrepHyper hp = make_hyper(s);
   PrepBwdPlan pl = prep_bwd_plan(s, VEC);
   SLX_REQUIRE(pl.kmax <= 4, SLX_E_UNSUPPORTED, "scanprep_bwd: N=%d too large for the lane mapping", d.N);
@@ -863,7 +885,7 @@ static int launch_prep_bwd(const slx_prep_shape *s, const PrepDims &d, const voi
     int rc_smem = ensure_dyn_smem(kern, pl.smem);                                                             \
     if (rc_smem) return rc_smem;                                                                              \
     kern<<<dim3(2 * pl.n_tiles, d.batch * d.H), 256, pl.smem, st>>>(                                          \
-        (const T *)params, (const T *)bc, bias, scale, (const T *)dU, dM, dK, (const T *)dB, (const T *)dC,   \
+        (const T *)params, (const T *)bc, pp, (const T *)dU, dM, dK, (const T *)dB, (const T *)dC,   \
         (T *)d_value, (T *)d_params, (T *)d_bc, part, d, hp, pl.rows_per_tile, pl.n_tiles);                   \
   }
   if (pl.kmax <= 1) SLX_PREP_BWD(1)
@@ -873,8 +895,7 @@ static int launch_prep_bwd(const slx_prep_shape *s, const PrepDims &d, const voi
   int rc = check_launch("scanprep_bwd");
   if (rc) return rc;
   int W = 4 * d.N + 13;
-  scanprep_reduce_kernel<<<dim3((W + 127) / 128, d.H), 128, 0, st>>>(part, d_bias, d_scale, d.batch, d.H, pl.n_tiles,
-                                                                      d.N);
+  scanprep_reduce_kernel<<<dim3((W + 127) / 128, d.H), 128, 0, st>>>(part, pg, d.batch, d.H, pl.n_tiles, d.N);
   return check_launch("scanprep_reduce");
 }
 
@@ -889,27 +910,98 @@ using namespace slx;
     default: { using T_ = __half; __VA_ARGS__; } break;              \
   }
 
+static PrepParams f32_prep_params(const slx_prep_shape *s, const float *bias, const float *scale) {
+  constexpr int kSlot[7] = {0, 1, 2, 5, 6, 7, 8};
+  PrepParams pp{};
+  for (int k = 0; k < 7; ++k) pp.bias[k] = bias ? bias + kSlot[k] : nullptr;
+  pp.b_scale = scale;
+  pp.c_scale = scale ? scale + 2 * s->N : nullptr;
+  pp.dtype = SLX_F32;
+  pp.bias_stride = 13;
+  pp.scale_stride = 4LL * s->N;
+  return pp;
+}
+static int make_prep_params(const slx_prep_shape *s, const slx_prep_params *p, PrepParams *pp) {
+  SLX_REQUIRE(p != nullptr, SLX_E_NULL, "scanprep: params is NULL");
+  SLX_REQUIRE(p->dtype >= SLX_F32 && p->dtype <= SLX_F16, SLX_E_DTYPE, "scanprep: bad parameter dtype %d", p->dtype);
+  for (int k = 0; k < 7; ++k) {
+    SLX_REQUIRE(p->bias[k] != nullptr, SLX_E_NULL, "scanprep: bias %d is NULL", k);
+    pp->bias[k] = p->bias[k];
+  }
+  SLX_REQUIRE(!s->normalize_bc || (p->b_scale && p->c_scale), SLX_E_NULL, "scanprep: scale is NULL with normalize_bc set");
+  pp->b_scale = p->b_scale;
+  pp->c_scale = p->c_scale;
+  pp->dtype = p->dtype;
+  pp->bias_stride = 1;
+  pp->scale_stride = 2LL * s->N;
+  return SLX_OK;
+}
+
+static int prep_fwd_impl(const slx_prep_shape *s, const void *value, const void *params, const void *bc,
+                         const PrepParams &pp, void *U, float *M, float *K, void *B, void *C, void *stream) {
+  PrepDims d;
+  int rc = check_prep(s, &d);
+  if (rc) return rc;
+  SLX_REQUIRE(value && params && bc && U && M && K && B && C, SLX_E_NULL, "scanprep_fwd: NULL tensor");
+  d.wide_params = params_rows_wide(s, params);
+  cudaStream_t st = as_stream(stream);
+  SLX_PREP_T(s->dtype, {
+    int vec = pick_vec<T_>(s, {value, bc, U, B, C});
+    if (!aligned16(pp.b_scale) || !aligned16(pp.c_scale)) vec = 1;  // the scales are read as vectors of their own dtype
+    constexpr int VFULL = 16 / (int)sizeof(T_);
+    if (vec == VFULL) rc = launch_prep_fwd<T_, VFULL>(s, d, value, params, bc, pp, U, M, K, B, C, st);
+    else if (vec == VFULL / 2) rc = launch_prep_fwd<T_, VFULL / 2>(s, d, value, params, bc, pp, U, M, K, B, C, st);
+    else rc = launch_prep_fwd<T_, 1>(s, d, value, params, bc, pp, U, M, K, B, C, st);
+  });
+  return rc;
+}
+
+static int prep_bwd_impl(const slx_prep_shape *s, const void *params, const void *bc, const PrepParams &pp,
+                         const void *dU, const float *dM, const float *dK, const void *dB, const void *dC,
+                         void *d_value, void *d_params, void *d_bc, const PrepParamGrads &pg, void *workspace,
+                         size_t workspace_bytes, void *stream) {
+  PrepDims d;
+  int rc = check_prep(s, &d);
+  if (rc) return rc;
+  SLX_REQUIRE(params && bc && dU && dM && dK && dB && dC && d_value && d_params && d_bc, SLX_E_NULL,
+              "scanprep_bwd: NULL tensor");
+  d.wide_params = params_rows_wide(s, params);
+  size_t need = slx_scanprep_bwd_workspace_bytes(s);
+  SLX_REQUIRE(workspace && workspace_bytes >= need, SLX_E_WORKSPACE, "scanprep_bwd: workspace of %zu bytes needed",
+              need);
+  cudaStream_t st = as_stream(stream);
+  float *part = static_cast<float *>(workspace);
+  SLX_PREP_T(s->dtype, {
+    int vec = pick_vec<T_>(s, {bc, dU, dB, dC, d_value, d_bc});
+    constexpr int VFULL = 16 / (int)sizeof(T_);
+    if (vec == VFULL)
+      rc = launch_prep_bwd<T_, VFULL>(s, d, params, bc, pp, dU, dM, dK, dB, dC, d_value, d_params, d_bc, pg, part, st);
+    else if (vec == VFULL / 2)
+      rc = launch_prep_bwd<T_, VFULL / 2>(s, d, params, bc, pp, dU, dM, dK, dB, dC, d_value, d_params, d_bc, pg, part,
+                                          st);
+    else rc = launch_prep_bwd<T_, 1>(s, d, params, bc, pp, dU, dM, dK, dB, dC, d_value, d_params, d_bc, pg, part, st);
+  });
+  return rc;
+}
+
 extern "C" {
 
 int slx_scanprep_fwd(const slx_prep_shape *s, const void *value, const void *params, const void *bc,
                      const float *bias, const float *scale, void *U, float *M, float *K, void *B, void *C,
                      void *stream) {
-  PrepDims d;
-  int rc = check_prep(s, &d);
-  if (rc) return rc;
-  SLX_REQUIRE(value && params && bc && bias && U && M && K && B && C, SLX_E_NULL, "scanprep_fwd: NULL tensor");
+  SLX_REQUIRE(s != nullptr, SLX_E_NULL, "shape is NULL");
+  SLX_REQUIRE(bias != nullptr, SLX_E_NULL, "scanprep_fwd: NULL tensor");
   SLX_REQUIRE(!s->normalize_bc || scale, SLX_E_NULL, "scanprep_fwd: scale is NULL with normalize_bc set");
-  d.wide_params = params_rows_wide(s, params);
-  cudaStream_t st = as_stream(stream);
-  SLX_PREP_T(s->dtype, {
-    int vec = pick_vec<T_>(s, {value, bc, U, B, C});
-    constexpr int VFULL = 16 / (int)sizeof(T_);
-    if (vec == VFULL) rc = launch_prep_fwd<T_, VFULL>(s, d, value, params, bc, bias, scale, U, M, K, B, C, st);
-    else if (vec == VFULL / 2)
-      rc = launch_prep_fwd<T_, VFULL / 2>(s, d, value, params, bc, bias, scale, U, M, K, B, C, st);
-    else rc = launch_prep_fwd<T_, 1>(s, d, value, params, bc, bias, scale, U, M, K, B, C, st);
-  });
-  return rc;
+  return prep_fwd_impl(s, value, params, bc, f32_prep_params(s, bias, scale), U, M, K, B, C, stream);
+}
+
+int slx_scanprep_fwd_params(const slx_prep_shape *s, const void *value, const void *params, const void *bc,
+                            const slx_prep_params *p, void *U, float *M, float *K, void *B, void *C, void *stream) {
+  SLX_REQUIRE(s != nullptr, SLX_E_NULL, "shape is NULL");
+  PrepParams pp;
+  int rc = make_prep_params(s, p, &pp);
+  if (rc) return rc;
+  return prep_fwd_impl(s, value, params, bc, pp, U, M, K, B, C, stream);
 }
 
 size_t slx_scanprep_bwd_workspace_bytes(const slx_prep_shape *s) {
@@ -923,32 +1015,37 @@ int slx_scanprep_bwd(const slx_prep_shape *s, const void *params, const void *bc
                      const float *scale, const void *dU, const float *dM, const float *dK, const void *dB,
                      const void *dC, void *d_value, void *d_params, void *d_bc, float *d_bias, float *d_scale,
                      void *workspace, size_t workspace_bytes, void *stream) {
-  PrepDims d;
-  int rc = check_prep(s, &d);
-  if (rc) return rc;
-  SLX_REQUIRE(params && bc && bias && dU && dM && dK && dB && dC && d_value && d_params && d_bc && d_bias, SLX_E_NULL,
-              "scanprep_bwd: NULL tensor");
+  SLX_REQUIRE(s != nullptr, SLX_E_NULL, "shape is NULL");
+  SLX_REQUIRE(bias && d_bias, SLX_E_NULL, "scanprep_bwd: NULL tensor");
   SLX_REQUIRE(!s->normalize_bc || (scale && d_scale), SLX_E_NULL, "scanprep_bwd: scale/d_scale NULL");
-  d.wide_params = params_rows_wide(s, params);
-  size_t need = slx_scanprep_bwd_workspace_bytes(s);
-  SLX_REQUIRE(workspace && workspace_bytes >= need, SLX_E_WORKSPACE, "scanprep_bwd: workspace of %zu bytes needed",
-              need);
-  cudaStream_t st = as_stream(stream);
-  float *part = static_cast<float *>(workspace);
-  SLX_PREP_T(s->dtype, {
-    int vec = pick_vec<T_>(s, {bc, dU, dB, dC, d_value, d_bc});
-    constexpr int VFULL = 16 / (int)sizeof(T_);
-    if (vec == VFULL)
-      rc = launch_prep_bwd<T_, VFULL>(s, d, params, bc, bias, scale, dU, dM, dK, dB, dC, d_value, d_params, d_bc,
-                                      d_bias, d_scale, part, st);
-    else if (vec == VFULL / 2)
-      rc = launch_prep_bwd<T_, VFULL / 2>(s, d, params, bc, bias, scale, dU, dM, dK, dB, dC, d_value, d_params, d_bc,
-                                          d_bias, d_scale, part, st);
-    else
-      rc = launch_prep_bwd<T_, 1>(s, d, params, bc, bias, scale, dU, dM, dK, dB, dC, d_value, d_params, d_bc, d_bias,
-                                  d_scale, part, st);
-  });
-  return rc;
+  PrepParamGrads pg{};
+  pg.bias13 = d_bias;
+  pg.b_scale = d_scale;
+  pg.c_scale = d_scale ? d_scale + 2 * s->N : nullptr;
+  pg.dtype = SLX_F32;
+  pg.scale_stride = 4LL * s->N;
+  return prep_bwd_impl(s, params, bc, f32_prep_params(s, bias, scale), dU, dM, dK, dB, dC, d_value, d_params, d_bc, pg,
+                       workspace, workspace_bytes, stream);
+}
+
+int slx_scanprep_bwd_params(const slx_prep_shape *s, const void *params, const void *bc, const slx_prep_params *p,
+                            const void *dU, const float *dM, const float *dK, const void *dB, const void *dC,
+                            void *d_value, void *d_params, void *d_bc, void *d_bias, void *d_b_scale, void *d_c_scale,
+                            void *workspace, size_t workspace_bytes, void *stream) {
+  SLX_REQUIRE(s != nullptr, SLX_E_NULL, "shape is NULL");
+  PrepParams pp;
+  int rc = make_prep_params(s, p, &pp);
+  if (rc) return rc;
+  SLX_REQUIRE(d_bias && (!s->normalize_bc || (d_b_scale && d_c_scale)), SLX_E_NULL, "scanprep_bwd: NULL gradient");
+  PrepParamGrads pg{};
+  const size_t row = (size_t)s->heads * (p->dtype == SLX_F32 ? 4 : 2);
+  for (int k = 0; k < 7; ++k) pg.bias[k] = static_cast<char *>(d_bias) + k * row;
+  pg.b_scale = d_b_scale;
+  pg.c_scale = d_c_scale;
+  pg.dtype = p->dtype;
+  pg.scale_stride = 2LL * s->N;
+  return prep_bwd_impl(s, params, bc, pp, dU, dM, dK, dB, dC, d_value, d_params, d_bc, pg, workspace, workspace_bytes,
+                       stream);
 }
 
 }  // extern "C"

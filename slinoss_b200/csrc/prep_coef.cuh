@@ -12,6 +12,30 @@ struct PrepHyper {
   float dt_min, dt_max, r_min, r_max, theta_bound, k_max, z_thr2;
 };
 
+// The layer's learnable scan-prep parameters as the kernels read them: the seven per-head biases (slots
+// 0,1,2,5,6,7,8 of the 13-wide row; element h at bias[k] + h * bias_stride) and the RMS-norm scales (plane j of
+// head h at b_scale or c_scale + h * scale_stride + (j & 1) * N), all in the parameters' own dtype.
+struct PrepParams {
+  const void *bias[7];
+  const void *b_scale, *c_scale;
+  int dtype, bias_stride;
+  long long scale_stride;
+};
+__device__ __forceinline__ void add_bias13(const PrepParams &pp, int h, float (&p)[13]) {
+  const size_t e = (size_t)h * pp.bias_stride;
+  p[0] += load_as_f(pp.bias[0], pp.dtype, e);
+  p[1] += load_as_f(pp.bias[1], pp.dtype, e);
+  p[2] += load_as_f(pp.bias[2], pp.dtype, e);
+  p[5] += load_as_f(pp.bias[3], pp.dtype, e);
+  p[6] += load_as_f(pp.bias[4], pp.dtype, e);
+  p[7] += load_as_f(pp.bias[5], pp.dtype, e);
+  p[8] += load_as_f(pp.bias[6], pp.dtype, e);
+}
+__device__ __forceinline__ const void *scale_plane(const PrepParams &pp, int j) { return j < 2 ? pp.b_scale : pp.c_scale; }
+__device__ __forceinline__ size_t scale_index(const PrepParams &pp, int h, int j, int N, int n) {
+  return (size_t)h * pp.scale_stride + (size_t)(j & 1) * N + n;
+}
+
 struct CoefOut {
   float2 rho, kp, kc;
 };

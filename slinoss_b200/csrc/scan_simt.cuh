@@ -44,6 +44,12 @@ template <>
 __device__ __forceinline__ float2 load_pair<__half>(const __half *p) {
   return __half22float2(*reinterpret_cast<const __half2 *>(p));
 }
+// The streaming row of batch-head offset `off` when it is held in the activation dtype (the same loads as any other
+// row then), NULL when it is absent or fp32.
+template <typename T>
+__device__ __forceinline__ const T *prev_row(const void *p, int dtype, size_t off) {
+  return (p != nullptr && dtype != SLX_F32) ? static_cast<const T *>(p) + off : nullptr;
+}
 template <typename T>
 __device__ __forceinline__ void store_pair(T *p, float2 v);
 template <>
@@ -118,7 +124,8 @@ struct OuterArgs {
   const T *X;       // (BH,T,D)
   const float *M;   // (BH,T,2)
   const float *K;   // (BH,T,2,2)  (mode 0)
-  const float *Bprev, *Uprev;  // (BH,D), (BH,P) fp32, nullable (mode 0)
+  const void *Bprev, *Uprev;  // (BH,D), (BH,P), nullable (mode 0)
+  int prev_dtype;
   float *out;       // (BH,NC,P,D)
   float *m_chunk;   // (BH,NC,2) (mode 0)
   ScanDims d;
@@ -159,7 +166,7 @@ __global__ void __launch_bounds__(kThreads) chunk_outer_kernel(OuterArgs<T> a) {
     for (int p = tid; p < d.P; p += kThreads) {
       float v = 0.f;
       if (t0 > 0) v = to_f(a.A[(tok0 - 1) * d.P + p]);
-      else if (a.Uprev) v = a.Uprev[(size_t)bh * d.P + p];
+      else if (a.Uprev) v = load_as_f(a.Uprev, a.prev_dtype, (size_t)bh * d.P + p);
       um1[p] = v;
     }
   }
@@ -215,7 +222,7 @@ __global__ void __launch_bounds__(kThreads) chunk_outer_kernel(OuterArgs<T> a) {
         float2 bv = make_float2(0.f, 0.f);
         if (dd < d.D) {
           if (t0 > 0) bv = load_pair<T>(a.X + (tok0 - 1) * d.D + dd);
-          else if (a.Bprev) bv = *reinterpret_cast<const float2 *>(a.Bprev + (size_t)bh * d.D + dd);
+          else if (a.Bprev) bv = load_as_f2(a.Bprev, a.prev_dtype, (size_t)bh * d.D + dd);
         }
         float2 v = cmul(k0p, bv);
         bh1[2 * n] = v.x;
@@ -257,7 +264,9 @@ __global__ void __launch_bounds__(kThreads) chunk_outer_kernel(OuterArgs<T> a) {
 template <typename T>
 struct ScanFwdArgs {
   const T *U, *B, *C;
-  const float *M, *K, *starts, *Bprev, *Uprev;
+  const float *M, *K, *starts;
+  const void *Bprev, *Uprev;
+  int prev_dtype;
   T *Y;
   int *bad;  // unused (the kernels report through g_scan_bad)
   ScanDims d;
@@ -315,7 +324,7 @@ __global__ void __launch_bounds__(kThreads) chunk_scan_fwd_kernel(ScanFwdArgs<T>
     float v = 0.f;
     if (p < d.P) {
       if (t0 > 0) v = to_f(a.U[(tok0 - 1) * d.P + p]);
-      else if (a.Uprev) v = a.Uprev[(size_t)bh * d.P + p];
+      else if (a.Uprev) v = load_as_f(a.Uprev, a.prev_dtype, (size_t)bh * d.P + p);
     }
     um1[p] = v;
   }
@@ -341,7 +350,7 @@ __global__ void __launch_bounds__(kThreads) chunk_scan_fwd_kernel(ScanFwdArgs<T>
       float2 bv = make_float2(0.f, 0.f);
       if (dd < d.D) {
         if (t0 > 0) bv = load_pair<T>(a.B + (tok0 - 1) * d.D + dd);
-        else if (a.Bprev) bv = *reinterpret_cast<const float2 *>(a.Bprev + (size_t)bh * d.D + dd);
+        else if (a.Bprev) bv = load_as_f2(a.Bprev, a.prev_dtype, (size_t)bh * d.D + dd);
       }
       bm1[2 * n] = bv.x;
       bm1[2 * n + 1] = bv.y;
@@ -440,7 +449,9 @@ __global__ void __launch_bounds__(kThreads) chunk_scan_fwd_kernel(ScanFwdArgs<T>
 template <typename T>
 struct ScanBwdArgs {
   const T *U, *B, *C, *dY;
-  const float *M, *K, *starts, *d_inc, *zdot, *Bprev, *Uprev;
+  const float *M, *K, *starts, *d_inc, *zdot;
+  const void *Bprev, *Uprev;
+  int prev_dtype;
   T *dU, *dB, *dC;
   float *dM, *dK, *carryB, *carryU;
   ScanDims d;
@@ -524,7 +535,7 @@ __global__ void __launch_bounds__(kThreads) chunk_scan_bwd_kernel(ScanBwdArgs<T>
     float v = 0.f;
     if (p < d.P) {
       if (t0 > 0) v = to_f(a.U[(tok0 - 1) * d.P + p]);
-      else if (a.Uprev) v = a.Uprev[(size_t)bh * d.P + p];
+      else if (a.Uprev) v = load_as_f(a.Uprev, a.prev_dtype, (size_t)bh * d.P + p);
     }
     um1[p] = v;
     duc[p] = 0.f;
@@ -596,7 +607,7 @@ __global__ void __launch_bounds__(kThreads) chunk_scan_bwd_kernel(ScanBwdArgs<T>
       float2 bv = make_float2(0.f, 0.f);
       if (dd < d.D) {
         if (t0 > 0) bv = load_pair<T>(a.B + (tok0 - 1) * d.D + dd);
-        else if (a.Bprev) bv = *reinterpret_cast<const float2 *>(a.Bprev + (size_t)bh * d.D + dd);
+        else if (a.Bprev) bv = load_as_f2(a.Bprev, a.prev_dtype, (size_t)bh * d.D + dd);
       }
       bm1[2 * n] = bv.x;
       bm1[2 * n + 1] = bv.y;

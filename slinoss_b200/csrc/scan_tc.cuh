@@ -213,13 +213,13 @@ __global__ void __launch_bounds__(kTcThreads, 2) chunk_scan_fwd_tc_kernel(ScanFw
     int p = tid - 64;
     float v = 0.f;
     if (t0 > 0) v = to_f(a.U[(tok0 - 1) * P + p]);
-    else if (a.Uprev) v = a.Uprev[(size_t)bh * P + p];
+    else if (a.Uprev) v = load_as_f(a.Uprev, a.prev_dtype, (size_t)bh * P + p);
     um1[p] = v;
   }
   if (tid < d.N) {
     float2 bv = make_float2(0.f, 0.f);
     if (t0 > 0) bv = load_pair<T>(a.B + (tok0 - 1) * d.D + 2 * tid);
-    else if (a.Bprev) bv = *reinterpret_cast<const float2 *>(a.Bprev + (size_t)bh * d.D + 2 * tid);
+    else if (a.Bprev) bv = load_as_f2(a.Bprev, a.prev_dtype, (size_t)bh * d.D + 2 * tid);
     bm1[tid] = bv;
   }
   umma::fence_before_sync();
@@ -496,8 +496,9 @@ __global__ void __launch_bounds__(kTcThreads, 2) chunk_outer_tc_kernel(OuterArgs
     } else if (tid - L < d.N) {
       const int n = tid - L;
       if (valid > 0) kpn = *reinterpret_cast<const float2 *>(a.K + tok0 * 4);
-      if (t0 > 0) bv = load_pair<T>(a.X + (tok0 - 1) * d.D + 2 * n);
-      else if (a.Bprev) bv = *reinterpret_cast<const float2 *>(a.Bprev + (size_t)bh * d.D + 2 * n);
+      const T *row = t0 > 0 ? a.X + (tok0 - 1) * d.D : prev_row<T>(a.Bprev, a.prev_dtype, (size_t)bh * d.D);
+      if (row) bv = load_pair<T>(row + 2 * n);
+      else if (a.Bprev) bv = *reinterpret_cast<const float2 *>((const float *)a.Bprev + (size_t)bh * d.D + 2 * n);
     }
   }
   if (warp == 2) chunk_prefix_fast128(mreg, lp, ph, mraw, &g_scan_bad);
@@ -514,8 +515,9 @@ __global__ void __launch_bounds__(kTcThreads, 2) chunk_outer_tc_kernel(OuterArgs
   if (MODE == 0 && tid >= 192) {
     int p = tid - 192;
     float v = 0.f;
-    if (t0 > 0) v = to_f(a.A[(tok0 - 1) * P + p]);
-    else if (a.Uprev) v = a.Uprev[(size_t)bh * P + p];
+    const T *row = t0 > 0 ? a.A + (tok0 - 1) * P : prev_row<T>(a.Uprev, a.prev_dtype, (size_t)bh * P);
+    if (row) v = to_f(row[p]);
+    else if (a.Uprev) v = ((const float *)a.Uprev)[(size_t)bh * P + p];
     um1[p] = v;
   }
   umma::fence_before_sync();

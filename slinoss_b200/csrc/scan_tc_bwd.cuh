@@ -154,14 +154,14 @@ __global__ void __launch_bounds__(kTcBwdThreads, 1) chunk_scan_bwd_tc_kernel(Sca
     int p = tid - 256;
     float v = 0.f;
     if (t0 > 0) v = to_f(a.U[(tok0 - 1) * P + p]);
-    else if (a.Uprev) v = a.Uprev[(size_t)bh * P + p];
+    else if (a.Uprev) v = load_as_f(a.Uprev, a.prev_dtype, (size_t)bh * P + p);
     um1[p] = v;
     duc[p] = 0.f;
   } else if (tid >= 320 && tid < 320 + d.N) {
     int n = tid - 320;
     float2 bv = make_float2(0.f, 0.f);
     if (t0 > 0) bv = load_pair<T>(a.B + (tok0 - 1) * d.D + 2 * n);
-    else if (a.Bprev) bv = *reinterpret_cast<const float2 *>(a.Bprev + (size_t)bh * d.D + 2 * n);
+    else if (a.Bprev) bv = load_as_f2(a.Bprev, a.prev_dtype, (size_t)bh * d.D + 2 * n);
     bm1[n] = bv;
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");  // U, dY tiles

@@ -255,14 +255,14 @@ __global__ void __launch_bounds__(kWsThreads, 1) chunk_scan_fwd_ws_kernel(ScanFw
           if (8 * q < d.D) {
             float tmp[8];
 #pragma unroll
-            for (int e = 0; e < 8; ++e) tmp[e] = a.Bprev ? a.Bprev[(size_t)bh * d.D + 8 * q + e] : 0.f;
+            for (int e = 0; e < 8; ++e) tmp[e] = a.Bprev ? load_as_f(a.Bprev, a.prev_dtype, (size_t)bh * d.D + 8 * q + e) : 0.f;
             *reinterpret_cast<uint4 *>(bpst + buf * 256 + 8 * q) = pack8<T>(tmp);
           }
         } else {
           const int q = tid - 288;
           float tmp[8];
 #pragma unroll
-          for (int e = 0; e < 8; ++e) tmp[e] = a.Uprev ? a.Uprev[(size_t)bh * P + 8 * q + e] : 0.f;
+          for (int e = 0; e < 8; ++e) tmp[e] = a.Uprev ? load_as_f(a.Uprev, a.prev_dtype, (size_t)bh * P + 8 * q + e) : 0.f;
           *reinterpret_cast<uint4 *>(upst + buf * 64 + 8 * q) = pack8<T>(tmp);
         }
       }

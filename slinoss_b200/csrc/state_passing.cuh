@@ -113,21 +113,59 @@ __device__ __forceinline__ float2 cdot(Float8 a, Float8 b) { return cadd(cdot(a.
 // (the affine offset of a segment in the context-parallel chain), and the pass writes nothing else.
 // The increments are stored as IT (float, or the activation dtype where the tensor-core chunk
 // kernel wrote them so); the recurrence is fp32 either way.
+// The streaming tensors on either end of the pass come and go in the caller's dtypes (StateEnds), and
+// the last (B, U) row of the sequence, which a stream carries on with the state, is copied on the side:
+// as separate conversion and copy kernels these cost a launch each, several times the pass itself on
+// short sequences.
+struct StateEnds {
+  const void *init;        // [opt] initial state
+  int init_dtype;
+  float *final_state;      // [opt] fp32
+  void *final_copy;        // [opt] the final state once more, as final_dtype
+  int final_dtype;
+  const void *B, *U;       // rows copied when B_last is set: 2-byte units per row, row T-1 of each (b, h)
+  void *B_last, *U_last;
+  int b_units, u_units, T;
+};
+template <typename V>
+__device__ __forceinline__ void load_state(const void *p, int dtype, size_t item, V &v) {
+  constexpr int VEC = sizeof(V) / sizeof(float);
+  if (dtype == SLX_BF16) st_load<__nv_bfloat16>(static_cast<const __nv_bfloat16 *>(p) + item * VEC, v);
+  else if (dtype == SLX_F16) st_load<__half>(static_cast<const __half *>(p) + item * VEC, v);
+  else v = static_cast<const V *>(p)[item];
+}
+template <typename V>
+__device__ __forceinline__ void store_state(void *p, int dtype, size_t item, const V &v) {
+  constexpr int VEC = sizeof(V) / sizeof(float);
+  if (dtype == SLX_BF16) st_store<__nv_bfloat16>(static_cast<__nv_bfloat16 *>(p) + item * VEC, v);
+  else if (dtype == SLX_F16) st_store<__half>(static_cast<__half *>(p) + item * VEC, v);
+  else static_cast<V *>(p)[item] = v;
+}
+
 template <int VEC, typename ST, typename IT>
 __global__ void __launch_bounds__(256) state_passing_fwd_kernel(const IT *inc, const float *__restrict__ m_chunk,
-                                                                const float *__restrict__ init, ST *starts,
-                                                                float *__restrict__ final_state, int NC,
+                                                                StateEnds ends, ST *starts, int NC,
                                                                 int n_vec /* P*D/VEC */) {
   using V = typename VecT<VEC>::type;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int bh = blockIdx.y;
+  if (ends.B_last && blockIdx.x == 0) {
+    const size_t row = (size_t)bh * ends.T + ends.T - 1;
+    const uint16_t *sb = static_cast<const uint16_t *>(ends.B) + row * ends.b_units;
+    const uint16_t *su = static_cast<const uint16_t *>(ends.U) + row * ends.u_units;
+    for (int e = threadIdx.x; e < ends.b_units; e += blockDim.x)
+      static_cast<uint16_t *>(ends.B_last)[(size_t)bh * ends.b_units + e] = sb[e];
+    for (int e = threadIdx.x; e < ends.u_units; e += blockDim.x)
+      static_cast<uint16_t *>(ends.U_last)[(size_t)bh * ends.u_units + e] = su[e];
+  }
   if (i >= n_vec) return;
   const size_t per = (size_t)n_vec;
   const IT *incv = inc + ((size_t)bh * NC * per + i) * VEC;  // + c * per * VEC per chunk
   ST *stv = starts ? starts + ((size_t)bh * NC * per + i) * VEC : nullptr;  // + c * per * VEC per chunk
   const size_t cs = per * VEC;
   const float2 *mc = reinterpret_cast<const float2 *>(m_chunk) + (size_t)bh * NC;
-  V z = init ? reinterpret_cast<const V *>(init)[(size_t)bh * per + i] : vzero(V());
+  V z = vzero(V());
+  if (ends.init) load_state(ends.init, ends.init_dtype, (size_t)bh * per + i, z);
   int c = 0;
   for (; c + 4 <= NC; c += 4) {
     V v0, v1, v2, v3;
@@ -152,7 +190,8 @@ __global__ void __launch_bounds__(256) state_passing_fwd_kernel(const IT *inc, c
     if (stv) st_store<ST>(stv + (size_t)c * cs, z);
     z = axpy_c(m, z, v);
   }
-  reinterpret_cast<V *>(final_state)[(size_t)bh * per + i] = z;
+  if (ends.final_state) reinterpret_cast<V *>(ends.final_state)[(size_t)bh * per + i] = z;
+  if (ends.final_copy) store_state(ends.final_copy, ends.final_dtype, (size_t)bh * per + i, z);
 }
 
 // Reverse pass: g = d_final; for c = NC-1..0:
@@ -166,8 +205,8 @@ template <int VEC, typename ST, typename IT>
 __global__ void __launch_bounds__(256) state_passing_bwd_kernel(const IT *dZ0, const float *__restrict__ m_chunk,
                                                                 const ST *__restrict__ starts,
                                                                 const float *__restrict__ final_state,
-                                                                const float *__restrict__ d_final, ST *d_inc,
-                                                                float *__restrict__ d_initial,
+                                                                const void *d_final, int d_final_dtype, ST *d_inc,
+                                                                void *d_initial, int d_initial_dtype,
                                                                 float *__restrict__ zdot_partials, int NC, int n_vec) {
   using V = typename VecT<VEC>::type;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -180,7 +219,8 @@ __global__ void __launch_bounds__(256) state_passing_bwd_kernel(const IT *dZ0, c
   const size_t ds = per * VEC;
   if (zdot_partials == nullptr) {  // reduce-only / no dot products: a plain reverse recurrence
     const float2 *mc0 = reinterpret_cast<const float2 *>(m_chunk) + (size_t)bh * NC;
-    V g0 = (d_final && live) ? reinterpret_cast<const V *>(d_final)[(size_t)bh * per + iv] : vzero(V());
+    V g0 = vzero(V());
+    if (d_final && live) load_state(d_final, d_final_dtype, (size_t)bh * per + iv, g0);
     int c = NC - 1;
     for (; c >= 3; c -= 4) {  // four loads in flight
       V d0, d1, d2, d3;
@@ -204,7 +244,7 @@ __global__ void __launch_bounds__(256) state_passing_bwd_kernel(const IT *dZ0, c
       if (div && live) st_store<ST>(div + (size_t)c * ds, g0);
       g0 = axpy_c(cconj(mc0[c]), g0, dz);
     }
-    if (d_initial && live) reinterpret_cast<V *>(d_initial)[(size_t)bh * per + iv] = g0;
+    if (d_initial && live) store_state(d_initial, d_initial_dtype, (size_t)bh * per + iv, g0);
     return;
   }
   // With the dot products: every warp writes its own partial of every chunk (no barrier in the
@@ -213,7 +253,8 @@ __global__ void __launch_bounds__(256) state_passing_bwd_kernel(const IT *dZ0, c
   const ST *stv = starts + ((size_t)bh * NC * per + iv) * VEC;
   const size_t cs = per * VEC;
   const float2 *mc = reinterpret_cast<const float2 *>(m_chunk) + (size_t)bh * NC;
-  V g = (d_final && live) ? reinterpret_cast<const V *>(d_final)[(size_t)bh * per + iv] : vzero(V());
+  V g = vzero(V());
+  if (d_final && live) load_state(d_final, d_final_dtype, (size_t)bh * per + iv, g);
   V endst = reinterpret_cast<const V *>(final_state)[(size_t)bh * per + iv];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
   const size_t nparts = (size_t)gridDim.x * nwarp;
@@ -253,7 +294,7 @@ __global__ void __launch_bounds__(256) state_passing_bwd_kernel(const IT *dZ0, c
     st_load<ST>(stv + (size_t)c * cs, st);
     step(c, dz, st, mc[c]);
   }
-  if (d_initial && live) reinterpret_cast<V *>(d_initial)[(size_t)bh * per + iv] = g;
+  if (d_initial && live) store_state(d_initial, d_initial_dtype, (size_t)bh * per + iv, g);
 }
 
 __global__ void zdot_reduce_kernel(const float *__restrict__ partials, float *__restrict__ zdot, int n_rows, int nblk) {
@@ -270,15 +311,16 @@ __global__ void zdot_reduce_kernel(const float *__restrict__ partials, float *__
 // gradient of the streaming inputs (B_prev, U_prev).
 template <typename T>
 __global__ void carry_fixup_kernel(const float *__restrict__ carryB, const float *__restrict__ carryU, T *dB, T *dU,
-                                   float *dB_prev, float *dU_prev, int T_len, int P, int D, int L, int NC) {
+                                   void *dB_prev, void *dU_prev, int d_prev_dtype, int T_len, int P, int D, int L,
+                                   int NC) {
   const int c = blockIdx.x, bh = blockIdx.y;
   const float *cb = carryB + ((size_t)bh * NC + c) * D;
   const float *cu = carryU + ((size_t)bh * NC + c) * P;
   if (c == 0) {
     if (dB_prev)
-      for (int i = threadIdx.x; i < D; i += blockDim.x) dB_prev[(size_t)bh * D + i] = cb[i];
+      for (int i = threadIdx.x; i < D; i += blockDim.x) store_as(dB_prev, d_prev_dtype, (size_t)bh * D + i, cb[i]);
     if (dU_prev)
-      for (int i = threadIdx.x; i < P; i += blockDim.x) dU_prev[(size_t)bh * P + i] = cu[i];
+      for (int i = threadIdx.x; i < P; i += blockDim.x) store_as(dU_prev, d_prev_dtype, (size_t)bh * P + i, cu[i]);
     return;
   }
   const size_t row = (size_t)bh * T_len + (size_t)c * L - 1;

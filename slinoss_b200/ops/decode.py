@@ -10,13 +10,11 @@ state is kept in fp32; passing ``final_state_out=initial_states`` (and likewise
 
 from __future__ import annotations
 
-from ctypes import byref
 from typing import Optional, Tuple
 
 import torch
 
 from .. import _lib
-from .scanprep import _flat_bias
 
 _DTYPES = (torch.float32, torch.bfloat16, torch.float16)
 
@@ -34,7 +32,6 @@ def _like(name: str, t: torch.Tensor, shape, dtype, device) -> torch.Tensor:
 
 
 @torch.compiler.disable
-@torch.no_grad()
 def mixer_decode_step_b200(value, params, bc, gate, skip, *, initial_states=None, B_prev=None,
                            U_prev=None, dt_min: float, dt_max: float, r_min: float, r_max: float,
                            theta_bound: float, k_max: float, eps: float, dt_bias, gamma_bias,
@@ -48,6 +45,29 @@ def mixer_decode_step_b200(value, params, bc, gate, skip, *, initial_states=None
                            ) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor]:
     """``value, gate (b,H,P)``, ``params (b,H,13)``, ``bc (b,H,4,N)``, ``skip (H,P)`` ->
     ``(gated (b, H*P), final_state (b,H,P,2N) fp32, b_last (b,H,2N), u_last (b,H,P))``."""
+    if normalize_bc and (b_scale is None or c_scale is None):
+        if value.device.type != "cuda":
+            raise ValueError("slinoss_b200 decode step requires CUDA tensors.")
+        raise ValueError("b_scale and c_scale are required when normalize_bc is set.")
+    hyper = (dt_min, dt_max, r_min, r_max, theta_bound, k_max, eps)
+    pars = (dt_bias, gamma_bias, omega_bias, mix_r_bias, mix_theta_bias, mix_k_prev_bias, mix_k_curr_bias)
+    if normalize_bc:
+        pars += (b_scale, c_scale)
+    if (output_dtype is None or output_dtype is value.dtype) and value.is_contiguous() and params.is_contiguous() \
+            and bc.is_contiguous() and gate.is_contiguous():
+        out = _lib.host().decode_step(value, params, bc, gate, skip, initial_states, B_prev, U_prev, normalize_bc, hyper,
+                                      pars, final_state_out, b_last_out, u_last_out)
+        if out is not None:
+            return out
+    return _decode_general(value, params, bc, gate, skip, initial_states, B_prev, U_prev, normalize_bc, hyper, pars,
+                           output_dtype, final_state_out, b_last_out, u_last_out)
+
+
+@torch.no_grad()
+def _decode_general(value, params, bc, gate, skip, initial_states, B_prev, U_prev, normalize_bc, hyper, pars,
+                    output_dtype, final_state_out, b_last_out, u_last_out):
+    """Arguments the native path does not take as they are: raises what is wrong with them, or converts the carried
+    tensors and the skip weights to the dtypes the kernel reads."""
     if value.device.type != "cuda":
         raise ValueError("slinoss_b200 decode step requires CUDA tensors.")
     if value.ndim != 3:
@@ -65,41 +85,27 @@ def mixer_decode_step_b200(value, params, bc, gate, skip, *, initial_states=None
     params = _like("params", params, (b, H, 13), dt, dev)
     bc = _like("bc", bc, (b, H, 4, N), dt, dev)
     gate = _like("gate", gate, (b, H, P), dt, dev)
-    skip = skip.detach().reshape(H, P).to(device=dev, dtype=dt).contiguous()
-    if normalize_bc and (b_scale is None or c_scale is None):
-        raise ValueError("b_scale and c_scale are required when normalize_bc is set.")
+    skip = skip.reshape(H, P).to(device=dev, dtype=dt).contiguous()
     if (B_prev is None) != (U_prev is None):
         raise ValueError("B_prev and U_prev must be passed together (or both omitted).")
-    bias = _flat_bias(H, (dt_bias, gamma_bias, omega_bias, mix_r_bias, mix_theta_bias, mix_k_prev_bias,
-                          mix_k_curr_bias), dev)
-    scale = None
-    if normalize_bc:
-        scale = torch.cat((b_scale.detach(), c_scale.detach()), dim=1).to(torch.float32).contiguous()
-    state_in = None
     if initial_states is not None:
-        state_in = _like("initial_states", initial_states, (b, H, P, 2 * N), None, dev)
-        if state_in.dtype != torch.float32:
-            state_in = state_in.to(torch.float32)
+        initial_states = _like("initial_states", initial_states, (b, H, P, 2 * N), None, dev).to(torch.float32)
     if B_prev is not None:
         B_prev = _like("B_prev", B_prev, (b, H, 2 * N), None, dev).to(dt)
         U_prev = _like("U_prev", U_prev, (b, H, P), None, dev).to(dt)
-    state_out = (torch.empty((b, H, P, 2 * N), device=dev, dtype=torch.float32) if final_state_out is None
-                 else _like("final_state_out", final_state_out, (b, H, P, 2 * N), torch.float32, dev))
-    b_last = (torch.empty((b, H, 2 * N), device=dev, dtype=dt) if b_last_out is None
-              else _like("b_last_out", b_last_out, (b, H, 2 * N), dt, dev))
-    u_last = (torch.empty((b, H, P), device=dev, dtype=dt) if u_last_out is None
-              else _like("u_last_out", u_last_out, (b, H, P), dt, dev))
-    out = torch.empty((b, H * P), device=dev, dtype=dt)
-    s = _lib.DecodeShape(b, H, P, N, _lib.dtype_code(dt), 1 if normalize_bc else 0, float(dt_min),
-                         float(dt_max), float(r_min), float(r_max), float(theta_bound), float(k_max),
-                         float(eps))
-    with _lib.guard(dev):
-        _lib.check(_lib.lib().slx_decode_step(
-            byref(s), value.data_ptr(), params.data_ptr(), bc.data_ptr(), gate.data_ptr(), skip.data_ptr(),
-            bias.data_ptr(), _lib.ptr(scale), _lib.ptr(state_in), _lib.ptr(B_prev), _lib.ptr(U_prev),
-            out.data_ptr(), state_out.data_ptr(), b_last.data_ptr(), u_last.data_ptr(),
-            _lib.stream_ptr(dev)), "decode step")
-    return out, state_out, b_last, u_last
+    if final_state_out is not None:
+        _like("final_state_out", final_state_out, (b, H, P, 2 * N), torch.float32, dev)
+    if b_last_out is not None:
+        _like("b_last_out", b_last_out, (b, H, 2 * N), dt, dev)
+    if u_last_out is not None:
+        _like("u_last_out", u_last_out, (b, H, P), dt, dev)
+    pars = tuple(p.to(device=dev, dtype=torch.float32) for p in pars)
+    pars = tuple(p.expand(H) for p in pars[:7]) + pars[7:]
+    out = _lib.host().decode_step(value, params, bc, gate, skip, initial_states, B_prev, U_prev, normalize_bc, hyper,
+                                  pars, final_state_out, b_last_out, u_last_out)
+    if out is None:
+        raise ValueError("decode step: the biases must be (heads,) and the scales (heads, 2, N), and every size positive.")
+    return out
 
 
 __all__ = ["mixer_decode_step_b200"]

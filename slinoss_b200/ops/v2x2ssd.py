@@ -5,7 +5,8 @@ reference's ``slinoss.ops.v2x2ssd.v2x2ssd_cute`` (slinoss/ops/v2x2ssd/cute/
 api.py:52-172); the stage functions mirror ``chunk_increment_cute`` /
 ``state_passing_cute`` / ``chunk_scan_cute`` (cute/kernels/fwd/__init__.py:740,
 897,1125).  All arithmetic happens in the sm_100a kernels behind the C ABI;
-this file validates, allocates outputs with torch and wires autograd.
+the native host path (csrc/host) checks the common case, allocates and wires autograd;
+this file holds the stages, the checks with the reference's messages and the conversions.
 """
 
 from __future__ import annotations
@@ -250,25 +251,8 @@ def _as_starts(chunk_starts: torch.Tensor, s: "_lib.ScanShape") -> torch.Tensor:
 
 
 def _fwd_impl(U, M, K, B, C, init32, bp32, up32, L):
-    """Three stages back to back.  Returns (Y, final32, chunk_starts, m_chunk)."""
-    b, h, T, P = map(int, U.shape)
-    D = int(B.shape[-1])
-    NC = (T + L - 1) // L
-    s = _shape(b, h, T, P, D // 2, L, U.dtype)
-    dev = U.device
-    Y = torch.empty_like(U)
-    final = torch.empty((b, h, P, D), device=dev, dtype=torch.float32)
-    starts = torch.empty((b, h, NC, P, D), device=dev, dtype=_lib.starts_dtype(s))
-    mch = torch.empty((b, h, NC, 2), device=dev, dtype=torch.float32)
-    # separate increment buffer (stored like the chunk starts): the two-buffer state pass is ~2.5x
-    # faster than the in-place one
-    inc = torch.empty((b, h, NC, P, D), device=dev, dtype=starts.dtype)
-    with _lib.guard(dev):
-        _lib.check(_lib.lib().slx_v2x2ssd_fwd(
-            byref(s), U.data_ptr(), M.data_ptr(), K.data_ptr(), B.data_ptr(), C.data_ptr(),
-            _lib.ptr(init32), _lib.ptr(bp32), _lib.ptr(up32), Y.data_ptr(), final.data_ptr(),
-            starts.data_ptr(), mch.data_ptr(), inc.data_ptr(), _lib.stream_ptr(dev)), "v2x2ssd forward")
-    return Y, final, starts, mch
+    """Three stages back to back, no autograd.  Returns (Y, final32, chunk_starts, m_chunk)."""
+    return _lib.host().scan_fwd_parts(U, M, K, B, C, init32, bp32, up32, L)
 
 
 def _bwd_begin(M, C, mch, dY, L, P):
@@ -292,100 +276,9 @@ def _bwd_begin(M, C, mch, dY, L, P):
 def _bwd_impl(U, M, K, B, C, bp32, up32, starts, mch, final32, dY, d_final32, L, *,
               want_initial: bool, want_prev: bool, workspace=None):
     b, h, T, P = map(int, U.shape)
-    D = int(B.shape[-1])
-    s = _shape(b, h, T, P, D // 2, L, U.dtype)
-    dev = U.device
-    dU, dB, dC = torch.empty_like(U), torch.empty_like(B), torch.empty_like(C)
-    dM = torch.empty((b, h, T, 2), device=dev, dtype=torch.float32)
-    dK = torch.empty((b, h, T, 2, 2), device=dev, dtype=torch.float32)
-    d_init = torch.empty((b, h, P, D), device=dev, dtype=torch.float32) if want_initial else None
-    dBp = torch.empty((b, h, D), device=dev, dtype=torch.float32) if want_prev else None
-    dUp = torch.empty((b, h, P), device=dev, dtype=torch.float32) if want_prev else None
-    L_ = _lib.lib()
-    nbytes = int(L_.slx_v2x2ssd_bwd_workspace_bytes(byref(s)))
-    starts = _as_starts(starts, s)
-    ws = torch.empty((nbytes,), device=dev, dtype=torch.uint8) if workspace is None else workspace
-    entry = L_.slx_v2x2ssd_bwd if workspace is None else L_.slx_v2x2ssd_bwd_finish  # dZ0 already there
-    with _lib.guard(dev):
-        _lib.check(entry(
-            byref(s), U.data_ptr(), M.data_ptr(), K.data_ptr(), B.data_ptr(), C.data_ptr(),
-            _lib.ptr(bp32), _lib.ptr(up32), starts.data_ptr(), mch.data_ptr(), final32.data_ptr(),
-            dY.data_ptr(), _lib.ptr(d_final32), dU.data_ptr(), dM.data_ptr(), dK.data_ptr(),
-            dB.data_ptr(), dC.data_ptr(), _lib.ptr(d_init), _lib.ptr(dBp), _lib.ptr(dUp),
-            ws.data_ptr(), nbytes, _lib.stream_ptr(dev)), "v2x2ssd backward")
-    return dU, dM, dK, dB, dC, d_init, dBp, dUp
-
-
-class _V2x2SSDFn(torch.autograd.Function):
-    """Autograd node; same inputs/outputs as the reference's
-    ``_V2x2SSDCuTeTrainingFn`` (cute/autograd.py:40-266)."""
-
-    @staticmethod
-    def forward(ctx, U, M, K, B, C, initial_states, B_prev, U_prev, L, odtype, return_state, residual="keep"):
-        init32, bp32, up32 = _f32(initial_states), _f32(B_prev), _f32(U_prev)
-        Y, final32, starts, mch = _fwd_impl(U.detach(), M.detach(), K.detach(), B.detach(),
-                                            C.detach(), init32, bp32, up32, L)
-        ctx.L = L
-        ctx.return_state = return_state
-        ctx.has_init = initial_states is not None
-        ctx.has_prev = B_prev is not None
-        ctx.init_dtype = None if initial_states is None else initial_states.dtype
-        ctx.prev_dtype = None if B_prev is None else B_prev.dtype
-        # What is kept of the chunk-start states (the largest residual, (b,h,NC,P,2N)): "keep" as the
-        # kernels exchange them (activation dtype on the tensor-core path, fp32 otherwise);
-        # "recompute" nothing: the backward rebuilds them from the inputs with one more
-        # chunk-increment and state pass.
-        ctx.residual = residual
-        if residual == "recompute":
-            starts = init32 if init32 is not None else final32.new_empty(0)
-        saved = [U, M, K, B, C, mch, starts, final32]
-        if ctx.has_prev:
-            saved += [bp32, up32]
-        ctx.save_for_backward(*[t.detach() for t in saved])
-        Y = Y.to(odtype)
-        if not return_state:
-            return Y
-        B_last = B.detach()[:, :, -1, :].to(odtype).contiguous()
-        U_last = U.detach()[:, :, -1, :].to(odtype).contiguous()
-        return Y, final32.to(odtype), B_last, U_last
-
-    @staticmethod
-    def backward(ctx, *grads):
-        saved = ctx.saved_tensors
-        U, M, K, B, C, mch, starts, final32 = saved[:8]
-        bp32, up32 = (saved[8], saved[9]) if ctx.has_prev else (None, None)
-        if ctx.return_state:
-            dY, d_final, dB_last, dU_last = grads
-        else:
-            (dY,) = grads
-            d_final = dB_last = dU_last = None
-        dU = dM = dK = dB = dC = d_init = dBp = dUp = None
-        if dY is not None or d_final is not None:
-            dYc = (torch.zeros_like(U) if dY is None else _aligned(dY.to(U.dtype).contiguous()))
-            dfin = None if d_final is None else d_final.to(torch.float32).contiguous()
-            if ctx.residual == "recompute":
-                init32 = starts if starts.numel() else None
-                b_, h_, T_, P_ = map(int, U.shape)
-                sdt = _lib.starts_dtype(_shape(b_, h_, T_, P_, int(B.shape[-1]) // 2, ctx.L, U.dtype))
-                inc, _ = chunk_increment_b200(U, M, K, B, B_prev=bp32, U_prev=up32, chunk_size=ctx.L, inc_dtype=sdt)
-                starts, _ = state_passing_b200(inc, mch, initial_states=init32, starts_dtype=sdt)
-                del inc
-            dU, dM, dK, dB, dC, d_init, dBp, dUp = _bwd_impl(
-                U, M, K, B, C, bp32, up32, starts, mch, final32, dYc, dfin, ctx.L,
-                want_initial=ctx.has_init, want_prev=ctx.has_prev)
-        if dB_last is not None:
-            if dB is None:
-                dB = torch.zeros_like(B)
-            dB[:, :, -1, :].add_(dB_last.to(B.dtype))
-        if dU_last is not None:
-            if dU is None:
-                dU = torch.zeros_like(U)
-            dU[:, :, -1, :].add_(dU_last.to(U.dtype))
-        if d_init is not None:
-            d_init = d_init.to(ctx.init_dtype)
-        if dBp is not None:
-            dBp, dUp = dBp.to(ctx.prev_dtype), dUp.to(ctx.prev_dtype)
-        return dU, dM, dK, dB, dC, d_init, dBp, dUp, None, None, None, None
+    starts = _as_starts(starts, _shape(b, h, T, P, int(B.shape[-1]) // 2, L, U.dtype))
+    return _lib.host().scan_bwd_parts(U, M, K, B, C, bp32, up32, starts, mch, final32, dY, d_final32, L, want_initial,
+                                      want_prev, workspace)
 
 
 @torch.compiler.disable
@@ -418,6 +311,20 @@ def v2x2ssd_b200(U, M, K, B, C, *, chunk_size: int, initial_states=None, B_prev=
     """
     if residual not in ("keep", "recompute"):
         raise ValueError(f"residual must be 'keep' or 'recompute'. Got {residual!r}.")
+    if not strict and (compute_dtype is None or compute_dtype is torch.float32) and (
+            output_dtype is None or output_dtype is U.dtype):
+        out = _lib.host().v2x2ssd(U, M, K, B, C, int(chunk_size), initial_states, B_prev, U_prev, return_state, retile,
+                                  residual == "recompute", None)
+        if out is not None:
+            return out
+    return _v2x2ssd_general(U, M, K, B, C, chunk_size, initial_states, B_prev, U_prev, compute_dtype, output_dtype,
+                            return_state, retile, strict, residual)
+
+
+def _v2x2ssd_general(U, M, K, B, C, chunk_size, initial_states, B_prev, U_prev, compute_dtype, output_dtype,
+                     return_state, retile, strict, residual):
+    """Arguments the native path does not take as they are: raises what is wrong with them, or brings them to one
+    activation dtype, fp32 parameters and 16-byte alignment and converts the results."""
     b, h, T, N, P = _validate_inputs(U, M, K, B, C, initial_states, B_prev, U_prev)
     if U.device.type != "cuda":
         raise ValueError("slinoss_b200 v2x2ssd requires CUDA tensors.")
@@ -438,37 +345,31 @@ def v2x2ssd_b200(U, M, K, B, C, *, chunk_size: int, initial_states=None, B_prev=
         raise TypeError(f"U/B/C must be float32, bfloat16 or float16. Got {act}.")
     if odtype == torch.float32 and act != torch.float32:
         act = torch.float32  # a wider output must not be rounded through the half store
-    Ua, Ba, Ca = (t if t.dtype == act else t.to(act) for t in (U, B, C))
-    Mf = M if M.dtype == torch.float32 else M.to(torch.float32)
-    Kf = K if K.dtype == torch.float32 else K.to(torch.float32)
-    Ua, Ba, Ca, Mf, Kf = (_aligned(t) for t in (Ua, Ba, Ca, Mf, Kf))
-    if retile and act in (torch.bfloat16, torch.float16) and P == 64 and D % 64 == 0 and D <= 256:
-        chunk_size = 128
-    needs_grad = torch.is_grad_enabled() and any(
-        t is not None and t.requires_grad for t in (U, M, K, B, C, initial_states, B_prev, U_prev))
+    Ua, Ba, Ca = (_aligned(t if t.dtype == act else t.to(act)) for t in (U, B, C))
+    Mf, Kf = (_aligned(t if t.dtype == torch.float32 else t.to(torch.float32)) for t in (M, K))
+    init, Bp, Up = initial_states, B_prev, U_prev
+    if init is not None:
+        init = _aligned(init if init.dtype in _ACT_DTYPES else init.to(torch.float32))
+    if Bp is not None and (Bp.dtype != Up.dtype or Bp.dtype not in (act, torch.float32)):
+        Bp, Up = Bp.to(torch.float32), Up.to(torch.float32)
+    if not (retile and act != torch.float32 and P == 64 and D % 64 == 0 and D <= 256):
+        _shape(b, h, T, P, N, int(chunk_size), act)  # chunk_size is one the kernels tile in
     if strict:
         _lib.read_scan_status(U.device)  # clear what earlier calls on this device may have left
         _lib.read_tc_status(U.device)
-
-    def _checked(out):
-        if strict:
-            if _lib.read_scan_status(U.device):
-                raise ValueError("M has an entry of magnitude exactly 0: the chunked scan needs abs(M) > 0.")
-            if _lib.read_tc_status(U.device):
-                raise RuntimeError("v2x2ssd: a bounded wait inside a tensor-core kernel ran out; the outputs "
-                                   "of the affected chunks are NaN.")
-        return out
-
-    if needs_grad:
-        return _checked(_V2x2SSDFn.apply(Ua, Mf, Kf, Ba, Ca, initial_states, B_prev, U_prev, int(chunk_size),
-                                         odtype, bool(return_state), residual))
-    Y, final32, _, _ = _fwd_impl(Ua, Mf, Kf, Ba, Ca, _f32(initial_states), _f32(B_prev),
-                                 _f32(U_prev), int(chunk_size))
-    Y = Y.to(odtype)
-    if not return_state:
-        return _checked(Y)
-    return _checked((Y, final32.to(odtype), B[:, :, -1, :].to(odtype).contiguous(),
-                     U[:, :, -1, :].to(odtype).contiguous()))
+    out = _lib.host().v2x2ssd(Ua, Mf, Kf, Ba, Ca, int(chunk_size), init, Bp, Up, return_state, retile,
+                              residual == "recompute", odtype if odtype in _ACT_DTYPES else torch.float32)
+    if out is None:
+        raise ValueError("slinoss_b200 v2x2ssd: sizes must be positive. "
+                         f"Got batch={b}, heads={h}, T={T}, P={P}, 2N={D}.")
+    out = tuple(t.to(odtype) for t in out) if return_state else out.to(odtype)
+    if strict:
+        if _lib.read_scan_status(U.device):
+            raise ValueError("M has an entry of magnitude exactly 0: the chunked scan needs abs(M) > 0.")
+        if _lib.read_tc_status(U.device):
+            raise RuntimeError("v2x2ssd: a bounded wait inside a tensor-core kernel ran out; the outputs "
+                               "of the affected chunks are NaN.")
+    return out
 
 
 __all__ = ["v2x2ssd_b200", "chunk_increment_b200", "state_passing_b200", "chunk_scan_b200"]
