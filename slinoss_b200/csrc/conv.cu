@@ -15,6 +15,7 @@
 // arithmetic on channel pairs (fma.rn.f32x2) and sizes its tiles so that the grid is a
 // whole number of waves.  The plain kernels (*_kernel, one channel per thread) serve
 // unaligned inputs.
+#include <algorithm>
 #include <initializer_list>
 #include <type_traits>
 #include <mutex>
@@ -85,7 +86,41 @@ __device__ __forceinline__ void ld_raw(const T *p, RowSlice<T, VEC> &r) {
 struct ConvDims {
   int batch, T, C, W, silu;
   long long xs, xbs;  // row stride / batch stride of x (elements)
+  int tile, n_tiles;  // tokens one thread walks, and how many such tiles cover T
 };
+
+// A thread's share: VEC channels of one tile of one batch row.  The shares are numbered channels first, then
+// tiles, then batch rows, and dealt to the threads of a flat grid: narrow layers fill their blocks (64 slices of a
+// 512-channel layer used half of every 128-thread block), and a block of a short sequence spans several tiles.
+template <int VEC>
+__device__ __forceinline__ bool conv_share(const ConvDims &d, int &b, int &tile_i, int &c0) {
+  const unsigned n_vec = (unsigned)(d.C + VEC - 1) / VEC;
+  const unsigned idx = blockIdx.x * kConvThreads + threadIdx.x;
+  const unsigned r = idx / n_vec;
+  c0 = (int)(idx - r * n_vec) * VEC;
+  b = (int)(r / (unsigned)d.n_tiles);
+  tile_i = (int)(r - (unsigned)b * d.n_tiles);
+  return b < d.batch;
+}
+
+// silu(x) and its derivative.  For half types the sigmoid comes from the fast exponential and reciprocal (relative
+// error about 1e-6, three digits below the rounding of the result); with the full-precision division the walk was
+// bound by its instruction count (forward 0.104 ms, backward 0.165 ms at b16 T4096 C1024).
+template <typename T>
+__device__ __forceinline__ float sigmoid_t(float x) {
+  if constexpr (sizeof(T) == 2) return __fdividef(1.f, 1.f + __expf(-x));
+  else return 1.f / (1.f + expf(-x));
+}
+template <typename T>
+__device__ __forceinline__ float silu_t(float x) {
+  if constexpr (sizeof(T) == 2) return __fdividef(x, 1.f + __expf(-x));
+  else return x / (1.f + expf(-x));
+}
+template <typename T>
+__device__ __forceinline__ float dsilu_t(float x) {
+  const float s = sigmoid_t<T>(x);
+  return s * (1.f + x * (1.f - s));
+}
 
 // x at token index tau (may be negative: reads the carried state, else zero)
 template <typename T, int VEC>
@@ -121,11 +156,10 @@ __global__ void __launch_bounds__(kConvThreads) cconv1d_fwd_kernel(const T *__re
                                                                    const T *__restrict__ weight,
                                                                    const T *__restrict__ bias,
                                                                    const T *__restrict__ state, T *__restrict__ y,
-                                                                   T *__restrict__ next_state, ConvDims d, int tile) {
-  const int c0 = (blockIdx.x * kConvThreads + threadIdx.x) * VEC;
-  if (c0 >= d.C) return;
-  const int b = blockIdx.z;
-  const int t_lo = blockIdx.y * tile, t_hi = min(d.T, t_lo + tile);
+                                                                   T *__restrict__ next_state, ConvDims d) {
+  int b, tile_i, c0;
+  if (!conv_share<VEC>(d, b, tile_i, c0)) return;
+  const int t_lo = tile_i * d.tile, t_hi = min(d.T, t_lo + d.tile);
   float w4[4][VEC], bv[VEC];
   load_taps<T, VEC>(weight, bias, d, c0, w4, bv);
   float x0[VEC], x1[VEC], x2[VEC], x3[VEC];
@@ -152,7 +186,7 @@ __global__ void __launch_bounds__(kConvThreads) cconv1d_fwd_kernel(const T *__re
         acc = fmaf(w4[1][e], x1[e], acc);
         acc = fmaf(w4[2][e], x2[e], acc);
         acc = fmaf(w4[3][e], x3[e], acc);
-        if (d.silu) acc = acc / (1.f + expf(-acc));
+        if (d.silu) acc = silu_t<T>(acc);
         o[e] = acc;
         x0[e] = x1[e];
         x1[e] = x2[e];
@@ -192,8 +226,7 @@ __device__ __forceinline__ void load_dyact(const T *dy, const ConvDims &d, int b
       pre = fmaf(w4[1][e], xb[e], pre);
       pre = fmaf(w4[2][e], xc[e], pre);
       pre = fmaf(w4[3][e], xd[e], pre);
-      float s = 1.f / (1.f + expf(-pre));
-      g[e] *= s * (1.f + pre * (1.f - s));
+      g[e] *= dsilu_t<T>(pre);
     }
   }
 }
@@ -218,8 +251,7 @@ __device__ __forceinline__ void apply_dyact(const ConvDims &d, int t, const floa
       pre = fmaf(w4[1][e], xb[e], pre);
       pre = fmaf(w4[2][e], xc[e], pre);
       pre = fmaf(w4[3][e], xd[e], pre);
-      float s = 1.f / (1.f + expf(-pre));
-      g[e] *= s * (1.f + pre * (1.f - s));
+      g[e] *= dsilu_t<T>(pre);
     }
   }
 }
@@ -271,9 +303,9 @@ __global__ void __launch_bounds__(kConvThreads) cconv1d_bwd_dstate_kernel(
 
 // Writes this tile's partial sums part[(b*n_tiles + tile)][C][5] = (dw4[0..3], dbias)
 template <int VEC>
-__device__ __forceinline__ void conv_bwd_partials(float *part, int C, int b, int c0, const float (&dw)[4][VEC],
+__device__ __forceinline__ void conv_bwd_partials(float *part, int C, int row, int c0, const float (&dw)[4][VEC],
                                                   const float (&db)[VEC]) {
-  float *pp = part + (((long long)b * gridDim.y + blockIdx.y) * C + c0) * 5;
+  float *pp = part + ((long long)row * C + c0) * 5;
 #pragma unroll
   for (int e = 0; e < VEC; ++e) {
 #pragma unroll
@@ -286,12 +318,10 @@ __device__ __forceinline__ void conv_bwd_partials(float *part, int C, int b, int
 template <typename T, int VEC>
 __global__ void __launch_bounds__(kConvThreads) cconv1d_bwd_kernel(
     const T *__restrict__ x, const T *__restrict__ weight, const T *__restrict__ bias, const T *__restrict__ state,
-    const T *__restrict__ dy, const T *__restrict__ d_next, T *__restrict__ dx, float *__restrict__ part, ConvDims d,
-    int tile) {
-  const int c0 = (blockIdx.x * kConvThreads + threadIdx.x) * VEC;
-  if (c0 >= d.C) return;
-  const int b = blockIdx.z;
-  const int t_lo = blockIdx.y * tile, t_hi = min(d.T, t_lo + tile);
+    const T *__restrict__ dy, const T *__restrict__ d_next, T *__restrict__ dx, float *__restrict__ part, ConvDims d) {
+  int b, tile_i, c0;
+  if (!conv_share<VEC>(d, b, tile_i, c0)) return;
+  const int t_lo = tile_i * d.tile, t_hi = min(d.T, t_lo + d.tile);
   float w4[4][VEC], bv[VEC];
   load_taps<T, VEC>(weight, bias, d, c0, w4, bv);
   float x0[VEC], x1[VEC], x2[VEC], x3[VEC];
@@ -366,7 +396,7 @@ __global__ void __launch_bounds__(kConvThreads) cconv1d_bwd_kernel(
     }
     }
   }
-  conv_bwd_partials<VEC>(part, d.C, b, c0, dw, db);
+  conv_bwd_partials<VEC>(part, d.C, b * d.n_tiles + tile_i, c0, dw, db);
 }
 
 // ---- staged variants: rows travel global -> shared by cp.async, several groups ahead of the walk ----
@@ -406,19 +436,17 @@ constexpr size_t conv_ring_bytes(int tensors) {
   return (size_t)RING * conv_group_rows<T, VEC>() * tensors * kConvThreads * sizeof(RowSlice<T, VEC>);
 }
 
-template <typename T, int VEC, int RING>
+template <typename T, int VEC, int RING, bool SILU>
 __global__ void __launch_bounds__(kConvThreads) cconv1d_bwd_staged_kernel(
     const T *__restrict__ x, const T *__restrict__ weight, const T *__restrict__ bias, const T *__restrict__ state,
-    const T *__restrict__ dy, const T *__restrict__ d_next, T *__restrict__ dx, float *__restrict__ part, ConvDims d,
-    int tile) {
+    const T *__restrict__ dy, const T *__restrict__ d_next, T *__restrict__ dx, float *__restrict__ part, ConvDims d) {
   using Slice = RowSlice<T, VEC>;
   constexpr int G = conv_group_rows<T, VEC>();
   extern __shared__ __align__(16) unsigned char conv_ring[];
-  const int c0 = (blockIdx.x * kConvThreads + threadIdx.x) * VEC;
-  if (c0 >= d.C) return;
+  int b, tile_i, c0;
+  if (!conv_share<VEC>(d, b, tile_i, c0)) return;
   Slice *ring = reinterpret_cast<Slice *>(conv_ring) + threadIdx.x;  // [RING*G rows][x, dy][thread]
-  const int b = blockIdx.z;
-  const int t_lo = blockIdx.y * tile, t_hi = min(d.T, t_lo + tile);
+  const int t_lo = tile_i * d.tile, t_hi = min(d.T, t_lo + d.tile);
   const int t_end = min(d.T + 3, t_hi + 3);
   const int n_grp = (t_end - t_lo + G - 1) / G;
   const T *xb = x + (long long)b * d.xbs + c0;
@@ -497,16 +525,15 @@ __global__ void __launch_bounds__(kConvThreads) cconv1d_bwd_staged_kernel(
     // rows past the sequence arrive as zeros, so g3 = 0 there without a test
 #pragma unroll
     for (int h = 0; h < H; ++h) g3[h] = make_float2(to_f(gr.v[2 * h]), to_f(gr.v[2 * h + 1]));
-    if (d.silu) {
+    if (SILU) {
 #pragma unroll
       for (int h = 0; h < H; ++h) {
         float2 pre = __ffma2_rn(w4[0][h], x0[h], bv[h]);
         pre = __ffma2_rn(w4[1][h], x1[h], pre);
         pre = __ffma2_rn(w4[2][h], x2[h], pre);
         pre = __ffma2_rn(w4[3][h], x3[h], pre);
-        const float sx = 1.f / (1.f + expf(-pre.x)), sy = 1.f / (1.f + expf(-pre.y));
-        g3[h].x *= sx * (1.f + pre.x * (1.f - sx));
-        g3[h].y *= sy * (1.f + pre.y * (1.f - sy));
+        g3[h].x *= dsilu_t<T>(pre.x);
+        g3[h].y *= dsilu_t<T>(pre.y);
       }
     }
     if (INNER || t < t_hi) {
@@ -580,24 +607,23 @@ __global__ void __launch_bounds__(kConvThreads) cconv1d_bwd_staged_kernel(
   }
   cp_async_wait<0>();
 #undef SLX_CONV_ISSUE
-  conv_bwd_partials<VEC>(part, d.C, b, c0, dwf, dbf);
+  conv_bwd_partials<VEC>(part, d.C, b * d.n_tiles + tile_i, c0, dwf, dbf);
 }
 
-template <typename T, int VEC, int RING>
+template <typename T, int VEC, int RING, bool SILU>
 __global__ void __launch_bounds__(kConvThreads) cconv1d_fwd_staged_kernel(const T *__restrict__ x,
                                                                           const T *__restrict__ weight,
                                                                           const T *__restrict__ bias,
                                                                           const T *__restrict__ state,
                                                                           T *__restrict__ y, T *__restrict__ next_state,
-                                                                          ConvDims d, int tile) {
+                                                                          ConvDims d) {
   using Slice = RowSlice<T, VEC>;
   constexpr int G = conv_group_rows<T, VEC>();
   extern __shared__ __align__(16) unsigned char conv_ring[];
-  const int c0 = (blockIdx.x * kConvThreads + threadIdx.x) * VEC;
-  if (c0 >= d.C) return;
+  int b, tile_i, c0;
+  if (!conv_share<VEC>(d, b, tile_i, c0)) return;
   Slice *ring = reinterpret_cast<Slice *>(conv_ring) + threadIdx.x;  // [RING*G rows][thread]
-  const int b = blockIdx.z;
-  const int t_lo = blockIdx.y * tile, t_hi = min(d.T, t_lo + tile);
+  const int t_lo = tile_i * d.tile, t_hi = min(d.T, t_lo + d.tile);
   const int n_grp = (t_hi - t_lo + G - 1) / G;
   const T *xb = x + (long long)b * d.xbs + c0;
 #define SLX_CONV_ISSUE(grp_)                                                                                  \
@@ -640,7 +666,7 @@ __global__ void __launch_bounds__(kConvThreads) cconv1d_fwd_staged_kernel(const 
       acc = fmaf(w4[1][e], x1[e], acc);
       acc = fmaf(w4[2][e], x2[e], acc);
       acc = fmaf(w4[3][e], x3[e], acc);
-      if (d.silu) acc = acc / (1.f + expf(-acc));
+      if (SILU) acc = silu_t<T>(acc);
       o[e] = acc;
       x0[e] = x1[e];
       x1[e] = x2[e];
@@ -758,12 +784,26 @@ static int check_conv(const slx_conv_shape *s, ConvDims *d) {
   return SLX_OK;
 }
 
-// Smallest tile of the token axis: the backward workspace is sized for it (one set of partial sums per tile).
+// Tile of the token axis.  A thread's walk is serial, so while the problem does not fill the GPU its time is the
+// length of the walk: the tile starts at 8 tokens (16 backward) and doubles until the shares of the call fit the
+// threads the GPU keeps resident with these kernels' copy rings, up to 64 (128 backward), where the three rows of
+// halo per tile and the backward's partial sums stop mattering.  (b2 T1000 C512: 63-token walks left 32 blocks for
+// 148 SMs, 0.038 ms.)
 constexpr int kConvTileFwd = 64, kConvTileBwd = 128;
+constexpr long long kConvResident = 148LL * 4 * kConvThreads;  // threads in flight with four rings to an SM
+constexpr size_t kNoAllocFloats = 1u << 20;  // partial sums that slx_cconv1d_bwd_noalloc can hold
 
-static int conv_tile(int T, bool bwd) {
-  int tile = bwd ? kConvTileBwd : kConvTileFwd;
-  return tile < T ? tile : T;
+static int conv_tile(const ConvDims &d, int vec, bool bwd) {
+  const long long n_vec = (d.C + vec - 1) / vec;
+  const int most = bwd ? kConvTileBwd : kConvTileFwd;
+  int tile = bwd ? 16 : 8;
+  auto tiles = [&](int t) { return (long long)d.batch * ((d.T + t - 1) / t); };
+  while (tile < most && n_vec * tiles(tile) > kConvResident) tile *= 2;
+  // the partial sums of a problem that fits the built-in buffer at the largest tile fit it at the chosen one
+  if (bwd)
+    while (tile < most && (size_t)tiles(tile) * d.C * 5 > kNoAllocFloats && (size_t)tiles(most) * d.C * 5 <= kNoAllocFloats)
+      tile *= 2;
+  return tile < d.T ? tile : d.T;
 }
 
 // CTAs of `kernel` (kConvThreads threads, `smem` dynamic bytes) that the current device holds at once
@@ -772,22 +812,30 @@ static long conv_slots(K kernel, size_t smem) {
   return resident_ctas(kernel, kConvThreads, smem);
 }
 
-// Tile of the token axis for a grid of base_ctas x ceil(T / tile) CTAs.  With the smallest tile the grid
-// may come to a few waves plus a thin last one; then the tile is grown (up to 512 tokens) to the size at
-// which the grid is k full waves, for the smallest such k.
-static int conv_tile_balanced(int T, int min_tile, long base_ctas, long slots) {
-  if (T <= min_tile) return T;
-  const long n_min = (T + min_tile - 1) / min_tile;
-  if (slots <= 0 || base_ctas * n_min <= slots) return min_tile;
-  for (long k = 1; k <= 16; ++k) {
-    const long nt = k * slots / base_ctas;
+// With the largest regular tile the grid may come to a few waves plus a thin last one; then the tile is grown (up
+// to 512 tokens) to the size at which the grid is k full waves, for the smallest such k.
+static int conv_tile_balanced(const ConvDims &d, int vec, long slots) {
+  const int tile0 = conv_tile(d, vec, true);
+  if (tile0 < kConvTileBwd || slots <= 0) return tile0;
+  const double per_tile = (double)((d.C + vec - 1) / vec) * d.batch / kConvThreads;  // CTAs per tile of the token axis
+  if (per_tile * ((d.T + tile0 - 1) / tile0) <= slots) return tile0;
+  for (int k = 1; k <= 16; ++k) {
+    const int nt = (int)(k * slots / per_tile);
     if (nt < 1) continue;
-    long tile = (T + nt - 1) / nt;
+    int tile = (d.T + nt - 1) / nt;
     tile = (tile + 7) / 8 * 8;
-    if (tile < min_tile) return min_tile;
-    if (tile <= 512) return (int)tile;
+    if (tile < tile0) return tile0;
+    if (tile <= 512) return tile;
   }
-  return min_tile;
+  return tile0;
+}
+static void set_conv_tile(ConvDims *d, int tile) {
+  d->tile = tile;
+  d->n_tiles = (d->T + tile - 1) / tile;
+}
+static unsigned conv_grid(const ConvDims &d, int vec) {
+  const long long shares = (long long)((d.C + vec - 1) / vec) * d.n_tiles * d.batch;
+  return (unsigned)((shares + kConvThreads - 1) / kConvThreads);
 }
 
 template <typename T>
@@ -819,26 +867,20 @@ int slx_cconv1d_fwd(const slx_conv_shape *s, const void *x, const void *weight, 
   SLX_REQUIRE(x && weight && y, SLX_E_NULL, "cconv1d_fwd: NULL tensor");
   cudaStream_t st = as_stream(stream);
   SLX_CONV_T(s->dtype, {
-    constexpr int VFULL = kConvVec;
     const T_ *xp = (const T_ *)x, *wp = (const T_ *)weight, *bp = (const T_ *)bias, *sp = (const T_ *)state;
     if (conv_vec_ok<T_>(s, {x, y})) {
       // 16-byte slices (8 channels of a half type): fewer instructions per channel than the backward's 8-byte ones
       constexpr int VW = 16 / (int)sizeof(T_);
-      const int nblk = (d.C / VW + kConvThreads - 1) / kConvThreads;
       constexpr size_t ring = conv_ring_bytes<T_, VW, kConvRingFwd>(1);
-      auto kern = cconv1d_fwd_staged_kernel<T_, VW, kConvRingFwd>;
+      auto kern = d.silu ? cconv1d_fwd_staged_kernel<T_, VW, kConvRingFwd, true>
+                         : cconv1d_fwd_staged_kernel<T_, VW, kConvRingFwd, false>;
       rc = ensure_dyn_smem(kern, ring);
       if (rc) return rc;
-      const int tile = conv_tile(d.T, false);  // growing the tile to whole waves measured no faster here
-      const int n_tiles = (d.T + tile - 1) / tile;
-      kern<<<dim3(nblk, n_tiles, d.batch), kConvThreads, ring, st>>>(xp, wp, bp, sp, (T_ *)y, (T_ *)next_state, d,
-                                                                     tile);
+      set_conv_tile(&d, conv_tile(d, VW, false));  // growing the tile to whole waves measured no faster here
+      kern<<<conv_grid(d, VW), kConvThreads, ring, st>>>(xp, wp, bp, sp, (T_ *)y, (T_ *)next_state, d);
     } else {
-      const int nblk = (d.C + kConvThreads - 1) / kConvThreads;
-      const int tile = conv_tile(d.T, false);
-      const int n_tiles = (d.T + tile - 1) / tile;
-      cconv1d_fwd_kernel<T_, 1><<<dim3(nblk, n_tiles, d.batch), kConvThreads, 0, st>>>(xp, wp, bp, sp, (T_ *)y,
-                                                                                     (T_ *)next_state, d, tile);
+      set_conv_tile(&d, conv_tile(d, 1, false));
+      cconv1d_fwd_kernel<T_, 1><<<conv_grid(d, 1), kConvThreads, 0, st>>>(xp, wp, bp, sp, (T_ *)y, (T_ *)next_state, d);
     }
   });
   return check_launch("cconv1d_fwd");
@@ -863,9 +905,9 @@ int slx_cconv1d_update(const slx_conv_shape *s, const void *x, const void *weigh
 size_t slx_cconv1d_bwd_workspace_bytes(const slx_conv_shape *s) {
   ConvDims d;
   if (check_conv(s, &d)) return 0;
-  const int tile = conv_tile(d.T, true);
-  const int n_tiles = (d.T + tile - 1) / tile;
-  return sizeof(float) * (size_t)d.batch * n_tiles * d.C * 5;
+  // the aligned kernels take kConvVec channels per share, the plain ones one: the smaller tile of the two
+  const int tile = std::min(conv_tile(d, kConvVec, true), conv_tile(d, 1, true));
+  return sizeof(float) * (size_t)d.batch * ((d.T + tile - 1) / tile) * d.C * 5;
 }
 
 int slx_cconv1d_bwd_as(const slx_conv_shape *s, const void *x, const void *weight, const void *bias, const void *state,
@@ -880,38 +922,34 @@ int slx_cconv1d_bwd_as(const slx_conv_shape *s, const void *x, const void *weigh
               need);
   cudaStream_t st = as_stream(stream);
   float *part = static_cast<float *>(workspace);
-  int n_tiles = 0;  // at most ceil(T / kConvTileBwd), which the workspace is sized for
   SLX_CONV_T(s->dtype, {
     constexpr int VFULL = kConvVec;
     const T_ *xp = (const T_ *)x, *wp = (const T_ *)weight, *bp = (const T_ *)bias, *sp = (const T_ *)state;
     const T_ *gp = (const T_ *)dy, *np = (const T_ *)d_next_state;
+    const int per_row = (d.C + kConvThreads - 1) / kConvThreads;
     if (conv_vec_ok<T_>(s, {x, dy, dx})) {
-      const int nblk = (d.C / VFULL + kConvThreads - 1) / kConvThreads;
       constexpr size_t ring = conv_ring_bytes<T_, VFULL>(2);
-      auto kern = cconv1d_bwd_staged_kernel<T_, VFULL, kConvRing>;
+      auto kern = d.silu ? cconv1d_bwd_staged_kernel<T_, VFULL, kConvRing, true>
+                         : cconv1d_bwd_staged_kernel<T_, VFULL, kConvRing, false>;
       rc = ensure_dyn_smem(kern, ring);
       if (rc) return rc;
-      const int tile = conv_tile_balanced(d.T, kConvTileBwd, (long)nblk * d.batch, conv_slots(kern, ring));
-      n_tiles = (d.T + tile - 1) / tile;
-      kern<<<dim3(nblk, n_tiles, d.batch), kConvThreads, ring, st>>>(xp, wp, bp, sp, gp, np, (T_ *)dx, part, d, tile);
+      set_conv_tile(&d, conv_tile_balanced(d, VFULL, conv_slots(kern, ring)));
+      kern<<<conv_grid(d, VFULL), kConvThreads, ring, st>>>(xp, wp, bp, sp, gp, np, (T_ *)dx, part, d);
       if (dstate)
-        cconv1d_bwd_dstate_kernel<T_, VFULL><<<dim3(nblk, 1, d.batch), kConvThreads, 0, st>>>(xp, wp, bp, sp, gp, np,
-                                                                                            dstate, grad_dtype, d);
+        cconv1d_bwd_dstate_kernel<T_, VFULL><<<dim3((per_row + VFULL - 1) / VFULL, 1, d.batch), kConvThreads, 0, st>>>(
+            xp, wp, bp, sp, gp, np, dstate, grad_dtype, d);
     } else {
-      const int nblk = (d.C + kConvThreads - 1) / kConvThreads;
-      const int tile = conv_tile(d.T, true);
-      n_tiles = (d.T + tile - 1) / tile;
-      cconv1d_bwd_kernel<T_, 1><<<dim3(nblk, n_tiles, d.batch), kConvThreads, 0, st>>>(xp, wp, bp, sp, gp, np,
-                                                                                     (T_ *)dx, part, d, tile);
+      set_conv_tile(&d, conv_tile(d, 1, true));
+      cconv1d_bwd_kernel<T_, 1><<<conv_grid(d, 1), kConvThreads, 0, st>>>(xp, wp, bp, sp, gp, np, (T_ *)dx, part, d);
       if (dstate)
-        cconv1d_bwd_dstate_kernel<T_, 1><<<dim3(nblk, 1, d.batch), kConvThreads, 0, st>>>(xp, wp, bp, sp, gp, np,
-                                                                                        dstate, grad_dtype, d);
+        cconv1d_bwd_dstate_kernel<T_, 1><<<dim3(per_row, 1, d.batch), kConvThreads, 0, st>>>(xp, wp, bp, sp, gp, np,
+                                                                                           dstate, grad_dtype, d);
     }
   });
   rc = check_launch("cconv1d_bwd");
   if (rc) return rc;
   cconv1d_reduce_kernel<<<(d.C * 5 + 31) / 32, dim3(32, kConvReduceRows), 0, st>>>(part, dweight, dbias, grad_dtype,
-                                                                                   d.batch * n_tiles, d.C, d.W);
+                                                                                   d.batch * d.n_tiles, d.C, d.W);
   return check_launch("cconv1d_reduce");
 }
 
@@ -928,7 +966,6 @@ int slx_cconv1d_bwd(const slx_conv_shape *s, const void *x, const void *weight, 
 // Scratch for the weight/bias partial sums lives in the library image itself: kNoAllocFloats
 // floats (4 MiB) per GPU that loads the library, held until the process exits.
 namespace slx {
-constexpr size_t kNoAllocFloats = 1u << 20;
 static __device__ __align__(256) float g_conv_noalloc_scratch[kNoAllocFloats];
 
 // In host code the array's name is only a stand-in for the symbol; the device address has to be
