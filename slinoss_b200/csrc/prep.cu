@@ -189,14 +189,202 @@ struct PrepDims {
   int batch, T, H, P, N;
   int normalize;
   long long vs, ps, bs;  // row strides (elements)
-  int wide_params;        // the covering 16-byte vectors of every params row lie inside the tensor
+  int wide_params;        // params rows start on 16-byte boundaries (half types)
 };
+// the 16-byte vectors that cover head h's 13 values lie inside its row of the tensor
+__device__ __forceinline__ bool row13_wide(const PrepDims &d, int h) {
+  return d.wide_params && (26 * (h + 1) + 15) / 16 * 16 <= 26 * d.H;
+}
 
-// Rows are ordered (b, h, t) so that a CTA's consecutive rows write contiguous
-// output.  A group of G lanes handles one row; lane q of the group owns the
+// ---- asynchronous copies of one lane's 16-byte slice (AL = alignment of the source: 16, or 8 as two halves) ----
+template <int AL>
+__device__ __forceinline__ void copy_slice(void *smem_dst, const void *gsrc) {
+  const unsigned dst = (unsigned)__cvta_generic_to_shared(smem_dst);
+  if constexpr (AL == 16) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(gsrc) : "memory");
+  } else {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(gsrc) : "memory");
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst + 8), "l"((const char *)gsrc + 8) : "memory");
+  }
+}
+__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// Sums over the G lanes of a group of four values at once: the lanes first trade values until each holds one of the
+// four partial sums (3 shuffles), finish that one (log2 G - 2), apply `f` to it and hand the result round (4).
+template <int G, typename F>
+__device__ __forceinline__ void group_sum4(float (&v)[4], F f) {
+  static_assert(G >= 4, "four lanes hold the four sums");
+  const int lane = threadIdx.x & 31;
+  const bool b0 = lane & 1, b1 = lane & 2;
+  const float p0 = (b0 ? v[2] : v[0]) + __shfl_xor_sync(0xffffffffu, b0 ? v[0] : v[2], 1);
+  const float p1 = (b0 ? v[3] : v[1]) + __shfl_xor_sync(0xffffffffu, b0 ? v[1] : v[3], 1);
+  float w = (b1 ? p1 : p0) + __shfl_xor_sync(0xffffffffu, b1 ? p0 : p1, 2);
+#pragma unroll
+  for (int off = 4; off < G; off <<= 1) w += __shfl_xor_sync(0xffffffffu, w, off);
+  w = f(w);
+  const int base = lane & ~3;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) v[j] = __shfl_sync(0xffffffffu, w, base + (j >> 1) + ((j & 1) << 1));
+}
+
+// Forward, rows that one 16-byte slice per lane covers (VEC elements per lane, G lanes per row, G * VEC >= N and P).
+// HBM-bound.  Rows are ordered (b, h, t), so that a CTA's consecutive rows write contiguous output.
+//   * Every lane copies its own five slices of a row (value and the four bc planes) into a ring of kPrepRing rows,
+//     so that two rows per group are on their way while one is worked on, without registers held for them and
+//     without a barrier; the first two are requested before the coefficient map, whose ~500 scalar instructions
+//     (one row per thread) run while they travel.
+//   * Rows per CTA shrink from 256 to 32 while the CTAs do not fill the GPU: a short prompt is latency-bound.
+//   * The RMS scales of the group's head stay in registers until the head changes.
+// Before (rows requested one ahead through registers, always 256 rows per CTA, 16 lanes per row): @@
+constexpr int kPrepRing = 3;
+template <typename T, int VEC, int G, int AL>
+__global__ void __launch_bounds__(256, 3) scanprep_fwd_kernel(const T *__restrict__ value, const T *__restrict__ params,
+                                                              const T *__restrict__ bc, PrepParams pp,
+                                                              T *__restrict__ U, float *__restrict__ M,
+                                                              float *__restrict__ K, T *__restrict__ Bo,
+                                                              T *__restrict__ Co, PrepDims d, PrepHyper hp,
+                                                              int rows_per_cta) {
+  constexpr int NG = 256 / G;  // row groups per CTA
+  extern __shared__ uint4 prep_ring[];  // [kPrepRing][5][256 threads]
+  __shared__ float sbias[258 * 7];      // biases of the CTA's (batch, head)s: at most 257, two for T >= 256
+  const int q = threadIdx.x % G, grp = threadIdx.x / G;
+  const int n0 = q * VEC;
+  const int D = 2 * d.N;
+  const long long n_rows = (long long)d.batch * d.H * d.T;
+  const long long row0 = (long long)blockIdx.x * rows_per_cta;
+  const int rows = (int)min((long long)rows_per_cta, n_rows - row0);
+  const int bh0 = (int)(row0 / d.T), tfirst = (int)(row0 - (long long)bh0 * d.T);
+  const bool on_n = n0 < d.N, on_p = n0 < d.P;
+
+  // the group's walk: rows grp, grp + NG, ... of the CTA
+  struct Walk {
+    int t, bh;
+    long long in_row;
+    int h;
+  };
+  auto settle = [&](Walk &w) {
+    while (w.t >= d.T) {
+      w.t -= d.T;
+      ++w.bh;
+    }
+    const int b = w.bh / d.H;
+    w.h = w.bh - b * d.H;
+    w.in_row = (long long)b * d.T + w.t;
+  };
+  auto advance = [&](Walk &w) {
+    w.t += NG;
+    if (w.t < d.T) w.in_row += NG;
+    else settle(w);
+  };
+  Walk ahead{tfirst + grp, bh0, 0, 0};
+  settle(ahead);
+  uint4 *slot = prep_ring + threadIdx.x;
+  auto request = [&](int i) {  // row grp + i * NG into ring slot i % kPrepRing
+    if (grp + i * NG < rows) {
+      uint4 *s = slot + (i % kPrepRing) * 5 * 256;
+      if (on_n) {
+        const T *bcr = bc + ahead.in_row * d.bs + (long long)ahead.h * 4 * d.N + n0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) copy_slice<AL>(s + j * 256, bcr + j * d.N);
+      }
+      if (on_p) copy_slice<AL>(s + 4 * 256, value + ahead.in_row * d.vs + (long long)ahead.h * d.P + n0);
+      advance(ahead);
+    }
+    copy_commit();
+  };
+#pragma unroll
+  for (int i = 0; i < kPrepRing - 1; ++i) request(i);
+
+  // ---- coefficient map, one row per thread ----
+  {
+    const int n_bh = (tfirst + rows - 1) / d.T + 1;
+    const int tt = tfirst + threadIdx.x, i = tt / d.T, t = tt - i * d.T;
+    float p[13];
+    if ((int)threadIdx.x < rows) {
+      const int bh = bh0 + i, b = bh / d.H, h = bh - b * d.H;
+      load_row13<T>(params + ((long long)b * d.T + t) * d.ps + (long long)h * 13, row13_wide(d, h), p);
+    }
+    for (int e = threadIdx.x; e < n_bh; e += 256) {
+      const size_t at = (size_t)((bh0 + e) % d.H) * pp.bias_stride;
+#pragma unroll
+      for (int k = 0; k < 7; ++k) sbias[7 * e + k] = load_as_f(pp.bias[k], pp.dtype, at);
+    }
+    __syncthreads();
+    if ((int)threadIdx.x < rows) {
+      const long long row = row0 + threadIdx.x;
+      const float *bi = sbias + 7 * i;
+      p[0] += bi[0]; p[1] += bi[1]; p[2] += bi[2]; p[5] += bi[3]; p[6] += bi[4]; p[7] += bi[5]; p[8] += bi[6];
+      const CoefOut o = coef_forward(p, hp, nullptr);
+      *reinterpret_cast<float2 *>(M + row * 2) = o.rho;
+      *reinterpret_cast<float4 *>(K + row * 4) = make_float4(o.kp.x, o.kp.y, o.kc.x, o.kc.y);
+    }
+  }
+
+  // ---- the wide rows ----
+  Walk cur{tfirst + grp, bh0, 0, 0};
+  settle(cur);
+  float sc[4][VEC];
+  int sc_h = -1;
+  const int n_iter = (rows + NG - 1) / NG;  // the same for every group: the shuffles below need whole warps
+  for (int i = 0; i < n_iter; ++i) {
+    request(i + kPrepRing - 1);  // into the slot read in the previous iteration
+    copy_wait<kPrepRing - 1>();
+    const bool live = grp + i * NG < rows;
+    const uint4 *s = slot + (i % kPrepRing) * 5 * 256;
+    const long long row = row0 + grp + (long long)i * NG;
+    if (live && on_p) *reinterpret_cast<uint4 *>(U + row * d.P + n0) = s[4 * 256];
+    uint4 raw[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) raw[j] = (live && on_n) ? s[j * 256] : make_uint4(0, 0, 0, 0);
+    auto elem = [&](int j, int e) { return to_f(reinterpret_cast<const T *>(&raw[j])[e]); };
+    float ss[4] = {1.f, 1.f, 1.f, 1.f};
+    if (d.normalize) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        float a = 0.f;
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) a = fmaf(elem(j, e), elem(j, e), a);
+        ss[j] = a;
+      }
+      group_sum4<G>(ss, [&](float w) { return rsqrtf(w / (float)d.N + 1e-5f); });
+      if (live && on_n && sc_h != cur.h) {
+        sc_h = cur.h;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) load_scale<VEC>(pp, sc_h, j, d.N, n0, sc[j]);
+      }
+    }
+    if (live && on_n) {
+#pragma unroll
+      for (int m = 0; m < 2; ++m) {  // B from planes 0, 1 and C from planes 2, 3, interleaved
+        float o[2][VEC];
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) {
+          float re = elem(2 * m, e), im = elem(2 * m + 1, e);
+          if (d.normalize) {
+            re = (re * ss[2 * m]) * sc[2 * m][e];
+            im = (im * ss[2 * m + 1]) * sc[2 * m + 1][e];
+          }
+          const int k = 2 * e;
+          o[k / VEC][k % VEC] = re;
+          o[(k + 1) / VEC][(k + 1) % VEC] = im;
+        }
+        T *dst = (m == 0 ? Bo : Co) + row * D + 2 * n0;
+        store_vec<T, VEC>(dst, o[0]);
+        store_vec<T, VEC>(dst + VEC, o[1]);
+      }
+    }
+    if (live) advance(cur);
+  }
+  copy_wait<0>();
+}
+
+// Forward, any width and alignment (rows the kernel above does not cover).  Rows are ordered (b, h, t) so that a
+// CTA's consecutive rows write contiguous output.  A group of G lanes handles one row; lane q of the group owns the
 // state lanes n in [VEC*(q + G*k), VEC*(q + G*k) + VEC).
 template <typename T, int VEC, int G>
-__global__ void __launch_bounds__(256) scanprep_fwd_kernel(const T *__restrict__ value, const T *__restrict__ params,
+__global__ void __launch_bounds__(256) scanprep_fwd_any_kernel(const T *__restrict__ value, const T *__restrict__ params,
                                                            const T *__restrict__ bc, PrepParams pp, T *__restrict__ U,
                                                            float *__restrict__ M, float *__restrict__ K,
                                                            T *__restrict__ Bo, T *__restrict__ Co, PrepDims d,
@@ -219,7 +407,7 @@ __global__ void __launch_bounds__(256) scanprep_fwd_kernel(const T *__restrict__
         const int b = (int)(row / ((long long)d.T * d.H));
         float p[13];
         const T *pr = params + ((long long)b * d.T + t) * d.ps + (long long)h * 13;
-        load_row13<T>(pr, d.wide_params != 0, p);
+        load_row13<T>(pr, row13_wide(d, h), p);
         add_bias13(pp, h, p);
         CoefOut o = coef_forward(p, hp, nullptr);
         *reinterpret_cast<float2 *>(M + row * 2) = o.rho;
@@ -235,28 +423,6 @@ __global__ void __launch_bounds__(256) scanprep_fwd_kernel(const T *__restrict__
       gh = (int)((r / d.T) % d.H);
       gb = (int)(r / ((long long)d.T * d.H));
     }
-    constexpr bool kPacked = (VEC > 1) && (VEC * sizeof(T) == 16);
-    const bool one_sweep = d.N <= G * VEC;
-    // raw 16-byte slices of the next row (value + four bc planes), requested one row ahead
-    uint4 nx[5];
-    auto fetch_row = [&](long long row, int b, int h, int t) {
-      if constexpr (kPacked) {
-#pragma unroll
-        for (int j = 0; j < 5; ++j) nx[j] = make_uint4(0, 0, 0, 0);
-        if (row < n_rows) {
-          const long long in_row = (long long)b * d.T + t;
-          const int n0 = q * VEC;
-          if (n0 < d.P) nx[4] = *reinterpret_cast<const uint4 *>(value + in_row * d.vs + (long long)h * d.P + n0);
-          if (n0 < d.N) {
-            const T *bcr = bc + in_row * d.bs + (long long)h * 4 * d.N;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) nx[j] = *reinterpret_cast<const uint4 *>(bcr + j * d.N + n0);
-          }
-        }
-      }
-    };
-    const bool packed_path = kPacked && one_sweep && d.P <= G * VEC;
-    if (packed_path) fetch_row(grow0, gb, gh, gt);
     for (int k = 0; k < RPG; ++k) {
       const long long row = grow0 + k;
       const bool live = row < n_rows;
@@ -271,58 +437,6 @@ __global__ void __launch_bounds__(256) scanprep_fwd_kernel(const T *__restrict__
         }
       }
       const long long in_row = (long long)b * d.T + t;
-      if constexpr (kPacked) {
-        if (packed_path) {
-          uint4 cur[5];
-#pragma unroll
-          for (int j = 0; j < 5; ++j) cur[j] = nx[j];
-          if (k + 1 < RPG) fetch_row(row + 1, gb, gh, gt);
-          const int n0 = q * VEC;
-          if (live && n0 < d.P) *reinterpret_cast<uint4 *>(U + rr * d.P + n0) = cur[4];
-          const bool mine = live && n0 < d.N;
-          float y[4][VEC];
-          float ss[4];
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const T *e = reinterpret_cast<const T *>(&cur[j]);
-            float a = 0.f;
-#pragma unroll
-            for (int i = 0; i < VEC; ++i) {
-              y[j][i] = to_f(e[i]);
-              a = fmaf(y[j][i], y[j][i], a);
-            }
-            ss[j] = a;
-          }
-          if (d.normalize) {
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              ss[j] = rsqrtf(group_sum_f<G>(ss[j]) / (float)d.N + 1e-5f);
-              if (mine) {
-                float sc[VEC];
-                load_scale<VEC>(pp, h, j, d.N, n0, sc);
-#pragma unroll
-                for (int i = 0; i < VEC; ++i) y[j][i] = (y[j][i] * ss[j]) * sc[i];
-              }
-            }
-          }
-          if (mine) {
-            float ob[2][VEC], oc[2][VEC];
-#pragma unroll
-            for (int i = 0; i < VEC; ++i) {
-              int o = 2 * i;
-              ob[o / VEC][o % VEC] = y[0][i];
-              ob[(o + 1) / VEC][(o + 1) % VEC] = y[1][i];
-              oc[o / VEC][o % VEC] = y[2][i];
-              oc[(o + 1) / VEC][(o + 1) % VEC] = y[3][i];
-            }
-            store_vec<T, VEC>(Bo + rr * D + 2 * n0, ob[0]);
-            store_vec<T, VEC>(Bo + rr * D + 2 * n0 + VEC, ob[1]);
-            store_vec<T, VEC>(Co + rr * D + 2 * n0, oc[0]);
-            store_vec<T, VEC>(Co + rr * D + 2 * n0 + VEC, oc[1]);
-          }
-          continue;
-        }
-      }
       // ---- U: copy P values ----
       if (live) {
         const T *src = value + in_row * d.vs + (long long)h * d.P;
@@ -335,35 +449,35 @@ __global__ void __launch_bounds__(256) scanprep_fwd_kernel(const T *__restrict__
       }
       // ---- B, C ----
       const T *bcr = bc + in_row * d.bs + (long long)h * 4 * d.N;
-      if (one_sweep) {
-        // one sweep: every lane keeps its four row slices in registers
-        const int n0 = q * VEC;
-        const bool mine = live && n0 < d.N;
-        float y[4][VEC];
-        float ss[4] = {0.f, 0.f, 0.f, 0.f};
+      float ss[4] = {0.f, 0.f, 0.f, 0.f};
+      if (d.normalize) {
+        if (live) {
+          for (int n0 = q * VEC; n0 < d.N; n0 += G * VEC) {
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          if (mine) load_vec<T, VEC>(bcr + j * d.N + n0, y[j]);
-          else {
+            for (int j = 0; j < 4; ++j) {
+              float v[VEC];
+              load_vec<T, VEC>(bcr + j * d.N + n0, v);
 #pragma unroll
-            for (int i = 0; i < VEC; ++i) y[j][i] = 0.f;
+              for (int i = 0; i < VEC; ++i) ss[j] = fmaf(v[i], v[i], ss[j]);
+            }
           }
-#pragma unroll
-          for (int i = 0; i < VEC; ++i) ss[j] = fmaf(y[j][i], y[j][i], ss[j]);
         }
-        if (d.normalize) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) ss[j] = rsqrtf(group_sum_f<G>(ss[j]) / (float)d.N + 1e-5f);
+      }
+      if (live) {
+        for (int n0 = q * VEC; n0 < d.N; n0 += G * VEC) {
+          float y[4][VEC];
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
-            ss[j] = rsqrtf(group_sum_f<G>(ss[j]) / (float)d.N + 1e-5f);
-            if (mine) {
+            load_vec<T, VEC>(bcr + j * d.N + n0, y[j]);
+            if (d.normalize) {
               float sc[VEC];
               load_scale<VEC>(pp, h, j, d.N, n0, sc);
 #pragma unroll
               for (int i = 0; i < VEC; ++i) y[j][i] = (y[j][i] * ss[j]) * sc[i];
             }
           }
-        }
-        if (mine) {
           float ob[2][VEC], oc[2][VEC];
 #pragma unroll
           for (int i = 0; i < VEC; ++i) {
@@ -377,51 +491,6 @@ __global__ void __launch_bounds__(256) scanprep_fwd_kernel(const T *__restrict__
           store_vec<T, VEC>(Bo + rr * D + 2 * n0 + VEC, ob[1]);
           store_vec<T, VEC>(Co + rr * D + 2 * n0, oc[0]);
           store_vec<T, VEC>(Co + rr * D + 2 * n0 + VEC, oc[1]);
-        }
-      } else {
-        float ss[4] = {0.f, 0.f, 0.f, 0.f};
-        if (d.normalize) {
-          if (live) {
-            for (int n0 = q * VEC; n0 < d.N; n0 += G * VEC) {
-#pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                float v[VEC];
-                load_vec<T, VEC>(bcr + j * d.N + n0, v);
-#pragma unroll
-                for (int i = 0; i < VEC; ++i) ss[j] = fmaf(v[i], v[i], ss[j]);
-              }
-            }
-          }
-#pragma unroll
-          for (int j = 0; j < 4; ++j) ss[j] = rsqrtf(group_sum_f<G>(ss[j]) / (float)d.N + 1e-5f);
-        }
-        if (live) {
-          for (int n0 = q * VEC; n0 < d.N; n0 += G * VEC) {
-            float y[4][VEC];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              load_vec<T, VEC>(bcr + j * d.N + n0, y[j]);
-              if (d.normalize) {
-                float sc[VEC];
-                load_scale<VEC>(pp, h, j, d.N, n0, sc);
-#pragma unroll
-                for (int i = 0; i < VEC; ++i) y[j][i] = (y[j][i] * ss[j]) * sc[i];
-              }
-            }
-            float ob[2][VEC], oc[2][VEC];
-#pragma unroll
-            for (int i = 0; i < VEC; ++i) {
-              int o = 2 * i;
-              ob[o / VEC][o % VEC] = y[0][i];
-              ob[(o + 1) / VEC][(o + 1) % VEC] = y[1][i];
-              oc[o / VEC][o % VEC] = y[2][i];
-              oc[(o + 1) / VEC][(o + 1) % VEC] = y[3][i];
-            }
-            store_vec<T, VEC>(Bo + rr * D + 2 * n0, ob[0]);
-            store_vec<T, VEC>(Bo + rr * D + 2 * n0 + VEC, ob[1]);
-            store_vec<T, VEC>(Co + rr * D + 2 * n0, oc[0]);
-            store_vec<T, VEC>(Co + rr * D + 2 * n0 + VEC, oc[1]);
-          }
         }
       }
     }
@@ -716,7 +785,7 @@ __device__ __forceinline__ void scanprep_bwd_coef_tile(const T *__restrict__ par
       const long long orow = ((long long)bh) * d.T + t;
       float p[13], dp[13];
       const T *pr = params + in_row * d.ps + (long long)h * 13;
-      load_row13<T>(pr, d.wide_params != 0, p);
+      load_row13<T>(pr, row13_wide(d, h), p);
       add_bias13(pp, h, p);
       CoefCtx ctx;
       coef_forward(p, hp, &ctx);
@@ -812,11 +881,10 @@ static int check_prep(const slx_prep_shape *s, PrepDims *d) {
 
 static bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
-// every aligned 16-byte vector that covers a 13-value params row of a half type lies inside its
-// own (16-byte aligned, 16-byte multiple) row of the tensor
+// params rows of a half type that start on 16-byte boundaries: a head's 13 values can be picked out of the aligned
+// vectors that cover them (row13_wide says for which heads those lie inside the row)
 static int params_rows_wide(const slx_prep_shape *s, const void *params) {
-  return s->dtype != SLX_F32 && aligned16(params) && (s->params_stride * 2) % 16 == 0 &&
-         ((long long)s->heads * 13 * 2) % 16 == 0;
+  return s->dtype != SLX_F32 && aligned16(params) && (s->params_stride * 2) % 16 == 0;
 }
 
 // vector width (elements) usable for this problem: 16-byte vectors when every row start and row
@@ -839,17 +907,56 @@ template <int VEC>
 constexpr int prep_group() { return VEC == 1 ? 32 : 16; }
 
 template <typename T, int VEC>
-static int launch_prep_fwd(const slx_prep_shape *s, const PrepDims &d, const void *value, const void *params,
-                           const void *bc, const PrepParams &pp, void *U, float *M, float *K,
-                           void *B, void *C, cudaStream_t st) {
+static int launch_prep_fwd_any(const slx_prep_shape *s, const PrepDims &d, const void *value, const void *params,
+                               const void *bc, const PrepParams &pp, void *U, float *M, float *K, void *B, void *C,
+                               cudaStream_t st) {
   PrepHyper hp = make_hyper(s);
   constexpr int G = prep_group<VEC>();
   long long n_rows = (long long)d.batch * d.H * d.T;
   long long blocks = (n_rows + 255) / 256;
   if (blocks > 148LL * 32) blocks = 148LL * 32;
-  scanprep_fwd_kernel<T, VEC, G><<<(unsigned)blocks, 256, 0, st>>>(
+  scanprep_fwd_any_kernel<T, VEC, G><<<(unsigned)blocks, 256, 0, st>>>(
       (const T *)value, (const T *)params, (const T *)bc, pp, (T *)U, M, K, (T *)B, (T *)C, d, hp);
   return check_launch("scanprep_fwd");
+}
+
+// Rows per CTA of the one-slice forward: as many as make the grid whole waves of three CTAs per SM, at most 256 (one
+// per thread in the coefficient map), at least 32.
+static int prep_rows_per_cta(long long n_rows) {
+  const long long slots = 148LL * 3, waves = (n_rows + slots * 256 - 1) / (slots * 256);
+  long long r = (n_rows + slots * waves - 1) / (slots * waves);
+  r = (r + 7) / 8 * 8;
+  return (int)(r < 32 ? 32 : r);
+}
+template <typename T, int G, int AL>
+static int launch_prep_fwd(const slx_prep_shape *s, const PrepDims &d, const void *value, const void *params,
+                           const void *bc, const PrepParams &pp, void *U, float *M, float *K, void *B, void *C,
+                           cudaStream_t st) {
+  constexpr size_t ring = (size_t)kPrepRing * 5 * 256 * 16;
+  auto kern = scanprep_fwd_kernel<T, 16 / (int)sizeof(T), G, AL>;
+  int rc = ensure_dyn_smem(kern, ring);
+  if (rc) return rc;
+  const long long n_rows = (long long)d.batch * d.H * d.T;
+  const int rows = prep_rows_per_cta(n_rows);
+  kern<<<(unsigned)((n_rows + rows - 1) / rows), 256, ring, st>>>((const T *)value, (const T *)params, (const T *)bc, pp,
+                                                                 (T *)U, M, K, (T *)B, (T *)C, d, make_hyper(s), rows);
+  return check_launch("scanprep_fwd");
+}
+template <typename T, int AL, typename... A>
+static int launch_prep_fwd_lanes(int lanes, const A &...args) {
+  switch (lanes) {
+    case 4: return launch_prep_fwd<T, 4, AL>(args...);
+    case 8: return launch_prep_fwd<T, 8, AL>(args...);
+    case 16: return launch_prep_fwd<T, 16, AL>(args...);
+    default: return launch_prep_fwd<T, 32, AL>(args...);
+  }
+}
+// lanes per row of the one-slice kernels (0: the row is wider than a warp's slices)
+template <typename T>
+static int prep_lanes(const slx_prep_shape *s) {
+  constexpr int v = 16 / (int)sizeof(T);
+  const int need = ((s->N > s->P ? s->N : s->P) + v - 1) / v;
+  return need <= 4 ? 4 : need <= 8 ? 8 : need <= 16 ? 16 : need <= 32 ? 32 : 0;
 }
 
 struct PrepBwdPlan {
@@ -946,12 +1053,25 @@ static int prep_fwd_impl(const slx_prep_shape *s, const void *value, const void 
   d.wide_params = params_rows_wide(s, params);
   cudaStream_t st = as_stream(stream);
   SLX_PREP_T(s->dtype, {
-    int vec = pick_vec<T_>(s, {value, bc, U, B, C});
-    if (!aligned16(pp.b_scale) || !aligned16(pp.c_scale)) vec = 1;  // the scales are read as vectors of their own dtype
     constexpr int VFULL = 16 / (int)sizeof(T_);
-    if (vec == VFULL) rc = launch_prep_fwd<T_, VFULL>(s, d, value, params, bc, pp, U, M, K, B, C, st);
-    else if (vec == VFULL / 2) rc = launch_prep_fwd<T_, VFULL / 2>(s, d, value, params, bc, pp, U, M, K, B, C, st);
-    else rc = launch_prep_fwd<T_, 1>(s, d, value, params, bc, pp, U, M, K, B, C, st);
+    const int G = prep_lanes<T_>(s);
+    // 16-byte slices need N and P in whole slices, rows and pointers aligned to 16 bytes or (copied as two halves) 8:
+    // a projection row of 4 but not 8 half values' multiple, e.g. 2*768 + 12*13 in front of bc
+    int al = 0;
+    if (s->N % VFULL == 0 && s->P % VFULL == 0 && aligned16(U) && aligned16(B) && aligned16(C) && aligned16(pp.b_scale) &&
+        aligned16(pp.c_scale)) {
+      const long long bits = (long long)(reinterpret_cast<uintptr_t>(value) | reinterpret_cast<uintptr_t>(bc)) |
+                             s->value_stride * (long long)sizeof(T_) | s->bc_stride * (long long)sizeof(T_);
+      al = bits % 16 == 0 ? 16 : bits % 8 == 0 ? 8 : 0;
+    }
+    if (al && G) {
+      rc = al == 16 ? launch_prep_fwd_lanes<T_, 16>(G, s, d, value, params, bc, pp, U, M, K, B, C, st)
+                    : launch_prep_fwd_lanes<T_, 8>(G, s, d, value, params, bc, pp, U, M, K, B, C, st);
+    } else if (al == 16) {
+      rc = launch_prep_fwd_any<T_, VFULL>(s, d, value, params, bc, pp, U, M, K, B, C, st);
+    } else {
+      rc = launch_prep_fwd_any<T_, 1>(s, d, value, params, bc, pp, U, M, K, B, C, st);
+    }
   });
   return rc;
 }
