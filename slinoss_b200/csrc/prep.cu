@@ -94,6 +94,9 @@ __device__ __forceinline__ void store_vec(T *p, const float (&v)[VEC]) {
 #pragma unroll
     for (int i = 0; i < VEC; ++i) e[i] = from_f<T>(v[i]);
     *reinterpret_cast<uint2 *>(p) = raw;
+  } else if constexpr (VEC * sizeof(T) == 32 && sizeof(T) == 4) {
+    reinterpret_cast<float4 *>(p)[0] = make_float4(v[0], v[1], v[2], v[3]);
+    reinterpret_cast<float4 *>(p)[1] = make_float4(v[4], v[5], v[6], v[7]);
   } else {
 #pragma unroll
     for (int i = 0; i < VEC; ++i) p[i] = from_f<T>(v[i]);
@@ -212,7 +215,7 @@ template <int N>
 __device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 // Sums over the G lanes of a group of four values at once: the lanes first trade values until each holds one of the
-// four partial sums (3 shuffles), finish that one (log2 G - 2), apply `f` to it and hand the result round (4).
+// four partial sums (3 shuffles; even lanes values 0 and 1, odd lanes 2 and 3), finish that one (log2 G - 2), apply `f` to it and hand the result round (4).
 template <int G, typename F>
 __device__ __forceinline__ void group_sum4(float (&v)[4], F f) {
   static_assert(G >= 4, "four lanes hold the four sums");
@@ -237,7 +240,8 @@ __device__ __forceinline__ void group_sum4(float (&v)[4], F f) {
 //     (one row per thread) run while they travel.
 //   * Rows per CTA shrink from 256 to 32 while the CTAs do not fill the GPU: a short prompt is latency-bound.
 //   * The RMS scales of the group's head stay in registers until the head changes.
-// Before (rows requested one ahead through registers, always 256 rows per CTA, 16 lanes per row): @@
+// b16 T4096 16 heads N128: 0.406 ms (0.94 of the copy rate; 0.504 with rows requested one ahead through registers, 16
+// lanes per row whatever its width and 256 rows per CTA); b2 T1000 8 heads N64: 0.009 ms (0.025).
 constexpr int kPrepRing = 3;
 template <typename T, int VEC, int G, int AL>
 __global__ void __launch_bounds__(256, 3) scanprep_fwd_kernel(const T *__restrict__ value, const T *__restrict__ params,
@@ -504,15 +508,186 @@ __device__ __forceinline__ void scanprep_bwd_coef_tile(const T *__restrict__ par
                                                        const PrepDims &d, const PrepHyper &hp, int rows_per_tile,
                                                        int tile, int n_tiles);
 
-// Backward.  grid = (2 * tiles over T, batch*H).  CTAs with blockIdx.x < n_tiles stream the wide
-// rows; the others run the coefficient-map VJP of the same tiles (scanprep_bwd_coef_tile): its long
-// scalar chains fill issue slots that the streaming CTAs leave idle while they wait on memory.
-// Every CTA works on one head, so the
-// per-head parameter gradients reduce inside the CTA first (registers ->
-// shared memory in a fixed order) and then across CTAs in a second kernel.
+// Backward, rows that one 16-byte slice per lane covers (as scanprep_fwd_kernel).  Reads nine slices per lane and row
+// (bc, dB, dC, dU), writes five.  grid = (2 * tiles over T, batch*H): the first half of a row of CTAs streams the wide
+// rows, the second runs the coefficient-map VJP of the same tiles, whose long scalar chains fill issue slots that
+// the streaming CTAs leave (run inside the streaming CTAs ahead of their rows it cost a third of the kernel's time).
+// A CTA works on one head, so that the parameter gradients reduce inside it first (registers, then shared memory in
+// a fixed order) and across CTAs in a second kernel.
+// HBM bounds the traffic, but the arithmetic on 64 values per lane and row is nearly as long: it works on (re, im)
+// pairs with two-wide fp32 instructions.  With r = 1/rms the two row sums, sum x^2 and sum g x (g = scale dy), are
+// taken together before r exists, so that the group synchronises once; then
+//   d_scale += dy x r,   dx = r g - x r^3 (sum g x) / N.
+// b16 T4096 16 heads N128: 0.707 ms (0.78 of the copy rate; 0.770 with rows requested when needed, 16 lanes per row and
+// 8-byte slices unless everything is 16-byte aligned); b8 T2048 12 heads N64: 0.101 ms (0.195).
 // Partial layout: part[(bh * n_tiles + tile)][4*N + 13].
+constexpr int kPrepBwdSlices = 9;
+#define SLX_OPAQUE4(u) asm volatile("" : "+r"((u).x), "+r"((u).y), "+r"((u).z), "+r"((u).w))
+template <typename T, int VEC, int G, int AL>
+__global__ void __launch_bounds__(256, 2) scanprep_bwd_kernel(const T *__restrict__ params, const T *__restrict__ bc,
+                                                              PrepParams pp, const T *__restrict__ dU,
+                                                              const float *__restrict__ dM,
+                                                              const float *__restrict__ dK, const T *__restrict__ dB,
+                                                              const T *__restrict__ dC, T *__restrict__ d_value,
+                                                              T *__restrict__ d_params, T *__restrict__ d_bc,
+                                                              float *__restrict__ part, PrepDims d, PrepHyper hp,
+                                                              int rows_per_tile, int n_tiles) {
+  if ((int)blockIdx.x >= n_tiles) {
+    scanprep_bwd_coef_tile<T>(params, pp, dM, dK, d_params, part, d, hp, rows_per_tile, (int)blockIdx.x - n_tiles,
+                              n_tiles);
+    return;
+  }
+  constexpr int NG = 256 / G;
+  extern __shared__ uint4 prep_ring[];  // [kPrepRing][9][256 threads] (afterwards the groups' d_scale sums), scales
+  // scale of the head as (re, im) pairs, two neighbouring state lanes per 16 bytes, laid out
+  // [B, C][VEC / 2][G lanes]: a warp reads consecutive 16-byte words
+  float4 *sscale = reinterpret_cast<float4 *>(prep_ring + kPrepRing * kPrepBwdSlices * 256);
+  const int q = threadIdx.x % G, grp = threadIdx.x / G;
+  const int n0 = q * VEC;
+  const int bh = blockIdx.y, b = bh / d.H, h = bh - b * d.H;
+  const int D = 2 * d.N, W = 4 * d.N + 13;
+  const int t_lo = blockIdx.x * rows_per_tile, rows = min(d.T - t_lo, rows_per_tile);
+  const bool on_n = n0 < d.N, on_p = n0 < d.P;
+  const long long in0 = (long long)b * d.T + t_lo, out0 = (long long)bh * d.T + t_lo;
+  uint4 *slot = prep_ring + threadIdx.x;
+  auto request = [&](int i) {  // row grp + i * NG of the tile into ring slot i % kPrepRing
+    const int r = grp + i * NG;
+    if (r < rows) {
+      uint4 *s = slot + (i % kPrepRing) * kPrepBwdSlices * 256;
+      if (on_n) {
+        const T *x = bc + (in0 + r) * d.bs + (long long)h * 4 * d.N + n0;
+        const T *gb = dB + (out0 + r) * D + 2 * n0, *gc = dC + (out0 + r) * D + 2 * n0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) copy_slice<AL>(s + j * 256, x + j * d.N);
+        copy_slice<16>(s + 4 * 256, gb);
+        copy_slice<16>(s + 5 * 256, gb + VEC);
+        copy_slice<16>(s + 6 * 256, gc);
+        copy_slice<16>(s + 7 * 256, gc + VEC);
+      }
+      if (on_p) copy_slice<16>(s + 8 * 256, dU + (out0 + r) * d.P + n0);
+    }
+    copy_commit();
+  };
+#pragma unroll
+  for (int i = 0; i < kPrepRing - 1; ++i) request(i);
+
+  if (d.normalize) {
+    for (int w = threadIdx.x; w < VEC * G; w += 256) {
+      const int m = w / (VEC / 2 * G), n = w % G * VEC + w / G % (VEC / 2) * 2;  // lanes n, n + 1
+      float v[4] = {0.f, 0.f, 0.f, 0.f};
+      if (n < d.N) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          v[k] = load_as_f(scale_plane(pp, 2 * m), pp.dtype, scale_index(pp, h, 2 * m + (k & 1), d.N, n + (k >> 1)));
+      }
+      sscale[w] = make_float4(v[0], v[1], v[2], v[3]);
+    }
+    __syncthreads();
+  }
+  float2 dsc[2][VEC];  // [B, C][lane]: (re, im)
+#pragma unroll
+  for (int m = 0; m < 2; ++m)
+#pragma unroll
+    for (int e = 0; e < VEC; ++e) dsc[m][e] = make_float2(0.f, 0.f);
+  const float inv_n = 1.f / (float)d.N;
+  const int n_iter = (rows + NG - 1) / NG;
+  for (int i = 0; i < n_iter; ++i) {
+    request(i + kPrepRing - 1);
+    copy_wait<kPrepRing - 1>();
+    const int r = grp + i * NG;
+    const bool live = r < rows, mine = live && on_n;
+    const uint4 *s = slot + (i % kPrepRing) * kPrepBwdSlices * 256;
+    if (live && on_p)
+      *reinterpret_cast<uint4 *>(d_value + (in0 + r) * ((long long)d.H * d.P) + (long long)h * d.P + n0) = s[8 * 256];
+    T *dst = d_bc + (in0 + r) * ((long long)d.H * 4 * d.N) + (long long)h * 4 * d.N + n0;
+#pragma unroll
+    for (int m = 0; m < 2; ++m) {  // B, then C: half the row's registers at a time (all of it spilled)
+      uint4 xr[2], gr[2];
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        xr[j] = mine ? s[(2 * m + j) * 256] : make_uint4(0, 0, 0, 0);
+        gr[j] = mine ? s[(4 + 2 * m + j) * 256] : make_uint4(0, 0, 0, 0);
+      }
+      // (re, im) of lane e: x from two planes, dy as it lies
+      auto x_of = [&](int e) {
+        return make_float2(to_f(reinterpret_cast<const T *>(&xr[0])[e]), to_f(reinterpret_cast<const T *>(&xr[1])[e]));
+      };
+      auto dy_of = [&](int e) {
+        const T *g = reinterpret_cast<const T *>(&gr[2 * e / VEC]) + 2 * e % VEC;
+        return make_float2(to_f(g[0]), to_f(g[1]));
+      };
+      auto sc_of = [&](int e) {
+        const float4 v = sscale[(m * (VEC / 2) + e / 2) * G + q];
+        return e & 1 ? make_float2(v.z, v.w) : make_float2(v.x, v.y);
+      };
+      float o[2][VEC];
+      if (d.normalize) {
+        float2 a = make_float2(0.f, 0.f), c = a;
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) {
+          const float2 x = x_of(e);
+          a = __ffma2_rn(x, x, a);
+          c = __ffma2_rn(__fmul2_rn(dy_of(e), sc_of(e)), x, c);
+        }
+        // the packed words stay opaque across the shuffles: expanding them again is a few shifts, holding the
+        // expanded values spilled
+        SLX_OPAQUE4(xr[0]);
+        SLX_OPAQUE4(xr[1]);
+        SLX_OPAQUE4(gr[0]);
+        SLX_OPAQUE4(gr[1]);
+        float v[4] = {a.x, a.y, c.x, c.y};
+        const bool is_square = !(threadIdx.x & 1);  // which of the four sums this lane finishes (group_sum4)
+        group_sum4<G>(v, [&](float w) { return is_square ? rsqrtf(w * inv_n + 1e-5f) : w * inv_n; });
+        const float2 rs = make_float2(v[0], v[1]);
+        const float2 cc = make_float2(-rs.x * rs.x * rs.x * v[2], -rs.y * rs.y * rs.y * v[3]);
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) {
+          const float2 x = x_of(e), dy = dy_of(e);
+          dsc[m][e] = __ffma2_rn(__fmul2_rn(dy, x), rs, dsc[m][e]);
+          const float2 dx = __ffma2_rn(x, cc, __fmul2_rn(rs, __fmul2_rn(dy, sc_of(e))));
+          o[0][e] = dx.x;
+          o[1][e] = dx.y;
+        }
+      } else {
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) {
+          const float2 dy = dy_of(e);
+          o[0][e] = dy.x;
+          o[1][e] = dy.y;
+        }
+      }
+      if (mine) {
+        store_vec<T, VEC>(dst + 2 * m * d.N, o[0]);
+        store_vec<T, VEC>(dst + (2 * m + 1) * d.N, o[1]);
+      }
+      asm volatile("" ::: "memory");
+    }
+  }
+  copy_wait<0>();
+  __syncthreads();  // every lane is done with its ring slots: the ring becomes the groups' sums
+  float *red = reinterpret_cast<float *>(prep_ring);  // [NG][4N]
+  if (on_n) {
+#pragma unroll
+    for (int m = 0; m < 2; ++m)
+#pragma unroll
+      for (int e = 0; e < VEC; ++e) {
+        red[(size_t)grp * 4 * d.N + 2 * m * d.N + n0 + e] = dsc[m][e].x;
+        red[(size_t)grp * 4 * d.N + (2 * m + 1) * d.N + n0 + e] = dsc[m][e].y;
+      }
+  }
+  __syncthreads();
+  float *outp = part + ((size_t)bh * n_tiles + blockIdx.x) * W;
+  for (int e = threadIdx.x; e < 4 * d.N; e += 256) {  // (the 13 bias slots are written by the coefficient CTAs)
+    float acc = 0.f;
+    for (int g = 0; g < NG; ++g) acc += red[(size_t)g * 4 * d.N + e];
+    outp[e] = acc;
+  }
+}
+
+// Backward, any width and alignment.  grid = (2 * tiles over T, batch*H).  CTAs with blockIdx.x < n_tiles stream the
+// wide rows; the others run the coefficient-map VJP of the same tiles.  Same partial layout.
 template <typename T, int VEC, int G, int KMAX>
-__global__ void __launch_bounds__(256, KMAX == 1 ? 2 : 1) scanprep_bwd_kernel(const T *__restrict__ params, const T *__restrict__ bc,
+__global__ void __launch_bounds__(256, KMAX == 1 ? 2 : 1) scanprep_bwd_any_kernel(const T *__restrict__ params, const T *__restrict__ bc,
                                                            PrepParams pp, const T *__restrict__ dU,
                                                            const float *__restrict__ dM, const float *__restrict__ dK,
                                                            const T *__restrict__ dB, const T *__restrict__ dC,
@@ -540,114 +715,6 @@ __global__ void __launch_bounds__(256, KMAX == 1 ? 2 : 1) scanprep_bwd_kernel(co
     for (int j = 0; j < 4; ++j)
 #pragma unroll
       for (int i = 0; i < VEC; ++i) dsc[k][j][i] = 0.f;
-  // Single-sweep path (one 16-byte vector per lane covers N): the row's raw bc and dB/dC stay
-  // packed in registers (8 x 16 bytes) and are expanded twice, once for the row sums and once
-  // for the output, instead of holding expanded fp32 copies; the head's scale sits in shared memory.
-  constexpr bool kPacked = (KMAX == 1) && (VEC > 1) && (VEC * sizeof(T) == 16);
-  float *sscale = red + (size_t)GPB * W;
-  if (kPacked && d.normalize) {
-    for (int e = threadIdx.x; e < 4 * d.N; e += 256) {
-      const int j = e / d.N, n = e - j * d.N;
-      sscale[e] = load_as_f(scale_plane(pp, j), pp.dtype, scale_index(pp, h, j, d.N, n));
-    }
-    __syncthreads();
-  }
-  if constexpr (kPacked) {
-    const int n0 = q * VEC;
-    const bool lane_on = n0 < d.N;
-    for (int tb = t_lo; tb < t_hi; tb += GPB) {
-      const int t = tb + grp;
-      const bool live = (t < t_hi);
-      const int tt = live ? t : t_lo;
-      const long long in_row = (long long)b * d.T + tt;
-      const long long orow = ((long long)bh) * d.T + tt;
-      const T *bcr = bc + in_row * d.bs + (long long)h * 4 * d.N;
-      T *dbcr = d_bc + in_row * ((long long)d.H * 4 * d.N) + (long long)h * 4 * d.N;
-      uint4 xr[4], gr[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) xr[j] = gr[j] = make_uint4(0, 0, 0, 0);
-      if (live && lane_on) {
-#pragma unroll
-        for (int j = 0; j < 4; ++j) xr[j] = *reinterpret_cast<const uint4 *>(bcr + j * d.N + n0);
-        gr[0] = *reinterpret_cast<const uint4 *>(dB + orow * D + 2 * n0);
-        gr[1] = *reinterpret_cast<const uint4 *>(dB + orow * D + 2 * n0 + VEC);
-        gr[2] = *reinterpret_cast<const uint4 *>(dC + orow * D + 2 * n0);
-        gr[3] = *reinterpret_cast<const uint4 *>(dC + orow * D + 2 * n0 + VEC);
-      }
-      if (live) {
-        const T *src = dU + orow * d.P;
-        T *dst = d_value + in_row * ((long long)d.H * d.P) + (long long)h * d.P;
-        for (int p0 = q * VEC; p0 < d.P; p0 += G * VEC)
-          *reinterpret_cast<uint4 *>(dst + p0) = *reinterpret_cast<const uint4 *>(src + p0);
-      }
-      auto elem = [](const uint4 &raw, int i) { return to_f(reinterpret_cast<const T *>(&raw)[i]); };
-      // dy of (plane j, lane i): de-interleave (re, im) pairs of dB (j < 2) or dC
-      auto dy_of = [&](int j, int i) {
-        const int o = 2 * i + (j & 1);
-        return elem(gr[(j < 2 ? 0 : 2) + o / VEC], o % VEC);
-      };
-      if (d.normalize) {
-        float ss[4], gx[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          float a = 0.f;
-#pragma unroll
-          for (int i = 0; i < VEC; ++i) {
-            const float v = elem(xr[j], i);
-            a = fmaf(v, v, a);
-          }
-          ss[j] = rsqrtf(group_sum_f<G>(a) / (float)d.N + 1e-5f);
-        }
-        // keep the packed words opaque between the passes: expanding them again costs a few
-        // shifts, holding 64 expanded values across the group sums costs the occupancy
-#define SLX_OPAQUE4(u) asm volatile("" : "+r"((u).x), "+r"((u).y), "+r"((u).z), "+r"((u).w))
-#pragma unroll
-        for (int j = 0; j < 4; ++j) SLX_OPAQUE4(xr[j]);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          float a = 0.f;
-          const float4 s0 = *reinterpret_cast<const float4 *>(sscale + j * d.N + (lane_on ? n0 : 0));
-          const float4 s1 = *reinterpret_cast<const float4 *>(sscale + j * d.N + (lane_on ? n0 : 0) + 4);
-          const float sc[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
-#pragma unroll
-          for (int i = 0; i < VEC; ++i) {
-            const float xv = elem(xr[j], i) * ss[j];
-            const float dy = dy_of(j, i);
-            dsc[0][j][i] = fmaf(dy, xv, dsc[0][j][i]);
-            a = fmaf(dy * sc[i], xv, a);
-          }
-          gx[j] = group_sum_f<G>(a) / (float)d.N;
-        }
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          SLX_OPAQUE4(xr[j]);
-          SLX_OPAQUE4(gr[j]);
-        }
-#undef SLX_OPAQUE4
-        if (live && lane_on) {
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const float4 s0 = *reinterpret_cast<const float4 *>(sscale + j * d.N + n0);
-            const float4 s1 = *reinterpret_cast<const float4 *>(sscale + j * d.N + n0 + 4);
-            const float sc[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
-            float o[VEC];
-#pragma unroll
-            for (int i = 0; i < VEC; ++i)
-              o[i] = ss[j] * (dy_of(j, i) * sc[i] - elem(xr[j], i) * ss[j] * gx[j]);
-            store_vec<T, VEC>(dbcr + j * d.N + n0, o);
-          }
-        }
-      } else if (live && lane_on) {
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          float o[VEC];
-#pragma unroll
-          for (int i = 0; i < VEC; ++i) o[i] = dy_of(j, i);
-          store_vec<T, VEC>(dbcr + j * d.N + n0, o);
-        }
-      }
-    }
-  } else
   for (int tb = t_lo; tb < t_hi; tb += GPB) {
     const int t = tb + grp;
     const bool live = t < t_hi;
@@ -763,8 +830,7 @@ __global__ void __launch_bounds__(256, KMAX == 1 ? 2 : 1) scanprep_bwd_kernel(co
 
 // Coefficient-map VJP of the backward: one row per thread (rows_per_tile == blockDim.x),
 // d_params rows and the per-tile partial sums of the 13 bias gradients
-// (part[(bh * n_tiles + tile)][4N .. 4N+13)).  Little traffic, long scalar chains: run by CTAs of
-// their own inside the backward launch.
+// (part[(bh * n_tiles + tile)][4N .. 4N+13)).  Little traffic, long scalar chains.
 template <typename T>
 __device__ __forceinline__ void scanprep_bwd_coef_tile(const T *__restrict__ params, const PrepParams &pp,
                                                        const float *__restrict__ dM, const float *__restrict__ dK,
@@ -968,12 +1034,55 @@ static PrepBwdPlan prep_bwd_plan(const slx_prep_shape *s, int VEC) {
   PrepBwdPlan p;
   p.G = VEC == 1 ? 32 : 16;
   p.kmax = (s->N + VEC * p.G - 1) / (VEC * p.G);
-  p.rows_per_tile = 256;
+  // Tiles of at most 256 rows (one per thread in the coefficient part), as many as make whole waves of two CTAs per
+  // SM, of 32 rows at least.
+  const long long slots = 148LL * 2, bh = (long long)s->batch * s->heads;
+  const long long waves = (bh * ((s->T + 255) / 256) + slots - 1) / slots;
+  long long n = waves * slots / bh;
+  if (n < (s->T + 255) / 256) n = (s->T + 255) / 256;
+  long long r = ((s->T + n - 1) / n + 7) / 8 * 8;
+  p.rows_per_tile = (int)(r < 32 ? 32 : r > 256 ? 256 : r);
   p.n_tiles = (s->T + p.rows_per_tile - 1) / p.rows_per_tile;
   int W = 4 * s->N + 13;
-  p.smem = sizeof(float) * ((size_t)(256 / p.G) * W + 4 * (size_t)s->N);  // group partials + the head's scale
+  p.smem = sizeof(float) * (size_t)(256 / p.G) * W;  // group partials (any-width kernel)
   p.ws_bytes = sizeof(float) * (size_t)s->batch * s->heads * p.n_tiles * W;
   return p;
+}
+
+template <typename T>
+static int launch_prep_reduce(const PrepDims &d, const float *part, const PrepParamGrads &pg, int n_tiles,
+                              cudaStream_t st) {
+  const int W = 4 * d.N + 13;
+  scanprep_reduce_kernel<<<dim3((W + 127) / 128, d.H), 128, 0, st>>>(part, pg, d.batch, d.H, n_tiles, d.N);
+  return check_launch("scanprep_reduce");
+}
+
+template <typename T, int G, int AL>
+static int launch_prep_bwd_rows(const slx_prep_shape *s, const PrepDims &d, const void *params, const void *bc,
+                                const PrepParams &pp, const void *dU, const float *dM, const float *dK, const void *dB,
+                                const void *dC, void *d_value, void *d_params, void *d_bc, const PrepParamGrads &pg,
+                                float *part, cudaStream_t st) {
+  constexpr int VEC = 16 / (int)sizeof(T);
+  const PrepBwdPlan pl = prep_bwd_plan(s, VEC);
+  const size_t smem = (size_t)kPrepRing * kPrepBwdSlices * 256 * 16 + (size_t)VEC * G * 16;
+  static_assert((size_t)kPrepRing * kPrepBwdSlices * 256 * 16 >= sizeof(float) * 256 * 4 * VEC, "d_scale sums fit the ring");
+  auto kern = scanprep_bwd_kernel<T, VEC, G, AL>;
+  int rc = ensure_dyn_smem(kern, smem);
+  if (rc) return rc;
+  kern<<<dim3(2 * pl.n_tiles, d.batch * d.H), 256, smem, st>>>(
+      (const T *)params, (const T *)bc, pp, (const T *)dU, dM, dK, (const T *)dB, (const T *)dC, (T *)d_value,
+      (T *)d_params, (T *)d_bc, part, d, make_hyper(s), pl.rows_per_tile, pl.n_tiles);
+  rc = check_launch("scanprep_bwd");
+  return rc ? rc : launch_prep_reduce<T>(d, part, pg, pl.n_tiles, st);
+}
+template <typename T, int AL, typename... A>
+static int launch_prep_bwd_lanes(int lanes, const A &...args) {
+  switch (lanes) {
+    case 4: return launch_prep_bwd_rows<T, 4, AL>(args...);
+    case 8: return launch_prep_bwd_rows<T, 8, AL>(args...);
+    case 16: return launch_prep_bwd_rows<T, 16, AL>(args...);
+    default: return launch_prep_bwd_rows<T, 32, AL>(args...);
+  }
 }
 
 template <typename T, int VEC>
@@ -988,7 +1097,7 @@ static int launch_prep_bwd(const slx_prep_shape *s, const PrepDims &d, const voi
   constexpr int G = prep_group<VEC>();
 #define SLX_PREP_BWD(KM)                                                                                      \
   {                                                                                                           \
-    auto kern = scanprep_bwd_kernel<T, VEC, G, KM>;                                                           \
+    auto kern = scanprep_bwd_any_kernel<T, VEC, G, KM>;                                                           \
     int rc_smem = ensure_dyn_smem(kern, pl.smem);                                                             \
     if (rc_smem) return rc_smem;                                                                              \
     kern<<<dim3(2 * pl.n_tiles, d.batch * d.H), 256, pl.smem, st>>>(                                          \
@@ -1000,10 +1109,7 @@ static int launch_prep_bwd(const slx_prep_shape *s, const PrepDims &d, const voi
   else SLX_PREP_BWD(4)
 #undef SLX_PREP_BWD
   int rc = check_launch("scanprep_bwd");
-  if (rc) return rc;
-  int W = 4 * d.N + 13;
-  scanprep_reduce_kernel<<<dim3((W + 127) / 128, d.H), 128, 0, st>>>(part, pg, d.batch, d.H, pl.n_tiles, d.N);
-  return check_launch("scanprep_reduce");
+  return rc ? rc : launch_prep_reduce<T>(d, part, pg, pl.n_tiles, st);
 }
 
 }  // namespace slx
@@ -1094,7 +1200,17 @@ static int prep_bwd_impl(const slx_prep_shape *s, const void *params, const void
   SLX_PREP_T(s->dtype, {
     int vec = pick_vec<T_>(s, {bc, dU, dB, dC, d_value, d_bc});
     constexpr int VFULL = 16 / (int)sizeof(T_);
-    if (vec == VFULL)
+    const int G = prep_lanes<T_>(s);
+    const long long bits = (long long)reinterpret_cast<uintptr_t>(bc) | s->bc_stride * (long long)sizeof(T_);
+    const bool rows_ok = s->N % VFULL == 0 && s->P % VFULL == 0 && aligned16(dU) && aligned16(dB) && aligned16(dC) &&
+                         aligned16(d_value) && aligned16(d_bc) && aligned16(pp.b_scale) && aligned16(pp.c_scale);
+    if (G && rows_ok && bits % 16 == 0)
+      rc = launch_prep_bwd_lanes<T_, 16>(G, s, d, params, bc, pp, dU, dM, dK, dB, dC, d_value, d_params, d_bc, pg, part,
+                                         st);
+    else if (G && rows_ok && bits % 8 == 0)
+      rc = launch_prep_bwd_lanes<T_, 8>(G, s, d, params, bc, pp, dU, dM, dK, dB, dC, d_value, d_params, d_bc, pg, part,
+                                        st);
+    else if (vec == VFULL)
       rc = launch_prep_bwd<T_, VFULL>(s, d, params, bc, pp, dU, dM, dK, dB, dC, d_value, d_params, d_bc, pg, part, st);
     else if (vec == VFULL / 2)
       rc = launch_prep_bwd<T_, VFULL / 2>(s, d, params, bc, pp, dU, dM, dK, dB, dC, d_value, d_params, d_bc, pg, part,
