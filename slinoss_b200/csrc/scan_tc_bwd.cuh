@@ -3,25 +3,37 @@
 // scan_simt.cuh; every contraction runs on tcgen05 with fp32 accumulators in
 // tensor memory.  One CTA of 512 threads per (chunk, batch*head), one CTA per SM.
 //
+// Operands per 64-column slab of the state (rotated, half precision):
+//   Qbar_t = c_t conj(phi_t),  kappa_s = gamma_s b_s conj(phi_{s+1}),  Z0,  Lambda' = conj(phi_{L-1}) Lambda
+// and per chunk, with es_s = exp(lp_{L-1} - lp_{s+1}):
+//   dS' = decay * (dY U^T),   Ye_t = exp(lp_t) dY_t,   Ue_s = es_s u_s
+// Because p_{L-1}/p_{s+1} = es_s phi_{L-1} conj(phi_{s+1}), the increment path needs no operands of its own:
+//   dB_s   = conj(kappa coefficient) (dS'^T Qbar + Ue Lambda')_s + ...     (one accumulator X for both paths)
+//   dU_s   = es_s (kappa Lambda'^T)_s + (S'^T dY)_s + ...
+// and kappa [Qbar ; Lambda']^T is ONE product of N = 192 that gives S^T and kappa Lambda'^T together.
+//
 // Tensor-memory map (fp32 columns):
-//   [  0,128)  G = dY U^T, then S = Qbar kappa^T (accumulated over state slabs)
-//   [128,192)  dU, increment path:  Bhat Lambda^T
-//   [192,256)  dq  (slab)   = dS' kappa + (e^lp dY) Z0
-//   [256,320)  X   (slab)   = dS'^T Qbar
-//   [320,384)  UL  (slab)   = U Lambda
-//   [384,448)  dU, score path:      S'^T dY
+//   [  0,192)  [S^T | R] = kappa [Qbar ; Lambda']^T   (accumulated over the slabs)
+//   [192,448)  two buffers, one per slab parity, of  dq = dS' kappa + Ye Z0  and  X = dS'^T Qbar + Ue Lambda'
+//              (buffer 0 holds G = dY U^T first)
+//   [448,512)  S'^T dY
 //
 // The source token in front of the chunk (b_{-1}, u_{-1}) borrows key slot 127,
 // whose own merged-tap column is empty (no query follows the last token):
-//   dS'[t][127] = exp(lp_t - lp_0) dY_t.u_{-1},   kappa[127] = k^p_0 b_{-1} conj(phi_0)
-// so that row 127 of X is the column sum the carry gradient needs, the boundary
-// term of dq comes out of the same product, column 127 of S is the boundary
-// score and row 127 of S'^T dY is the dU carried to the previous token.
+//   dS'[t][127] = exp(lp_t - lp_0) dY_t.u_{-1},  kappa_127 = k^p_0 b_{-1} conj(phi_0),  Ue_127 = exp(lp_{L-1} - lp_0) u_{-1}
+// so that row 127 of X is the whole gradient it receives (times conj(phi_0)), the boundary term of dq comes out of
+// the same product, and row 127 of es R + S'^T dY is the dU carried to the previous token.  Token 127's own share of
+// the increment path, u_127 . Lambda and (k^c b)_127 . Lambda, is summed on the CUDA cores (carry helpers below).
 //
-// Thread roles: for staging, thread = (16-byte chunk j = tid%8, rows tid/8 and
-// tid/8+64); for tensor-memory epilogues, thread = (row 32*(warp%4)+lane,
-// column quarter warp/4).  Global loads a phase needs are issued before the
-// wait on the preceding products, so that their latency overlaps the tensor work.
+// What bounds it: neither HBM (35 %) nor the tensor pipe (a slab's 28 products take about 2 K cycles) but the
+// rotations and the epilogue on the CUDA cores, so everything else has to run in their shadow.  Operand tiles and
+// slab accumulators are double-buffered: while the tensor core works on slab i+1, all warps are in the epilogue of
+// slab i and the staging of slab i+2.  The raw (C, B) slab travels by TMA one slab ahead; dC / dB leave by TMA from
+// the operand tiles.  8192 chunks of D 256: 1.245 ms (1.394 with single buffers, where staging, products and epilogue of
+// a slab took turns).
+//
+// Thread mapping: thread = (row 32*(warp%4)+lane, 16-byte chunks 2*(warp/4) and +1 of the slab), the tensor-memory
+// lane mapping, for staging and epilogue alike, so that the raw b, c of a cell stay in registers from one to the other.
 #pragma once
 
 #include "scan_tc.cuh"
@@ -34,7 +46,24 @@ struct alignas(64) ScanBwdMaps {
 };
 
 constexpr int kTcBwdThreads = 512;
-constexpr size_t scan_bwd_tc_smem_bytes() { return 1024 + 144 * 1024 + 28 * 1024 + 32 * 1024; }
+constexpr uint32_t kBwdStage = 49152;  // [kappa 16 K][Qbar 16 K][Lambda' 8 K][Z0 8 K], one per slab parity
+constexpr uint32_t kBwdScalars = 81920 + 2 * kBwdStage + 32768;
+constexpr size_t scan_bwd_tc_smem_bytes() { return 1024 + kBwdScalars + 17920; }
+constexpr int kTmR = 128, kTmSlab = 192, kTmU = 448;  // accumulator columns (S^T at 0)
+
+// S^T -> S'^T of one 32-column block: row s, columns t = c0 + i.  lpb = lp_{s+1} (lp_0 for the boundary slot, whose
+// row takes every column).  FAST factors exp(lp_t - lpb) through the table e3[t] = exp(lp_t - lp_{32 (t / 32)}).
+template <bool FAST>
+__device__ __forceinline__ void decay_mask32_rows(float (&v)[32], int c0, int s, bool boundary, float lpb,
+                                                  const float *lp, const float *e3, float diag) {
+  const float rf = FAST ? __expf(lp[c0] - lpb) : 0.f;
+#pragma unroll
+  for (int i = 0; i < 32; ++i) {
+    const int t = c0 + i;
+    const float f = FAST ? rf * e3[t] : __expf(lp[t] - lpb);
+    v[i] = (t > s || boundary) ? v[i] * f : (t == s ? diag : 0.f);
+  }
+}
 
 template <typename T>
 __global__ void __launch_bounds__(kTcBwdThreads, 1) chunk_scan_bwd_tc_kernel(ScanBwdArgs<T> a,
@@ -43,35 +72,32 @@ __global__ void __launch_bounds__(kTcBwdThreads, 1) chunk_scan_bwd_tc_kernel(Sca
   extern __shared__ unsigned char smem_raw[];
   unsigned char *base =
       reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  unsigned char *tdY = base;                // [t][p]
-  unsigned char *tdYe = base + 16384;       // [t][p]  exp(lp_t) dY
-  unsigned char *tU = base + 32768;         // [s][p]
-  unsigned char *tdS = base + 49152;        // 2 x [t][64 s]   dS', later S'
-  unsigned char *tQ = base + 81920;         // [t][d]  Qbar slab
-  unsigned char *tK = base + 98304;         // [s][d]  kappa slab
-  unsigned char *tBh = base + 114688;       // [s][d]  w_s b_s slab
-  unsigned char *tZ = base + 131072;        // [p][d]  Z0 slab        (8 KB)
-  unsigned char *tLm = base + 139264;       // [p][d]  Lambda slab    (8 KB)
-  float *lp = reinterpret_cast<float *>(base + 147456);
-  float *gd = lp + L;                        // G[t][t]
-  float *gm1 = gd + L;                       // dY_t . u_{-1}
-  float *um1 = gm1 + L;                      // 64
-  float *duc = um1 + 64;                     // 64  increment path of the carried dU
-  float2 *ph = reinterpret_cast<float2 *>(duc + 64);
-  float2 *mraw = ph + L, *kc = mraw + L, *kp = kc + L, *gam = kp + L, *gk = gam + L, *wco = gk + L, *sg1 = wco + L;
-  float2 *bc = sg1 + L, *bX = bc + L, *gA = bX + L, *gsum = gA + L;
-  float2 *bm1 = gsum + L;                    // 128  b_{-1}
-  float2 *ul1 = bm1 + 128;                   // 128  (u_{-1} . Lambda)[n]
-  float2 *bh1 = ul1 + 128;                   // 128  w_{-1} b_{-1}
-  float2 *misc = bh1 + 128;                  // [0] bLam(last row) [1] dk^p_0 [2] w_{-1} [3] p_{L-1}/p_0
-  float *ulw = reinterpret_cast<float *>(misc + 4);  // [16][64] per-warp partials of u_{-1}.Lambda
-  float *e2 = ulw + 16 * 64;                          // 128: decay table (decay_mask32)
-  float *xb = e2 + L;                                 // 256: row 127 of X (boundary column sums), all slabs
-  float *ulf = xb + 256;                              // 256: u_{-1} . Lambda, all slabs
-  unsigned char *sC = base + 147456 + 28672;          // raw C slab (swizzled tile), filled by cp.async
-  unsigned char *sB = sC + 16384;                     // raw B slab
-  __shared__ uint64_t mbar;   // completion of the tensor products
-  __shared__ uint64_t tbar;   // arrival of a raw (C, B) slab by TMA
+  unsigned char *tdY = base;                   // [t][p]
+  unsigned char *tYe = base + 16384;           // [t][p]
+  unsigned char *tUe = base + 32768;           // [s][p]
+  unsigned char *tdS = base + 49152;           // 2 x [t][64 s]  dS', at the end 2 x [s][64 t]  S'^T
+  unsigned char *tSt = base + 81920;           // two staging buffers
+  unsigned char *tU = tSt + kBwdStage;         // [s][p]  U, needed for G only: lies in the second staging buffer
+  unsigned char *sC = tSt + 2 * kBwdStage;     // raw C slab (swizzled tile), by TMA
+  unsigned char *sB = sC + 16384;              // raw B slab
+  float *lp = reinterpret_cast<float *>(base + kBwdScalars);
+  float *gd = lp + L;                          // G[t][t]
+  float *gm1 = gd + L;                         // dY_t . u_{-1}
+  float *um1 = gm1 + L;                        // 64   u_{-1}
+  float *u127 = um1 + 64;                      // 64   u of the chunk's last token (zero past the end)
+  float *dla = u127 + 64;                      // 64   (k^c b)_127 . Lambda[p]
+  float *e2 = dla + 64;                        // 128  decay table of dS' (decay_mask32)
+  float *e3 = e2 + L;                          // 128  decay table of S'^T
+  float *xb = e3 + L;                          // 256  row 127 of X, all slabs
+  float *ulf = xb + 256;                       // 256  u_127 . Lambda, all slabs
+  float *ulw = ulf + 256;                      // [16][64] per-warp partials of u_127 . Lambda
+  float2 *gA = reinterpret_cast<float2 *>(ulw), *bX = gA + L;  // (after the slabs)
+  float2 *ph = reinterpret_cast<float2 *>(ulw + 16 * 64);
+  float2 *mraw = ph + L, *kc = mraw + L, *kp = kc + L, *bc = kp + L, *gsum = bc + L;
+  float2 *bm1 = gsum + L;                      // 128  b_{-1}
+  float2 *kcb = bm1 + 128;                     // 128  (k^c b)_127
+  float2 *misc = kcb + 128;                    // [0] conj(b_127) . (u_127 . Lambda)   [1..4] dk^p_0, by warp
+  __shared__ uint64_t bars[4];  // [0], [1] products of a slab, by parity; [2] G, then S'^T dY; [3] raw slab by TMA
   __shared__ uint32_t tmem_slot;
 
   const ScanDims d = a.d;
@@ -81,31 +107,32 @@ __global__ void __launch_bounds__(kTcBwdThreads, 1) chunk_scan_bwd_tc_kernel(Sca
   const int valid = min(L, d.T - t0);
   const size_t tok0 = (size_t)bh * d.T + t0;
   const int NB = d.D / 64;
-  const uint32_t mbar_s = umma::smem_u32(&mbar), tbar_s = umma::smem_u32(&tbar);
+  const uint32_t bar0 = umma::smem_u32(&bars[0]), gbar = bar0 + 16, tbar = bar0 + 24;
   constexpr int fmt = umma::HalfFmt<T>::value;
 
 #define SLX_STAMP(i) SLX_DIAG_STAMP(i)
   SLX_STAMP(0);
-  const int j = tid & 7, r0 = tid >> 3;  // r0 in [0,64)
   // on this path the chunk-start states are stored in the activation dtype (api: slx_scan_starts_dtype)
   const T *z0 = reinterpret_cast<const T *>(a.starts) + ((size_t)bh * d.NC + c) * P * d.D;
   const T *lam = reinterpret_cast<const T *>(a.d_inc) + ((size_t)bh * d.NC + c) * P * d.D;  // same dtype as z0
   float2 mreg[4];  // the prefix warp's multipliers, requested ahead of the bulk copies
   if (warp == 2) chunk_prefix_load4(a.M + tok0 * 2, valid, mreg);
-  // U and dY land in their operand tiles by asynchronous copy (rows past the chunk end are
-  // zero-filled); the first raw (C, B) slab follows as a second group
+  // U and dY land in their tiles by asynchronous copy (rows past the chunk end are zero-filled)
+  {
+    const int j = tid & 7, r0 = tid >> 3;
 #pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    const int r = r0 + 64 * i;
-    const int rr = r < valid ? r : 0;
-    const uint32_t nbytes = r < valid ? 16u : 0u;
-    const uint32_t off = umma::swz_off(r, j);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(umma::smem_u32(tU + off)),
-                 "l"(a.U + (tok0 + rr) * P + 8 * j), "r"(nbytes)
-                 : "memory");
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(umma::smem_u32(tdY + off)),
-                 "l"(a.dY + (tok0 + rr) * P + 8 * j), "r"(nbytes)
-                 : "memory");
+    for (int i = 0; i < 2; ++i) {
+      const int r = r0 + 64 * i;
+      const int rr = r < valid ? r : 0;
+      const uint32_t nbytes = r < valid ? 16u : 0u;
+      const uint32_t off = umma::swz_off(r, j);
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(umma::smem_u32(tU + off)),
+                   "l"(a.U + (tok0 + rr) * P + 8 * j), "r"(nbytes)
+                   : "memory");
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(umma::smem_u32(tdY + off)),
+                   "l"(a.dY + (tok0 + rr) * P + 8 * j), "r"(nbytes)
+                   : "memory");
+    }
   }
   asm volatile("cp.async.commit_group;" ::: "memory");
   // One raw (C, B) slab = two TMA boxes of [128 tokens][64 columns] into the swizzled staging tiles,
@@ -113,14 +140,14 @@ __global__ void __launch_bounds__(kTcBwdThreads, 1) chunk_scan_bwd_tc_kernel(Sca
   auto prefetch_cb = [&](int sl) {
     if (tid == 32) {
       umma::fence_smem_to_async();  // the tiles' earlier (generic) readers are behind a barrier
-      umma::mbar_expect_tx(tbar_s, 2u * 16384u);
-      umma::tma_load_3d(umma::smem_u32(sC), &maps.C, sl * 64, t0, bh, tbar_s);
-      umma::tma_load_3d(umma::smem_u32(sB), &maps.B, sl * 64, t0, bh, tbar_s);
+      umma::mbar_expect_tx(tbar, 2u * 16384u);
+      umma::tma_load_3d(umma::smem_u32(sC), &maps.C, sl * 64, t0, bh, tbar);
+      umma::tma_load_3d(umma::smem_u32(sB), &maps.B, sl * 64, t0, bh, tbar);
     }
   };
   if (tid == 32) {
-    umma::mbar_init(mbar_s, 1);
-    umma::mbar_init(tbar_s, 1);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) umma::mbar_init(bar0 + 8 * i, 1);
     umma::fence_mbar_init();
     umma::tma_prefetch_map(&maps.C);
     umma::tma_prefetch_map(&maps.B);
@@ -128,7 +155,6 @@ __global__ void __launch_bounds__(kTcBwdThreads, 1) chunk_scan_bwd_tc_kernel(Sca
     umma::tma_prefetch_map(&maps.dB);
   }
   prefetch_cb(0);
-  uint32_t tphase = 0;
   // Z0 / Lambda slab: one 8-value (16-byte) item per thread, prefetched into registers
   const int zp = tid >> 3, zj = tid & 7;
   uint4 zr, lr;
@@ -156,13 +182,18 @@ __global__ void __launch_bounds__(kTcBwdThreads, 1) chunk_scan_bwd_tc_kernel(Sca
     if (t0 > 0) v = to_f(a.U[(tok0 - 1) * P + p]);
     else if (a.Uprev) v = load_as_f(a.Uprev, a.prev_dtype, (size_t)bh * P + p);
     um1[p] = v;
-    duc[p] = 0.f;
+    u127[p] = valid == L ? to_f(a.U[(tok0 + L - 1) * P + p]) : 0.f;
+    dla[p] = 0.f;
   } else if (tid >= 320 && tid < 320 + d.N) {
     int n = tid - 320;
-    float2 bv = make_float2(0.f, 0.f);
+    float2 bv = make_float2(0.f, 0.f), kb = bv;
     if (t0 > 0) bv = load_pair<T>(a.B + (tok0 - 1) * d.D + 2 * n);
     else if (a.Bprev) bv = load_as_f2(a.Bprev, a.prev_dtype, (size_t)bh * d.D + 2 * n);
+    if (valid == L)
+      kb = cmul(*reinterpret_cast<const float2 *>(a.K + (tok0 + L - 1) * 4 + 2),
+                load_pair<T>(a.B + (tok0 + L - 1) * d.D + 2 * n));
     bm1[n] = bv;
+    kcb[n] = kb;
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");  // U, dY tiles
   umma::fence_smem_to_async();
@@ -170,74 +201,485 @@ __global__ void __launch_bounds__(kTcBwdThreads, 1) chunk_scan_bwd_tc_kernel(Sca
   __syncthreads();
   umma::fence_after_sync();
   const uint32_t tmem = tmem_slot;
-  const uint32_t sdY = umma::smem_u32(tdY), sdYe = umma::smem_u32(tdYe), sU = umma::smem_u32(tU),
-                 sdS = umma::smem_u32(tdS), sQ = umma::smem_u32(tQ), sK = umma::smem_u32(tK),
-                 sBh = umma::smem_u32(tBh), sZ = umma::smem_u32(tZ), sLm = umma::smem_u32(tLm);
+  const uint32_t sdY = umma::smem_u32(tdY), sYe = umma::smem_u32(tYe), sUe = umma::smem_u32(tUe),
+                 sdS = umma::smem_u32(tdS), sSt = umma::smem_u32(tSt);
   SLX_STAMP(1);
-  // ---- G = dY U^T (runs while the per-token coefficients are computed) -----------------------
+  // ---- G = dY U^T (runs while the first slab is staged) --------------------------------------
   if (tid == 0) {
-    const uint32_t id = umma::make_idesc(128, 128, false, false, fmt);
+    const uint32_t id = umma::make_idesc(128, 128, false, false, fmt), sU = umma::smem_u32(tU);
 #pragma unroll
     for (int kk = 0; kk < 4; ++kk)
-      umma::mma_ss(tmem, umma::desc_kmajor(sdY, kk), umma::desc_kmajor(sU, kk), id, kk != 0);
-    umma::commit(mbar_s);
+      umma::mma_ss(tmem + kTmSlab, umma::desc_kmajor(sdY, kk), umma::desc_kmajor(sU, kk), id, kk != 0);
+    umma::commit(gbar);
   }
-  // exp(lp_t) dY and g_{-1}[t] = dY_t . u_{-1}
-#pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    int r = r0 + 64 * i;
-    const uint4 dyr = *reinterpret_cast<const uint4 *>(tdY + umma::swz_off(r, j));
-    const uint32_t *w = reinterpret_cast<const uint32_t *>(&dyr);
-    const float el = __expf(lp[r]);
-    float tmp[8], dot = 0.f;
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      float2 v = umma::unpack2(w[e], T());
-      dot = fmaf(v.x, um1[8 * j + 2 * e], fmaf(v.y, um1[8 * j + 2 * e + 1], dot));
-      tmp[2 * e] = el * v.x;
-      tmp[2 * e + 1] = el * v.y;
-    }
-    *reinterpret_cast<uint4 *>(tdYe + umma::swz_off(r, j)) = pack8<T>(tmp);
-#pragma unroll
-    for (int off = 4; off > 0; off >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, off);
-    if (j == 0) gm1[r] = dot;
-  }
-  if (tid < L) {
-    const int t = tid;
-    float2 g = make_float2(0.f, 0.f), w, s1 = g, gkv = g;
-    if (t + 1 < L) {
-      g = cadd(cmul(mraw[t + 1], kc[t]), kp[t + 1]);
-      gkv = cmulc(g, ph[t + 1]);
-      s1 = cscale(cmulc(ph[L - 1], ph[t + 1]), __expf(lp[L - 1] - lp[t + 1]));  // p_{L-1}/p_{t+1}
-      w = cmul(s1, g);
-    } else {
-      w = kc[t];
-      gkv = cmulc(kp[0], ph[0]);  // boundary slot: kappa[127] = k^p_0 b_{-1} conj(phi_0)
-    }
-    gam[t] = g;
-    gk[t] = gkv;
-    sg1[t] = s1;
-    wco[t] = w;
-    e2[t] = decay_table_entry(lp, t, L);
-  } else if (tid >= 256 && tid < 256 + d.N) {
-    const int n = tid - 256;
-    const float2 s0 = cscale(cmulc(ph[L - 1], ph[0]), __expf(lp[L - 1] - lp[0]));  // p_{L-1}/p_0
-    const float2 w1 = cmul(s0, kp[0]);
-    bh1[n] = cmul(w1, bm1[n]);
-    if (n == 0) {
-      misc[0] = misc[1] = make_float2(0.f, 0.f);
-      misc[2] = w1;
-      misc[3] = s0;
-    }
-  }
-  umma::fence_smem_to_async();
-  const bool fast_decay = !__syncthreads_or(tid < L && decay_step_out_of_range(lp, tid));
-
-  uint32_t phase = 0;
-  bool ok = true;
   const int q4 = warp & 3, qc = warp >> 2;  // lane quarter of tensor memory, column quarter
   const int row = 32 * q4 + lane;
-#include "scan_tc_bwd_body.inc"
+  const bool last_row = row == L - 1;
+  const float2 ph_r = ph[row];
+  const float2 phL = ph[L - 1];
+  const float2 kc_r = kc[row];
+  // gamma_s conj(phi_{s+1}); the boundary slot: k^p_0 conj(phi_0)
+  const float2 gk_r = last_row ? cmulc(kp[0], ph[0])
+                               : cmulc(cadd(cmul(mraw[row + 1], kc_r), kp[row + 1]), ph[row + 1]);
+  const float lpb = last_row ? lp[0] : lp[row + 1];
+  uint32_t ph_bits = 0;  // phases of the barriers: bit 0, 1 slab products, 2 gbar, 3 tbar
+  bool ok = true;
+  auto wait = [&](int which) {
+    ok = umma::mbar_wait(bar0 + 8 * which, (ph_bits >> which) & 1) && ok;
+    ph_bits ^= 1u << which;
+  };
+  float2 acc_bc = make_float2(0.f, 0.f);  // conj(b) c over this thread's cells
+  uint4 cr[2], br[2], cn[2], bn[2];       // raw cells: slab in its epilogue, slab being staged
+
+  // Operand tiles of slab sl from its raw cells, written to its staging buffer.  The bulk stores of dC / dB of
+  // slab sl-2 leave from the same tiles: the rotated cells wait in registers until those have read them.
+  auto stage = [&](int sl) {
+    wait(3);
+    uint4 qv[2], kv[2];
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const uint32_t off = umma::swz_off(row, 2 * qc + k);
+      cn[k] = *reinterpret_cast<const uint4 *>(sC + off);
+      bn[k] = *reinterpret_cast<const uint4 *>(sB + off);
+      uint4 src = bn[k];
+      if (last_row) {
+        float tmp[8];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float2 v = bm1[sl * 32 + 8 * qc + 4 * k + e];
+          tmp[2 * e] = v.x;
+          tmp[2 * e + 1] = v.y;
+        }
+        src = pack8<T>(tmp);
+      }
+      qv[k] = rotate_chunk<T>(cn[k], cconj(ph_r));
+      kv[k] = rotate_chunk<T>(src, gk_r);
+      cdot_chunk<T>(bn[k], cn[k], acc_bc);
+    }
+    const uint4 lv = rotate_chunk<T>(lr, cconj(phL));
+    unsigned char *buf = tSt + kBwdStage * (sl & 1);
+    if (sl >= 2) {
+      if (tid == 0) umma::tma_store_wait_read();
+      __syncthreads();
+    }
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const uint32_t off = umma::swz_off(row, 2 * qc + k);
+      *reinterpret_cast<uint4 *>(buf + off) = kv[k];
+      *reinterpret_cast<uint4 *>(buf + 16384 + off) = qv[k];
+    }
+    *reinterpret_cast<uint4 *>(buf + 32768 + umma::swz_off(zp, zj)) = lv;
+    *reinterpret_cast<uint4 *>(buf + 40960 + umma::swz_off(zp, zj)) = zr;
+    umma::fence_smem_to_async();
+    umma::fence_before_sync();
+  };
+  auto issue = [&](int sl) {  // one thread
+    umma::fence_after_sync();
+    constexpr uint32_t id_sr = umma::make_idesc(128, 192, false, false, fmt);
+    constexpr uint32_t id_km = umma::make_idesc(128, 64, false, true, fmt);
+    constexpr uint32_t id_mm = umma::make_idesc(128, 64, true, true, fmt);
+    const uint32_t sK = sSt + kBwdStage * (sl & 1), sQ = sK + 16384, sLm = sK + 32768, sZ = sK + 40960;
+    const uint32_t dq = tmem + kTmSlab + 128 * (sl & 1), X = dq + 64;
+    const uint64_t dSk = umma::desc_kmajor(sdS, 0), dSm = umma::desc_mnmajor(sdS, 0, 16384u);
+    const uint64_t dKm = umma::desc_mnmajor(sK, 0, 0), dKk = umma::desc_kmajor(sK, 0);
+    const uint64_t dQm = umma::desc_mnmajor(sQ, 0, 0), dQk = umma::desc_kmajor(sQ, 0);
+    const uint64_t dYk = umma::desc_kmajor(sYe, 0), dZm = umma::desc_mnmajor(sZ, 0, 0);
+    const uint64_t dUk = umma::desc_kmajor(sUe, 0), dLm = umma::desc_mnmajor(sLm, 0, 0);
+#pragma unroll
+    for (int kk = 0; kk < 8; ++kk) {
+      umma::mma_ss(dq, umma::desc_advance(dSk, 16384u * (kk >> 2) + umma::kStepK * (kk & 3)),
+                   umma::desc_advance(dKm, umma::kStepMN * kk), id_km, kk != 0);
+      umma::mma_ss(X, umma::desc_advance(dSm, umma::kStepMN * kk), umma::desc_advance(dQm, umma::kStepMN * kk), id_mm,
+                   kk != 0);
+    }
+#pragma unroll
+    for (int kk = 0; kk < 4; ++kk) {
+      umma::mma_ss(dq, umma::desc_advance(dYk, umma::kStepK * kk), umma::desc_advance(dZm, umma::kStepMN * kk), id_km, 1);
+      umma::mma_ss(X, umma::desc_advance(dUk, umma::kStepK * kk), umma::desc_advance(dLm, umma::kStepMN * kk), id_km, 1);
+      umma::mma_ss(tmem, umma::desc_advance(dKk, umma::kStepK * kk), umma::desc_advance(dQk, umma::kStepK * kk), id_sr,
+                   (sl | kk) != 0);
+    }
+    umma::commit(bar0 + 8 * (sl & 1));
+  };
+  // Token 127's own share of the increment path, from this thread's Lambda values (still in registers): per-warp
+  // partials of (u_127 . Lambda)[d] (rows zp of this warp, summed over the 4 lanes that share zj) and
+  // dla[p] += sum_d kcb[d] Lambda[p][d] (summed over the 8 lanes that share zp).
+  auto helper = [&](int sl) {
+    float tl[8];
+    {
+      const uint32_t *lw = reinterpret_cast<const uint32_t *>(&lr);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float2 v = umma::unpack2(lw[e], T());
+        tl[2 * e] = v.x;
+        tl[2 * e + 1] = v.y;
+      }
+    }
+    const float4 *kbv = reinterpret_cast<const float4 *>(reinterpret_cast<const float *>(kcb) + 64 * sl + 8 * zj);
+    const float4 h0 = kbv[0], h1 = kbv[1];
+    const float hb[8] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
+    const float uz = u127[zp];
+    float ds = 0.f, up[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      ds = fmaf(hb[e], tl[e], ds);
+      up[e] = uz * tl[e];
+      up[e] += __shfl_xor_sync(0xffffffffu, up[e], 8);
+      up[e] += __shfl_xor_sync(0xffffffffu, up[e], 16);
+    }
+#pragma unroll
+    for (int off = 4; off > 0; off >>= 1) ds += __shfl_xor_sync(0xffffffffu, ds, off);
+    if (zj == 0) dla[zp] += ds;
+    if (lane < 8) {
+      *reinterpret_cast<float4 *>(ulw + 64 * warp + 8 * lane) = make_float4(up[0], up[1], up[2], up[3]);
+      *reinterpret_cast<float4 *>(ulw + 64 * warp + 8 * lane + 4) = make_float4(up[4], up[5], up[6], up[7]);
+    }
+  };
+
+  // ---- Ye, Ue, the boundary dots, the decay tables; the first slab's operands ------------------
+  {
+    const int j = tid & 7, r0 = tid >> 3;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int r = r0 + 64 * i;
+      const uint32_t off = umma::swz_off(r, j);
+      const uint4 dyr = *reinterpret_cast<const uint4 *>(tdY + off), ur = *reinterpret_cast<const uint4 *>(tU + off);
+      const uint32_t *w = reinterpret_cast<const uint32_t *>(&dyr), *wu = reinterpret_cast<const uint32_t *>(&ur);
+      const float el = __expf(lp[r]), es = __expf(lp[L - 1] - (r == L - 1 ? lp[0] : lp[r + 1]));
+      float ty[8], tu[8], dot = 0.f;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float2 v = umma::unpack2(w[e], T());
+        float2 u = umma::unpack2(wu[e], T());
+        const float2 m = make_float2(um1[8 * j + 2 * e], um1[8 * j + 2 * e + 1]);
+        if (r == L - 1) u = m;
+        dot = fmaf(v.x, m.x, fmaf(v.y, m.y, dot));
+        ty[2 * e] = el * v.x;
+        ty[2 * e + 1] = el * v.y;
+        tu[2 * e] = es * u.x;
+        tu[2 * e + 1] = es * u.y;
+      }
+      *reinterpret_cast<uint4 *>(tYe + off) = pack8<T>(ty);
+      *reinterpret_cast<uint4 *>(tUe + off) = pack8<T>(tu);
+#pragma unroll
+      for (int o = 4; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
+      if (j == 0) gm1[r] = dot;
+    }
+  }
+  if (tid < L) {
+    e2[tid] = decay_table_entry(lp, tid, L);
+    e3[tid] = __expf(lp[tid] - lp[32 * (tid >> 5)]);
+  }
+  stage(0);
+  helper(0);
+  if (NB > 1) prefetch_zl(1);
+  const bool fast_decay = !__syncthreads_or(tid < L && decay_step_out_of_range(lp, tid));
+  if (NB > 1) prefetch_cb(1);  // every thread has its raw cells of the first slab
+  SLX_STAMP(2);
+
+  // ---- G -> dS' -----------------------------------------------------------------------------
+  wait(2);
+  umma::fence_after_sync();
+  {
+    const float lpt = lp[row];
+    const int c0 = 32 * qc;
+    float v[32];
+    if (qc <= q4) {
+      umma::tmem_ld32(umma::tmem_addr(tmem + kTmSlab, 32 * q4, c0), v);
+      if (qc == q4) {  // the diagonal lives in the block with qc == q4
+        float gdv = 0.f;
+#pragma unroll
+        for (int i = 0; i < 32; ++i)
+          if (i == lane) gdv = v[i];
+        gd[row] = gdv;
+      }
+      if (fast_decay) decay_mask32<true>(v, c0, row, lpt, lp, e2, 0.f);
+      else decay_mask32<false>(v, c0, row, lpt, lp, e2, 0.f);
+    } else {  // block entirely above the diagonal
+#pragma unroll
+      for (int i = 0; i < 32; ++i) v[i] = 0.f;
+    }
+    if (qc == 3) v[31] = __expf(lpt - lp[0]) * gm1[row];  // boundary slot (column 127)
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      *reinterpret_cast<uint4 *>(tdS + 16384 * (qc >> 1) + umma::swz_off(row, 4 * (qc & 1) + k)) = pack8<T>(v + 8 * k);
+  }
+  umma::fence_smem_to_async();
+  umma::fence_before_sync();
+  __syncthreads();
+  if (tid == 0) issue(0);
+  SLX_STAMP(3);
+  const float gd_r = gd[row];
+  const float2 cA_r = cscale(kc_r, gd_r);
+  const float2 cB_r = cscale(cconj(kc_r), gd_r);
+  const float2 cE_r = last_row ? cconj(kc_r) : cconj(gk_r);
+  float2 pgA = make_float2(0.f, 0.f), pP = pgA;
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    cr[k] = cn[k];
+    br[k] = bn[k];
+  }
+  for (int sl = 0; sl < NB; ++sl) {
+    SLX_STAMP(8 + 8 * sl);
+    // u_127 . Lambda of this slab: sum of the 16 per-warp partials (two warps, one column per thread)
+    if (tid >= 32 && tid < 96) {
+      const int dcol = tid - 32;
+      float acc = 0.f;
+#pragma unroll
+      for (int w = 0; w < 16; ++w) acc += ulw[64 * w + dcol];
+      ulf[64 * sl + dcol] = acc;
+    }
+    if (sl + 1 < NB) {
+      stage(sl + 1);
+      SLX_STAMP(9 + 8 * sl);
+      __syncthreads();
+      SLX_STAMP(10 + 8 * sl);
+      if (tid == 0) issue(sl + 1);
+      if (sl + 2 < NB) prefetch_cb(sl + 2);
+      helper(sl + 1);
+      if (sl + 2 < NB) prefetch_zl(sl + 2);
+    } else {
+      __syncthreads();
+    }
+    SLX_STAMP(11 + 8 * sl);
+    wait(sl & 1);
+    umma::fence_after_sync();
+    SLX_STAMP(12 + 8 * sl);
+    // ---- slab epilogue: dC, dB, per-token dots --------------------------------------------------
+    //   dC_t = phi_t dq_t + (k^c_t G_tt) b_t,   dB_s = (conj(k^c_s) G_ss) c_s + conj(gk_s) X_s
+    //   dots: gA += c conj(dC),  P += conj(b) X     (bX = phi_{s+1} P)
+    // Row 127 of X belongs to the token in front of the chunk; token 127 itself has u_127 . Lambda in its place,
+    // with conj(k^c) for conj(gk).
+    unsigned char *buf = tSt + kBwdStage * (sl & 1);
+    const uint32_t acc = tmem + kTmSlab + 128 * (sl & 1);
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      // eight accumulator columns (four complex lanes) of dq and X at a time
+      uint32_t r0[8], r1[8];
+      umma::tmem_ld8_issue(umma::tmem_addr(acc, 32 * q4, 16 * qc + 8 * k), r0);
+      umma::tmem_ld8_issue(umma::tmem_addr(acc, 32 * q4, 64 + 16 * qc + 8 * k), r1);
+      umma::tmem_ld8_wait(r0);
+      umma::tmem_ld8_wait(r1);
+      if (last_row) {
+        float4 *dst = reinterpret_cast<float4 *>(xb + 64 * sl + 16 * qc + 8 * k);
+        const float4 *src = reinterpret_cast<const float4 *>(ulf + 64 * sl + 16 * qc + 8 * k);
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          dst[i] = make_float4(__uint_as_float(r1[4 * i]), __uint_as_float(r1[4 * i + 1]),
+                               __uint_as_float(r1[4 * i + 2]), __uint_as_float(r1[4 * i + 3]));
+          const float4 u = src[i];
+          r1[4 * i] = __float_as_uint(u.x);
+          r1[4 * i + 1] = __float_as_uint(u.y);
+          r1[4 * i + 2] = __float_as_uint(u.z);
+          r1[4 * i + 3] = __float_as_uint(u.w);
+        }
+      }
+      const uint32_t *wb = reinterpret_cast<const uint32_t *>(&br[k]);
+      const uint32_t *wc = reinterpret_cast<const uint32_t *>(&cr[k]);
+      float odc[8], odb[8];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float2 bv = umma::unpack2(wb[e], T()), cv = umma::unpack2(wc[e], T());
+        const float2 dqv = make_float2(__uint_as_float(r0[2 * e]), __uint_as_float(r0[2 * e + 1]));
+        const float2 Xv = make_float2(__uint_as_float(r1[2 * e]), __uint_as_float(r1[2 * e + 1]));
+        const float2 dcv = cadd(cmul(ph_r, dqv), cmul(cA_r, bv));
+        pgA = cadd(pgA, cmulc(cv, dcv));
+        const float2 dbv = cadd(cmul(cB_r, cv), cmul(cE_r, Xv));
+        pP = cadd(pP, cmul(cconj(bv), Xv));
+        odc[2 * e] = dcv.x;
+        odc[2 * e + 1] = dcv.y;
+        odb[2 * e] = dbv.x;
+        odb[2 * e + 1] = dbv.y;
+      }
+      // the results take the place of the slab's (now idle) Qbar / kappa cells and leave from there
+      const uint32_t off = umma::swz_off(row, 2 * qc + k);
+      *reinterpret_cast<uint4 *>(buf + 16384 + off) = pack8<T>(odc);
+      *reinterpret_cast<uint4 *>(buf + off) = pack8<T>(odb);
+    }
+    umma::fence_smem_to_async();  // the dC / dB cells just written leave through the async proxy
+    umma::fence_before_sync();
+    SLX_STAMP(13 + 8 * sl);
+    __syncthreads();
+    SLX_STAMP(14 + 8 * sl);
+    if (tid == 0) {  // one thread sends both tiles (rows past the end of the sequence are clipped by the copy)
+      umma::tma_store_3d(&maps.dC, 64 * sl, t0, bh, sSt + kBwdStage * (sl & 1) + 16384);
+      umma::tma_store_3d(&maps.dB, 64 * sl, t0, bh, sSt + kBwdStage * (sl & 1));
+      umma::tma_store_commit();
+    }
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      cr[k] = cn[k];
+      br[k] = bn[k];
+    }
+  }
+  SLX_STAMP(4);
+
+  // ---- fold the column quarters of the per-token dots (scratch: the idle Lambda' and Z0 tiles) -----
+  float2 *part = reinterpret_cast<float2 *>(tSt + 32768);  // 3 x [4][128]: gA, bX, bc
+  const float2 ph_r1 = last_row ? make_float2(0.f, 0.f) : ph[row + 1];
+  part[128 * qc + row] = pgA;
+  part[512 + 128 * qc + row] = last_row ? pP : cmul(ph_r1, pP);  // row 127: conj(b_127) . (u_127 . Lambda)
+  part[1024 + 128 * qc + row] = acc_bc;
+  __syncthreads();
+  {
+    // every thread needs its row's bc (diagonal of S'^T); the first quarter keeps the sums for the token phase
+    const float2 s2 = cadd(cadd(part[1024 + row], part[1152 + row]), cadd(part[1280 + row], part[1408 + row]));
+    acc_bc = s2;
+    if (qc == 0) {
+      gA[row] = cadd(cadd(part[row], part[128 + row]), cadd(part[256 + row], part[384 + row]));
+      const float2 s1 = cadd(cadd(part[512 + row], part[640 + row]), cadd(part[768 + row], part[896 + row]));
+      bX[row] = s1;
+      if (last_row) misc[0] = s1;
+      bc[row] = s2;
+    }
+  }
+  // Gradient of the token before the chunk: xi_n = phi_0 X_127[n], dB_{-1}[n] = conj(k^p_0) xi_n,
+  // dk^p_0 = sum_n conj(b_{-1}[n]) xi_n
+  float *cB = a.carryB + ((size_t)bh * d.NC + c) * d.D;
+  if (tid >= 256 && tid < 256 + L) {
+    const int n = tid - 256;
+    float2 contrib = make_float2(0.f, 0.f);
+    if (n < d.N) {
+      const float2 xi = cmul(ph[0], make_float2(xb[2 * n], xb[2 * n + 1]));
+      *reinterpret_cast<float2 *>(cB + 2 * n) = cmul(cconj(kp[0]), xi);
+      contrib = cmul(cconj(bm1[n]), xi);
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+      contrib.x += __shfl_xor_sync(0xffffffffu, contrib.x, off);
+      contrib.y += __shfl_xor_sync(0xffffffffu, contrib.y, off);
+    }
+    if (lane == 0) misc[1 + warp - 8] = contrib;
+  }
+  SLX_STAMP(56);
+  // ---- S^T -> S'^T (forward scores; row 127 = boundary) --------------------------------
+  const float dg_r = kc_r.x * acc_bc.x + kc_r.y * acc_bc.y;  // Re(k^c conj(bc))
+  {
+    const int c0 = 32 * qc;
+    float v[32];
+    if (qc >= q4 || q4 == 3) {  // (the last row quarter holds the boundary row, which takes every column)
+      umma::tmem_ld32(umma::tmem_addr(tmem, 32 * q4, c0), v);
+      if (fast_decay) decay_mask32_rows<true>(v, c0, row, last_row, lpb, lp, e3, dg_r);
+      else decay_mask32_rows<false>(v, c0, row, last_row, lpb, lp, e3, dg_r);
+    } else {
+#pragma unroll
+      for (int i = 0; i < 32; ++i) v[i] = 0.f;
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      *reinterpret_cast<uint4 *>(tdS + 16384 * (qc >> 1) + umma::swz_off(row, 4 * (qc & 1) + k)) = pack8<T>(v + 8 * k);
+  }
+  umma::fence_smem_to_async();
+  umma::fence_before_sync();
+  __syncthreads();
+  if (tid == 0) {
+    umma::fence_after_sync();
+    const uint32_t id_km = umma::make_idesc(128, 64, false, true, fmt);
+#pragma unroll
+    for (int kk = 0; kk < 8; ++kk)
+      umma::mma_ss(tmem + kTmU, umma::desc_kmajor(sdS + 16384u * (kk >> 2), kk & 3), umma::desc_mnmajor(sdY, kk, 0),
+                   id_km, kk != 0);
+    umma::commit(gbar);
+  }
+  SLX_STAMP(57);
+  // ---- dK and the per-token terms of dM (overlaps the last product) -----------------------
+  if (tid < L) {
+    const int t = tid;
+    float2 dkc = cscale(bc[t], gd[t]);
+    if (t + 1 < L) dkc = cadd(dkc, cmul(cconj(mraw[t + 1]), bX[t]));
+    else dkc = cadd(dkc, misc[0]);
+    const float2 dkp = (t == 0) ? cadd(cadd(misc[1], misc[2]), cadd(misc[3], misc[4])) : bX[t - 1];
+    if (t < valid) *reinterpret_cast<float4 *>(a.dK + (tok0 + t) * 4) = make_float4(dkp.x, dkp.y, dkc.x, dkc.y);
+    float2 g = csub(gA[t], cadd(cmul(cconj(kc[t]), dkc), cmul(cconj(kp[t]), dkp)));
+    if (t == L - 1) {
+      const float *zd = a.zdot + ((size_t)bh * d.NC + c) * 2;
+      g = cadd(g, make_float2(zd[0], zd[1]));
+    }
+    gsum[t] = g;
+    asm volatile("bar.sync 1, 128;" ::: "memory");  // gsum of the four token warps is complete
+  }
+  // reverse cumulative sum of g over the chunk (warp 0: 4 tokens per lane + shuffle scan)
+  if (warp == 0) {
+    float2 loc[4];
+    float2 run = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int i = 3; i >= 0; --i) {
+      run = cadd(run, gsum[4 * lane + i]);
+      loc[i] = run;
+    }
+    float2 incl = run;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      float ox = __shfl_down_sync(0xffffffffu, incl.x, off), oy = __shfl_down_sync(0xffffffffu, incl.y, off);
+      if (lane + off < 32) incl = cadd(incl, make_float2(ox, oy));
+    }
+    const float2 excl = csub(incl, run);  // sum over the lanes above
+#pragma unroll
+    for (int i = 0; i < 4; ++i) gsum[4 * lane + i] = cadd(loc[i], excl);
+  }
+  // last-row dY (for the diagonal term of dU_127), fetched before the wait
+  float dy_last[16];
+#pragma unroll
+  for (int i = 0; i < 16; ++i) dy_last[i] = 0.f;
+  if (last_row && row < valid) {
+#pragma unroll
+    for (int i = 0; i < 16; ++i) dy_last[i] = to_f(a.dY[(tok0 + row) * P + 16 * qc + i]);
+  }
+  SLX_STAMP(58);
+  wait(2);
+  umma::fence_after_sync();
+  SLX_STAMP(59);
+  // ---- dU = increment path + score path; carry of dU ------------------------------------------
+  {
+    const float es = __expf(lp[L - 1] - lpb);
+    uint32_t r0[16], r1[16];
+    umma::tmem_ld16_issue(umma::tmem_addr(tmem + kTmR, 32 * q4, 16 * qc), r0);
+    umma::tmem_ld16_issue(umma::tmem_addr(tmem + kTmU, 32 * q4, 16 * qc), r1);
+    umma::tmem_ld16_wait(r0);
+    umma::tmem_ld16_wait(r1);
+    float du[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) du[i] = fmaf(es, __uint_as_float(r0[i]), __uint_as_float(r1[i]));
+    if (last_row) {  // the sum belongs to the token in front of the chunk
+      float *cU = a.carryU + ((size_t)bh * d.NC + c) * P + 16 * qc;
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        cU[i] = du[i];
+        du[i] = fmaf(dg_r, dy_last[i], dla[16 * qc + i]);
+      }
+    }
+    if (row < valid) {
+#pragma unroll
+      for (int k = 0; k < 2; ++k)
+        *reinterpret_cast<uint4 *>(a.dU + (tok0 + row) * P + 16 * qc + 8 * k) = pack8<T>(du + 8 * k);
+    }
+  }
+  umma::fence_before_sync();
+  __syncthreads();
+  if (tid < valid) {
+    const float2 m = mraw[tid];
+    const float inv = 1.f / (m.x * m.x + m.y * m.y);
+    *reinterpret_cast<float2 *>(a.dM + (tok0 + tid) * 2) = cscale(cmul(gsum[tid], m), inv);
+  }
+  SLX_STAMP(5);
+  if (tid == 0) umma::tma_store_wait_all();  // the bulk stores of dC / dB have completed
+  if (__syncthreads_or(!ok)) {
+    // a bounded wait ran out: every gradient row of this chunk came from unfinished products or copies;
+    // overwrite them (and the carries) with NaN so that the failure shows in the data as well as in the status word
+    const float nanf_ = __int_as_float(0x7fc00000);
+    const T nanv = from_f<T>(nanf_);
+    for (int e = tid; e < valid * P; e += kTcBwdThreads) a.dU[tok0 * P + e] = nanv;
+    for (int e = tid; e < valid * d.D; e += kTcBwdThreads) {
+      a.dB[tok0 * d.D + e] = nanv;
+      a.dC[tok0 * d.D + e] = nanv;
+    }
+    for (int e = tid; e < valid * 2; e += kTcBwdThreads) a.dM[tok0 * 2 + e] = nanf_;
+    for (int e = tid; e < valid * 4; e += kTcBwdThreads) a.dK[tok0 * 4 + e] = nanf_;
+    for (int e = tid; e < d.D; e += kTcBwdThreads) cB[e] = nanf_;
+    for (int e = tid; e < P; e += kTcBwdThreads) a.carryU[((size_t)bh * d.NC + c) * P + e] = nanf_;
+    if (tid == 0) atomicExch(&g_tc_status, 1);
+  }
+  if (warp == 0) umma::tmem_dealloc(tmem, 512);
 #undef SLX_STAMP
 }
 
