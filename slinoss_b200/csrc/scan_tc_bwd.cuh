@@ -1,7 +1,7 @@
 // Tensor-core per-chunk backward of the v2x2ssd scan (chunk 128, P 64, half
 // inputs, fp32 state).  Same mathematics as chunk_scan_bwd_kernel in
 // scan_simt.cuh; every contraction runs on tcgen05 with fp32 accumulators in
-// tensor memory.  One CTA of 512 threads per (chunk, batch*head), one CTA per SM.
+// tensor memory.  One CTA of 16 worker warps and an issuing warp per (chunk, batch*head), one CTA per SM.
 //
 // Operands per 64-column slab of the state (rotated, half precision):
 //   Qbar_t = c_t conj(phi_t),  kappa_s = gamma_s b_s conj(phi_{s+1}),  Z0,  Lambda' = conj(phi_{L-1}) Lambda
@@ -45,7 +45,7 @@ struct alignas(64) ScanBwdMaps {
   CUtensorMap C, B, dC, dB;
 };
 
-constexpr int kTcBwdThreads = 512;
+constexpr int kTcBwdWorkers = 512, kTcBwdThreads = kTcBwdWorkers + 32;  // the last warp issues products and loads
 constexpr uint32_t kBwdStage = 49152;  // [kappa 16 K][Qbar 16 K][Lambda' 8 K][Z0 8 K], one per slab parity
 constexpr uint32_t kBwdScalars = 81920 + 2 * kBwdStage + 32768;
 constexpr size_t scan_bwd_tc_smem_bytes() { return 1024 + kBwdScalars + 17920; }
@@ -102,6 +102,8 @@ __global__ void __launch_bounds__(kTcBwdThreads, 1) chunk_scan_bwd_tc_kernel(Sca
 
   const ScanDims d = a.d;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const bool issuer = warp == kTcBwdWorkers / 32;
+  auto workers_sync = [] { asm volatile("bar.sync 2, 512;" ::: "memory"); };
   const int c = blockIdx.x, bh = blockIdx.y;
   const int t0 = c * L;
   const int valid = min(L, d.T - t0);
@@ -118,7 +120,7 @@ __global__ void __launch_bounds__(kTcBwdThreads, 1) chunk_scan_bwd_tc_kernel(Sca
   float2 mreg[4];  // the prefix warp's multipliers, requested ahead of the bulk copies
   if (warp == 2) chunk_prefix_load4(a.M + tok0 * 2, valid, mreg);
   // U and dY land in their tiles by asynchronous copy (rows past the chunk end are zero-filled)
-  {
+  if (!issuer) {
     const int j = tid & 7, r0 = tid >> 3;
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
@@ -138,14 +140,12 @@ __global__ void __launch_bounds__(kTcBwdThreads, 1) chunk_scan_bwd_tc_kernel(Sca
   // One raw (C, B) slab = two TMA boxes of [128 tokens][64 columns] into the swizzled staging tiles,
   // issued by one thread; tokens past the end of the sequence arrive as zeros.
   auto prefetch_cb = [&](int sl) {
-    if (tid == 32) {
-      umma::fence_smem_to_async();  // the tiles' earlier (generic) readers are behind a barrier
-      umma::mbar_expect_tx(tbar, 2u * 16384u);
-      umma::tma_load_3d(umma::smem_u32(sC), &maps.C, sl * 64, t0, bh, tbar);
-      umma::tma_load_3d(umma::smem_u32(sB), &maps.B, sl * 64, t0, bh, tbar);
-    }
+    umma::fence_smem_to_async();  // the tiles' earlier (generic) readers are behind a barrier
+    umma::mbar_expect_tx(tbar, 2u * 16384u);
+    umma::tma_load_3d(umma::smem_u32(sC), &maps.C, sl * 64, t0, bh, tbar);
+    umma::tma_load_3d(umma::smem_u32(sB), &maps.B, sl * 64, t0, bh, tbar);
   };
-  if (tid == 32) {
+  if (tid == kTcBwdWorkers) {
 #pragma unroll
     for (int i = 0; i < 4; ++i) umma::mbar_init(bar0 + 8 * i, 1);
     umma::fence_mbar_init();
@@ -153,8 +153,8 @@ __global__ void __launch_bounds__(kTcBwdThreads, 1) chunk_scan_bwd_tc_kernel(Sca
     umma::tma_prefetch_map(&maps.B);
     umma::tma_prefetch_map(&maps.dC);
     umma::tma_prefetch_map(&maps.dB);
+    prefetch_cb(0);
   }
-  prefetch_cb(0);
   // Z0 / Lambda slab: one 8-value (16-byte) item per thread, prefetched into registers
   const int zp = tid >> 3, zj = tid & 7;
   uint4 zr, lr;
@@ -162,9 +162,12 @@ __global__ void __launch_bounds__(kTcBwdThreads, 1) chunk_scan_bwd_tc_kernel(Sca
     zr = *reinterpret_cast<const uint4 *>(z0 + (size_t)zp * d.D + sl * 64 + 8 * zj);
     lr = *reinterpret_cast<const uint4 *>(lam + (size_t)zp * d.D + sl * 64 + 8 * zj);
   };
-  prefetch_zl(0);
+  if (!issuer) prefetch_zl(0);
 
-  if (warp == 0) umma::tmem_alloc(&tmem_slot, 512);
+  if (issuer) {
+    __syncwarp();
+    umma::tmem_alloc(&tmem_slot, 512);
+  }
   if (warp == 2) chunk_prefix_fast128(mreg, lp, ph, mraw, &g_scan_bad);
   if (tid >= 128 && tid < 256) {
     int t = tid - 128;
@@ -204,13 +207,70 @@ __global__ void __launch_bounds__(kTcBwdThreads, 1) chunk_scan_bwd_tc_kernel(Sca
   const uint32_t sdY = umma::smem_u32(tdY), sYe = umma::smem_u32(tYe), sUe = umma::smem_u32(tUe),
                  sdS = umma::smem_u32(tdS), sSt = umma::smem_u32(tSt);
   SLX_STAMP(1);
-  // ---- G = dY U^T (runs while the first slab is staged) --------------------------------------
-  if (tid == 0) {
-    const uint32_t id = umma::make_idesc(128, 128, false, false, fmt), sU = umma::smem_u32(tU);
+  // The products of slab sl, by one thread.  Issuing is slow (the queue in front of the tensor core is short): done by
+  // a worker it held that warp, and with it every barrier, for 3 K cycles a slab; hence a warp of its own.
+  auto issue = [&](int sl) {
+    umma::fence_after_sync();
+    constexpr uint32_t id_sr = umma::make_idesc(128, 192, false, false, fmt);
+    constexpr uint32_t id_km = umma::make_idesc(128, 64, false, true, fmt);
+    constexpr uint32_t id_mm = umma::make_idesc(128, 64, true, true, fmt);
+    const uint32_t sK = sSt + kBwdStage * (sl & 1), sQ = sK + 16384, sLm = sK + 32768, sZ = sK + 40960;
+    const uint32_t dq = tmem + kTmSlab + 128 * (sl & 1), X = dq + 64;
+    const uint64_t dSk = umma::desc_kmajor(sdS, 0), dSm = umma::desc_mnmajor(sdS, 0, 16384u);
+    const uint64_t dKm = umma::desc_mnmajor(sK, 0, 0), dKk = umma::desc_kmajor(sK, 0);
+    const uint64_t dQm = umma::desc_mnmajor(sQ, 0, 0), dQk = umma::desc_kmajor(sQ, 0);
+    const uint64_t dYk = umma::desc_kmajor(sYe, 0), dZm = umma::desc_mnmajor(sZ, 0, 0);
+    const uint64_t dUk = umma::desc_kmajor(sUe, 0), dLm = umma::desc_mnmajor(sLm, 0, 0);
 #pragma unroll
-    for (int kk = 0; kk < 4; ++kk)
-      umma::mma_ss(tmem + kTmSlab, umma::desc_kmajor(sdY, kk), umma::desc_kmajor(sU, kk), id, kk != 0);
-    umma::commit(gbar);
+    for (int kk = 0; kk < 8; ++kk) {
+      umma::mma_ss(dq, umma::desc_advance(dSk, 16384u * (kk >> 2) + umma::kStepK * (kk & 3)),
+                   umma::desc_advance(dKm, umma::kStepMN * kk), id_km, kk != 0);
+      umma::mma_ss(X, umma::desc_advance(dSm, umma::kStepMN * kk), umma::desc_advance(dQm, umma::kStepMN * kk), id_mm,
+                   kk != 0);
+    }
+#pragma unroll
+    for (int kk = 0; kk < 4; ++kk) {
+      umma::mma_ss(dq, umma::desc_advance(dYk, umma::kStepK * kk), umma::desc_advance(dZm, umma::kStepMN * kk), id_km, 1);
+      umma::mma_ss(X, umma::desc_advance(dUk, umma::kStepK * kk), umma::desc_advance(dLm, umma::kStepMN * kk), id_km, 1);
+      umma::mma_ss(tmem, umma::desc_advance(dKk, umma::kStepK * kk), umma::desc_advance(dQk, umma::kStepK * kk), id_sr,
+                   (sl | kk) != 0);
+    }
+    umma::commit(bar0 + 8 * (sl & 1));
+  };
+  if (issuer) {
+    if (lane == 0) {
+      const uint32_t id = umma::make_idesc(128, 128, false, false, fmt), sU = umma::smem_u32(tU);
+#pragma unroll
+      for (int kk = 0; kk < 4; ++kk)  // G = dY U^T, while the first slab is staged
+        umma::mma_ss(tmem + kTmSlab, umma::desc_kmajor(sdY, kk), umma::desc_kmajor(sU, kk), id, kk != 0);
+      umma::commit(gbar);
+    }
+    __syncwarp();
+    __syncthreads_or(0);
+    for (int sl = 0; sl <= NB; ++sl) {
+      // the raw tile of slab sl+1 is free once every worker has its cells of slab sl
+      if (sl == 0 && NB > 1 && lane == 0) prefetch_cb(1);
+      __syncthreads();  // slab sl is staged (sl == NB: u_127 . Lambda of the last slab is complete)
+      if (lane == 0 && sl < NB) {
+        if (sl > 0 && sl + 1 < NB) prefetch_cb(sl + 1);
+        issue(sl);
+      }
+      __syncwarp();
+    }
+    __syncthreads();  // S'^T is complete
+    if (lane == 0) {
+      umma::fence_after_sync();
+      const uint32_t id_km = umma::make_idesc(128, 64, false, true, fmt);
+#pragma unroll
+      for (int kk = 0; kk < 8; ++kk)
+        umma::mma_ss(tmem + kTmU, umma::desc_kmajor(sdS + 16384u * (kk >> 2), kk & 3), umma::desc_mnmajor(sdY, kk, 0),
+                     id_km, kk != 0);
+      umma::commit(gbar);
+    }
+    __syncwarp();
+    __syncthreads();  // every worker has read its accumulators
+    umma::tmem_dealloc(tmem, 512);
+    return;
   }
   const int q4 = warp & 3, qc = warp >> 2;  // lane quarter of tensor memory, column quarter
   const int row = 32 * q4 + lane;
@@ -260,7 +320,7 @@ __global__ void __launch_bounds__(kTcBwdThreads, 1) chunk_scan_bwd_tc_kernel(Sca
     unsigned char *buf = tSt + kBwdStage * (sl & 1);
     if (sl >= 2) {
       if (tid == 0) umma::tma_store_wait_read();
-      __syncthreads();
+      workers_sync();
     }
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
@@ -272,34 +332,6 @@ __global__ void __launch_bounds__(kTcBwdThreads, 1) chunk_scan_bwd_tc_kernel(Sca
     *reinterpret_cast<uint4 *>(buf + 40960 + umma::swz_off(zp, zj)) = zr;
     umma::fence_smem_to_async();
     umma::fence_before_sync();
-  };
-  auto issue = [&](int sl) {  // one thread
-    umma::fence_after_sync();
-    constexpr uint32_t id_sr = umma::make_idesc(128, 192, false, false, fmt);
-    constexpr uint32_t id_km = umma::make_idesc(128, 64, false, true, fmt);
-    constexpr uint32_t id_mm = umma::make_idesc(128, 64, true, true, fmt);
-    const uint32_t sK = sSt + kBwdStage * (sl & 1), sQ = sK + 16384, sLm = sK + 32768, sZ = sK + 40960;
-    const uint32_t dq = tmem + kTmSlab + 128 * (sl & 1), X = dq + 64;
-    const uint64_t dSk = umma::desc_kmajor(sdS, 0), dSm = umma::desc_mnmajor(sdS, 0, 16384u);
-    const uint64_t dKm = umma::desc_mnmajor(sK, 0, 0), dKk = umma::desc_kmajor(sK, 0);
-    const uint64_t dQm = umma::desc_mnmajor(sQ, 0, 0), dQk = umma::desc_kmajor(sQ, 0);
-    const uint64_t dYk = umma::desc_kmajor(sYe, 0), dZm = umma::desc_mnmajor(sZ, 0, 0);
-    const uint64_t dUk = umma::desc_kmajor(sUe, 0), dLm = umma::desc_mnmajor(sLm, 0, 0);
-#pragma unroll
-    for (int kk = 0; kk < 8; ++kk) {
-      umma::mma_ss(dq, umma::desc_advance(dSk, 16384u * (kk >> 2) + umma::kStepK * (kk & 3)),
-                   umma::desc_advance(dKm, umma::kStepMN * kk), id_km, kk != 0);
-      umma::mma_ss(X, umma::desc_advance(dSm, umma::kStepMN * kk), umma::desc_advance(dQm, umma::kStepMN * kk), id_mm,
-                   kk != 0);
-    }
-#pragma unroll
-    for (int kk = 0; kk < 4; ++kk) {
-      umma::mma_ss(dq, umma::desc_advance(dYk, umma::kStepK * kk), umma::desc_advance(dZm, umma::kStepMN * kk), id_km, 1);
-      umma::mma_ss(X, umma::desc_advance(dUk, umma::kStepK * kk), umma::desc_advance(dLm, umma::kStepMN * kk), id_km, 1);
-      umma::mma_ss(tmem, umma::desc_advance(dKk, umma::kStepK * kk), umma::desc_advance(dQk, umma::kStepK * kk), id_sr,
-                   (sl | kk) != 0);
-    }
-    umma::commit(bar0 + 8 * (sl & 1));
   };
   // Token 127's own share of the increment path, from this thread's Lambda values (still in registers): per-warp
   // partials of (u_127 . Lambda)[d] (rows zp of this warp, summed over the 4 lanes that share zj) and
@@ -374,7 +406,6 @@ __global__ void __launch_bounds__(kTcBwdThreads, 1) chunk_scan_bwd_tc_kernel(Sca
   helper(0);
   if (NB > 1) prefetch_zl(1);
   const bool fast_decay = !__syncthreads_or(tid < L && decay_step_out_of_range(lp, tid));
-  if (NB > 1) prefetch_cb(1);  // every thread has its raw cells of the first slab
   SLX_STAMP(2);
 
   // ---- G -> dS' -----------------------------------------------------------------------------
@@ -407,7 +438,6 @@ __global__ void __launch_bounds__(kTcBwdThreads, 1) chunk_scan_bwd_tc_kernel(Sca
   umma::fence_smem_to_async();
   umma::fence_before_sync();
   __syncthreads();
-  if (tid == 0) issue(0);
   SLX_STAMP(3);
   const float gd_r = gd[row];
   const float2 cA_r = cscale(kc_r, gd_r);
@@ -434,8 +464,6 @@ __global__ void __launch_bounds__(kTcBwdThreads, 1) chunk_scan_bwd_tc_kernel(Sca
       SLX_STAMP(9 + 8 * sl);
       __syncthreads();
       SLX_STAMP(10 + 8 * sl);
-      if (tid == 0) issue(sl + 1);
-      if (sl + 2 < NB) prefetch_cb(sl + 2);
       helper(sl + 1);
       if (sl + 2 < NB) prefetch_zl(sl + 2);
     } else {
@@ -499,7 +527,7 @@ __global__ void __launch_bounds__(kTcBwdThreads, 1) chunk_scan_bwd_tc_kernel(Sca
     umma::fence_smem_to_async();  // the dC / dB cells just written leave through the async proxy
     umma::fence_before_sync();
     SLX_STAMP(13 + 8 * sl);
-    __syncthreads();
+    workers_sync();
     SLX_STAMP(14 + 8 * sl);
     if (tid == 0) {  // one thread sends both tiles (rows past the end of the sequence are clipped by the copy)
       umma::tma_store_3d(&maps.dC, 64 * sl, t0, bh, sSt + kBwdStage * (sl & 1) + 16384);
@@ -520,7 +548,7 @@ __global__ void __launch_bounds__(kTcBwdThreads, 1) chunk_scan_bwd_tc_kernel(Sca
   part[128 * qc + row] = pgA;
   part[512 + 128 * qc + row] = last_row ? pP : cmul(ph_r1, pP);  // row 127: conj(b_127) . (u_127 . Lambda)
   part[1024 + 128 * qc + row] = acc_bc;
-  __syncthreads();
+  workers_sync();
   {
     // every thread needs its row's bc (diagonal of S'^T); the first quarter keeps the sums for the token phase
     const float2 s2 = cadd(cadd(part[1024 + row], part[1152 + row]), cadd(part[1280 + row], part[1408 + row]));
@@ -572,15 +600,6 @@ __global__ void __launch_bounds__(kTcBwdThreads, 1) chunk_scan_bwd_tc_kernel(Sca
   umma::fence_smem_to_async();
   umma::fence_before_sync();
   __syncthreads();
-  if (tid == 0) {
-    umma::fence_after_sync();
-    const uint32_t id_km = umma::make_idesc(128, 64, false, true, fmt);
-#pragma unroll
-    for (int kk = 0; kk < 8; ++kk)
-      umma::mma_ss(tmem + kTmU, umma::desc_kmajor(sdS + 16384u * (kk >> 2), kk & 3), umma::desc_mnmajor(sdY, kk, 0),
-                   id_km, kk != 0);
-    umma::commit(gbar);
-  }
   SLX_STAMP(57);
   // ---- dK and the per-token terms of dM (overlaps the last product) -----------------------
   if (tid < L) {
@@ -663,23 +682,28 @@ __global__ void __launch_bounds__(kTcBwdThreads, 1) chunk_scan_bwd_tc_kernel(Sca
   }
   SLX_STAMP(5);
   if (tid == 0) umma::tma_store_wait_all();  // the bulk stores of dC / dB have completed
-  if (__syncthreads_or(!ok)) {
+  int bad;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.s32 p, %1, 0;\n\tbar.red.or.pred q, 2, 512, p;\n\tselp.s32 %0, 1, 0, q;\n\t}"
+      : "=r"(bad)
+      : "r"(ok ? 0 : 1)
+      : "memory");
+  if (bad) {
     // a bounded wait ran out: every gradient row of this chunk came from unfinished products or copies;
     // overwrite them (and the carries) with NaN so that the failure shows in the data as well as in the status word
     const float nanf_ = __int_as_float(0x7fc00000);
     const T nanv = from_f<T>(nanf_);
-    for (int e = tid; e < valid * P; e += kTcBwdThreads) a.dU[tok0 * P + e] = nanv;
-    for (int e = tid; e < valid * d.D; e += kTcBwdThreads) {
+    for (int e = tid; e < valid * P; e += kTcBwdWorkers) a.dU[tok0 * P + e] = nanv;
+    for (int e = tid; e < valid * d.D; e += kTcBwdWorkers) {
       a.dB[tok0 * d.D + e] = nanv;
       a.dC[tok0 * d.D + e] = nanv;
     }
-    for (int e = tid; e < valid * 2; e += kTcBwdThreads) a.dM[tok0 * 2 + e] = nanf_;
-    for (int e = tid; e < valid * 4; e += kTcBwdThreads) a.dK[tok0 * 4 + e] = nanf_;
-    for (int e = tid; e < d.D; e += kTcBwdThreads) cB[e] = nanf_;
-    for (int e = tid; e < P; e += kTcBwdThreads) a.carryU[((size_t)bh * d.NC + c) * P + e] = nanf_;
+    for (int e = tid; e < valid * 2; e += kTcBwdWorkers) a.dM[tok0 * 2 + e] = nanf_;
+    for (int e = tid; e < valid * 4; e += kTcBwdWorkers) a.dK[tok0 * 4 + e] = nanf_;
+    for (int e = tid; e < d.D; e += kTcBwdWorkers) cB[e] = nanf_;
+    for (int e = tid; e < P; e += kTcBwdWorkers) a.carryU[((size_t)bh * d.NC + c) * P + e] = nanf_;
     if (tid == 0) atomicExch(&g_tc_status, 1);
   }
-  if (warp == 0) umma::tmem_dealloc(tmem, 512);
 #undef SLX_STAMP
 }
 
