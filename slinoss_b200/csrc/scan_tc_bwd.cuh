@@ -29,7 +29,7 @@
 // rotations and the epilogue on the CUDA cores, so everything else has to run in their shadow.  Operand tiles and
 // slab accumulators are double-buffered: while the tensor core works on slab i+1, all warps are in the epilogue of
 // slab i and the staging of slab i+2.  The raw (C, B) slab travels by TMA one slab ahead; dC / dB leave by TMA from
-// the operand tiles.  8192 chunks of D 256: 1.245 ms (1.394 with single buffers, where staging, products and epilogue of
+// the operand tiles.  8192 chunks of D 256: 1.094 ms (1.394 with single buffers, where staging, products and epilogue of
 // a slab took turns).
 //
 // Thread mapping: thread = (row 32*(warp%4)+lane, 16-byte chunks 2*(warp/4) and +1 of the slab), the tensor-memory
@@ -96,7 +96,7 @@ __global__ void __launch_bounds__(kTcBwdThreads, 1) chunk_scan_bwd_tc_kernel(Sca
   float2 *mraw = ph + L, *kc = mraw + L, *kp = kc + L, *bc = kp + L, *gsum = bc + L;
   float2 *bm1 = gsum + L;                      // 128  b_{-1}
   float2 *kcb = bm1 + 128;                     // 128  (k^c b)_127
-  float2 *misc = kcb + 128;                    // [0] conj(b_127) . (u_127 . Lambda)   [1..4] dk^p_0, by warp
+  float2 *misc = kcb + 128;                    // [0] conj(b_127) . (u_127 . Lambda)   [1..4] dk^p_0, by warp   [5] zdot
   __shared__ uint64_t bars[4];  // [0], [1] products of a slab, by parity; [2] G, then S'^T dY; [3] raw slab by TMA
   __shared__ uint32_t tmem_slot;
 
@@ -197,6 +197,8 @@ __global__ void __launch_bounds__(kTcBwdThreads, 1) chunk_scan_bwd_tc_kernel(Sca
                 load_pair<T>(a.B + (tok0 + L - 1) * d.D + 2 * n));
     bm1[n] = bv;
     kcb[n] = kb;
+  } else if (tid == 448) {
+    misc[5] = *reinterpret_cast<const float2 *>(a.zdot + ((size_t)bh * d.NC + c) * 2);
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");  // U, dY tiles
   umma::fence_smem_to_async();
@@ -356,16 +358,18 @@ __global__ void __launch_bounds__(kTcBwdThreads, 1) chunk_scan_bwd_tc_kernel(Sca
     for (int e = 0; e < 8; ++e) {
       ds = fmaf(hb[e], tl[e], ds);
       up[e] = uz * tl[e];
-      up[e] += __shfl_xor_sync(0xffffffffu, up[e], 8);
-      up[e] += __shfl_xor_sync(0xffffffffu, up[e], 16);
     }
+    // sums over the four lanes that share zj: the lanes trade halves, so that each ends with two of the eight columns
+    const bool hi8 = lane & 8, hi16 = lane & 16;
+    float w4[4], w2[2];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) w4[e] = (hi8 ? up[4 + e] : up[e]) + __shfl_xor_sync(0xffffffffu, hi8 ? up[e] : up[4 + e], 8);
+#pragma unroll
+    for (int e = 0; e < 2; ++e) w2[e] = (hi16 ? w4[2 + e] : w4[e]) + __shfl_xor_sync(0xffffffffu, hi16 ? w4[e] : w4[2 + e], 16);
 #pragma unroll
     for (int off = 4; off > 0; off >>= 1) ds += __shfl_xor_sync(0xffffffffu, ds, off);
     if (zj == 0) dla[zp] += ds;
-    if (lane < 8) {
-      *reinterpret_cast<float4 *>(ulw + 64 * warp + 8 * lane) = make_float4(up[0], up[1], up[2], up[3]);
-      *reinterpret_cast<float4 *>(ulw + 64 * warp + 8 * lane + 4) = make_float4(up[4], up[5], up[6], up[7]);
-    }
+    *reinterpret_cast<float2 *>(ulw + 64 * warp + 8 * zj + (hi8 ? 4 : 0) + (hi16 ? 2 : 0)) = make_float2(w2[0], w2[1]);
   };
 
   // ---- Ye, Ue, the boundary dots, the decay tables; the first slab's operands ------------------
@@ -510,10 +514,10 @@ __global__ void __launch_bounds__(kTcBwdThreads, 1) chunk_scan_bwd_tc_kernel(Sca
         const float2 bv = umma::unpack2(wb[e], T()), cv = umma::unpack2(wc[e], T());
         const float2 dqv = make_float2(__uint_as_float(r0[2 * e]), __uint_as_float(r0[2 * e + 1]));
         const float2 Xv = make_float2(__uint_as_float(r1[2 * e]), __uint_as_float(r1[2 * e + 1]));
-        const float2 dcv = cadd(cmul(ph_r, dqv), cmul(cA_r, bv));
-        pgA = cadd(pgA, cmulc(cv, dcv));
-        const float2 dbv = cadd(cmul(cB_r, cv), cmul(cE_r, Xv));
-        pP = cadd(pP, cmul(cconj(bv), Xv));
+        const float2 dcv = cmadd(ph_r, dqv, cmul(cA_r, bv));
+        pgA = cmadd(cv, cconj(dcv), pgA);
+        const float2 dbv = cmadd(cE_r, Xv, cmul(cB_r, cv));
+        pP = cmadd(cconj(bv), Xv, pP);
         odc[2 * e] = dcv.x;
         odc[2 * e + 1] = dcv.y;
         odb[2 * e] = dbv.x;
@@ -611,8 +615,7 @@ __global__ void __launch_bounds__(kTcBwdThreads, 1) chunk_scan_bwd_tc_kernel(Sca
     if (t < valid) *reinterpret_cast<float4 *>(a.dK + (tok0 + t) * 4) = make_float4(dkp.x, dkp.y, dkc.x, dkc.y);
     float2 g = csub(gA[t], cadd(cmul(cconj(kc[t]), dkc), cmul(cconj(kp[t]), dkp)));
     if (t == L - 1) {
-      const float *zd = a.zdot + ((size_t)bh * d.NC + c) * 2;
-      g = cadd(g, make_float2(zd[0], zd[1]));
+      g = cadd(g, misc[5]);
     }
     gsum[t] = g;
     asm volatile("bar.sync 1, 128;" ::: "memory");  // gsum of the four token warps is complete
@@ -636,14 +639,6 @@ __global__ void __launch_bounds__(kTcBwdThreads, 1) chunk_scan_bwd_tc_kernel(Sca
 #pragma unroll
     for (int i = 0; i < 4; ++i) gsum[4 * lane + i] = cadd(loc[i], excl);
   }
-  // last-row dY (for the diagonal term of dU_127), fetched before the wait
-  float dy_last[16];
-#pragma unroll
-  for (int i = 0; i < 16; ++i) dy_last[i] = 0.f;
-  if (last_row && row < valid) {
-#pragma unroll
-    for (int i = 0; i < 16; ++i) dy_last[i] = to_f(a.dY[(tok0 + row) * P + 16 * qc + i]);
-  }
   SLX_STAMP(58);
   wait(2);
   umma::fence_after_sync();
@@ -662,9 +657,18 @@ __global__ void __launch_bounds__(kTcBwdThreads, 1) chunk_scan_bwd_tc_kernel(Sca
     if (last_row) {  // the sum belongs to the token in front of the chunk
       float *cU = a.carryU + ((size_t)bh * d.NC + c) * P + 16 * qc;
 #pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        cU[i] = du[i];
-        du[i] = fmaf(dg_r, dy_last[i], dla[16 * qc + i]);
+      for (int k = 0; k < 2; ++k) {
+        const uint4 dyr = *reinterpret_cast<const uint4 *>(tdY + umma::swz_off(L - 1, 2 * qc + k));
+        const uint32_t *w = reinterpret_cast<const uint32_t *>(&dyr);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float2 dyv = umma::unpack2(w[e], T());
+          const int i = 8 * k + 2 * e;
+          cU[i] = du[i];
+          cU[i + 1] = du[i + 1];
+          du[i] = fmaf(dg_r, dyv.x, dla[16 * qc + i]);
+          du[i + 1] = fmaf(dg_r, dyv.y, dla[16 * qc + i + 1]);
+        }
       }
     }
     if (row < valid) {
