@@ -75,16 +75,24 @@ static int set_smem(K kernel, size_t bytes) {
   }
 
 // ---- stage launchers ----------------------------------------------------------
-template <typename T, int L, int MODE>
-static int launch_outer(const ScanDims &d, const void *A, const void *X, const float *M, const float *K,
+template <typename T, int L, int TP, int MODE>
+static int launch_outer_p(const ScanDims &d, const void *A, const void *X, const float *M, const float *K,
                         const PrevRow &pv, float *out, float *m_chunk, cudaStream_t st) {
   OuterArgs<T> a{(const T *)A, (const T *)X, M, K, pv.B, pv.U, pv.dtype, out, m_chunk, d};
-  auto kern = chunk_outer_kernel<T, L, MODE>;
-  size_t smem = outer_smem_bytes<L>();
+  auto kern = chunk_outer_kernel<T, L, TP, MODE>;
+  size_t smem = outer_smem_bytes<L, TP>();
   int rc = set_smem(kern, smem);
   if (rc) return rc;
   kern<<<dim3(d.NC, d.BH), kThreads, smem, st>>>(a);
   return check_launch(MODE == 0 ? "chunk_increment_fwd" : "chunk_scan_bwd_dz0");
+}
+
+// head-dim tiles are 32 or 64 wide
+template <typename T, int L, int MODE>
+static int launch_outer(const ScanDims &d, const void *A, const void *X, const float *M, const float *K,
+                        const PrevRow &pv, float *out, float *m_chunk, cudaStream_t st) {
+  return d.P <= 32 ? launch_outer_p<T, L, 2, MODE>(d, A, X, M, K, pv, out, m_chunk, st)
+                   : launch_outer_p<T, L, 4, MODE>(d, A, X, M, K, pv, out, m_chunk, st);
 }
 
 template <typename T, int L>
@@ -92,8 +100,8 @@ static int launch_scan_fwd(const ScanDims &d, const void *U, const float *M, con
                            const void *C, const float *starts, const PrevRow &pv, void *Y,
                            cudaStream_t st) {
   ScanFwdArgs<T> a{(const T *)U, (const T *)B, (const T *)C, M, K, starts, pv.B, pv.U, pv.dtype, (T *)Y, nullptr, d};
-  auto kern = chunk_scan_fwd_kernel<T, L>;
-  size_t smem = scan_fwd_smem_bytes<L>();
+  auto kern = d.P <= 32 ? chunk_scan_fwd_kernel<T, L, 2> : chunk_scan_fwd_kernel<T, L, 4>;
+  size_t smem = d.P <= 32 ? scan_fwd_smem_bytes<L, 2>() : scan_fwd_smem_bytes<L, 4>();
   int rc = set_smem(kern, smem);
   if (rc) return rc;
   kern<<<dim3(d.NC, d.BH), kThreads, smem, st>>>(a);
@@ -102,8 +110,8 @@ static int launch_scan_fwd(const ScanDims &d, const void *U, const float *M, con
 
 template <typename T, int L>
 static int launch_scan_bwd(const ScanDims &d, const ScanBwdArgs<T> &a, cudaStream_t st) {
-  auto kern = chunk_scan_bwd_kernel<T, L>;
-  size_t smem = scan_bwd_smem_bytes<L>();
+  auto kern = d.P <= 32 ? chunk_scan_bwd_kernel<T, L, 2> : chunk_scan_bwd_kernel<T, L, 4>;
+  size_t smem = d.P <= 32 ? scan_bwd_smem_bytes<L, 2>() : scan_bwd_smem_bytes<L, 4>();
   int rc = set_smem(kern, smem);
   if (rc) return rc;
   kern<<<dim3(d.NC, d.BH), kThreads, smem, st>>>(a);

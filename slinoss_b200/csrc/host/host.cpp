@@ -9,6 +9,7 @@
 // matching shapes and dtypes) and returns None for anything else; the Python function above it then raises the
 // error, or converts the arguments and calls again.
 #include <ATen/ATen.h>
+#include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
@@ -314,6 +315,14 @@ bool scan_inputs_plain(const Tensor &U, const Tensor &M, const Tensor &K, const 
   return true;
 }
 
+// Tiling of the CUDA-core chunk kernels.  Their work per token is least at 64 tokens: at 128 the causal triangle doubles
+// and one CTA fills an SM (2, 8, T 2048, N 64, forward + backward: 466 us against 286), below it the chunk states and
+// the state pass weigh more (32 tokens: 320).  A CTA's time is proportional to its tokens, though, so calls with less
+// than a chunk of 64 per SM are tiled in 32 (1, 2, T 500, N 64: 99 -> 66 us; 1, 8, T 1024: 109 -> 105).
+int64_t cuda_core_chunk(int64_t heads, int64_t T) {
+  return heads * ((T + 63) / 64) < at::cuda::getCurrentDeviceProperties()->multiProcessorCount ? 32 : 64;
+}
+
 // (U, M, K, B, C) -> Y or (Y, final, B_last, U_last) in the activation dtype, with autograd.  None: not the
 // plain case.
 py::object v2x2ssd(const Tensor &U, const Tensor &M, const Tensor &K, const Tensor &B, const Tensor &C, int64_t L,
@@ -322,8 +331,10 @@ py::object v2x2ssd(const Tensor &U, const Tensor &M, const Tensor &K, const Tens
   if (!scan_inputs_plain(U, M, K, B, C, init, Bp, Up)) return py::none();
   const int64_t P = U.size(3), D = B.size(3);
   // chunk_size only says how the sequence is tiled; the tcgen05 kernels tile in 128 tokens
-  if (L > 0 && retile && U.scalar_type() != at::kFloat && P == 64 && D % 64 == 0 && D <= 256) L = 128;
+  const bool tensor_cores = U.scalar_type() != at::kFloat && P == 64 && D % 64 == 0 && D <= 256;
+  if (L > 0 && retile && tensor_cores) L = 128;
   if (L != 16 && L != 32 && L != 64 && L != 128) return py::none();
+  if (retile && !tensor_cores) L = cuda_core_chunk(U.size(0) * U.size(1), U.size(2));
   const at::ScalarType final_type = final_type_in.value_or(U.scalar_type());
   if (code_of(final_type) < 0) return py::none();
   const ScanDims d = scan_dims(U, B, L);

@@ -292,8 +292,9 @@ def v2x2ssd_b200(U, M, K, B, C, *, chunk_size: int, initial_states=None, B_prev=
     ``chunk_size`` only says how the sequence is tiled; none of the returned values depends
     on it beyond rounding.  With ``retile`` (default) half-precision inputs of head dim 64 and
     state width up to 256 are tiled in the 128-token chunks of the tcgen05 kernels whatever
-    ``chunk_size`` asks for (the reference's default is 64); ``retile=False`` keeps the
-    requested tiling (fp32-exact kernels for anything but 128).
+    ``chunk_size`` asks for (the reference's default is 64), and the fp32-exact kernels, which
+    take everything else, in chunks of 64 tokens, or of 32 where 64 would leave SMs idle;
+    ``retile=False`` keeps the requested tiling (fp32-exact kernels for anything but 128).
 
     A transition ``M`` of magnitude exactly 0 makes the reference raise ``ValueError``
     (reference.py:480-485).  The kernels cannot raise: they fill the affected outputs with NaN
