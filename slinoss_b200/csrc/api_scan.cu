@@ -358,7 +358,7 @@ static int launch_state_bwd_t(int BH, int NC, int P, int N, const IT *dZ0, const
   int rc = check_launch("state_passing_bwd");
   if (rc || partials == nullptr) return rc;
   int rows = BH * NC;
-  zdot_reduce_kernel<<<(rows + 255) / 256, 256, 0, st>>>(partials, zdot, rows, nblk * 8);
+  zdot_reduce_kernel<<<(rows + 7) / 8, 256, 0, st>>>(partials, zdot, rows, nblk * 8);
   return check_launch("zdot_reduce");
 }
 // dz0_dtype is fp32 or starts_dtype (checked by the callers)

@@ -297,13 +297,20 @@ __global__ void __launch_bounds__(256) state_passing_bwd_kernel(const IT *dZ0, c
   if (d_initial && live) store_state(d_initial, d_initial_dtype, (size_t)bh * per + iv, g);
 }
 
+// A warp per chunk, lanes over its partials and a butterfly: the order is fixed.  One thread per chunk left the loads to
+// a few warps (512 chunks of 64 partials: 10 us; now 2.3, 8192 chunks: 11 us and 3.8).
 __global__ void zdot_reduce_kernel(const float *__restrict__ partials, float *__restrict__ zdot, int n_rows, int nblk) {
-  int r = blockIdx.x * blockDim.x + threadIdx.x;
+  const int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (r >= n_rows) return;
   const float2 *p = reinterpret_cast<const float2 *>(partials) + (size_t)r * nblk;
   float2 acc = make_float2(0.f, 0.f);
-  for (int b = 0; b < nblk; ++b) acc = cadd(acc, p[b]);
-  reinterpret_cast<float2 *>(zdot)[r] = acc;
+  for (int b = lane; b < nblk; b += 32) acc = cadd(acc, p[b]);
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) {
+    acc.x += __shfl_xor_sync(0xffffffffu, acc.x, off);
+    acc.y += __shfl_xor_sync(0xffffffffu, acc.y, off);
+  }
+  if (lane == 0) reinterpret_cast<float2 *>(zdot)[r] = acc;
 }
 
 // Adds the gradient a chunk sends to the token before it (prev-tap terms of its
