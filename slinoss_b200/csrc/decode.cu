@@ -10,9 +10,19 @@
 //   y[p]            = sum_n Re(conj(c[n]) z'[p][n])
 //   out[p]          = (y[p] + skip[p] u[p]) * silu(gate[p])
 // One CTA per (batch, head).  The fp32 state (P x 2N) is the only large operand: every warp
-// streams whole rows with 16-byte accesses (a row is contiguous), four rows in flight, and
-// reduces its own y[p] by shuffles, so there is no cross-warp reduction and no atomics.
-// The step is bound by HBM: 2 * P * 2N * 4 bytes per (batch, head).
+// streams whole rows with 16-byte accesses (a row is contiguous) and reduces its own y[p] by
+// shuffles, so there is no cross-warp reduction and no atomics.
+// The step is bound by HBM: 2 * P * 2N * 4 bytes per (batch, head).  The CTAs that fit the GPU
+// walk over the heads: eight warps stream states, four others meanwhile prepare the operands of
+// the next head (a serial chain of norms and the coefficient map, as long as the streaming
+// itself) and finish the outputs of the last.  The state comes through shared memory by
+// asynchronous copies, each thread reading back only what it copied itself, and the requests
+// run ahead into the next head, so that the loads never stop.
+// Batch 256, 32 heads, P 64, 2N 256: 238 us (4.5 TB/s) with a CTA per head that loaded four rows per
+// warp at a time after its parameters -> 203 us (5.3 TB/s); 8 heads of 2N 128: 6.4 -> 6.5 us.
+// A CTA per head with all of its state requested first took 311 us: the chain of the parameters
+// was then exposed three CTAs deep.  Three CTAs per SM of three steps each are the optimum of
+// {2, 3, 4} x {2, 3, 4}: fewer CTAs leave the writes uneven, four do not leave the registers.
 #include "common.cuh"
 #include "prep_coef.cuh"
 
@@ -24,131 +34,223 @@ struct DecodeDims {
   int skip_dtype;
 };
 
-constexpr int kDecodeThreads = 256;
-constexpr int kDecodeRowsAhead = 4;
+constexpr int kDecodeWarps = 8;                           // warps that stream the state
+constexpr int kDecodeStream = 32 * kDecodeWarps;
+constexpr int kDecodePrep = 128;                          // threads that prepare the next and finish the last head
+constexpr int kDecodeThreads = kDecodeStream + kDecodePrep;
+constexpr int kDecodeRows = 4;                            // rows of a step, per warp
+constexpr int kDecodeSteps = 3;                           // steps requested ahead
+constexpr int kDecodeRing = 16 * kDecodeSteps * kDecodeRows * kDecodeStream;
+
+__device__ __forceinline__ void cp_async16(void *dst, const void *src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+__device__ __forceinline__ void decode_prep_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kDecodePrep) : "memory"); }
+
+// One head's operands in shared memory, two of them in turn
+struct DecodeBuf {
+  float *c, *kb, *kbp;                // [D] c, k^c b, k^p b_prev
+  float *u, *up, *y, *gate, *skip;    // [P]
+  float2 *rho;                        // [1]
+  float *rstd;                        // [4]
+  __device__ DecodeBuf(float *base, int D, int P) {
+    c = base; kb = c + D; kbp = kb + D;
+    u = kbp + D; up = u + P; y = up + P; gate = y + P; skip = gate + P;
+    rstd = skip + P + P % 2; rho = reinterpret_cast<float2 *>(rstd + 4);
+  }
+};
+__host__ __device__ inline size_t decode_buf_floats(int D, int P) { return ((size_t)3 * D + 5 * P + 7 + 3) / 4 * 4; }
 
 template <typename T>
-__global__ void __launch_bounds__(kDecodeThreads) decode_step_kernel(
+__global__ void __launch_bounds__(kDecodeThreads, 3) decode_step_kernel(
     const T *__restrict__ value, const T *__restrict__ params, const T *__restrict__ bc, const T *__restrict__ gate,
     const void *__restrict__ skip, PrepParams pp, const float *state_in,
     const T *b_prev, const T *u_prev, T *__restrict__ out, float *state_out, T *b_last, T *u_last, DecodeDims d,
     PrepHyper hp) {
-  extern __shared__ float sm[];
-  const int D = 2 * d.N;
-  float *sb = sm;            // [D]  b (interleaved complex), already rounded to T
-  float *sc = sb + D;        // [D]  c
-  float *skb = sc + D;       // [D]  k^c b
-  float *skbp = skb + D;     // [D]  k^p b_prev
-  float *su = skbp + D;      // [P]  u
-  float *sup = su + d.P;     // [P]  u_prev
-  float *sy = sup + d.P;     // [P]  y
-  float *scoef = sy + d.P;   // [6]  rho, k^p, k^c
-  float *srstd = scoef + 8;  // [4]
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int bh = blockIdx.x, h = bh % d.H, b_ = bh / d.H;
-  const T *vrow = value + (size_t)b_ * d.vs + (size_t)h * d.P;
+  extern __shared__ __align__(16) float sm[];
+  const int D = 2 * d.N, n_items = D / 4, n_heads = d.batch * d.H;
+  const int ring_floats = state_in ? kDecodeRing / 4 : 0;
+  const DecodeBuf buf0(sm + ring_floats, D, d.P), buf1(sm + ring_floats + decode_buf_floats(D, d.P), D, d.P);
+  __shared__ float2 coef[3 * 32];  // rho, k^p, k^c of up to 32 of the CTA's heads
+  const int tid = threadIdx.x;
+  const bool streams = tid < kDecodeStream;
+  const int lane = tid & 31, warp = tid >> 5;
 
-  if (tid == 0) {
-    float p[13];
+  // ---- state requests of a streaming thread.  Step = (head, rows ip + 8 r of this warp, item iq of every lane), the
+  // item fastest; they run ahead of the steps that are worked on, into the next head
+  float4 *ring = reinterpret_cast<float4 *>(sm) + tid;  // [steps][rows][threads]
+  int ih = blockIdx.x, ip = kDecodeRows * warp, iq = lane, islot = 0;
+  auto request = [&]() {
+    if (state_in && ih < n_heads && iq < n_items) {
+      const float *zin = state_in + (size_t)ih * d.P * D + 4 * iq;
 #pragma unroll
-    for (int i = 0; i < 13; ++i) p[i] = to_f(params[(size_t)b_ * d.ps + (size_t)h * 13 + i]);
-    add_bias13(pp, h, p);
-    const CoefOut o = coef_forward(p, hp, nullptr);
-    scoef[0] = o.rho.x; scoef[1] = o.rho.y; scoef[2] = o.kp.x; scoef[3] = o.kp.y; scoef[4] = o.kc.x; scoef[5] = o.kc.y;
-  }
-  // rms-norm statistics: warp j < 4 owns plane j of bc
-  const T *bcr = bc + (size_t)b_ * d.bs + (size_t)h * 4 * d.N;
-  if (warp < 4) {
+      for (int r = 0; r < kDecodeRows; ++r) {
+        const int p = ip + r;
+        if (p < d.P) cp_async16(ring + (islot * kDecodeRows + r) * kDecodeStream, zin + (size_t)p * D);
+      }
+    }
+    cp_async_commit();
+    islot = islot + 1 == kDecodeSteps ? 0 : islot + 1;
+    iq += 32;
+    if (iq - lane >= n_items) {
+      iq = lane;
+      ip += kDecodeWarps * kDecodeRows;
+      if (ip - kDecodeRows * warp >= d.P) {
+        ip = kDecodeRows * warp;
+        ih += gridDim.x;
+      }
+    }
+  };
+
+  // ---- operands of one head, by the preparing threads
+  const int t = tid - kDecodeStream;
+  auto prepare = [&](int bh, int k, const DecodeBuf &s) {  // the CTA's k-th
+    // the coefficient map is a long serial chain: a lane per head, for this and the 31 after it (in the last warp, which
+    // has the fewest other loads to wait for)
+    const int ahead = bh + (int)gridDim.x * lane;
+    if ((k & 31) == 0 && t >= kDecodePrep - 32 && ahead < n_heads) {
+      const int h = ahead % d.H, b_ = ahead / d.H;
+      float p[13];
+#pragma unroll
+      for (int i = 0; i < 13; ++i) p[i] = to_f(params[(size_t)b_ * d.ps + (size_t)h * 13 + i]);
+      add_bias13(pp, h, p);
+      const CoefOut o = coef_forward(p, hp, nullptr);
+      coef[3 * lane] = o.rho;
+      coef[3 * lane + 1] = o.kp;
+      coef[3 * lane + 2] = o.kc;
+    }
+    const int h = bh % d.H, b_ = bh / d.H;
+    const T *bcr = bc + (size_t)b_ * d.bs + (size_t)h * 4 * d.N;
+    float raw[4], scl[4];
+    float2 bp = make_float2(0.f, 0.f);
+    auto load_n = [&](int n) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        raw[j] = to_f(bcr[j * d.N + n]);
+        scl[j] = d.normalize ? load_as_f(scale_plane(pp, j), pp.dtype, scale_index(pp, h, j, d.N, n)) : 1.f;
+      }
+      if (b_prev) bp = make_float2(to_f(b_prev[(size_t)bh * D + 2 * n]), to_f(b_prev[(size_t)bh * D + 2 * n + 1]));
+    };
+    if (t < d.N) load_n(t);  // requested before anything is waited for
+    for (int p = t; p < d.P; p += kDecodePrep) {
+      const float u = to_f(value[(size_t)b_ * d.vs + (size_t)h * d.P + p]);
+      s.u[p] = u;
+      s.up[p] = u_prev ? to_f(u_prev[(size_t)bh * d.P + p]) : 0.f;
+      s.gate[p] = to_f(gate[(size_t)b_ * d.gs + (size_t)h * d.P + p]);
+      // skip takes part rounded to the activation dtype, whatever it is stored in
+      s.skip[p] = to_f(from_f<T>(load_as_f(skip, d.skip_dtype, (size_t)h * d.P + p)));
+      if (u_last) u_last[(size_t)bh * d.P + p] = from_f<T>(u);
+    }
+    // rms-norm statistics: warp j owns plane j of bc
     float ss = 0.f;
     for (int n = lane; n < d.N; n += 32) {
-      const float v = to_f(bcr[warp * d.N + n]);
+      const float v = to_f(bcr[(t >> 5) * d.N + n]);
       ss = fmaf(v, v, ss);
     }
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, off);
-    if (lane == 0) srstd[warp] = d.normalize ? rsqrtf(ss / (float)d.N + 1e-5f) : 1.f;
-  }
-  for (int p = tid; p < d.P; p += kDecodeThreads) {
-    su[p] = to_f(vrow[p]);
-    sup[p] = u_prev ? to_f(u_prev[(size_t)bh * d.P + p]) : 0.f;
-  }
-  __syncthreads();
-  const float2 kp = make_float2(scoef[2], scoef[3]), kc = make_float2(scoef[4], scoef[5]);
-  for (int n = tid; n < d.N; n += kDecodeThreads) {
-    float y[4];
+    if (lane == 0) s.rstd[t >> 5] = d.normalize ? rsqrtf(ss / (float)d.N + 1e-5f) : 1.f;
+    decode_prep_sync();
+    const float2 kp = coef[3 * (k & 31) + 1], kc = coef[3 * (k & 31) + 2];
+    if (t == 0) s.rho[0] = coef[3 * (k & 31)];
+    for (int n = t; n < d.N; n += kDecodePrep) {
+      if (n != t) load_n(n);
+      float y[4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      float v = to_f(bcr[j * d.N + n]);
-      if (d.normalize) v = (v * srstd[j]) * load_as_f(scale_plane(pp, j), pp.dtype, scale_index(pp, h, j, d.N, n));
-      y[j] = to_f(from_f<T>(v));  // the reference casts the normalised rows back before the scan
-    }
-    const float2 b = make_float2(y[0], y[1]);
-    float2 bp = make_float2(0.f, 0.f);
-    if (b_prev) bp = make_float2(to_f(b_prev[(size_t)bh * D + 2 * n]), to_f(b_prev[(size_t)bh * D + 2 * n + 1]));
-    const float2 kb = cmul(kc, b), kbp = cmul(kp, bp);
-    sb[2 * n] = b.x; sb[2 * n + 1] = b.y;
-    sc[2 * n] = y[2]; sc[2 * n + 1] = y[3];
-    skb[2 * n] = kb.x; skb[2 * n + 1] = kb.y;
-    skbp[2 * n] = kbp.x; skbp[2 * n + 1] = kbp.y;
-  }
-  __syncthreads();
-
-  // ---- stream the state: warp w owns rows w, w+8, ...; a lane owns the float4 items q = lane + 32 i
-  const float2 m = make_float2(scoef[0], scoef[1]);
-  const int n_items = D / 4;
-  const float *zin = state_in ? state_in + (size_t)bh * d.P * D : nullptr;
-  float *zout = state_out + (size_t)bh * d.P * D;
-  constexpr int NW = kDecodeThreads / 32;
-  for (int p0 = warp; p0 < d.P; p0 += NW * kDecodeRowsAhead) {
-    float acc[kDecodeRowsAhead];
-#pragma unroll
-    for (int r = 0; r < kDecodeRowsAhead; ++r) acc[r] = 0.f;
-    for (int q0 = lane; q0 < n_items; q0 += 32) {
-      float4 z[kDecodeRowsAhead];
-#pragma unroll
-      for (int r = 0; r < kDecodeRowsAhead; ++r) {
-        const int p = p0 + r * NW;
-        z[r] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (p < d.P && zin) z[r] = *reinterpret_cast<const float4 *>(zin + (size_t)p * D + 4 * q0);
+      for (int j = 0; j < 4; ++j) {
+        float v = raw[j];
+        if (d.normalize) v = (v * s.rstd[j]) * scl[j];
+        y[j] = to_f(from_f<T>(v));  // the reference casts the normalised rows back before the scan
       }
-      const float4 vkb = *reinterpret_cast<const float4 *>(skb + 4 * q0);
-      const float4 vkbp = *reinterpret_cast<const float4 *>(skbp + 4 * q0);
-      const float4 vc = *reinterpret_cast<const float4 *>(sc + 4 * q0);
+      const float2 b = make_float2(y[0], y[1]);
+      *reinterpret_cast<float2 *>(s.c + 2 * n) = make_float2(y[2], y[3]);
+      *reinterpret_cast<float2 *>(s.kb + 2 * n) = cmul(kc, b);
+      *reinterpret_cast<float2 *>(s.kbp + 2 * n) = cmul(kp, bp);
+      if (b_last) {
+        b_last[(size_t)bh * D + 2 * n] = from_f<T>(b.x);
+        b_last[(size_t)bh * D + 2 * n + 1] = from_f<T>(b.y);
+      }
+    }
+  };
+  auto finish = [&](int bh, const DecodeBuf &s) {
+    for (int p = t; p < d.P; p += kDecodePrep) {
+      const float g = s.gate[p], y = s.y[p] + s.skip[p] * s.u[p];
+      out[(size_t)bh * d.P + p] = from_f<T>(y * (g / (1.f + expf(-g))));
+    }
+  };
+
+  if (streams) {
 #pragma unroll
-      for (int r = 0; r < kDecodeRowsAhead; ++r) {
-        const int p = p0 + r * NW;
-        if (p < d.P) {
-          const float u = su[p], up = sup[p];
-          float4 o;
-          o.x = fmaf(m.x, z[r].x, fmaf(-m.y, z[r].y, fmaf(up, vkbp.x, u * vkb.x)));
-          o.y = fmaf(m.x, z[r].y, fmaf(m.y, z[r].x, fmaf(up, vkbp.y, u * vkb.y)));
-          o.z = fmaf(m.x, z[r].z, fmaf(-m.y, z[r].w, fmaf(up, vkbp.z, u * vkb.z)));
-          o.w = fmaf(m.x, z[r].w, fmaf(m.y, z[r].z, fmaf(up, vkbp.w, u * vkb.w)));
-          *reinterpret_cast<float4 *>(zout + (size_t)p * D + 4 * q0) = o;
-          acc[r] += fmaf(vc.x, o.x, fmaf(vc.y, o.y, fmaf(vc.z, o.z, vc.w * o.w)));
+    for (int k = 0; k < kDecodeSteps; ++k) request();
+  } else {
+    prepare(blockIdx.x, 0, buf0);
+  }
+  __syncthreads();
+  int slot = 0, it = 0, bh = blockIdx.x;
+  for (; bh < n_heads; bh += gridDim.x, ++it) {
+    const DecodeBuf &s = it & 1 ? buf1 : buf0;
+    if (streams) {
+      // warp w owns rows 4 w .. 4 w + 3 of every 32; a lane owns the float4 items q = lane + 32 i
+      const float2 m = s.rho[0];
+      float *zout = state_out + (size_t)bh * d.P * D;
+      for (int p0 = kDecodeRows * warp; p0 - kDecodeRows * warp < d.P; p0 += kDecodeWarps * kDecodeRows) {
+        float acc[kDecodeRows];
+#pragma unroll
+        for (int r = 0; r < kDecodeRows; ++r) acc[r] = 0.f;
+        for (int q0 = lane; q0 - lane < n_items; q0 += 32) {
+          cp_async_wait<kDecodeSteps - 1>();  // this thread's own copies of the step
+          float4 z[kDecodeRows];
+#pragma unroll
+          for (int r = 0; r < kDecodeRows; ++r)
+            z[r] = state_in ? ring[(slot * kDecodeRows + r) * kDecodeStream] : make_float4(0.f, 0.f, 0.f, 0.f);
+          slot = slot + 1 == kDecodeSteps ? 0 : slot + 1;
+          request();
+          if (q0 >= n_items) continue;
+          const float4 vkb = *reinterpret_cast<const float4 *>(s.kb + 4 * q0);
+          const float4 vkbp = *reinterpret_cast<const float4 *>(s.kbp + 4 * q0);
+          const float4 vc = *reinterpret_cast<const float4 *>(s.c + 4 * q0);
+#pragma unroll
+          for (int r = 0; r < kDecodeRows; ++r) {
+            const int p = p0 + r;
+            if (p < d.P) {
+              const float u = s.u[p], up = s.up[p];
+              float4 o;
+              o.x = fmaf(m.x, z[r].x, fmaf(-m.y, z[r].y, fmaf(up, vkbp.x, u * vkb.x)));
+              o.y = fmaf(m.x, z[r].y, fmaf(m.y, z[r].x, fmaf(up, vkbp.y, u * vkb.y)));
+              o.z = fmaf(m.x, z[r].z, fmaf(-m.y, z[r].w, fmaf(up, vkbp.z, u * vkb.z)));
+              o.w = fmaf(m.x, z[r].w, fmaf(m.y, z[r].z, fmaf(up, vkbp.w, u * vkb.w)));
+              *reinterpret_cast<float4 *>(zout + (size_t)p * D + 4 * q0) = o;
+              acc[r] += fmaf(vc.x, o.x, fmaf(vc.y, o.y, fmaf(vc.z, o.z, vc.w * o.w)));
+            }
+          }
+        }
+#pragma unroll
+        for (int r = 0; r < kDecodeRows; ++r) {
+          float a = acc[r];
+#pragma unroll
+          for (int off = 16; off > 0; off >>= 1) a += __shfl_xor_sync(0xffffffffu, a, off);
+          const int p = p0 + r;
+          if (lane == 0 && p < d.P) s.y[p] = a;
         }
       }
+    } else {
+      const DecodeBuf &o = it & 1 ? buf0 : buf1;
+      if (it > 0) {
+        finish(bh - gridDim.x, o);
+        decode_prep_sync();  // the buffer is free
+      }
+      if (bh + (int)gridDim.x < n_heads) prepare(bh + gridDim.x, it + 1, o);
     }
-#pragma unroll
-    for (int r = 0; r < kDecodeRowsAhead; ++r) {
-      float a = acc[r];
-#pragma unroll
-      for (int off = 16; off > 0; off >>= 1) a += __shfl_xor_sync(0xffffffffu, a, off);
-      const int p = p0 + r * NW;
-      if (lane == 0 && p < d.P) sy[p] = a;
-    }
+    __syncthreads();
   }
-  __syncthreads();
-  for (int p = tid; p < d.P; p += kDecodeThreads) {
-    const float g = to_f(gate[(size_t)b_ * d.gs + (size_t)h * d.P + p]);
-    // skip takes part rounded to the activation dtype, whatever it is stored in
-    const float sk = to_f(from_f<T>(load_as_f(skip, d.skip_dtype, (size_t)h * d.P + p)));
-    const float y = sy[p] + sk * su[p];
-    out[(size_t)bh * d.P + p] = from_f<T>(y * (g / (1.f + expf(-g))));
-    if (u_last) u_last[(size_t)bh * d.P + p] = from_f<T>(su[p]);
-  }
-  if (b_last)
-    for (int i = tid; i < D; i += kDecodeThreads) b_last[(size_t)bh * D + i] = from_f<T>(sb[i]);
+  if (!streams && it > 0) finish(bh - gridDim.x, (it - 1) & 1 ? buf1 : buf0);
+  cp_async_wait<0>();
 }
 
 }  // namespace slx
@@ -184,21 +286,26 @@ static int decode_impl(const slx_decode_shape *s, const void *value, const void 
     if (thr < 1e-4f) thr = 1e-4f;
     hp.z_thr2 = thr * thr;
   }
-  const size_t smem = sizeof(float) * ((size_t)8 * s->N + 3 * (size_t)s->P + 16);
-  SLX_REQUIRE(smem <= 48 * 1024, SLX_E_UNSUPPORTED, "decode_step: N=%d, P=%d need %zu bytes of shared memory",
-              s->N, s->P, smem);
-  const long long ctas = (long long)s->batch * s->heads;
-  SLX_REQUIRE(ctas <= 2147483647LL, SLX_E_UNSUPPORTED, "decode_step: batch*heads too large");
+  const size_t vecs = sizeof(float) * ((size_t)8 * s->N + 3 * (size_t)s->P + 16);
+  SLX_REQUIRE(vecs <= 48 * 1024, SLX_E_UNSUPPORTED, "decode_step: N=%d, P=%d need %zu bytes of shared memory",
+              s->N, s->P, vecs);
+  const size_t smem = (state_in ? kDecodeRing : 0) + 2 * sizeof(float) * decode_buf_floats(2 * s->N, s->P);
+  const long long heads = (long long)s->batch * s->heads;
+  SLX_REQUIRE(heads <= 2147483647LL, SLX_E_UNSUPPORTED, "decode_step: batch*heads too large");
   cudaStream_t st = as_stream(stream);
-#define SLX_DECODE(TT)                                                                                            \
-  decode_step_kernel<TT><<<(unsigned)ctas, kDecodeThreads, smem, st>>>(                                           \
-      (const TT *)value, (const TT *)params, (const TT *)bc, (const TT *)gate, skip, pp, state_in,                \
-      (const TT *)b_prev, (const TT *)u_prev, (TT *)out, state_out, (TT *)b_last, (TT *)u_last, d, hp)
-  if (s->dtype == SLX_F32) SLX_DECODE(float);
-  else if (s->dtype == SLX_BF16) SLX_DECODE(__nv_bfloat16);
-  else SLX_DECODE(__half);
-#undef SLX_DECODE
-  return check_launch("decode_step");
+  auto launch = [&](auto t) {
+    using TT = decltype(t);
+    auto kern = decode_step_kernel<TT>;
+    if (int rc = ensure_dyn_smem(kern, smem)) return rc;
+    const long resident = resident_ctas(kern, kDecodeThreads, smem);
+    const unsigned grid = (unsigned)(resident > 0 && resident < heads ? resident : heads);
+    kern<<<grid, kDecodeThreads, smem, st>>>(
+        (const TT *)value, (const TT *)params, (const TT *)bc, (const TT *)gate, skip, pp, state_in,
+        (const TT *)b_prev, (const TT *)u_prev, (TT *)out, state_out, (TT *)b_last, (TT *)u_last, d, hp);
+    return check_launch("decode_step");
+  };
+  if (s->dtype == SLX_F32) return launch(float());
+  return s->dtype == SLX_BF16 ? launch(__nv_bfloat16()) : launch(__half());
 }
 
 extern "C" int slx_decode_step(const slx_decode_shape *s, const void *value, const void *params, const void *bc,
