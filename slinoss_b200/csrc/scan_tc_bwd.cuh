@@ -3,34 +3,36 @@
 // scan_simt.cuh; every contraction runs on tcgen05 with fp32 accumulators in
 // tensor memory.  One CTA of 16 worker warps and an issuing warp per (chunk, batch*head), one CTA per SM.
 //
-// Operands per 64-column slab of the state (rotated, half precision):
-//   Qbar_t = c_t conj(phi_t),  kappa_s = gamma_s b_s conj(phi_{s+1}),  Z0,  Lambda' = conj(phi_{L-1}) Lambda
-// and per chunk, with es_s = exp(lp_{L-1} - lp_{s+1}):
-//   dS' = decay * (dY U^T),   Ye_t = exp(lp_t) dY_t,   Ue_s = es_s u_s
-// Because p_{L-1}/p_{s+1} = es_s phi_{L-1} conj(phi_{s+1}), the increment path needs no operands of its own:
-//   dB_s   = conj(kappa coefficient) (dS'^T Qbar + Ue Lambda')_s + ...     (one accumulator X for both paths)
-//   dU_s   = es_s (kappa Lambda'^T)_s + (S'^T dY)_s + ...
-// and kappa [Qbar ; Lambda']^T is ONE product of N = 192 that gives S^T and kappa Lambda'^T together.
+// Operands per 64-column slab of the state (half precision, every one rounded once from fp32 or as it is stored):
+//   Qbar_t = c_t conj(phi_t),  kappa_s = gamma_s b_s conj(phi_{s+1}),  Bhat_s = w_s b_s,  Z0,  Lambda
+// with w_s = gamma_s p_{L-1}/p_{s+1} (k^c for the last token), and per chunk
+//   dS' = decay * (dY U^T),   Ye_t = exp(lp_t) dY_t,   U
 //
 // Tensor-memory map (fp32 columns):
-//   [  0,192)  [S^T | R] = kappa [Qbar ; Lambda']^T   (accumulated over the slabs)
-//   [192,448)  two buffers, one per slab parity, of  dq = dS' kappa + Ye Z0  and  X = dS'^T Qbar + Ue Lambda'
-//              (buffer 0 holds G = dY U^T first)
-//   [448,512)  S'^T dY
+//   [  0,128)  S^T = kappa Qbar^T                    (accumulated over the slabs)
+//   [128,192)  dU, increment path:  Bhat Lambda^T    (accumulated over the slabs)
+//   [192,448)  two buffers, one per slab parity, of  dq = dS' kappa + Ye Z0  and  X = dS'^T Qbar
+//              (buffer 0 holds G = dY U^T first, and S'^T dY at the end)
+//   [448,512)  UL = U Lambda of one slab
 //
 // The source token in front of the chunk (b_{-1}, u_{-1}) borrows key slot 127,
 // whose own merged-tap column is empty (no query follows the last token):
-//   dS'[t][127] = exp(lp_t - lp_0) dY_t.u_{-1},  kappa_127 = k^p_0 b_{-1} conj(phi_0),  Ue_127 = exp(lp_{L-1} - lp_0) u_{-1}
-// so that row 127 of X is the whole gradient it receives (times conj(phi_0)), the boundary term of dq comes out of
-// the same product, and row 127 of es R + S'^T dY is the dU carried to the previous token.  Token 127's own share of
-// the increment path, u_127 . Lambda and (k^c b)_127 . Lambda, is summed on the CUDA cores (carry helpers below).
+//   dS'[t][127] = exp(lp_t - lp_0) dY_t.u_{-1},   kappa_127 = k^p_0 b_{-1} conj(phi_0)
+// so that row 127 of X is the column sum the carry gradient needs, the boundary term of dq comes out of the same
+// product, and row 127 of S'^T dY is the dU carried to the previous token.  What that token gets from the increment
+// path, u_{-1} . Lambda and (w_{-1} b_{-1}) . Lambda, is summed on the CUDA cores (carry helpers below).
 //
-// What bounds it: neither HBM (35 %) nor the tensor pipe (a slab's 28 products take about 2 K cycles) but the
-// rotations and the epilogue on the CUDA cores, so everything else has to run in their shadow.  Operand tiles and
-// slab accumulators are double-buffered: while the tensor core works on slab i+1, all warps are in the epilogue of
-// slab i and the staging of slab i+2.  The raw (C, B) slab travels by TMA one slab ahead; dC / dB leave by TMA from
-// the operand tiles.  8192 chunks of D 256: 1.094 ms (1.394 with single buffers, where staging, products and epilogue of
-// a slab took turns).
+// What bounds it: neither HBM (35 %) nor the tensor pipe (a slab's 32 products take about 2 K cycles) but the
+// rotations and the epilogue on the CUDA cores, so everything else has to run in their shadow.  The tiles of kappa,
+// Qbar, Lambda and Z0 and the accumulators dq and X are double-buffered: while the tensor core works on slab i+1, all
+// warps are in the epilogue of slab i and the staging of slab i+2.  Bhat and UL have one buffer, which is what shared
+// and tensor memory still hold: their two products are issued behind the epilogue of the slab before and run under
+// the staging of the next.  dY gives its tile to Ye and is fetched again (from L2) for the last product.  The raw
+// (C, B) slab travels by TMA one slab ahead; dC / dB leave by TMA from the operand tiles.
+// 8192 chunks of D 256: 1.207 ms (1.395 with single buffers, where staging, products and epilogue of a slab took
+// turns).  Scaling the increment path's operands to meet the score path's (X += round(es u) round(conj(phi_{L-1})
+// Lambda), dU from kappa and the same Lambda) needs neither Bhat nor UL and took 1.095 ms, but rounds two operands a
+// second time: with |m| in (0.99, 1) and a large gradient of the final state dK was 2.9 times as far from float64.
 //
 // Thread mapping: thread = (row 32*(warp%4)+lane, 16-byte chunks 2*(warp/4) and +1 of the slab), the tensor-memory
 // lane mapping, for staging and epilogue alike, so that the raw b, c of a cell stay in registers from one to the other.
@@ -46,10 +48,10 @@ struct alignas(64) ScanBwdMaps {
 };
 
 constexpr int kTcBwdWorkers = 512, kTcBwdThreads = kTcBwdWorkers + 32;  // the last warp issues products and loads
-constexpr uint32_t kBwdStage = 49152;  // [kappa 16 K][Qbar 16 K][Lambda' 8 K][Z0 8 K], one per slab parity
+constexpr uint32_t kBwdStage = 49152;  // [kappa 16 K][Qbar 16 K][Lambda 8 K][Z0 8 K], one per slab parity
 constexpr uint32_t kBwdScalars = 81920 + 2 * kBwdStage + 32768;
 constexpr size_t scan_bwd_tc_smem_bytes() { return 1024 + kBwdScalars + 17920; }
-constexpr int kTmR = 128, kTmSlab = 192, kTmU = 448;  // accumulator columns (S^T at 0)
+constexpr int kTmR = 128, kTmSlab = 192, kTmUL = 448, kTmU = kTmSlab;  // accumulator columns (S^T at 0)
 
 // S^T -> S'^T of one 32-column block: row s, columns t = c0 + i.  lpb = lp_{s+1} (lp_0 for the boundary slot, whose
 // row takes every column).  FAST factors exp(lp_t - lpb) through the table e3[t] = exp(lp_t - lp_{32 (t / 32)}).
@@ -72,31 +74,29 @@ __global__ void __launch_bounds__(kTcBwdThreads, 1) chunk_scan_bwd_tc_kernel(Sca
   extern __shared__ unsigned char smem_raw[];
   unsigned char *base =
       reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  unsigned char *tdY = base;                   // [t][p]
-  unsigned char *tYe = base + 16384;           // [t][p]
-  unsigned char *tUe = base + 32768;           // [s][p]
-  unsigned char *tdS = base + 49152;           // 2 x [t][64 s]  dS', at the end 2 x [s][64 t]  S'^T
+  unsigned char *tYe = base;                   // [t][p]  dY until G is done, then Ye
+  unsigned char *tU = base + 16384;            // [s][p]
+  unsigned char *tdS = base + 32768;           // 2 x [t][64 s]  dS', at the end 2 x [s][64 t]  S'^T
+  unsigned char *tBh = base + 65536;           // [s][d]  Bhat
   unsigned char *tSt = base + 81920;           // two staging buffers
-  unsigned char *tU = tSt + kBwdStage;         // [s][p]  U, needed for G only: lies in the second staging buffer
-  unsigned char *sC = tSt + 2 * kBwdStage;     // raw C slab (swizzled tile), by TMA
+  unsigned char *sC = tSt + 2 * kBwdStage;     // raw C slab (swizzled tile), by TMA; dY once more at the end
   unsigned char *sB = sC + 16384;              // raw B slab
   float *lp = reinterpret_cast<float *>(base + kBwdScalars);
   float *gd = lp + L;                          // G[t][t]
   float *gm1 = gd + L;                         // dY_t . u_{-1}
   float *um1 = gm1 + L;                        // 64   u_{-1}
-  float *u127 = um1 + 64;                      // 64   u of the chunk's last token (zero past the end)
-  float *dla = u127 + 64;                      // 64   (k^c b)_127 . Lambda[p]
-  float *e2 = dla + 64;                        // 128  decay table of dS' (decay_mask32)
+  float *duc = um1 + 64;                       // 64   (w_{-1} b_{-1}) . Lambda[p]
+  float *e2 = duc + 64;                        // 128  decay table of dS' (decay_mask32)
   float *e3 = e2 + L;                          // 128  decay table of S'^T
   float *xb = e3 + L;                          // 256  row 127 of X, all slabs
-  float *ulf = xb + 256;                       // 256  u_127 . Lambda, all slabs
-  float *ulw = ulf + 256;                      // [16][64] per-warp partials of u_127 . Lambda
+  float *ulf = xb + 256;                       // 256  u_{-1} . Lambda, all slabs
+  float *ulw = ulf + 256;                      // [16][64] per-warp partials of u_{-1} . Lambda
   float2 *gA = reinterpret_cast<float2 *>(ulw), *bX = gA + L;  // (after the slabs)
   float2 *ph = reinterpret_cast<float2 *>(ulw + 16 * 64);
   float2 *mraw = ph + L, *kc = mraw + L, *kp = kc + L, *bc = kp + L, *gsum = bc + L;
   float2 *bm1 = gsum + L;                      // 128  b_{-1}
-  float2 *kcb = bm1 + 128;                     // 128  (k^c b)_127
-  float2 *misc = kcb + 128;                    // [0] conj(b_127) . (u_127 . Lambda)   [1..4] dk^p_0, by warp   [5] zdot
+  float2 *bh1 = bm1 + 128;                     // 128  w_{-1} b_{-1}
+  float2 *misc = bh1 + 128;                    // [0] conj(b_127) . (u_127 . Lambda)   [1..4] dk^p_0, by warp   [5] zdot
   __shared__ uint64_t bars[4];  // [0], [1] products of a slab, by parity; [2] G, then S'^T dY; [3] raw slab by TMA
   __shared__ uint32_t tmem_slot;
 
@@ -120,21 +120,21 @@ __global__ void __launch_bounds__(kTcBwdThreads, 1) chunk_scan_bwd_tc_kernel(Sca
   float2 mreg[4];  // the prefix warp's multipliers, requested ahead of the bulk copies
   if (warp == 2) chunk_prefix_load4(a.M + tok0 * 2, valid, mreg);
   // U and dY land in their tiles by asynchronous copy (rows past the chunk end are zero-filled)
-  if (!issuer) {
+  auto fetch_rows = [&](unsigned char *tile, const T *src) {
     const int j = tid & 7, r0 = tid >> 3;
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
       const int r = r0 + 64 * i;
       const int rr = r < valid ? r : 0;
       const uint32_t nbytes = r < valid ? 16u : 0u;
-      const uint32_t off = umma::swz_off(r, j);
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(umma::smem_u32(tU + off)),
-                   "l"(a.U + (tok0 + rr) * P + 8 * j), "r"(nbytes)
-                   : "memory");
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(umma::smem_u32(tdY + off)),
-                   "l"(a.dY + (tok0 + rr) * P + 8 * j), "r"(nbytes)
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(umma::smem_u32(tile + umma::swz_off(r, j))),
+                   "l"(src + (tok0 + rr) * P + 8 * j), "r"(nbytes)
                    : "memory");
     }
+  };
+  if (!issuer) {
+    fetch_rows(tU, a.U);
+    fetch_rows(tYe, a.dY);
   }
   asm volatile("cp.async.commit_group;" ::: "memory");
   // One raw (C, B) slab = two TMA boxes of [128 tokens][64 columns] into the swizzled staging tiles,
@@ -185,18 +185,13 @@ __global__ void __launch_bounds__(kTcBwdThreads, 1) chunk_scan_bwd_tc_kernel(Sca
     if (t0 > 0) v = to_f(a.U[(tok0 - 1) * P + p]);
     else if (a.Uprev) v = load_as_f(a.Uprev, a.prev_dtype, (size_t)bh * P + p);
     um1[p] = v;
-    u127[p] = valid == L ? to_f(a.U[(tok0 + L - 1) * P + p]) : 0.f;
-    dla[p] = 0.f;
+    duc[p] = 0.f;
   } else if (tid >= 320 && tid < 320 + d.N) {
     int n = tid - 320;
-    float2 bv = make_float2(0.f, 0.f), kb = bv;
+    float2 bv = make_float2(0.f, 0.f);
     if (t0 > 0) bv = load_pair<T>(a.B + (tok0 - 1) * d.D + 2 * n);
     else if (a.Bprev) bv = load_as_f2(a.Bprev, a.prev_dtype, (size_t)bh * d.D + 2 * n);
-    if (valid == L)
-      kb = cmul(*reinterpret_cast<const float2 *>(a.K + (tok0 + L - 1) * 4 + 2),
-                load_pair<T>(a.B + (tok0 + L - 1) * d.D + 2 * n));
     bm1[n] = bv;
-    kcb[n] = kb;
   } else if (tid == 448) {
     misc[5] = *reinterpret_cast<const float2 *>(a.zdot + ((size_t)bh * d.NC + c) * 2);
   }
@@ -206,23 +201,23 @@ __global__ void __launch_bounds__(kTcBwdThreads, 1) chunk_scan_bwd_tc_kernel(Sca
   __syncthreads();
   umma::fence_after_sync();
   const uint32_t tmem = tmem_slot;
-  const uint32_t sdY = umma::smem_u32(tdY), sYe = umma::smem_u32(tYe), sUe = umma::smem_u32(tUe),
-                 sdS = umma::smem_u32(tdS), sSt = umma::smem_u32(tSt);
+  const uint32_t sYe = umma::smem_u32(tYe), sU = umma::smem_u32(tU), sdS = umma::smem_u32(tdS),
+                 sBh = umma::smem_u32(tBh), sSt = umma::smem_u32(tSt);
   SLX_STAMP(1);
   // The products of slab sl, by one thread.  Issuing is slow (the queue in front of the tensor core is short): done by
   // a worker it held that warp, and with it every barrier, for 3 K cycles a slab; hence a warp of its own.
-  auto issue = [&](int sl) {
+  constexpr uint32_t id_kk = umma::make_idesc(128, 64, false, false, fmt);
+  constexpr uint32_t id_km = umma::make_idesc(128, 64, false, true, fmt);
+  constexpr uint32_t id_mm = umma::make_idesc(128, 64, true, true, fmt);
+  constexpr uint32_t id_sq = umma::make_idesc(128, 128, false, false, fmt);
+  auto issue = [&](int sl) {  // dq, X and S^T: operands and accumulators of the slab's parity
     umma::fence_after_sync();
-    constexpr uint32_t id_sr = umma::make_idesc(128, 192, false, false, fmt);
-    constexpr uint32_t id_km = umma::make_idesc(128, 64, false, true, fmt);
-    constexpr uint32_t id_mm = umma::make_idesc(128, 64, true, true, fmt);
-    const uint32_t sK = sSt + kBwdStage * (sl & 1), sQ = sK + 16384, sLm = sK + 32768, sZ = sK + 40960;
+    const uint32_t sK = sSt + kBwdStage * (sl & 1), sQ = sK + 16384, sZ = sK + 40960;
     const uint32_t dq = tmem + kTmSlab + 128 * (sl & 1), X = dq + 64;
     const uint64_t dSk = umma::desc_kmajor(sdS, 0), dSm = umma::desc_mnmajor(sdS, 0, 16384u);
     const uint64_t dKm = umma::desc_mnmajor(sK, 0, 0), dKk = umma::desc_kmajor(sK, 0);
     const uint64_t dQm = umma::desc_mnmajor(sQ, 0, 0), dQk = umma::desc_kmajor(sQ, 0);
     const uint64_t dYk = umma::desc_kmajor(sYe, 0), dZm = umma::desc_mnmajor(sZ, 0, 0);
-    const uint64_t dUk = umma::desc_kmajor(sUe, 0), dLm = umma::desc_mnmajor(sLm, 0, 0);
 #pragma unroll
     for (int kk = 0; kk < 8; ++kk) {
       umma::mma_ss(dq, umma::desc_advance(dSk, 16384u * (kk >> 2) + umma::kStepK * (kk & 3)),
@@ -233,36 +228,51 @@ __global__ void __launch_bounds__(kTcBwdThreads, 1) chunk_scan_bwd_tc_kernel(Sca
 #pragma unroll
     for (int kk = 0; kk < 4; ++kk) {
       umma::mma_ss(dq, umma::desc_advance(dYk, umma::kStepK * kk), umma::desc_advance(dZm, umma::kStepMN * kk), id_km, 1);
-      umma::mma_ss(X, umma::desc_advance(dUk, umma::kStepK * kk), umma::desc_advance(dLm, umma::kStepMN * kk), id_km, 1);
-      umma::mma_ss(tmem, umma::desc_advance(dKk, umma::kStepK * kk), umma::desc_advance(dQk, umma::kStepK * kk), id_sr,
+      umma::mma_ss(tmem, umma::desc_advance(dKk, umma::kStepK * kk), umma::desc_advance(dQk, umma::kStepK * kk), id_sq,
                    (sl | kk) != 0);
     }
-    umma::commit(bar0 + 8 * (sl & 1));
+  };
+  auto issue_increment = [&](int sl) {  // UL and the dU of the increment path, whose buffers are single
+    umma::fence_after_sync();
+    const uint32_t sLm = sSt + kBwdStage * (sl & 1) + 32768;
+    const uint64_t dUk = umma::desc_kmajor(sU, 0), dBk = umma::desc_kmajor(sBh, 0);
+    const uint64_t dLm = umma::desc_mnmajor(sLm, 0, 0), dLk = umma::desc_kmajor(sLm, 0);
+#pragma unroll
+    for (int kk = 0; kk < 4; ++kk) {
+      umma::mma_ss(tmem + kTmUL, umma::desc_advance(dUk, umma::kStepK * kk), umma::desc_advance(dLm, umma::kStepMN * kk),
+                   id_km, kk != 0);
+      umma::mma_ss(tmem + kTmR, umma::desc_advance(dBk, umma::kStepK * kk), umma::desc_advance(dLk, umma::kStepK * kk),
+                   id_kk, (sl | kk) != 0);
+    }
+    umma::commit(bar0 + 8 * (sl & 1));  // completes with every product of the slab
   };
   if (issuer) {
     if (lane == 0) {
-      const uint32_t id = umma::make_idesc(128, 128, false, false, fmt), sU = umma::smem_u32(tU);
 #pragma unroll
       for (int kk = 0; kk < 4; ++kk)  // G = dY U^T, while the first slab is staged
-        umma::mma_ss(tmem + kTmSlab, umma::desc_kmajor(sdY, kk), umma::desc_kmajor(sU, kk), id, kk != 0);
+        umma::mma_ss(tmem + kTmSlab, umma::desc_kmajor(sYe, kk), umma::desc_kmajor(sU, kk), id_sq, kk != 0);
       umma::commit(gbar);
     }
     __syncwarp();
     __syncthreads_or(0);
-    for (int sl = 0; sl <= NB; ++sl) {
-      // the raw tile of slab sl+1 is free once every worker has its cells of slab sl
-      if (sl == 0 && NB > 1 && lane == 0) prefetch_cb(1);
-      __syncthreads();  // slab sl is staged (sl == NB: u_127 . Lambda of the last slab is complete)
-      if (lane == 0 && sl < NB) {
+    // the raw tile of slab sl+1 is free once every worker has its cells of slab sl
+    if (NB > 1 && lane == 0) prefetch_cb(1);
+    for (int sl = 0; sl < NB; ++sl) {
+      __syncthreads();  // slab sl is staged
+      if (lane == 0) {
         if (sl > 0 && sl + 1 < NB) prefetch_cb(sl + 1);
         issue(sl);
       }
       __syncwarp();
+      if (sl > 0) __syncthreads();  // slab sl-1 has left its accumulators, Bhat of slab sl is staged
+      if (lane == 0) issue_increment(sl);
+      __syncwarp();
     }
-    __syncthreads();  // S'^T is complete
+    __syncthreads();  // the last slab has left its accumulators
+    __syncthreads();  // S'^T and dY are complete
     if (lane == 0) {
       umma::fence_after_sync();
-      const uint32_t id_km = umma::make_idesc(128, 64, false, true, fmt);
+      const uint32_t sdY = umma::smem_u32(sC);
 #pragma unroll
       for (int kk = 0; kk < 8; ++kk)
         umma::mma_ss(tmem + kTmU, umma::desc_kmajor(sdS + 16384u * (kk >> 2), kk & 3), umma::desc_mnmajor(sdY, kk, 0),
@@ -278,11 +288,14 @@ __global__ void __launch_bounds__(kTcBwdThreads, 1) chunk_scan_bwd_tc_kernel(Sca
   const int row = 32 * q4 + lane;
   const bool last_row = row == L - 1;
   const float2 ph_r = ph[row];
-  const float2 phL = ph[L - 1];
   const float2 kc_r = kc[row];
-  // gamma_s conj(phi_{s+1}); the boundary slot: k^p_0 conj(phi_0)
-  const float2 gk_r = last_row ? cmulc(kp[0], ph[0])
-                               : cmulc(cadd(cmul(mraw[row + 1], kc_r), kp[row + 1]), ph[row + 1]);
+  // gamma_s conj(phi_{s+1}), the boundary slot: k^p_0 conj(phi_0);  w_s, the last token: k^c
+  float2 gk_r = cmulc(kp[0], ph[0]), w_r = kc_r;
+  if (!last_row) {
+    const float2 gam = cadd(cmul(mraw[row + 1], kc_r), kp[row + 1]);
+    gk_r = cmulc(gam, ph[row + 1]);
+    w_r = cmul(cscale(cmulc(ph[L - 1], ph[row + 1]), __expf(lp[L - 1] - lp[row + 1])), gam);
+  }
   const float lpb = last_row ? lp[0] : lp[row + 1];
   uint32_t ph_bits = 0;  // phases of the barriers: bit 0, 1 slab products, 2 gbar, 3 tbar
   bool ok = true;
@@ -318,7 +331,6 @@ __global__ void __launch_bounds__(kTcBwdThreads, 1) chunk_scan_bwd_tc_kernel(Sca
       kv[k] = rotate_chunk<T>(src, gk_r);
       cdot_chunk<T>(bn[k], cn[k], acc_bc);
     }
-    const uint4 lv = rotate_chunk<T>(lr, cconj(phL));
     unsigned char *buf = tSt + kBwdStage * (sl & 1);
     if (sl >= 2) {
       if (tid == 0) umma::tma_store_wait_read();
@@ -330,14 +342,20 @@ __global__ void __launch_bounds__(kTcBwdThreads, 1) chunk_scan_bwd_tc_kernel(Sca
       *reinterpret_cast<uint4 *>(buf + off) = kv[k];
       *reinterpret_cast<uint4 *>(buf + 16384 + off) = qv[k];
     }
-    *reinterpret_cast<uint4 *>(buf + 32768 + umma::swz_off(zp, zj)) = lv;
+    *reinterpret_cast<uint4 *>(buf + 32768 + umma::swz_off(zp, zj)) = lr;
     *reinterpret_cast<uint4 *>(buf + 40960 + umma::swz_off(zp, zj)) = zr;
     umma::fence_smem_to_async();
     umma::fence_before_sync();
   };
-  // Token 127's own share of the increment path, from this thread's Lambda values (still in registers): per-warp
-  // partials of (u_127 . Lambda)[d] (rows zp of this warp, summed over the 4 lanes that share zj) and
-  // dla[p] += sum_d kcb[d] Lambda[p][d] (summed over the 8 lanes that share zp).
+  // Bhat of the slab just staged, from the raw cells in registers
+  auto stage_bhat = [&]() {
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+      *reinterpret_cast<uint4 *>(tBh + umma::swz_off(row, 2 * qc + k)) = rotate_chunk<T>(bn[k], w_r);
+  };
+  // The increment path of the token in front of the chunk, from this thread's Lambda values (still in registers):
+  // per-warp partials of (u_{-1} . Lambda)[d] (rows zp of this warp, summed over the 4 lanes that share zj) and
+  // duc[p] += sum_d bh1[d] Lambda[p][d] (summed over the 8 lanes that share zp).
   auto helper = [&](int sl) {
     float tl[8];
     {
@@ -349,10 +367,10 @@ __global__ void __launch_bounds__(kTcBwdThreads, 1) chunk_scan_bwd_tc_kernel(Sca
         tl[2 * e + 1] = v.y;
       }
     }
-    const float4 *kbv = reinterpret_cast<const float4 *>(reinterpret_cast<const float *>(kcb) + 64 * sl + 8 * zj);
+    const float4 *kbv = reinterpret_cast<const float4 *>(reinterpret_cast<const float *>(bh1) + 64 * sl + 8 * zj);
     const float4 h0 = kbv[0], h1 = kbv[1];
     const float hb[8] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
-    const float uz = u127[zp];
+    const float uz = um1[zp];
     float ds = 0.f, up[8];
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
@@ -368,35 +386,24 @@ __global__ void __launch_bounds__(kTcBwdThreads, 1) chunk_scan_bwd_tc_kernel(Sca
     for (int e = 0; e < 2; ++e) w2[e] = (hi16 ? w4[2 + e] : w4[e]) + __shfl_xor_sync(0xffffffffu, hi16 ? w4[e] : w4[2 + e], 16);
 #pragma unroll
     for (int off = 4; off > 0; off >>= 1) ds += __shfl_xor_sync(0xffffffffu, ds, off);
-    if (zj == 0) dla[zp] += ds;
+    if (zj == 0) duc[zp] += ds;
     *reinterpret_cast<float2 *>(ulw + 64 * warp + 8 * zj + (hi8 ? 4 : 0) + (hi16 ? 2 : 0)) = make_float2(w2[0], w2[1]);
   };
 
-  // ---- Ye, Ue, the boundary dots, the decay tables; the first slab's operands ------------------
+  // ---- the boundary dots, the decay tables; the first slab's operands ------------------
   {
     const int j = tid & 7, r0 = tid >> 3;
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
       const int r = r0 + 64 * i;
-      const uint32_t off = umma::swz_off(r, j);
-      const uint4 dyr = *reinterpret_cast<const uint4 *>(tdY + off), ur = *reinterpret_cast<const uint4 *>(tU + off);
-      const uint32_t *w = reinterpret_cast<const uint32_t *>(&dyr), *wu = reinterpret_cast<const uint32_t *>(&ur);
-      const float el = __expf(lp[r]), es = __expf(lp[L - 1] - (r == L - 1 ? lp[0] : lp[r + 1]));
-      float ty[8], tu[8], dot = 0.f;
+      const uint4 dyr = *reinterpret_cast<const uint4 *>(tYe + umma::swz_off(r, j));
+      const uint32_t *w = reinterpret_cast<const uint32_t *>(&dyr);
+      float dot = 0.f;
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         const float2 v = umma::unpack2(w[e], T());
-        float2 u = umma::unpack2(wu[e], T());
-        const float2 m = make_float2(um1[8 * j + 2 * e], um1[8 * j + 2 * e + 1]);
-        if (r == L - 1) u = m;
-        dot = fmaf(v.x, m.x, fmaf(v.y, m.y, dot));
-        ty[2 * e] = el * v.x;
-        ty[2 * e + 1] = el * v.y;
-        tu[2 * e] = es * u.x;
-        tu[2 * e + 1] = es * u.y;
+        dot = fmaf(v.x, um1[8 * j + 2 * e], fmaf(v.y, um1[8 * j + 2 * e + 1], dot));
       }
-      *reinterpret_cast<uint4 *>(tYe + off) = pack8<T>(ty);
-      *reinterpret_cast<uint4 *>(tUe + off) = pack8<T>(tu);
 #pragma unroll
       for (int o = 4; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
       if (j == 0) gm1[r] = dot;
@@ -405,16 +412,40 @@ __global__ void __launch_bounds__(kTcBwdThreads, 1) chunk_scan_bwd_tc_kernel(Sca
   if (tid < L) {
     e2[tid] = decay_table_entry(lp, tid, L);
     e3[tid] = __expf(lp[tid] - lp[32 * (tid >> 5)]);
+  } else if (tid >= 256 && tid < 256 + d.N) {
+    const float2 s0 = cscale(cmulc(ph[L - 1], ph[0]), __expf(lp[L - 1] - lp[0]));  // p_{L-1}/p_0
+    bh1[tid - 256] = cmul(cmul(s0, kp[0]), bm1[tid - 256]);
   }
   stage(0);
+  stage_bhat();
+  umma::fence_smem_to_async();
+  const bool fast_decay = !__syncthreads_or(tid < L && decay_step_out_of_range(lp, tid));
   helper(0);
   if (NB > 1) prefetch_zl(1);
-  const bool fast_decay = !__syncthreads_or(tid < L && decay_step_out_of_range(lp, tid));
   SLX_STAMP(2);
 
-  // ---- G -> dS' -----------------------------------------------------------------------------
+  // ---- G -> dS'; dY -> Ye in its place ----------------------------------------------------------
   wait(2);
   umma::fence_after_sync();
+  {
+    const int j = tid & 7, r0 = tid >> 3;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int r = r0 + 64 * i;
+      uint4 *cell = reinterpret_cast<uint4 *>(tYe + umma::swz_off(r, j));
+      const uint4 dyr = *cell;
+      const uint32_t *w = reinterpret_cast<const uint32_t *>(&dyr);
+      const float el = __expf(lp[r]);
+      float ty[8];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float2 v = umma::unpack2(w[e], T());
+        ty[2 * e] = el * v.x;
+        ty[2 * e + 1] = el * v.y;
+      }
+      *cell = pack8<T>(ty);
+    }
+  }
   {
     const float lpt = lp[row];
     const int c0 = 32 * qc;
@@ -445,9 +476,8 @@ __global__ void __launch_bounds__(kTcBwdThreads, 1) chunk_scan_bwd_tc_kernel(Sca
   SLX_STAMP(3);
   const float gd_r = gd[row];
   const float2 cA_r = cscale(kc_r, gd_r);
-  const float2 cB_r = cscale(cconj(kc_r), gd_r);
-  const float2 cE_r = last_row ? cconj(kc_r) : cconj(gk_r);
-  float2 pgA = make_float2(0.f, 0.f), pP = pgA;
+
+  float2 pgA = make_float2(0.f, 0.f), pX = pgA, pUL = pgA;
 #pragma unroll
   for (int k = 0; k < 2; ++k) {
     cr[k] = cn[k];
@@ -455,7 +485,7 @@ __global__ void __launch_bounds__(kTcBwdThreads, 1) chunk_scan_bwd_tc_kernel(Sca
   }
   for (int sl = 0; sl < NB; ++sl) {
     SLX_STAMP(8 + 8 * sl);
-    // u_127 . Lambda of this slab: sum of the 16 per-warp partials (two warps, one column per thread)
+    // u_{-1} . Lambda of this slab: sum of the 16 per-warp partials (two warps, one column per thread)
     if (tid >= 32 && tid < 96) {
       const int dcol = tid - 32;
       float acc = 0.f;
@@ -471,40 +501,39 @@ __global__ void __launch_bounds__(kTcBwdThreads, 1) chunk_scan_bwd_tc_kernel(Sca
       helper(sl + 1);
       if (sl + 2 < NB) prefetch_zl(sl + 2);
     } else {
-      __syncthreads();
+      // the raw tiles are free: dY comes back for the last product
+      fetch_rows(sC, a.dY);
+      asm volatile("cp.async.commit_group;" ::: "memory");
     }
     SLX_STAMP(11 + 8 * sl);
     wait(sl & 1);
     umma::fence_after_sync();
     SLX_STAMP(12 + 8 * sl);
     // ---- slab epilogue: dC, dB, per-token dots --------------------------------------------------
-    //   dC_t = phi_t dq_t + (k^c_t G_tt) b_t,   dB_s = (conj(k^c_s) G_ss) c_s + conj(gk_s) X_s
-    //   dots: gA += c conj(dC),  P += conj(b) X     (bX = phi_{s+1} P)
-    // Row 127 of X belongs to the token in front of the chunk; token 127 itself has u_127 . Lambda in its place,
-    // with conj(k^c) for conj(gk).
+    //   dC_t = phi_t dq_t + (k^c_t G_tt) b_t,
+    //   dB_s = (conj(k^c_s) G_ss) c_s + conj(gk_s) X_s + conj(w_s) UL_s
+    //   dots: gA += c conj(dC),  conj(b) X,  conj(b) UL
+    // Row 127 of X belongs to the token in front of the chunk; the last token takes no part in X.
     unsigned char *buf = tSt + kBwdStage * (sl & 1);
     const uint32_t acc = tmem + kTmSlab + 128 * (sl & 1);
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
-      // eight accumulator columns (four complex lanes) of dq and X at a time
-      uint32_t r0[8], r1[8];
+      // eight accumulator columns (four complex lanes) of dq, X and UL at a time
+      uint32_t r0[8], r1[8], r2[8];
       umma::tmem_ld8_issue(umma::tmem_addr(acc, 32 * q4, 16 * qc + 8 * k), r0);
       umma::tmem_ld8_issue(umma::tmem_addr(acc, 32 * q4, 64 + 16 * qc + 8 * k), r1);
+      umma::tmem_ld8_issue(umma::tmem_addr(tmem + kTmUL, 32 * q4, 16 * qc + 8 * k), r2);
       umma::tmem_ld8_wait(r0);
       umma::tmem_ld8_wait(r1);
+      umma::tmem_ld8_wait(r2);
       if (last_row) {
         float4 *dst = reinterpret_cast<float4 *>(xb + 64 * sl + 16 * qc + 8 * k);
-        const float4 *src = reinterpret_cast<const float4 *>(ulf + 64 * sl + 16 * qc + 8 * k);
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
+        for (int i = 0; i < 2; ++i)
           dst[i] = make_float4(__uint_as_float(r1[4 * i]), __uint_as_float(r1[4 * i + 1]),
                                __uint_as_float(r1[4 * i + 2]), __uint_as_float(r1[4 * i + 3]));
-          const float4 u = src[i];
-          r1[4 * i] = __float_as_uint(u.x);
-          r1[4 * i + 1] = __float_as_uint(u.y);
-          r1[4 * i + 2] = __float_as_uint(u.z);
-          r1[4 * i + 3] = __float_as_uint(u.w);
-        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) r1[i] = 0;
       }
       const uint32_t *wb = reinterpret_cast<const uint32_t *>(&br[k]);
       const uint32_t *wc = reinterpret_cast<const uint32_t *>(&cr[k]);
@@ -514,10 +543,12 @@ __global__ void __launch_bounds__(kTcBwdThreads, 1) chunk_scan_bwd_tc_kernel(Sca
         const float2 bv = umma::unpack2(wb[e], T()), cv = umma::unpack2(wc[e], T());
         const float2 dqv = make_float2(__uint_as_float(r0[2 * e]), __uint_as_float(r0[2 * e + 1]));
         const float2 Xv = make_float2(__uint_as_float(r1[2 * e]), __uint_as_float(r1[2 * e + 1]));
+        const float2 ULv = make_float2(__uint_as_float(r2[2 * e]), __uint_as_float(r2[2 * e + 1]));
         const float2 dcv = cmadd(ph_r, dqv, cmul(cA_r, bv));
         pgA = cmadd(cv, cconj(dcv), pgA);
-        const float2 dbv = cmadd(cE_r, Xv, cmul(cB_r, cv));
-        pP = cmadd(cconj(bv), Xv, pP);
+        const float2 dbv = cmadd(cconj(gk_r), Xv, cmadd(cconj(w_r), ULv, cmul(cconj(cA_r), cv)));
+        pX = cmadd(cconj(bv), Xv, pX);
+        pUL = cmadd(cconj(bv), ULv, pUL);
         odc[2 * e] = dcv.x;
         odc[2 * e + 1] = dcv.y;
         odb[2 * e] = dbv.x;
@@ -528,10 +559,11 @@ __global__ void __launch_bounds__(kTcBwdThreads, 1) chunk_scan_bwd_tc_kernel(Sca
       *reinterpret_cast<uint4 *>(buf + 16384 + off) = pack8<T>(odc);
       *reinterpret_cast<uint4 *>(buf + off) = pack8<T>(odb);
     }
-    umma::fence_smem_to_async();  // the dC / dB cells just written leave through the async proxy
+    if (sl + 1 < NB) stage_bhat();  // of slab sl+1: the product that read the last one is done
+    umma::fence_smem_to_async();  // Bhat, and the dC / dB cells, which leave through the async proxy
     umma::fence_before_sync();
     SLX_STAMP(13 + 8 * sl);
-    workers_sync();
+    __syncthreads();
     SLX_STAMP(14 + 8 * sl);
     if (tid == 0) {  // one thread sends both tiles (rows past the end of the sequence are clipped by the copy)
       umma::tma_store_3d(&maps.dC, 64 * sl, t0, bh, sSt + kBwdStage * (sl & 1) + 16384);
@@ -546,11 +578,15 @@ __global__ void __launch_bounds__(kTcBwdThreads, 1) chunk_scan_bwd_tc_kernel(Sca
   }
   SLX_STAMP(4);
 
-  // ---- fold the column quarters of the per-token dots (scratch: the idle Lambda' and Z0 tiles) -----
+  // ---- fold the column quarters of the per-token dots (scratch: the idle Lambda and Z0 tiles) -----
   float2 *part = reinterpret_cast<float2 *>(tSt + 32768);  // 3 x [4][128]: gA, bX, bc
-  const float2 ph_r1 = last_row ? make_float2(0.f, 0.f) : ph[row + 1];
   part[128 * qc + row] = pgA;
-  part[512 + 128 * qc + row] = last_row ? pP : cmul(ph_r1, pP);  // row 127: conj(b_127) . (u_127 . Lambda)
+  // conj(b_s) xi_s = phi_{s+1} conj(b) X + conj(p_{L-1}/p_{s+1}) conj(b) UL; row 127: conj(b_127) . (u_127 . Lambda)
+  if (!last_row) {
+    const float2 sg = cscale(cmulc(ph[L - 1], ph[row + 1]), __expf(lp[L - 1] - lp[row + 1]));
+    pUL = cmadd(ph[row + 1], pX, cmul(cconj(sg), pUL));
+  }
+  part[512 + 128 * qc + row] = pUL;
   part[1024 + 128 * qc + row] = acc_bc;
   workers_sync();
   {
@@ -565,14 +601,16 @@ __global__ void __launch_bounds__(kTcBwdThreads, 1) chunk_scan_bwd_tc_kernel(Sca
       bc[row] = s2;
     }
   }
-  // Gradient of the token before the chunk: xi_n = phi_0 X_127[n], dB_{-1}[n] = conj(k^p_0) xi_n,
-  // dk^p_0 = sum_n conj(b_{-1}[n]) xi_n
+  // Gradient of the token before the chunk: xi_n = phi_0 X_127[n] + conj(p_{L-1}/p_0) (u_{-1} . Lambda)[n],
+  // dB_{-1}[n] = conj(k^p_0) xi_n, dk^p_0 = sum_n conj(b_{-1}[n]) xi_n
   float *cB = a.carryB + ((size_t)bh * d.NC + c) * d.D;
   if (tid >= 256 && tid < 256 + L) {
     const int n = tid - 256;
     float2 contrib = make_float2(0.f, 0.f);
     if (n < d.N) {
-      const float2 xi = cmul(ph[0], make_float2(xb[2 * n], xb[2 * n + 1]));
+      const float2 s0 = cscale(cmulc(ph[L - 1], ph[0]), __expf(lp[L - 1] - lp[0]));
+      const float2 xi = cmadd(ph[0], make_float2(xb[2 * n], xb[2 * n + 1]),
+                              cmul(cconj(s0), make_float2(ulf[2 * n], ulf[2 * n + 1])));
       *reinterpret_cast<float2 *>(cB + 2 * n) = cmul(cconj(kp[0]), xi);
       contrib = cmul(cconj(bm1[n]), xi);
     }
@@ -601,6 +639,7 @@ __global__ void __launch_bounds__(kTcBwdThreads, 1) chunk_scan_bwd_tc_kernel(Sca
     for (int k = 0; k < 4; ++k)
       *reinterpret_cast<uint4 *>(tdS + 16384 * (qc >> 1) + umma::swz_off(row, 4 * (qc & 1) + k)) = pack8<T>(v + 8 * k);
   }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");  // dY
   umma::fence_smem_to_async();
   umma::fence_before_sync();
   __syncthreads();
@@ -645,7 +684,6 @@ __global__ void __launch_bounds__(kTcBwdThreads, 1) chunk_scan_bwd_tc_kernel(Sca
   SLX_STAMP(59);
   // ---- dU = increment path + score path; carry of dU ------------------------------------------
   {
-    const float es = __expf(lp[L - 1] - lpb);
     uint32_t r0[16], r1[16];
     umma::tmem_ld16_issue(umma::tmem_addr(tmem + kTmR, 32 * q4, 16 * qc), r0);
     umma::tmem_ld16_issue(umma::tmem_addr(tmem + kTmU, 32 * q4, 16 * qc), r1);
@@ -653,23 +691,26 @@ __global__ void __launch_bounds__(kTcBwdThreads, 1) chunk_scan_bwd_tc_kernel(Sca
     umma::tmem_ld16_wait(r1);
     float du[16];
 #pragma unroll
-    for (int i = 0; i < 16; ++i) du[i] = fmaf(es, __uint_as_float(r0[i]), __uint_as_float(r1[i]));
-    if (last_row) {  // the sum belongs to the token in front of the chunk
+    for (int i = 0; i < 16; ++i) du[i] = __uint_as_float(r0[i]);
+    if (last_row) {  // the score path's sum belongs to the token in front of the chunk
       float *cU = a.carryU + ((size_t)bh * d.NC + c) * P + 16 * qc;
 #pragma unroll
       for (int k = 0; k < 2; ++k) {
-        const uint4 dyr = *reinterpret_cast<const uint4 *>(tdY + umma::swz_off(L - 1, 2 * qc + k));
+        const uint4 dyr = *reinterpret_cast<const uint4 *>(sC + umma::swz_off(L - 1, 2 * qc + k));
         const uint32_t *w = reinterpret_cast<const uint32_t *>(&dyr);
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
           const float2 dyv = umma::unpack2(w[e], T());
           const int i = 8 * k + 2 * e;
-          cU[i] = du[i];
-          cU[i + 1] = du[i + 1];
-          du[i] = fmaf(dg_r, dyv.x, dla[16 * qc + i]);
-          du[i + 1] = fmaf(dg_r, dyv.y, dla[16 * qc + i + 1]);
+          cU[i] = __uint_as_float(r1[i]) + duc[16 * qc + i];
+          cU[i + 1] = __uint_as_float(r1[i + 1]) + duc[16 * qc + i + 1];
+          du[i] = fmaf(dg_r, dyv.x, du[i]);
+          du[i + 1] = fmaf(dg_r, dyv.y, du[i + 1]);
         }
       }
+    } else {
+#pragma unroll
+      for (int i = 0; i < 16; ++i) du[i] += __uint_as_float(r1[i]);
     }
     if (row < valid) {
 #pragma unroll
