@@ -445,7 +445,7 @@ static int chunk_increment_impl(const slx_scan_shape *s, const void *U, const fl
   SLX_REQUIRE(inc_dtype == SLX_F32 || (use_tc(s) && inc_dtype == s->dtype), SLX_E_DTYPE,
               "chunk_increment_fwd: inc_dtype %d must be fp32, or the activation dtype on the tensor-core path",
               inc_dtype);
-  SLX_REQUIRE_ALIGNED("chunk_increment_fwd", U, M, K, B, inc, m_chunk);
+  SLX_REQUIRE_ALIGNED("chunk_increment_fwd", U, M, K, B, pv.B, pv.U, inc, m_chunk);
   SLX_REQUIRE(pv.B == nullptr || pv.dtype == SLX_F32 || pv.dtype == s->dtype, SLX_E_DTYPE,
               "B_prev and U_prev must be fp32 or of the activation dtype");
   SLX_REQUIRE((pv.B == nullptr) == (pv.U == nullptr), SLX_E_NULL, "B_prev and U_prev must be passed together");
@@ -466,7 +466,7 @@ static int chunk_scan_impl(const slx_scan_shape *s, const void *U, const float *
   int rc = check_shape(s, &d);
   if (rc) return rc;
   SLX_REQUIRE(U && M && K && B && C && chunk_starts && Y, SLX_E_NULL, "chunk_scan_fwd: NULL tensor");
-  SLX_REQUIRE_ALIGNED("chunk_scan_fwd", U, M, K, B, C, chunk_starts, Y);
+  SLX_REQUIRE_ALIGNED("chunk_scan_fwd", U, M, K, B, C, chunk_starts, pv.B, pv.U, Y);
   SLX_REQUIRE(pv.B == nullptr || pv.dtype == SLX_F32 || pv.dtype == s->dtype, SLX_E_DTYPE,
               "B_prev and U_prev must be fp32 or of the activation dtype");
   SLX_REQUIRE((pv.B == nullptr) == (pv.U == nullptr), SLX_E_NULL, "B_prev and U_prev must be passed together");
@@ -495,7 +495,8 @@ static int chunk_scan_bwd_impl(const slx_scan_shape *s, const void *U, const flo
   SLX_REQUIRE(U && M && K && B && C && chunk_starts && d_inc && zdot && dY && dU && dM && dK && dB && dC && carryB &&
                   carryU,
               SLX_E_NULL, "chunk_scan_bwd: NULL tensor");
-  SLX_REQUIRE_ALIGNED("chunk_scan_bwd", U, M, K, B, C, chunk_starts, d_inc, dY, dU, dM, dK, dB, dC, carryB, carryU);
+  SLX_REQUIRE_ALIGNED("chunk_scan_bwd", U, M, K, B, C, pv.B, pv.U, chunk_starts, d_inc, dY, dU, dM, dK, dB, dC, carryB,
+                      carryU);
   SLX_REQUIRE(pv.B == nullptr || pv.dtype == SLX_F32 || pv.dtype == s->dtype, SLX_E_DTYPE,
               "B_prev and U_prev must be fp32 or of the activation dtype");
   SLX_REQUIRE((pv.B == nullptr) == (pv.U == nullptr), SLX_E_NULL, "B_prev and U_prev must be passed together");
@@ -723,7 +724,7 @@ static int v2x2ssd_bwd_impl(const slx_scan_shape *s, const void *U, const float 
   if (e == nullptr) e = &none;
   SLX_REQUIRE(U && M && K && B && C && chunk_starts && m_chunk && final_state && dY && dU && dM && dK && dB && dC,
               SLX_E_NULL, "v2x2ssd_bwd: NULL tensor");
-  SLX_REQUIRE_ALIGNED("v2x2ssd_bwd", final_state, e->d_final, e->d_initial);
+  SLX_REQUIRE_ALIGNED("v2x2ssd_bwd", e->B_prev, e->U_prev, final_state, e->d_final, e->d_initial);
   SLX_REQUIRE((e->B_prev == nullptr) == (e->U_prev == nullptr), SLX_E_NULL, "B_prev and U_prev must be passed together");
   const BwdWs w = bwd_ws(d, s->starts_dtype);
   SLX_REQUIRE(workspace != nullptr && workspace_bytes >= w.total, SLX_E_WORKSPACE,

@@ -308,7 +308,7 @@ bool scan_inputs_plain(const Tensor &U, const Tensor &M, const Tensor &K, const 
   if (Bp) {
     const int64_t sb[3] = {b, h, D}, su[3] = {b, h, P};
     if (!is(*Bp, dev) || !is(*Up, dev) || !shaped(*Bp, sb) || !shaped(*Up, su) || !Bp->is_contiguous() ||
-        !Up->is_contiguous() || (Bp->scalar_type() != act && Bp->scalar_type() != at::kFloat) ||
+        !Up->is_contiguous() || !aligned(*Bp) || !aligned(*Up) || (Bp->scalar_type() != act && Bp->scalar_type() != at::kFloat) ||
         Bp->scalar_type() != Up->scalar_type())
       return false;
   }

@@ -353,6 +353,7 @@ def _v2x2ssd_general(U, M, K, B, C, chunk_size, initial_states, B_prev, U_prev, 
         init = _aligned(init if init.dtype in _ACT_DTYPES else init.to(torch.float32))
     if Bp is not None and (Bp.dtype != Up.dtype or Bp.dtype not in (act, torch.float32)):
         Bp, Up = Bp.to(torch.float32), Up.to(torch.float32)
+    Bp, Up = _aligned(Bp), _aligned(Up)
     if not (retile and act != torch.float32 and P == 64 and D % 64 == 0 and D <= 256):
         _shape(b, h, T, P, N, int(chunk_size), act)  # chunk_size is one the kernels tile in
     if strict:
