@@ -394,10 +394,21 @@ py::tuple scan_bwd_parts(const Tensor &U, const Tensor &M, const Tensor &K, cons
 // ------------------------------------------------------------------------------------------------------------
 constexpr int kParamDim = 13;
 
-// (b, T, width) with dense rows equally spaced over (b, T)
-bool dense_rows(const Tensor &x, int64_t width) {
-  return x.dim() >= 3 && x.stride(-1) == 1 && x.stride(1) >= width && (x.size(0) == 1 || x.stride(0) == x.size(1) * x.stride(1));
+// Elements between the rows of a (b, T, ...) tensor whose rows are dense inside and equally spaced over (b, T), or 0.
+// The stride of an axis of one element means nothing (and contiguous() leaves it as it is), so it is not looked at.
+int64_t row_stride(const Tensor &x) {
+  int64_t width = 1;
+  for (int64_t i = x.dim() - 1; i >= 2; --i) {
+    if (x.size(i) != 1 && x.stride(i) != width) return 0;
+    width *= x.size(i);
+  }
+  const int64_t b = x.size(0), T = x.size(1);
+  if (b == 1 && T == 1) return width;
+  const int64_t s = x.stride(T > 1 ? 1 : 0);
+  return s < width || (b > 1 && T > 1 && x.stride(0) != T * s) ? 0 : s;
 }
+// x itself where its rows are like that, else a copy
+Tensor with_rows(const Tensor &x) { return row_stride(x) ? x : x.detach().contiguous(); }
 
 struct PrepConfig {
   int64_t H, N, P;
@@ -453,7 +464,7 @@ slx_prep_params params_struct(const std::vector<Tensor> &p, bool normalize) {
 
 struct PrepBackward : public Node {
   PrepConfig cfg{};
-  int64_t b = 0, T = 0, ps = 0, bs = 0;
+  int64_t b = 0, T = 0;
   std::vector<int64_t> bc_sizes;
   SavedVariable params_, bc_;
   std::vector<SavedVariable> pars_;
@@ -467,7 +478,7 @@ struct PrepBackward : public Node {
   }
   variable_list apply(variable_list &&grads) override {
     std::lock_guard<std::mutex> lock(mutex_);
-    Tensor params = saved(params_), bc = saved(bc_);
+    Tensor params = with_rows(saved(params_)), bc = with_rows(saved(bc_));
     std::vector<Tensor> pars(9);
     const size_t n = cfg.normalize ? 9 : 7;
     for (size_t i = 0; i < n; ++i) pars[i] = saved(pars_[i]);
@@ -486,7 +497,7 @@ struct PrepBackward : public Node {
       d_bs = empty({H, 2, N}, pt, dev);
       d_cs = empty({H, 2, N}, pt, dev);
     }
-    const slx_prep_shape s = prep_shape(cfg, b, T, code_of(act), H * P, ps, bs);
+    const slx_prep_shape s = prep_shape(cfg, b, T, code_of(act), H * P, row_stride(params), row_stride(bc));
     const slx_prep_params pp = params_struct(pars, cfg.normalize);
     const size_t nbytes = slx_scanprep_bwd_workspace_bytes(&s);
     Tensor ws = empty({(int64_t)nbytes}, at::kByte, dev);
@@ -527,16 +538,12 @@ py::object scanprep(const Tensor &value, const Tensor &params, const Tensor &bc,
   if (params.scalar_type() != act || bc.scalar_type() != act || params.device() != dev || bc.device() != dev)
     return py::none();
   if (!prep_params_plain(pars, normalize, dev, H, N)) return py::none();
-  auto rows = [](const Tensor &x, int64_t w) { return dense_rows(x, w) ? x : x.detach().contiguous(); };
-  Tensor v = rows(value, H * P), p = rows(params, H * kParamDim), c = bc;
-  const bool bc_ok = bc.stride(4) == 1 && bc.stride(3) == N && (H == 1 || bc.stride(2) == 4 * N) && bc.stride(1) >= H * 4 * N &&
-                     (b == 1 || bc.stride(0) == T * bc.stride(1));
-  if (!bc_ok) c = bc.detach().contiguous();
+  const Tensor v = with_rows(value), p = with_rows(params), c = with_rows(bc);
   const PrepConfig cfg = prep_config(H, N, P, normalize, hp);
   Tensor U = empty({b, H, T, P}, act, dev), M = empty({b, H, T, 2}, at::kFloat, dev),
          K = empty({b, H, T, 2, 2}, at::kFloat, dev), B = empty({b, H, T, 2 * N}, act, dev),
          C = empty({b, H, T, 2 * N}, act, dev);
-  const slx_prep_shape s = prep_shape(cfg, b, T, code_of(act), v.stride(1), p.stride(1), c.stride(1));
+  const slx_prep_shape s = prep_shape(cfg, b, T, code_of(act), row_stride(v), row_stride(p), row_stride(c));
   const std::vector<Tensor> up = uniform_params(pars, normalize);
   const slx_prep_params pp = params_struct(up, normalize);
   {
@@ -557,8 +564,6 @@ py::object scanprep(const Tensor &value, const Tensor &params, const Tensor &bc,
     node->cfg = cfg;
     node->b = b;
     node->T = T;
-    node->ps = p.stride(1);
-    node->bs = c.stride(1);
     node->bc_sizes.assign(bsz, bsz + 5);
     node->params_ = keep(p);
     node->bc_ = keep(c);
@@ -748,6 +753,25 @@ py::object cconv1d_update(const Tensor &x_in, const Tensor &weight, const OptTen
 // ------------------------------------------------------------------------------------------------------------
 // skip and gate
 // ------------------------------------------------------------------------------------------------------------
+// Strides of the gate over (tokens, batch): it may be a column slice of a wider row, with rows on 16-byte boundaries.
+// As in row_stride, an axis of one element has the stride that a dense tensor would have.
+struct GateRows {
+  int64_t token, batch;
+};
+GateRows gate_rows(const Tensor &g) {
+  GateRows r;
+  r.token = g.size(1) > 1 ? g.stride(1) : g.size(2);
+  r.batch = g.size(0) > 1 ? g.stride(0) : g.size(1) * r.token;
+  return r;
+}
+Tensor with_gate_rows(const Tensor &g) {
+  const GateRows r = gate_rows(g);
+  const bool ok = g.stride(2) == 1 && r.token % 8 == 0 && r.batch % 8 == 0 && r.token >= g.size(2) && aligned(g);
+  if (ok) return g;
+  Tensor c = g.detach().contiguous();
+  return aligned(c) ? c : c.clone();
+}
+
 struct GateBackward : public Node {
   SavedVariable y_, u_, gate_, skip_;
   at::ScalarType u_type, g_type, s_type;
@@ -760,7 +784,7 @@ struct GateBackward : public Node {
   variable_list apply(variable_list &&grads) override {
     std::lock_guard<std::mutex> lock(mutex_);
     if (!grads[0].defined()) return variable_list(4);
-    Tensor y = saved(y_), u = saved(u_), gate = saved(gate_), skip = saved(skip_);
+    Tensor y = saved(y_), u = saved(u_), gate = with_gate_rows(saved(gate_)), skip = saved(skip_);
     const int64_t b = y.size(0), H = y.size(1), T = y.size(2), P = y.size(3);
     const at::ScalarType act = y.scalar_type();
     const at::Device dev = y.device();
@@ -768,7 +792,8 @@ struct GateBackward : public Node {
     const at::ScalarType kt = code_of(s_type) >= 0 ? s_type : at::kFloat;
     Tensor dy = empty(y.sizes(), act, dev), du = empty(y.sizes(), act, dev), dg = empty({b, T, H * P}, act, dev),
            dsk = empty(skip_sizes, kt, dev);
-    const slx_glue_shape s{(int32_t)b, (int32_t)T, (int32_t)H, (int32_t)P, code_of(act), gate.stride(1), gate.stride(0)};
+    const slx_glue_shape s{(int32_t)b, (int32_t)T, (int32_t)H, (int32_t)P, code_of(act), gate_rows(gate).token,
+                           gate_rows(gate).batch};
     const size_t nbytes = slx_gate_skip_bwd_workspace_bytes(&s);
     Tensor ws = empty({(int64_t)nbytes}, at::kByte, dev);
     {
@@ -798,15 +823,13 @@ py::object gate_skip(const Tensor &y_in, const Tensor &u_in, const Tensor &gate_
     return aligned(r) ? r : r.clone();
   };
   const Tensor y = plain(y_in), u = plain(u_in);
-  // the gate may be a column slice of a wider row with 16-byte aligned rows
-  Tensor gate = gate_in.scalar_type() == act ? gate_in : gate_in.detach().to(act);
-  if (gate.stride(2) != 1 || gate.stride(1) % 8 != 0 || gate.stride(0) % 8 != 0 || gate.stride(1) < H * P || !aligned(gate))
-    gate = gate.detach().contiguous();
+  const Tensor gate = with_gate_rows(gate_in.scalar_type() == act ? gate_in : gate_in.detach().to(act));
   Tensor skip = skip_in;
   if (code_of(skip.scalar_type()) < 0) skip = skip.detach().to(at::kFloat);
   if (!skip.is_contiguous()) skip = skip.detach().contiguous();
   Tensor out = empty(gsz, act, dev);
-  const slx_glue_shape s{(int32_t)b, (int32_t)T, (int32_t)H, (int32_t)P, code_of(act), gate.stride(1), gate.stride(0)};
+  const slx_glue_shape s{(int32_t)b, (int32_t)T, (int32_t)H, (int32_t)P, code_of(act), gate_rows(gate).token,
+                         gate_rows(gate).batch};
   {
     c10::cuda::CUDAGuard guard(dev);
     check(slx_gate_skip_fwd_as(&s, ptr(y), ptr(u), ptr(gate), ptr(skip), code_of(skip.scalar_type()), ptr(out),
@@ -849,6 +872,7 @@ PYBIND11_MODULE(_host, m) {
   m.def("scan_fwd_parts", python(&scan_fwd_parts));
   m.def("scan_bwd_parts", python(&scan_bwd_parts));
   m.def("scanprep", python(&scanprep));
+  m.def("row_stride", &row_stride);
   m.def("decode_step", python(&decode_step));
   m.def("cconv1d", python(&cconv1d));
   m.def("cconv1d_update", python(&cconv1d_update));

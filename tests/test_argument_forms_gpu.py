@@ -63,3 +63,54 @@ def test_streaming_rows_at_any_address(dtype, N, T):
     assert torch.equal(out[0], Y) and torch.equal(out[1], fin)
     names = ("dU", "dM", "dK", "dB", "dC", "d_initial", "dB_prev", "dU_prev")
     assert all(torch.equal(a, g[k]) for k, a in zip(names, grads))
+
+
+def _one_token_forms(t):
+    """(b, 1, ...) tensors with the values of ``t`` and other strides: the size-one axis leading in storage, trailing."""
+    lead = t.transpose(0, 1).contiguous().transpose(0, 1)
+    trail = torch.empty((*t.shape[:1], *t.shape[2:], 1), dtype=t.dtype, device=t.device).movedim(-1, 1).copy_(t)
+    wide = torch.empty((t.shape[0], 3, *t.shape[2:]), dtype=t.dtype, device=t.device)[:, 1:2].copy_(t)
+    return lead, trail, wide
+
+
+def test_row_stride_of_one_token():
+    """The distance of the rows that the scan preparation is given (no GPU needed)."""
+    from slinoss_b200 import _lib
+
+    rs = _lib.host().row_stride
+    x = torch.zeros(4, 1, 24)
+    assert [rs(t) for t in (x, *_one_token_forms(x))] == [24, 24, 24, 72]
+    assert rs(x.view(4, 1, 3, 2, 4).transpose(0, 1).contiguous().transpose(0, 1)) == 24
+    assert rs(torch.zeros(1, 1, 24)) == 24 and rs(torch.zeros(1, 24, 1).transpose(1, 2)) == 24
+    assert rs(torch.zeros(2, 5, 30)[..., 3:27]) == 30 and rs(torch.zeros(2, 5, 24)[:, :4]) == 0
+    assert rs(torch.zeros(1, 5, 24)[:, :4]) == 24 and rs(torch.zeros(5, 2, 24).transpose(0, 1)) == 0
+    assert rs(torch.zeros(1, 1, 24).expand(3, 1, 24)) == 0 and rs(torch.zeros(2, 24, 5).transpose(1, 2)) == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [BF16, F32])
+@pytest.mark.parametrize("form", range(3))
+def test_scanprep_and_gate_of_one_token(dtype, form):
+    import slinoss_b200 as sb
+
+    b, H, P, N = 3, 2, 16, 8
+    g = torch.Generator().manual_seed(form)
+    r = lambda *s: torch.randn(*s, generator=g).to(dtype).cuda()
+    hp = dict(n_heads=H, d_state=N, d_head=P, normalize_bc=True, dt_min=1e-4, dt_max=1e-1, r_min=0.9, r_max=1.0,
+              theta_bound=3.0, k_max=0.5, eps=1e-8, b_scale=r(H, 2, N), c_scale=r(H, 2, N),
+              **{k: r(H) for k in ("dt_bias", "gamma_bias", "omega_bias", "mix_r_bias", "mix_theta_bias",
+                                   "mix_k_prev_bias", "mix_k_curr_bias")})
+    args = [r(b, 1, H * P), r(b, 1, H * 13), r(b, 1, H, 4, N)]
+    gate, skip, y, u = r(b, 1, H * P), r(H * P), r(b, H, 1, P), r(b, H, 1, P)
+
+    def both(value, params, bc, gate):
+        leaves = [t.detach().requires_grad_(True) for t in (value, params, bc, gate)]
+        o = sb.scanprep_b200(*leaves[:3], **hp)
+        outs = [o.U, o.M, o.K, o.B, o.C, sb.gate_skip_b200(y, u, leaves[3], skip)]
+        return outs + list(torch.autograd.grad([t.float().square().sum() for t in outs], leaves))
+
+    want = both(*args, gate)
+    for k, t in enumerate([*args, gate]):
+        mixed = [*args, gate]
+        mixed[k] = _one_token_forms(t)[form]
+        assert all(torch.equal(a, w) for a, w in zip(both(*mixed), want)), k
