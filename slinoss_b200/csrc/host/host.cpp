@@ -63,8 +63,8 @@ void *stream_of(const at::Device &dev) { return c10::cuda::getCurrentCUDAStream(
 bool is(const Tensor &t, const at::Device &dev) { return t.defined() && t.device() == dev; }
 bool shaped(const Tensor &t, at::IntArrayRef sizes) { return t.sizes() == sizes; }
 
-// an incoming gradient in the dtype and layout the kernels read
-Tensor grad_in(const Tensor &g, at::ScalarType t) {
+// a tensor in the dtype and layout the kernels read
+Tensor as_read(const Tensor &g, at::ScalarType t) {
   Tensor r = g.scalar_type() == t ? g : g.to(t);
   r = r.contiguous();
   return aligned(r) ? r : r.clone();
@@ -89,7 +89,9 @@ struct ScanDims {
   at::ScalarType act;
 };
 
-ScanDims scan_dims(const Tensor &U, const Tensor &B, int64_t L) {
+// starts_dtype (the code in which chunk starts are held, and with it the kernel family): that of chunk starts in hand, or
+// the library's current choice for the shape.
+ScanDims scan_dims(const Tensor &U, const Tensor &B, int64_t L, std::optional<int> starts_dtype = std::nullopt) {
   ScanDims d;
   d.b = U.size(0);
   d.h = U.size(1);
@@ -102,7 +104,7 @@ ScanDims scan_dims(const Tensor &U, const Tensor &B, int64_t L) {
   d.act = U.scalar_type();
   d.s = slx_scan_shape{(int32_t)(d.b * d.h), (int32_t)d.T, (int32_t)d.P, (int32_t)(d.D / 2), (int32_t)L,
                        code_of(d.act), SLX_F32};
-  d.s.starts_dtype = slx_scan_starts_dtype(&d.s);
+  d.s.starts_dtype = starts_dtype ? *starts_dtype : slx_scan_starts_dtype(&d.s);
   return d;
 }
 
@@ -236,10 +238,10 @@ struct ScanBackward : public Node {
         Up = saved(Up_);
       }
       const ScanDims d = scan_dims(U, B, L);
-      Tensor dY = dY_in.defined() ? grad_in(dY_in, d.act) : at::zeros_like(U);
+      Tensor dY = dY_in.defined() ? as_read(dY_in, d.act) : at::zeros_like(U);
       Tensor d_fin;
       if (d_fin_in.defined())
-        d_fin = grad_in(d_fin_in, code_of(d_fin_in.scalar_type()) < 0 ? at::kFloat : d_fin_in.scalar_type());
+        d_fin = as_read(d_fin_in, code_of(d_fin_in.scalar_type()) < 0 ? at::kFloat : d_fin_in.scalar_type());
       Tensor starts;
       std::optional<at::ScalarType> init_type;
       OptTensor init;
@@ -267,7 +269,8 @@ struct ScanBackward : public Node {
                                      fptr(m2), ptr(inc), stream_of(d.dev)),
               "v2x2ssd chunk starts");
       } else {
-        starts = saved(starts_);
+        // the process may have chosen other kernels since the forward, which hold chunk starts in another dtype
+        starts = as_read(saved(starts_), type_of(d.s.starts_dtype));
       }
       ScanGrads g = scan_backward(d, U, M, K, B, C, Bp, Up, starts, mch, final32, dY, d_fin, init_type, has_prev,
                                   std::nullopt);
@@ -383,7 +386,8 @@ py::tuple scan_bwd_parts(const Tensor &U, const Tensor &M, const Tensor &K, cons
                          bool want_initial, bool want_prev, const OptTensor &workspace) {
   std::optional<at::ScalarType> it;
   if (want_initial) it = at::kFloat;
-  ScanGrads g = scan_backward(scan_dims(U, B, L), U, M, K, B, C, Bp.value_or(Tensor()), Up.value_or(Tensor()), starts,
+  // (the stage entry points convert the chunk starts to the current kernels' dtype first)
+  ScanGrads g = scan_backward(scan_dims(U, B, L, code_of(starts.scalar_type())), U, M, K, B, C, Bp.value_or(Tensor()), Up.value_or(Tensor()), starts,
                               mch, final32, dY, d_final.value_or(Tensor()), it, want_prev && Bp.has_value(), workspace);
   auto opt = [](const Tensor &t) -> py::object { return t.defined() ? py::cast(t) : py::none(); };
   return py::make_tuple(g.dU, g.dM, g.dK, g.dB, g.dC, opt(g.d_init), opt(g.dBp), opt(g.dUp));
@@ -486,7 +490,7 @@ struct PrepBackward : public Node {
     const at::ScalarType act = params.scalar_type(), pt = pars[0].scalar_type();
     const at::Device dev = params.device();
     auto in = [&](size_t i, at::IntArrayRef sizes, at::ScalarType t) {
-      return grads[i].defined() ? grad_in(grads[i], t) : at::zeros(sizes, at::TensorOptions().dtype(t).device(dev));
+      return grads[i].defined() ? as_read(grads[i], t) : at::zeros(sizes, at::TensorOptions().dtype(t).device(dev));
     };
     const int64_t H = cfg.H, N = cfg.N, P = cfg.P;
     Tensor dU = in(0, {b, H, T, P}, act), dM = in(1, {b, H, T, 2}, at::kFloat), dK = in(2, {b, H, T, 2, 2}, at::kFloat),
@@ -661,7 +665,7 @@ struct ConvBackward : public Node {
     if (has_bias) bias = as_type(saved(bias_), act);
     if (has_state) state = as_type(saved(state_), act);
     const int64_t b = x.size(0), T = x.size(1), C = x.size(2), W = w.size(1);
-    Tensor dy = grads[0].defined() ? grad_in(grads[0], act)
+    Tensor dy = grads[0].defined() ? as_read(grads[0], act)
                                    : at::zeros({b, T, C}, at::TensorOptions().dtype(act).device(dev));
     Tensor dn;
     if (grads[1].defined()) dn = as_type(grads[1], act);
@@ -788,7 +792,7 @@ struct GateBackward : public Node {
     const int64_t b = y.size(0), H = y.size(1), T = y.size(2), P = y.size(3);
     const at::ScalarType act = y.scalar_type();
     const at::Device dev = y.device();
-    Tensor go = grad_in(grads[0], act);
+    Tensor go = as_read(grads[0], act);
     const at::ScalarType kt = code_of(s_type) >= 0 ? s_type : at::kFloat;
     Tensor dy = empty(y.sizes(), act, dev), du = empty(y.sizes(), act, dev), dg = empty({b, T, H * P}, act, dev),
            dsk = empty(skip_sizes, kt, dev);

@@ -114,3 +114,28 @@ def test_scanprep_and_gate_of_one_token(dtype, form):
         mixed = [*args, gate]
         mixed[k] = _one_token_forms(t)[form]
         assert all(torch.equal(a, w) for a, w in zip(both(*mixed), want)), k
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("before,after", [(1, 0), (0, 1), (2, 0), (1, 2)])
+def test_kernel_family_chosen_between_forward_and_backward(before, after):
+    """Chunk starts are held in the dtype of the family that wrote them: the backward runs on the family chosen by then."""
+    import slinoss_b200 as sb
+    from slinoss_b200 import _lib
+
+    inp = make_scan_inputs(1, 2, 300, 32, 64, BF16, seed=1, with_init=True)
+    names = ("U", "M", "K", "B", "C", "initial_states")
+
+    def grads(forward, backward):
+        old = _lib.set_tensor_path(forward)
+        try:
+            leaves = [inp[k].detach().requires_grad_(True) for k in names]
+            Y = sb.v2x2ssd_b200(*leaves[:5], chunk_size=128, initial_states=leaves[5])
+            _lib.set_tensor_path(backward)
+            return torch.autograd.grad(Y, leaves, inp["dY"])
+        finally:
+            _lib.set_tensor_path(old)
+
+    for k, a, b in zip(names, grads(before, after), grads(after, after)):
+        # the families' chunk starts differ by their storage, half against fp32: 2^-9 of a value
+        assert (a.float() - b.float()).norm() < 4e-3 * b.float().norm(), k
