@@ -7,12 +7,14 @@
 //
 // Every entry point takes the form in which programs normally call the op (one device, contiguous, 16-byte aligned,
 // matching shapes and dtypes) and returns None for anything else; the Python function above it then raises the
-// error, or converts the arguments and calls again.
+// error, or converts the arguments and calls again.  The interpreter lock is not held meanwhile: an allocation or a full
+// launch queue may wait for the GPU, and what it waits for may be another thread's to launch.
 #include <ATen/ATen.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/function.h>
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/saved_variable.h>
@@ -24,7 +26,6 @@
 
 #include "../../../include/slinoss_b200.h"
 
-namespace py = pybind11;
 using at::Tensor;
 using torch::autograd::Node;
 using torch::autograd::SavedVariable;
@@ -326,20 +327,20 @@ int64_t cuda_core_chunk(int64_t heads, int64_t T) {
   return heads * ((T + 63) / 64) < at::cuda::getCurrentDeviceProperties()->multiProcessorCount ? 32 : 64;
 }
 
-// (U, M, K, B, C) -> Y or (Y, final, B_last, U_last) in the activation dtype, with autograd.  None: not the
+// (U, M, K, B, C) -> [Y] or [Y, final, B_last, U_last] in the activation dtype, with autograd.  None: not the
 // plain case.
-py::object v2x2ssd(const Tensor &U, const Tensor &M, const Tensor &K, const Tensor &B, const Tensor &C, int64_t L,
+std::optional<std::vector<Tensor>> v2x2ssd(const Tensor &U, const Tensor &M, const Tensor &K, const Tensor &B, const Tensor &C, int64_t L,
                    const OptTensor &init, const OptTensor &Bp, const OptTensor &Up, bool return_state, bool retile,
                    bool recompute, std::optional<at::ScalarType> final_type_in) {
-  if (!scan_inputs_plain(U, M, K, B, C, init, Bp, Up)) return py::none();
+  if (!scan_inputs_plain(U, M, K, B, C, init, Bp, Up)) return std::nullopt;
   const int64_t P = U.size(3), D = B.size(3);
   // chunk_size only says how the sequence is tiled; the tcgen05 kernels tile in 128 tokens
   const bool tensor_cores = U.scalar_type() != at::kFloat && P == 64 && D % 64 == 0 && D <= 256;
   if (L > 0 && retile && tensor_cores) L = 128;
-  if (L != 16 && L != 32 && L != 64 && L != 128) return py::none();
+  if (L != 16 && L != 32 && L != 64 && L != 128) return std::nullopt;
   if (retile && !tensor_cores) L = cuda_core_chunk(U.size(0) * U.size(1), U.size(2));
   const at::ScalarType final_type = final_type_in.value_or(U.scalar_type());
-  if (code_of(final_type) < 0) return py::none();
+  if (code_of(final_type) < 0) return std::nullopt;
   const ScanDims d = scan_dims(U, B, L);
   const bool grad = torch::autograd::compute_requires_grad(U, M, K, B, C, init.value_or(Tensor()),
                                                            Bp.value_or(Tensor()), Up.value_or(Tensor()));
@@ -370,17 +371,18 @@ py::object v2x2ssd(const Tensor &U, const Tensor &M, const Tensor &K, const Tens
     if (return_state)
       for (Tensor *t : {&r.final_copy, &r.B_last, &r.U_last}) torch::autograd::set_history(*t, node);
   }
-  if (!return_state) return py::cast(r.Y);
-  return py::make_tuple(r.Y, r.final_copy, r.B_last, r.U_last);
+  if (!return_state) return std::vector<Tensor>{r.Y};
+  return std::vector<Tensor>{r.Y, r.final_copy, r.B_last, r.U_last};
 }
 
 // building blocks of the context-parallel mode: fp32 streaming tensors, no autograd
-py::tuple scan_fwd_parts(const Tensor &U, const Tensor &M, const Tensor &K, const Tensor &B, const Tensor &C,
+using Parts4 = std::tuple<Tensor, Tensor, Tensor, Tensor>;
+Parts4 scan_fwd_parts(const Tensor &U, const Tensor &M, const Tensor &K, const Tensor &B, const Tensor &C,
                          const OptTensor &init, const OptTensor &Bp, const OptTensor &Up, int64_t L) {
   ScanForward r = scan_forward(scan_dims(U, B, L), U, M, K, B, C, init, Bp, Up, true, false, at::kFloat);
-  return py::make_tuple(r.Y, r.final32, r.starts, r.mch);
+  return {r.Y, r.final32, r.starts, r.mch};
 }
-py::tuple scan_bwd_parts(const Tensor &U, const Tensor &M, const Tensor &K, const Tensor &B, const Tensor &C,
+std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor> scan_bwd_parts(const Tensor &U, const Tensor &M, const Tensor &K, const Tensor &B, const Tensor &C,
                          const OptTensor &Bp, const OptTensor &Up, const Tensor &starts, const Tensor &mch,
                          const Tensor &final32, const Tensor &dY, const OptTensor &d_final, int64_t L,
                          bool want_initial, bool want_prev, const OptTensor &workspace) {
@@ -389,8 +391,7 @@ py::tuple scan_bwd_parts(const Tensor &U, const Tensor &M, const Tensor &K, cons
   // (the stage entry points convert the chunk starts to the current kernels' dtype first)
   ScanGrads g = scan_backward(scan_dims(U, B, L, code_of(starts.scalar_type())), U, M, K, B, C, Bp.value_or(Tensor()), Up.value_or(Tensor()), starts,
                               mch, final32, dY, d_final.value_or(Tensor()), it, want_prev && Bp.has_value(), workspace);
-  auto opt = [](const Tensor &t) -> py::object { return t.defined() ? py::cast(t) : py::none(); };
-  return py::make_tuple(g.dU, g.dM, g.dK, g.dB, g.dC, opt(g.d_init), opt(g.dBp), opt(g.dUp));
+  return {g.dU, g.dM, g.dK, g.dB, g.dC, g.d_init, g.dBp, g.dUp};  // (undefined tensors arrive as None)
 }
 
 // ------------------------------------------------------------------------------------------------------------
@@ -530,18 +531,18 @@ struct PrepBackward : public Node {
 };
 
 // value (b,T,H*P), params (b,T,H*13), bc (b,T,H,4,N); pars = the seven biases, then b_scale, c_scale
-py::object scanprep(const Tensor &value, const Tensor &params, const Tensor &bc, int64_t H, int64_t N, int64_t P,
+std::optional<std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor>> scanprep(const Tensor &value, const Tensor &params, const Tensor &bc, int64_t H, int64_t N, int64_t P,
                     bool normalize, const Hyper &hp, const std::vector<Tensor> &pars) {
-  if (!value.is_cuda() || value.dim() != 3 || params.dim() != 3 || bc.dim() != 5) return py::none();
+  if (!value.is_cuda() || value.dim() != 3 || params.dim() != 3 || bc.dim() != 5) return std::nullopt;
   const at::Device dev = value.device();
   const at::ScalarType act = value.scalar_type();
   const int64_t b = value.size(0), T = value.size(1);
-  if (b == 0 || T == 0 || H <= 0 || N <= 0 || P <= 0 || code_of(act) < 0) return py::none();
+  if (b == 0 || T == 0 || H <= 0 || N <= 0 || P <= 0 || code_of(act) < 0) return std::nullopt;
   const int64_t vsz[3] = {b, T, H * P}, psz[3] = {b, T, H * kParamDim}, bsz[5] = {b, T, H, 4, N};
-  if (!shaped(value, vsz) || !shaped(params, psz) || !shaped(bc, bsz)) return py::none();
+  if (!shaped(value, vsz) || !shaped(params, psz) || !shaped(bc, bsz)) return std::nullopt;
   if (params.scalar_type() != act || bc.scalar_type() != act || params.device() != dev || bc.device() != dev)
-    return py::none();
-  if (!prep_params_plain(pars, normalize, dev, H, N)) return py::none();
+    return std::nullopt;
+  if (!prep_params_plain(pars, normalize, dev, H, N)) return std::nullopt;
   const Tensor v = with_rows(value), p = with_rows(params), c = with_rows(bc);
   const PrepConfig cfg = prep_config(H, N, P, normalize, hp);
   Tensor U = empty({b, H, T, P}, act, dev), M = empty({b, H, T, 2}, at::kFloat, dev),
@@ -579,7 +580,7 @@ py::object scanprep(const Tensor &value, const Tensor &params, const Tensor &bc,
     }
     for (Tensor *t : {&U, &M, &K, &B, &C}) torch::autograd::set_history(*t, node);
   }
-  return py::make_tuple(U, M, K, B, C);
+  return std::make_tuple(U, M, K, B, C);
 }
 
 // ------------------------------------------------------------------------------------------------------------
@@ -594,34 +595,34 @@ bool dense_batch(const Tensor &x, int64_t inner) {
   }
   return x.size(0) == 1 || x.stride(0) >= inner;
 }
-py::object decode_step(const Tensor &value, const Tensor &params, const Tensor &bc, const Tensor &gate,
+std::optional<Parts4> decode_step(const Tensor &value, const Tensor &params, const Tensor &bc, const Tensor &gate,
                        const Tensor &skip, const OptTensor &state_in, const OptTensor &Bp, const OptTensor &Up,
                        bool normalize, const Hyper &hp, const std::vector<Tensor> &pars, const OptTensor &state_out_in,
                        const OptTensor &b_last_in, const OptTensor &u_last_in) {
-  if (!value.is_cuda() || value.dim() != 3 || bc.dim() != 4) return py::none();
+  if (!value.is_cuda() || value.dim() != 3 || bc.dim() != 4) return std::nullopt;
   const at::Device dev = value.device();
   const at::ScalarType act = value.scalar_type();
   const int64_t b = value.size(0), H = value.size(1), P = value.size(2), N = bc.size(3);
-  if (code_of(act) < 0 || b == 0 || H == 0 || P == 0 || N == 0) return py::none();
+  if (code_of(act) < 0 || b == 0 || H == 0 || P == 0 || N == 0) return std::nullopt;
   const int64_t vsz[3] = {b, H, P}, psz[3] = {b, H, kParamDim}, bsz[4] = {b, H, 4, N}, ssz[4] = {b, H, P, 2 * N},
                 lsz[3] = {b, H, 2 * N};
-  if (!shaped(params, psz) || !shaped(bc, bsz) || !shaped(gate, vsz) || skip.numel() != H * P) return py::none();
+  if (!shaped(params, psz) || !shaped(bc, bsz) || !shaped(gate, vsz) || skip.numel() != H * P) return std::nullopt;
   for (const Tensor *t : {&params, &bc, &gate, &skip})
-    if (t->device() != dev) return py::none();
+    if (t->device() != dev) return std::nullopt;
   for (const Tensor *t : {&params, &bc, &gate})
-    if (t->scalar_type() != act) return py::none();
-  if (code_of(skip.scalar_type()) < 0 || !skip.is_contiguous()) return py::none();
+    if (t->scalar_type() != act) return std::nullopt;
+  if (code_of(skip.scalar_type()) < 0 || !skip.is_contiguous()) return std::nullopt;
   if (!dense_batch(value, H * P) || !dense_batch(params, H * kParamDim) || !dense_batch(bc, H * 4 * N) ||
       !dense_batch(gate, H * P))
-    return py::none();
-  if (!prep_params_plain(pars, normalize, dev, H, N)) return py::none();
+    return std::nullopt;
+  if (!prep_params_plain(pars, normalize, dev, H, N)) return std::nullopt;
   auto fits = [&](const OptTensor &t, at::IntArrayRef sz, at::ScalarType ty) {
     return !t || (is(*t, dev) && shaped(*t, sz) && t->is_contiguous() && t->scalar_type() == ty);
   };
-  if (Bp.has_value() != Up.has_value()) return py::none();
+  if (Bp.has_value() != Up.has_value()) return std::nullopt;
   if (!fits(state_in, ssz, at::kFloat) || !fits(Bp, lsz, act) || !fits(Up, vsz, act) ||
       !fits(state_out_in, ssz, at::kFloat) || !fits(b_last_in, lsz, act) || !fits(u_last_in, vsz, act))
-    return py::none();
+    return std::nullopt;
   Tensor out = empty({b, H * P}, act, dev);
   Tensor state_out = state_out_in ? *state_out_in : empty(ssz, at::kFloat, dev);
   Tensor b_last = b_last_in ? *b_last_in : empty(lsz, act, dev);
@@ -637,7 +638,7 @@ py::object decode_step(const Tensor &value, const Tensor &params, const Tensor &
                                code_of(skip.scalar_type()), &pp, static_cast<const float *>(cptr(state_in)), cptr(Bp),
                                cptr(Up), ptr(out), fptr(state_out), ptr(b_last), ptr(u_last), stream_of(dev)),
         "decode step");
-  return py::make_tuple(out, state_out, b_last, u_last);
+  return Parts4{out, state_out, b_last, u_last};
 }
 
 // ------------------------------------------------------------------------------------------------------------
@@ -690,16 +691,16 @@ struct ConvBackward : public Node {
   }
 };
 
-py::object cconv1d(const Tensor &x_in, const Tensor &weight, const OptTensor &bias, const OptTensor &state, bool silu) {
-  if (!x_in.is_cuda() || x_in.dim() != 3 || weight.dim() != 2) return py::none();
+std::optional<std::tuple<Tensor, Tensor>> cconv1d(const Tensor &x_in, const Tensor &weight, const OptTensor &bias, const OptTensor &state, bool silu) {
+  if (!x_in.is_cuda() || x_in.dim() != 3 || weight.dim() != 2) return std::nullopt;
   const at::Device dev = x_in.device();
   const at::ScalarType act = x_in.scalar_type();
   const int64_t b = x_in.size(0), T = x_in.size(1), C = x_in.size(2), W = weight.size(1);
   if (code_of(act) < 0 || b == 0 || T == 0 || C == 0 || W < 2 || W > 4 || weight.size(0) != C || weight.device() != dev)
-    return py::none();
-  if (bias && (!is(*bias, dev) || bias->numel() != C)) return py::none();
+    return std::nullopt;
+  if (bias && (!is(*bias, dev) || bias->numel() != C)) return std::nullopt;
   const int64_t ssz[3] = {b, C, W - 1};
-  if (state && (!is(*state, dev) || !shaped(*state, ssz))) return py::none();
+  if (state && (!is(*state, dev) || !shaped(*state, ssz))) return std::nullopt;
   // a column slice of a wider matrix is read where it is; anything else is copied
   const bool rows = x_in.stride(2) == 1 && (T == 1 || x_in.stride(1) >= C);
   const Tensor x = rows ? x_in : x_in.detach().contiguous();
@@ -728,22 +729,22 @@ py::object cconv1d(const Tensor &x_in, const Tensor &weight, const OptTensor &bi
     torch::autograd::set_history(y, node);
     torch::autograd::set_history(nxt, node);
   }
-  return py::make_tuple(y, nxt);
+  return std::make_tuple(y, nxt);
 }
 
 // x (b,C), rolling state (b,C,W-1) -> (y, next state); `inplace`: the state tensor itself is rolled
-py::object cconv1d_update(const Tensor &x_in, const Tensor &weight, const OptTensor &bias, const OptTensor &state,
+std::optional<std::tuple<Tensor, Tensor>> cconv1d_update(const Tensor &x_in, const Tensor &weight, const OptTensor &bias, const OptTensor &state,
                           bool silu, bool inplace) {
-  if (!x_in.is_cuda() || x_in.dim() != 2 || weight.dim() != 2) return py::none();
+  if (!x_in.is_cuda() || x_in.dim() != 2 || weight.dim() != 2) return std::nullopt;
   const at::Device dev = x_in.device();
   const at::ScalarType act = x_in.scalar_type();
   const int64_t b = x_in.size(0), C = x_in.size(1), W = weight.size(1);
   if (code_of(act) < 0 || b == 0 || C == 0 || W < 2 || W > 4 || weight.size(0) != C || weight.device() != dev)
-    return py::none();
-  if (bias && (!is(*bias, dev) || bias->numel() != C)) return py::none();
+    return std::nullopt;
+  if (bias && (!is(*bias, dev) || bias->numel() != C)) return std::nullopt;
   const int64_t ssz[3] = {b, C, W - 1};
-  if (state && (!is(*state, dev) || !shaped(*state, ssz))) return py::none();
-  if (inplace && (!state || state->scalar_type() != act || !state->is_contiguous())) return py::none();
+  if (state && (!is(*state, dev) || !shaped(*state, ssz))) return std::nullopt;
+  if (inplace && (!state || state->scalar_type() != act || !state->is_contiguous())) return std::nullopt;
   const Tensor x = x_in.stride(1) == 1 ? x_in : x_in.contiguous();
   const Tensor w = as_type(weight, act), bs = bias ? as_type(*bias, act) : Tensor(),
                st = state ? as_type(*state, act) : Tensor();
@@ -751,7 +752,7 @@ py::object cconv1d_update(const Tensor &x_in, const Tensor &weight, const OptTen
   const slx_conv_shape s{(int32_t)b, 1, (int32_t)C, (int32_t)W, code_of(act), silu ? 1 : 0, C, x.stride(0)};
   c10::cuda::CUDAGuard guard(dev);
   check(slx_cconv1d_update(&s, ptr(x), ptr(w), ptr(bs), ptr(st), ptr(y), ptr(nxt), stream_of(dev)), "cconv1d update");
-  return py::make_tuple(y, nxt);
+  return std::make_tuple(y, nxt);
 }
 
 // ------------------------------------------------------------------------------------------------------------
@@ -811,17 +812,17 @@ struct GateBackward : public Node {
   }
 };
 
-py::object gate_skip(const Tensor &y_in, const Tensor &u_in, const Tensor &gate_in, const Tensor &skip_in) {
-  if (!y_in.is_cuda() || y_in.dim() != 4 || gate_in.dim() != 3) return py::none();
+OptTensor gate_skip(const Tensor &y_in, const Tensor &u_in, const Tensor &gate_in, const Tensor &skip_in) {
+  if (!y_in.is_cuda() || y_in.dim() != 4 || gate_in.dim() != 3) return std::nullopt;
   const at::Device dev = y_in.device();
   const at::ScalarType act = y_in.scalar_type();
   const int64_t b = y_in.size(0), H = y_in.size(1), T = y_in.size(2), P = y_in.size(3);
   const int64_t gsz[3] = {b, T, H * P};
   if (code_of(act) < 0 || b == 0 || T == 0 || H == 0 || P == 0 || P % 8 != 0 || !shaped(u_in, y_in.sizes()) ||
       !shaped(gate_in, gsz) || skip_in.numel() != H * P)
-    return py::none();
+    return std::nullopt;
   for (const Tensor *t : {&u_in, &gate_in, &skip_in})
-    if (t->device() != dev) return py::none();
+    if (t->device() != dev) return std::nullopt;
   auto plain = [&](const Tensor &t) {
     Tensor r = as_type(t, act);
     return aligned(r) ? r : r.clone();
@@ -852,33 +853,19 @@ py::object gate_skip(const Tensor &y_in, const Tensor &u_in, const Tensor &gate_
     node->skip_sizes = skip_in.sizes().vec();
     torch::autograd::set_history(out, node);
   }
-  return py::cast(out);
-}
-
-// argument errors that the C ABI reports reach Python as the exceptions the ops document
-template <typename R, typename... A>
-auto python(R (*fn)(A...)) {
-  return [fn](A... args) -> R {
-    try {
-      return fn(args...);
-    } catch (const c10::ValueError &e) {
-      throw py::value_error(e.what_without_backtrace());
-    } catch (const c10::TypeError &e) {
-      throw py::type_error(e.what_without_backtrace());
-    }
-  };
+  return out;
 }
 
 }  // namespace
 
 PYBIND11_MODULE(_host, m) {
-  m.def("v2x2ssd", python(&v2x2ssd));
-  m.def("scan_fwd_parts", python(&scan_fwd_parts));
-  m.def("scan_bwd_parts", python(&scan_bwd_parts));
-  m.def("scanprep", python(&scanprep));
-  m.def("row_stride", &row_stride);
-  m.def("decode_step", python(&decode_step));
-  m.def("cconv1d", python(&cconv1d));
-  m.def("cconv1d_update", python(&cconv1d_update));
-  m.def("gate_skip", python(&gate_skip));
+  m.def("v2x2ssd", torch::wrap_pybind_function_no_gil(&v2x2ssd));
+  m.def("scan_fwd_parts", torch::wrap_pybind_function_no_gil(&scan_fwd_parts));
+  m.def("scan_bwd_parts", torch::wrap_pybind_function_no_gil(&scan_bwd_parts));
+  m.def("scanprep", torch::wrap_pybind_function_no_gil(&scanprep));
+  m.def("row_stride", torch::wrap_pybind_function(&row_stride));
+  m.def("decode_step", torch::wrap_pybind_function_no_gil(&decode_step));
+  m.def("cconv1d", torch::wrap_pybind_function_no_gil(&cconv1d));
+  m.def("cconv1d_update", torch::wrap_pybind_function_no_gil(&cconv1d_update));
+  m.def("gate_skip", torch::wrap_pybind_function_no_gil(&gate_skip));
 }

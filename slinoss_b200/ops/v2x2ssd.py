@@ -317,7 +317,7 @@ def v2x2ssd_b200(U, M, K, B, C, *, chunk_size: int, initial_states=None, B_prev=
         out = _lib.host().v2x2ssd(U, M, K, B, C, int(chunk_size), initial_states, B_prev, U_prev, return_state, retile,
                                   residual == "recompute", None)
         if out is not None:
-            return out
+            return tuple(out) if return_state else out[0]
     return _v2x2ssd_general(U, M, K, B, C, chunk_size, initial_states, B_prev, U_prev, compute_dtype, output_dtype,
                             return_state, retile, strict, residual)
 
@@ -364,14 +364,14 @@ def _v2x2ssd_general(U, M, K, B, C, chunk_size, initial_states, B_prev, U_prev, 
     if out is None:
         raise ValueError("slinoss_b200 v2x2ssd: sizes must be positive. "
                          f"Got batch={b}, heads={h}, T={T}, P={P}, 2N={D}.")
-    out = tuple(t.to(odtype) for t in out) if return_state else out.to(odtype)
+    out = tuple(t.to(odtype) for t in out)
     if strict:
         if _lib.read_scan_status(U.device):
             raise ValueError("M has an entry of magnitude exactly 0: the chunked scan needs abs(M) > 0.")
         if _lib.read_tc_status(U.device):
             raise RuntimeError("v2x2ssd: a bounded wait inside a tensor-core kernel ran out; the outputs "
                                "of the affected chunks are NaN.")
-    return out
+    return out if return_state else out[0]
 
 
 __all__ = ["v2x2ssd_b200", "chunk_increment_b200", "state_passing_b200", "chunk_scan_b200"]

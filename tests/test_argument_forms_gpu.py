@@ -139,3 +139,40 @@ def test_kernel_family_chosen_between_forward_and_backward(before, after):
     for k, a, b in zip(names, grads(before, after), grads(after, after)):
         # the families' chunk starts differ by their storage, half against fp32: 2^-9 of a value
         assert (a.float() - b.float()).norm() < 4e-3 * b.float().norm(), k
+
+
+@pytest.mark.gpu
+def test_other_threads_run_while_a_launch_waits():
+    """The interpreter lock is free while an op waits for room in the launch queue."""
+    import threading
+    import time
+
+    import slinoss_b200 as sb
+
+    x, w = torch.zeros(1, 8, device="cuda"), torch.zeros(8, 4, device="cuda")
+    state = torch.zeros(1, 8, 3, device="cuda")
+    sb.cconv1d_update_b200(x, w, None, state, inplace=True)
+    torch.cuda.synchronize()
+    gaps, done = [], threading.Event()
+
+    def tick():
+        last = time.perf_counter()
+        while not done.is_set():
+            time.sleep(0.001)
+            now = time.perf_counter()
+            gaps.append(now - last)
+            last = now
+
+    torch.cuda._sleep(int(1.5e9))  # the GPU is busy for most of a second
+    thread = threading.Thread(target=tick)
+    thread.start()
+    start = time.perf_counter()
+    for _ in range(4000):  # more than the queue holds
+        sb.cconv1d_update_b200(x, w, None, state, inplace=True)
+    waited = time.perf_counter() - start
+    done.set()
+    thread.join()
+    torch.cuda.synchronize()
+    if waited < 0.4:
+        pytest.skip("the launches did not have to wait")
+    assert max(gaps) < 0.5 * waited, (max(gaps), waited)
