@@ -72,6 +72,9 @@ Tensor as_read(const Tensor &g, at::ScalarType t) {
 }
 Tensor saved(SavedVariable &v) { return v.unpack(); }
 SavedVariable keep(const Tensor &t) { return t.defined() ? SavedVariable(t, false) : SavedVariable(); }
+// A small tensor that its owner may overwrite before the backward runs (a stream's carried rows, in place; parameters): a
+// half one is kept by value, an fp32 one by reference, so that autograd reports the overwriting.
+SavedVariable keep_value(const Tensor &t) { return keep(t.scalar_type() == at::kFloat ? t : t.detach().clone()); }
 
 template <typename N>
 std::shared_ptr<N> make_node(torch::autograd::edge_list edges) {
@@ -217,7 +220,8 @@ struct ScanBackward : public Node {
   int64_t L = 0;
   bool recompute = false;
   SavedVariable U_, M_, K_, B_, C_, mch_, starts_, final_, init_, Bp_, Up_;
-  bool has_init = false, has_prev = false;
+  std::optional<at::ScalarType> init_type;  // of the initial states, where there are any
+  bool has_prev = false;
   std::string name() const override { return "V2x2ssdBackward"; }
 
   void release_variables() override {
@@ -244,21 +248,17 @@ struct ScanBackward : public Node {
       if (d_fin_in.defined())
         d_fin = as_read(d_fin_in, code_of(d_fin_in.scalar_type()) < 0 ? at::kFloat : d_fin_in.scalar_type());
       Tensor starts;
-      std::optional<at::ScalarType> init_type;
-      OptTensor init;
-      if (has_init) {
-        init = saved(init_);
-        init_type = init->scalar_type();
-      }
       if (recompute) {
         const at::ScalarType st = type_of(d.s.starts_dtype);
         const int64_t sizes[5] = {d.b, d.h, d.NC, d.P, d.D};
         starts = empty(sizes, st, d.dev);
         Tensor inc = empty(sizes, st, d.dev), m2 = empty({d.b, d.h, d.NC, 2}, at::kFloat, d.dev);
         slx_scan_ends e{};
-        if (init) {
-          e.initial_states = init->data_ptr();
-          e.initial_dtype = code_of(*init_type);
+        Tensor init;
+        if (init_type) {
+          init = saved(init_);
+          e.initial_states = ptr(init);
+          e.initial_dtype = code_of(init.scalar_type());
         }
         if (has_prev) {
           e.B_prev = ptr(Bp);
@@ -358,14 +358,14 @@ std::optional<std::vector<Tensor>> v2x2ssd(const Tensor &U, const Tensor &M, con
     node->mch_ = keep(r.mch);
     node->final_ = keep(r.final32.is_same(r.final_copy) ? r.final32.detach() : r.final32);
     // What is kept of the chunk-start states, the largest residual: as the kernels exchange them, or (recompute)
-    // nothing: the backward rebuilds them with one more chunk-increment and state pass.
+    // nothing: the backward rebuilds them with one more chunk-increment and state pass, from the initial states.
     if (!recompute) node->starts_ = keep(r.starts);
-    node->has_init = init.has_value();
+    if (init) node->init_type = init->scalar_type();
+    if (init && recompute) node->init_ = keep_value(*init);
     node->has_prev = Bp.has_value();
-    if (init) node->init_ = keep(*init);
     if (Bp) {
-      node->Bp_ = keep(*Bp);
-      node->Up_ = keep(*Up);
+      node->Bp_ = keep_value(*Bp);
+      node->Up_ = keep_value(*Up);
     }
     torch::autograd::set_history(r.Y, node);
     if (return_state)
@@ -467,28 +467,47 @@ slx_prep_params params_struct(const std::vector<Tensor> &p, bool normalize) {
   return s;
 }
 
+// The same parameters by value, in one tensor: [scales of B and C,] biases.  What the backward keeps: a program may
+// update them before it runs.
+Tensor flat_params(const std::vector<Tensor> &p, bool normalize) {
+  at::AutoDispatchBelowAutograd no_graph;
+  std::vector<Tensor> flat;
+  for (int i = normalize ? 7 : 9; i < 9; ++i) flat.push_back(p[i].view({-1}));
+  for (int i = 0; i < 7; ++i) flat.push_back(p[i].dim() == 1 ? p[i] : p[i].view({-1}));
+  return at::cat(flat);
+}
+slx_prep_params flat_params_struct(const Tensor &flat, bool normalize, int64_t H, int64_t N) {
+  slx_prep_params s{};
+  const char *at = static_cast<const char *>(flat.data_ptr());
+  const int64_t size = flat.element_size();
+  if (normalize) {
+    s.b_scale = at;
+    s.c_scale = at + 2 * H * N * size;
+    at += 4 * H * N * size;
+  }
+  for (int i = 0; i < 7; ++i) s.bias[i] = at + i * H * size;
+  s.dtype = code_of(flat.scalar_type());
+  return s;
+}
+
 struct PrepBackward : public Node {
   PrepConfig cfg{};
   int64_t b = 0, T = 0;
   std::vector<int64_t> bc_sizes;
-  SavedVariable params_, bc_;
-  std::vector<SavedVariable> pars_;
+  SavedVariable params_, bc_, pars_;  // pars_: the parameters by value, as flat_params lays them out
   std::vector<at::ScalarType> par_types;
   std::string name() const override { return "ScanPrepBackward"; }
   void release_variables() override {
     std::lock_guard<std::mutex> lock(mutex_);
     params_.reset_data();
     bc_.reset_data();
-    for (auto &v : pars_) v.reset_data();
+    pars_.reset_data();
   }
   variable_list apply(variable_list &&grads) override {
     std::lock_guard<std::mutex> lock(mutex_);
     Tensor params = with_rows(saved(params_)), bc = with_rows(saved(bc_));
-    std::vector<Tensor> pars(9);
-    const size_t n = cfg.normalize ? 9 : 7;
-    for (size_t i = 0; i < n; ++i) pars[i] = saved(pars_[i]);
-    pars = uniform_params(pars, cfg.normalize);
-    const at::ScalarType act = params.scalar_type(), pt = pars[0].scalar_type();
+    const Tensor pars = saved(pars_);
+    const at::ScalarType act = params.scalar_type(), pt = pars.scalar_type();
     const at::Device dev = params.device();
     auto in = [&](size_t i, at::IntArrayRef sizes, at::ScalarType t) {
       return grads[i].defined() ? as_read(grads[i], t) : at::zeros(sizes, at::TensorOptions().dtype(t).device(dev));
@@ -503,7 +522,7 @@ struct PrepBackward : public Node {
       d_cs = empty({H, 2, N}, pt, dev);
     }
     const slx_prep_shape s = prep_shape(cfg, b, T, code_of(act), H * P, row_stride(params), row_stride(bc));
-    const slx_prep_params pp = params_struct(pars, cfg.normalize);
+    const slx_prep_params pp = flat_params_struct(pars, cfg.normalize, H, N);
     const size_t nbytes = slx_scanprep_bwd_workspace_bytes(&s);
     Tensor ws = empty({(int64_t)nbytes}, at::kByte, dev);
     {
@@ -572,12 +591,8 @@ std::optional<std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor>> scanprep(const
     node->bc_sizes.assign(bsz, bsz + 5);
     node->params_ = keep(p);
     node->bc_ = keep(c);
-    const size_t n = normalize ? 9 : 7;
-    node->pars_.reserve(n);
-    for (size_t i = 0; i < n; ++i) {
-      node->pars_.push_back(keep(pars[i]));
-      node->par_types.push_back(pars[i].scalar_type());
-    }
+    node->pars_ = keep(flat_params(up, normalize));
+    for (size_t i = 0; i < (normalize ? 9 : 7); ++i) node->par_types.push_back(pars[i].scalar_type());
     for (Tensor *t : {&U, &M, &K, &B, &C}) torch::autograd::set_history(*t, node);
   }
   return std::make_tuple(U, M, K, B, C);
@@ -662,9 +677,9 @@ struct ConvBackward : public Node {
     Tensor x = saved(x_);
     const at::ScalarType act = x.scalar_type();
     const at::Device dev = x.device();
-    Tensor w = as_type(saved(w_), act), bias, state;
-    if (has_bias) bias = as_type(saved(bias_), act);
-    if (has_state) state = as_type(saved(state_), act);
+    Tensor w = saved(w_), bias, state;  // in x's dtype
+    if (has_bias) bias = saved(bias_);
+    if (has_state) state = saved(state_);
     const int64_t b = x.size(0), T = x.size(1), C = x.size(2), W = w.size(1);
     Tensor dy = grads[0].defined() ? as_read(grads[0], act)
                                    : at::zeros({b, T, C}, at::TensorOptions().dtype(act).device(dev));
@@ -723,9 +738,9 @@ std::optional<std::tuple<Tensor, Tensor>> cconv1d(const Tensor &x_in, const Tens
     if (bias) node->b_type = bias->scalar_type();
     if (state) node->s_type = state->scalar_type();
     node->x_ = keep(x);
-    node->w_ = keep(weight);
-    if (bias) node->bias_ = keep(*bias);
-    if (state) node->state_ = keep(*state);
+    node->w_ = keep(w);
+    node->bias_ = keep(bs);
+    node->state_ = keep(st);
     torch::autograd::set_history(y, node);
     torch::autograd::set_history(nxt, node);
   }
@@ -846,7 +861,7 @@ OptTensor gate_skip(const Tensor &y_in, const Tensor &u_in, const Tensor &gate_i
     node->y_ = keep(y);
     node->u_ = keep(u);
     node->gate_ = keep(gate);
-    node->skip_ = keep(skip);
+    node->skip_ = keep_value(skip);
     node->u_type = u_in.scalar_type();
     node->g_type = gate_in.scalar_type();
     node->s_type = skip_in.scalar_type();

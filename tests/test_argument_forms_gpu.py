@@ -176,3 +176,58 @@ def test_other_threads_run_while_a_launch_waits():
     if waited < 0.4:
         pytest.skip("the launches did not have to wait")
     assert max(gaps) < 0.5 * waited, (max(gaps), waited)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("residual", ["keep", "recompute"])
+def test_carried_tensors_may_be_overwritten_before_the_backward(residual):
+    """A stream that keeps its carried tensors in place: the backward needs the rows and states that the forward read."""
+    import slinoss_b200 as sb
+
+    inp = make_scan_inputs(1, 2, 140, 32, 64, BF16, seed=2, streaming=True, with_init=True)
+    inp["initial_states"] = inp["initial_states"].to(BF16)
+    names = ("U", "M", "K", "B", "C")
+
+    def grads(overwrite):
+        leaves = [inp[k].detach().requires_grad_(True) for k in names]
+        carried = {k: inp[k].clone() for k in ("initial_states", "B_prev", "U_prev")}
+        Y, *nxt = sb.v2x2ssd_b200(*leaves, chunk_size=128, return_state=True, residual=residual, **carried)
+        if overwrite:
+            for t, n in zip(carried.values(), nxt):
+                t.copy_(n.detach())
+        return torch.autograd.grad(Y, leaves, inp["dY"])
+
+    assert all(torch.equal(a, b) for a, b in zip(grads(True), grads(False)))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [BF16, F32])
+def test_parameters_may_be_updated_before_the_backward(dtype):
+    import slinoss_b200 as sb
+
+    b, T, H, P, N = 2, 9, 2, 16, 8
+    g = torch.Generator().manual_seed(5)
+    r = lambda *s, dt=BF16: torch.randn(*s, generator=g).to(dt).cuda()
+    value, params, bc = r(b, T, H * P), r(b, T, H * 13), r(b, T, H, 4, N)
+    gate, y = r(b, T, H * P), r(b, H, T, P)
+    names = ("dt_bias", "gamma_bias", "omega_bias", "mix_r_bias", "mix_theta_bias", "mix_k_prev_bias",
+             "mix_k_curr_bias")
+    pars = {k: r(H, dt=dtype) for k in names}
+    pars.update(b_scale=r(H, 2, N, dt=dtype), c_scale=r(H, 2, N, dt=dtype))
+    skip, w = r(H * P), r(H * P, 4, dt=F32)  # (fp32 skip weights and taps of x's own dtype are kept by reference)
+
+    def grads(update):
+        leaves = [t.clone().requires_grad_(True) for t in (value, params, bc, gate)]
+        ps = {k: t.clone().requires_grad_(True) for k, t in pars.items()}
+        ws = [t.clone().requires_grad_(True) for t in (skip, w)]
+        x, _ = sb.cconv1d_b200(leaves[0], ws[1], None, activation="silu")
+        o = sb.scanprep_b200(x, leaves[1], leaves[2], n_heads=H, d_state=N, d_head=P, normalize_bc=True, dt_min=1e-4,
+                             dt_max=1e-1, r_min=0.9, r_max=1.0, theta_bound=3.0, k_max=0.5, eps=1e-8, **ps)
+        outs = [o.U, o.M, o.K, o.B, o.C, sb.gate_skip_b200(y, o.U, leaves[3], ws[0])]
+        if update:
+            with torch.no_grad():
+                for t in (*ps.values(), *ws):
+                    t.mul_(0.5)
+        return torch.autograd.grad([t.float().square().sum() for t in outs], [*leaves, *ps.values(), *ws])
+
+    assert all(torch.equal(a, b) for a, b in zip(grads(True), grads(False)))
