@@ -14,6 +14,7 @@ from typing import Optional, Tuple
 import torch
 
 from .. import _lib
+from . import _trace
 
 
 def _check(x, weight, conv_state, rank: str, ndim: int) -> None:
@@ -40,6 +41,8 @@ def cconv1d_b200(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Ten
                  activation: Optional[str] = None) -> Tuple[torch.Tensor, torch.Tensor]:
     if activation not in (None, "silu", "swish"):
         raise NotImplementedError("activation must be None, silu, or swish")
+    if _trace.tracing():
+        return _trace.recorded(lambda *a: cconv1d_b200(*a, activation=activation), x, weight, bias, conv_state)
     out = _lib.host().cconv1d(x, weight, bias, conv_state, activation is not None)
     if out is not None:
         return out

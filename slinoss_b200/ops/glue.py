@@ -7,6 +7,7 @@ from __future__ import annotations
 import torch
 
 from .. import _lib
+from . import _trace
 
 
 @torch.compiler.disable
@@ -14,6 +15,8 @@ def gate_skip_b200(scan_y: torch.Tensor, scan_u: torch.Tensor, gate: torch.Tenso
     """``(scan_y + scan_u * skip)`` re-laid from ``(b,H,T,P)`` to ``(b,T,H*P)`` and multiplied by
     ``silu(gate)``; ``gate (b,T,H*P)`` may be a column slice of the input projection's output,
     ``skip (H*P,)``.  Differentiable in all four."""
+    if _trace.tracing():
+        return _trace.recorded(lambda *a: (gate_skip_b200(*a),), scan_y, scan_u, gate, skip)[0]
     out = _lib.host().gate_skip(scan_y, scan_u, gate, skip)
     if out is not None:
         return out

@@ -15,6 +15,7 @@ import torch
 
 from .. import _lib
 from ..types import ScanInputs
+from . import _trace
 
 PARAM_DIM = 13
 
@@ -33,6 +34,15 @@ def scanprep_b200(value, params, bc, *, n_heads: int, d_state: int, d_head: int,
     if normalize_bc:
         pars += (b_scale, c_scale)
     hyper = (dt_min, dt_max, r_min, r_max, theta_bound, k_max, eps)
+    if _trace.tracing():
+        def call(value, params, bc, *pars):
+            names = ("dt_bias", "gamma_bias", "omega_bias", "mix_r_bias", "mix_theta_bias", "mix_k_prev_bias",
+                     "mix_k_curr_bias", "b_scale", "c_scale")
+            o = scanprep_b200(value, params, bc, n_heads=n_heads, d_state=d_state, d_head=d_head,
+                              normalize_bc=normalize_bc, dt_min=dt_min, dt_max=dt_max, r_min=r_min, r_max=r_max,
+                              theta_bound=theta_bound, k_max=k_max, eps=eps, **dict(zip(names, pars)))
+            return o.U, o.M, o.K, o.B, o.C
+        return ScanInputs(*_trace.recorded(call, value, params, bc, *pars))
     out = _lib.host().scanprep(value, params, bc, n_heads, d_state, d_head, normalize_bc, hyper, pars)
     if out is not None:
         return ScanInputs(*out)

@@ -17,6 +17,7 @@ from typing import Optional, Tuple
 import torch
 
 from .. import _lib
+from . import _trace
 
 _ACT_DTYPES = (torch.float32, torch.bfloat16, torch.float16)
 _CHUNKS = (16, 32, 64, 128)
@@ -312,6 +313,14 @@ def v2x2ssd_b200(U, M, K, B, C, *, chunk_size: int, initial_states=None, B_prev=
     """
     if residual not in ("keep", "recompute"):
         raise ValueError(f"residual must be 'keep' or 'recompute'. Got {residual!r}.")
+    if _trace.tracing():
+        def call(U, M, K, B, C, init, Bp, Up):
+            o = v2x2ssd_b200(U, M, K, B, C, chunk_size=chunk_size, initial_states=init, B_prev=Bp, U_prev=Up,
+                             compute_dtype=compute_dtype, output_dtype=output_dtype, return_state=return_state,
+                             retile=retile, strict=strict, residual=residual)
+            return o if return_state else (o,)
+        out = _trace.recorded(call, U, M, K, B, C, initial_states, B_prev, U_prev)
+        return out if return_state else out[0]
     if not strict and (compute_dtype is None or compute_dtype is torch.float32) and (
             output_dtype is None or output_dtype is U.dtype):
         out = _lib.host().v2x2ssd(U, M, K, B, C, int(chunk_size), initial_states, B_prev, U_prev, return_state, retile,

@@ -231,3 +231,40 @@ def test_parameters_may_be_updated_before_the_backward(dtype):
         return torch.autograd.grad([t.float().square().sum() for t in outs], [*leaves, *ps.values(), *ws])
 
     assert all(torch.equal(a, b) for a, b in zip(grads(True), grads(False)))
+
+
+def _one_input_calls():
+    """name -> (op as a function of its main input, shape of that input)"""
+    import slinoss_b200 as sb
+
+    g = torch.Generator().manual_seed(8)
+    r = lambda *s: torch.randn(*s, generator=g).cuda()
+    b, T, H, P, N = 1, 20, 2, 16, 8
+    hp = dict(n_heads=H, d_state=N, d_head=P, normalize_bc=True, dt_min=1e-4, dt_max=1e-1, r_min=0.9, r_max=1.0,
+              theta_bound=3.0, k_max=0.5, eps=1e-8, b_scale=r(H, 2, N), c_scale=r(H, 2, N),
+              **{k: r(H) for k in ("dt_bias", "gamma_bias", "omega_bias", "mix_r_bias", "mix_theta_bias",
+                                   "mix_k_prev_bias", "mix_k_curr_bias")})
+    w, params, bc, gate, skip = r(H * P, 4), r(b, T, H * 13), r(b, T, H, 4, N), r(b, T, H * P), r(H * P)
+    M = torch.view_as_real(torch.polar(0.5 + 0.5 * torch.rand(b, H, T, generator=g), torch.randn(b, H, T, generator=g)))
+    scan = [M.contiguous().cuda(), r(b, H, T, 2, 2), r(b, H, T, 2 * N), r(b, H, T, 2 * N)]
+    return {
+        "conv": (lambda x: sb.cconv1d_b200(x, w, None, activation="silu")[0], (b, T, H * P)),
+        "prep": (lambda x: sb.scanprep_b200(gate, params, x, **hp).B, (b, T, H, 4, N)),
+        "gate": (lambda x: sb.gate_skip_b200(x, x, gate, skip), (b, H, T, P)),
+        "scan": (lambda x: sb.v2x2ssd_b200(x, *scan, chunk_size=16, return_state=True)[1], (b, H, T, P)),
+    }
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name", ["conv", "prep", "gate", "scan"])
+@pytest.mark.parametrize("grad", [False, True])
+@pytest.mark.filterwarnings("ignore")
+def test_traced_calls_run_again(name, grad):
+    fn, shape = _one_input_calls()[name]
+    x, y = torch.randn(2, *shape, device="cuda").requires_grad_(grad)
+    traced = torch.jit.trace(fn, x.detach().requires_grad_(grad), check_trace=False)
+    leaf = y.detach().requires_grad_(grad)
+    outs = traced(leaf), fn(leaf)
+    assert torch.equal(*outs)
+    if grad:
+        assert torch.equal(*(torch.autograd.grad(o.square().sum(), leaf)[0] for o in outs))
