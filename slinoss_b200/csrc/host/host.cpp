@@ -71,6 +71,16 @@ Tensor as_read(const Tensor &g, at::ScalarType t) {
   return aligned(r) ? r : r.clone();
 }
 Tensor saved(SavedVariable &v) { return v.unpack(); }
+// Forward-mode derivatives are not implemented: an error, not an output without its tangent.
+void refuse_tangent(const Tensor &t) {
+  TORCH_CHECK_NOT_IMPLEMENTED(!t.defined() || !t._fw_grad(0).defined(),
+                              "slinoss_b200 ops have no forward-mode derivative; use reverse mode.");
+}
+template <typename... T>
+void refuse_tangents(const T &...t) {
+  (refuse_tangent(t), ...);
+}
+Tensor or_undefined(const OptTensor &t) { return t.value_or(Tensor()); }
 SavedVariable keep(const Tensor &t) { return t.defined() ? SavedVariable(t, false) : SavedVariable(); }
 // A small tensor that its owner may overwrite before the backward runs (a stream's carried rows, in place; parameters): a
 // half one is kept by value, an fp32 one by reference, so that autograd reports the overwriting.
@@ -342,12 +352,13 @@ std::optional<std::vector<Tensor>> v2x2ssd(const Tensor &U, const Tensor &M, con
   const at::ScalarType final_type = final_type_in.value_or(U.scalar_type());
   if (code_of(final_type) < 0) return std::nullopt;
   const ScanDims d = scan_dims(U, B, L);
-  const bool grad = torch::autograd::compute_requires_grad(U, M, K, B, C, init.value_or(Tensor()),
-                                                           Bp.value_or(Tensor()), Up.value_or(Tensor()));
+  refuse_tangents(U, M, K, B, C, or_undefined(init), or_undefined(Bp), or_undefined(Up));
+  const bool grad =
+      torch::autograd::compute_requires_grad(U, M, K, B, C, or_undefined(init), or_undefined(Bp), or_undefined(Up));
   ScanForward r = scan_forward(d, U, M, K, B, C, init, Bp, Up, grad, return_state, final_type);
   if (grad) {
     auto node = make_node<ScanBackward>(torch::autograd::collect_next_edges(
-        U, M, K, B, C, init.value_or(Tensor()), Bp.value_or(Tensor()), Up.value_or(Tensor())));
+        U, M, K, B, C, or_undefined(init), or_undefined(Bp), or_undefined(Up)));
     node->L = L;
     node->recompute = recompute;
     node->U_ = keep(U);
@@ -389,8 +400,8 @@ std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor> scan_
   std::optional<at::ScalarType> it;
   if (want_initial) it = at::kFloat;
   // (the stage entry points convert the chunk starts to the current kernels' dtype first)
-  ScanGrads g = scan_backward(scan_dims(U, B, L, code_of(starts.scalar_type())), U, M, K, B, C, Bp.value_or(Tensor()), Up.value_or(Tensor()), starts,
-                              mch, final32, dY, d_final.value_or(Tensor()), it, want_prev && Bp.has_value(), workspace);
+  ScanGrads g = scan_backward(scan_dims(U, B, L, code_of(starts.scalar_type())), U, M, K, B, C, or_undefined(Bp), or_undefined(Up), starts,
+                              mch, final32, dY, or_undefined(d_final), it, want_prev && Bp.has_value(), workspace);
   return {g.dU, g.dM, g.dK, g.dB, g.dC, g.d_init, g.dBp, g.dUp};  // (undefined tensors arrive as None)
 }
 
@@ -562,6 +573,8 @@ std::optional<std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor>> scanprep(const
   if (params.scalar_type() != act || bc.scalar_type() != act || params.device() != dev || bc.device() != dev)
     return std::nullopt;
   if (!prep_params_plain(pars, normalize, dev, H, N)) return std::nullopt;
+  refuse_tangents(value, params, bc);
+  for (const Tensor &t : pars) refuse_tangent(t);
   const Tensor v = with_rows(value), p = with_rows(params), c = with_rows(bc);
   const PrepConfig cfg = prep_config(H, N, P, normalize, hp);
   Tensor U = empty({b, H, T, P}, act, dev), M = empty({b, H, T, 2}, at::kFloat, dev),
@@ -716,6 +729,7 @@ std::optional<std::tuple<Tensor, Tensor>> cconv1d(const Tensor &x_in, const Tens
   if (bias && (!is(*bias, dev) || bias->numel() != C)) return std::nullopt;
   const int64_t ssz[3] = {b, C, W - 1};
   if (state && (!is(*state, dev) || !shaped(*state, ssz))) return std::nullopt;
+  refuse_tangents(x_in, weight, or_undefined(bias), or_undefined(state));
   // a column slice of a wider matrix is read where it is; anything else is copied
   const bool rows = x_in.stride(2) == 1 && (T == 1 || x_in.stride(1) >= C);
   const Tensor x = rows ? x_in : x_in.detach().contiguous();
@@ -728,9 +742,9 @@ std::optional<std::tuple<Tensor, Tensor>> cconv1d(const Tensor &x_in, const Tens
     c10::cuda::CUDAGuard guard(dev);
     check(slx_cconv1d_fwd(&s, ptr(x), ptr(w), ptr(bs), ptr(st), ptr(y), ptr(nxt), stream_of(dev)), "cconv1d forward");
   }
-  if (torch::autograd::compute_requires_grad(x_in, weight, bias.value_or(Tensor()), state.value_or(Tensor()))) {
-    auto node = make_node<ConvBackward>(torch::autograd::collect_next_edges(x_in, weight, bias.value_or(Tensor()),
-                                                                            state.value_or(Tensor())));
+  if (torch::autograd::compute_requires_grad(x_in, weight, or_undefined(bias), or_undefined(state))) {
+    auto node = make_node<ConvBackward>(
+        torch::autograd::collect_next_edges(x_in, weight, or_undefined(bias), or_undefined(state)));
     node->silu = silu;
     node->has_bias = bias.has_value();
     node->has_state = state.has_value();
@@ -838,6 +852,7 @@ OptTensor gate_skip(const Tensor &y_in, const Tensor &u_in, const Tensor &gate_i
     return std::nullopt;
   for (const Tensor *t : {&u_in, &gate_in, &skip_in})
     if (t->device() != dev) return std::nullopt;
+  refuse_tangents(y_in, u_in, gate_in, skip_in);
   auto plain = [&](const Tensor &t) {
     Tensor r = as_type(t, act);
     return aligned(r) ? r : r.clone();

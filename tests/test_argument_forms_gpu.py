@@ -268,3 +268,16 @@ def test_traced_calls_run_again(name, grad):
     assert torch.equal(*outs)
     if grad:
         assert torch.equal(*(torch.autograd.grad(o.square().sum(), leaf)[0] for o in outs))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name", ["conv", "prep", "gate", "scan"])
+@pytest.mark.parametrize("grad", [False, True])
+def test_tangents_are_refused(name, grad):
+    """Forward-mode derivatives are not implemented: an error, not an output without its tangent."""
+    import torch.autograd.forward_ad as forward_ad
+
+    fn, shape = _one_input_calls()[name]
+    x, t = torch.randn(2, *shape, device="cuda")
+    with forward_ad.dual_level(), pytest.raises(NotImplementedError):
+        fn(forward_ad.make_dual(x.requires_grad_(grad), t))
