@@ -53,7 +53,7 @@ inline cudaStream_t as_stream(void *s) { return reinterpret_cast<cudaStream_t>(s
 // remembered, so that a launch costs no driver call beyond the launch itself.
 struct KernelSetup {
   size_t smem = 0;   // largest dynamic shared-memory size granted so far
-  long slots = -1;   // CTAs the device holds at once (occupancy query), -1 = not asked yet
+  std::map<std::pair<int, size_t>, long> slots;  // CTAs the device holds at once, by (threads, dynamic bytes) asked for
 };
 inline std::mutex &kernel_setup_mutex() {
   static std::mutex mu;
@@ -87,15 +87,15 @@ inline long resident_ctas(K kernel, int threads, size_t smem) {
   }
   std::lock_guard<std::mutex> lock(kernel_setup_mutex());
   KernelSetup &ks = kernel_setup_table()[{reinterpret_cast<const void *>(kernel), dev}];
-  if (ks.slots >= 0) return ks.slots;
+  const auto known = ks.slots.find({threads, smem});
+  if (known != ks.slots.end()) return known->second;
   int sms = 0, per_sm = 0;
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem) != cudaSuccess) {
     cudaGetLastError();
     return 0;
   }
-  ks.slots = (long)sms * per_sm;
-  return ks.slots;
+  return ks.slots[{threads, smem}] = (long)sms * per_sm;
 }
 
 // ---- element access in the activation dtype ---------------------------------

@@ -281,3 +281,43 @@ def test_tangents_are_refused(name, grad):
     x, t = torch.randn(2, *shape, device="cuda")
     with forward_ad.dual_level(), pytest.raises(NotImplementedError):
         fn(forward_ad.make_dual(x.requires_grad_(grad), t))
+
+
+def _kernels(fn):
+    """(name, grid) of the kernels that ``fn`` launches, in order."""
+    import json
+    import tempfile
+
+    fn()
+    torch.cuda.synchronize()
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        fn()
+        torch.cuda.synchronize()
+    with tempfile.NamedTemporaryFile(suffix=".json") as f:
+        prof.export_chrome_trace(f.name)
+        events = json.load(open(f.name))["traceEvents"]
+    found = sorted((e["ts"], e["name"], e["args"]["grid"]) for e in events if e.get("cat") == "kernel")
+    if not found:
+        pytest.skip("the profiler shows no kernels here")
+    return [(n, g) for _, n, g in found]
+
+
+@pytest.mark.gpu
+def test_decode_grid_follows_the_state_width():
+    """Wide states leave fewer CTAs per SM; the narrow ones before and after keep three."""
+    import slinoss_b200 as sb
+
+    def grid(N):
+        b, H, P = 1024, 1, 64
+        z = lambda *s: torch.zeros(*s, device="cuda")
+        bias = {k: z(H) for k in ("dt_bias", "gamma_bias", "omega_bias", "mix_r_bias", "mix_theta_bias",
+                                  "mix_k_prev_bias", "mix_k_curr_bias")}
+        kern = _kernels(lambda: sb.mixer_decode_step_b200(
+            z(b, H, P), z(b, H, 13), z(b, H, 4, N), z(b, H, P), z(H, P), initial_states=z(b, H, P, 2 * N),
+            B_prev=z(b, H, 2 * N), U_prev=z(b, H, P), dt_min=1e-4, dt_max=0.1, r_min=0.9, r_max=1.0, theta_bound=3.0,
+            k_max=0.5, eps=1e-8, b_scale=z(H, 2, N), c_scale=z(H, 2, N), **bias))
+        return [g[0] for n, g in kern if "decode_step" in n][-1]
+
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert [grid(N) for N in (64, 1024, 64)] == [3 * sms, grid(1024), 3 * sms]
+    assert grid(1024) in (sms, 2 * sms)
