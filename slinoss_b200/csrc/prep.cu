@@ -1170,11 +1170,15 @@ static int prep_fwd_impl(const slx_prep_shape *s, const void *value, const void 
                              s->value_stride * (long long)sizeof(T_) | s->bc_stride * (long long)sizeof(T_);
       al = bits % 16 == 0 ? 16 : bits % 8 == 0 ? 8 : 0;
     }
+    // the rows of the any-width kernel, and the scales that it reads in the same vectors
+    const int vec = aligned16(pp.b_scale) && aligned16(pp.c_scale) ? pick_vec<T_>(s, {value, bc, U, B, C}) : 1;
     if (al && G) {
       rc = al == 16 ? launch_prep_fwd_lanes<T_, 16>(G, s, d, value, params, bc, pp, U, M, K, B, C, st)
                     : launch_prep_fwd_lanes<T_, 8>(G, s, d, value, params, bc, pp, U, M, K, B, C, st);
-    } else if (al == 16) {
+    } else if (vec == VFULL) {
       rc = launch_prep_fwd_any<T_, VFULL>(s, d, value, params, bc, pp, U, M, K, B, C, st);
+    } else if (vec == VFULL / 2) {
+      rc = launch_prep_fwd_any<T_, VFULL / 2>(s, d, value, params, bc, pp, U, M, K, B, C, st);
     } else {
       rc = launch_prep_fwd_any<T_, 1>(s, d, value, params, bc, pp, U, M, K, B, C, st);
     }

@@ -321,3 +321,32 @@ def test_decode_grid_follows_the_state_width():
     sms = torch.cuda.get_device_properties(0).multi_processor_count
     assert [grid(N) for N in (64, 1024, 64)] == [3 * sms, grid(1024), 3 * sms]
     assert grid(1024) in (sms, 2 * sms)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype,N,P,vec", [(F16, 36, 12, 4), (BF16, 512, 64, 4), (F32, 6, 2, 2)])
+def test_scanprep_rows_on_8_byte_boundaries(dtype, N, P, vec):
+    """Rows wider than a warp's slices, or of half a slice's multiple: the forward reads 8 bytes at a time."""
+    import slinoss_b200 as sb
+
+    b, T, H = 2, 37, 4
+    g = torch.Generator().manual_seed(N)
+    r = lambda *s: torch.randn(*s, generator=g).to(dtype).cuda()
+    hp = dict(n_heads=H, d_state=N, d_head=P, normalize_bc=True, dt_min=1e-4, dt_max=1e-1, r_min=0.9, r_max=1.0,
+              theta_bound=3.0, k_max=0.5, eps=1e-8, b_scale=r(H, 2, N), c_scale=r(H, 2, N),
+              **{k: r(H) for k in ("dt_bias", "gamma_bias", "omega_bias", "mix_r_bias", "mix_theta_bias",
+                                   "mix_k_prev_bias", "mix_k_curr_bias")})
+    per = 16 // (2 if dtype != F32 else 4)  # values of 16 bytes
+    value, bc = r(b, T, H * P + per // 2)[..., :H * P], r(b, T, H * 4 * N + per // 2)[..., :H * 4 * N].view(b, T, H, 4, N)
+    params = r(b, T, H * 13)
+    call = lambda: sb.scanprep_b200(value, params, bc, **hp)
+    names = [n for n, _ in _kernels(call) if "scanprep_fwd" in n]
+    assert len(names) == 1 and f", {vec}, 16>" in names[0], names
+    got = call()
+    x = bc.double()
+    x = x * torch.rsqrt(x.square().mean(-1, keepdim=True) + 1e-5)
+    want = x * torch.cat([hp["b_scale"], hp["c_scale"]], 1).double()[None, None]
+    want = want.view(b, T, H, 2, 2, N).permute(3, 0, 2, 1, 5, 4).reshape(2, b, H, T, 2 * N)
+    assert torch.equal(got.U, value.view(b, T, H, P).transpose(1, 2))
+    for a, w in zip((got.B, got.C), want):  # one rounding of the result; fp32: of each of its few operations
+        assert (a.double() - w).norm() < (1e-6 if dtype == F32 else 2.0 ** -8) * w.norm()
