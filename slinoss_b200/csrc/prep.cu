@@ -639,7 +639,8 @@ __global__ void __launch_bounds__(256, 2) scanprep_bwd_kernel(const T *__restric
         const bool is_square = !(threadIdx.x & 1);  // which of the four sums this lane finishes (group_sum4)
         group_sum4<G>(v, [&](float w) { return is_square ? rsqrtf(w * inv_n + 1e-5f) : w * inv_n; });
         const float2 rs = make_float2(v[0], v[1]);
-        const float2 cc = make_float2(-rs.x * rs.x * rs.x * v[2], -rs.y * rs.y * rs.y * v[3]);
+        // (r v first: r^3 alone leaves the range of fp32 for rows of magnitude 1e13)
+        const float2 cc = make_float2(-(rs.x * v[2]) * (rs.x * rs.x), -(rs.y * v[3]) * (rs.y * rs.y));
 #pragma unroll
         for (int e = 0; e < VEC; ++e) {
           const float2 x = x_of(e), dy = dy_of(e);

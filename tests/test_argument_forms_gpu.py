@@ -350,3 +350,27 @@ def test_scanprep_rows_on_8_byte_boundaries(dtype, N, P, vec):
     assert torch.equal(got.U, value.view(b, T, H, P).transpose(1, 2))
     for a, w in zip((got.B, got.C), want):  # one rounding of the result; fp32: of each of its few operations
         assert (a.double() - w).norm() < (1e-6 if dtype == F32 else 2.0 ** -8) * w.norm()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [BF16, F32])
+def test_scanprep_gradient_of_huge_rows(dtype):
+    """RMS norm does not see the scale of its row: the gradient is that of the scaled-down row, scaled down."""
+    import slinoss_b200 as sb
+
+    b, T, H, P, N = 1, 8, 2, 16, 16
+    g = torch.Generator().manual_seed(4)
+    r = lambda *s: torch.randn(*s, generator=g).to(dtype).cuda()
+    hp = dict(n_heads=H, d_state=N, d_head=P, normalize_bc=True, dt_min=1e-4, dt_max=1e-1, r_min=0.9, r_max=1.0,
+              theta_bound=3.0, k_max=0.5, eps=1e-8, b_scale=r(H, 2, N), c_scale=r(H, 2, N),
+              **{k: r(H) for k in ("dt_bias", "gamma_bias", "omega_bias", "mix_r_bias", "mix_theta_bias",
+                                   "mix_k_prev_bias", "mix_k_curr_bias")})
+    value, params, bc, dB = r(b, T, H * P), r(b, T, H * 13), r(b, T, H, 4, N), r(b, H, T, 2 * N)
+
+    def grad(scale):
+        x = (bc * scale).requires_grad_(True)
+        return torch.autograd.grad(sb.scanprep_b200(value, params, x, **hp).B, x, dB)[0].double() * scale
+
+    # powers of two: the two differ by the norm's eps (1e-5 of x^2 = 1) and by the rounding of the result
+    a, w = grad(2.0 ** 56), grad(2.0 ** 10)
+    assert (a - w).norm() < (1e-6 if dtype == F32 else 2.0 ** -8) * w.norm()
