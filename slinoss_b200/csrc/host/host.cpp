@@ -448,8 +448,13 @@ bool prep_params_plain(const std::vector<Tensor> &pars, bool normalize, const at
   if (pars.size() < n) return false;
   for (size_t i = 0; i < n; ++i) {
     const Tensor &t = pars[i];
-    if (!t.defined() || t.device() != dev || code_of(t.scalar_type()) < 0 || t.numel() != (i < 7 ? H : 2 * H * N))
-      return false;
+    if (!t.defined() || t.device() != dev || code_of(t.scalar_type()) < 0) return false;
+    // biases (H) or (1, H), scales (H, 2, N) or (H, 2 N)
+    const int64_t n_dim = t.dim();
+    const bool ok = i < 7 ? n_dim >= 1 && t.size(-1) == H && t.numel() == H
+                          : t.numel() == 2 * H * N && ((n_dim == 3 && t.size(0) == H && t.size(1) == 2) ||
+                                                       (n_dim == 2 && t.size(0) == H));
+    if (!ok) return false;
   }
   return true;
 }

@@ -374,3 +374,22 @@ def test_scanprep_gradient_of_huge_rows(dtype):
     # powers of two: the two differ by the norm's eps (1e-5 of x^2 = 1) and by the rounding of the result
     a, w = grad(2.0 ** 56), grad(2.0 ** 10)
     assert (a - w).norm() < (1e-6 if dtype == F32 else 2.0 ** -8) * w.norm()
+
+
+@pytest.mark.gpu
+def test_scanprep_refuses_parameters_of_other_shapes():
+    import slinoss_b200 as sb
+
+    b, T, H, P, N = 1, 3, 3, 16, 8
+    r = lambda *s: torch.randn(*s, device="cuda")
+    names = ("dt_bias", "gamma_bias", "omega_bias", "mix_r_bias", "mix_theta_bias", "mix_k_prev_bias",
+             "mix_k_curr_bias")
+    pars = dict({k: r(H) for k in names}, b_scale=r(H, 2, N), c_scale=r(H, 2, N))
+    call = lambda **kw: sb.scanprep_b200(
+        r(b, T, H * P), r(b, T, H * 13), r(b, T, H, 4, N), n_heads=H, d_state=N, d_head=P, dt_min=1e-4, dt_max=1e-1,
+        r_min=0.9, r_max=1.0, theta_bound=3.0, k_max=0.5, eps=1e-8, **{**pars, **kw})
+    for kw in (dict(dt_bias=r(1)), dict(mix_r_bias=r(())), dict(omega_bias=r(1, H)), dict(b_scale=r(H, 2 * N))):
+        call(**kw)
+    for kw in (dict(dt_bias=r(H, 1)), dict(b_scale=r(2 * H * N)), dict(c_scale=r(2, H, N)), dict(c_scale=r(H, 2, N + 1))):
+        with pytest.raises((ValueError, RuntimeError)):
+            call(**kw)
