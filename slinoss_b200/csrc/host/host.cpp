@@ -333,8 +333,8 @@ bool scan_inputs_plain(const Tensor &U, const Tensor &M, const Tensor &K, const 
 // and one CTA fills an SM (2, 8, T 2048, N 64, forward + backward: 466 us against 286), below it the chunk states and
 // the state pass weigh more (32 tokens: 320).  A CTA's time is proportional to its tokens, though, so calls with less
 // than a chunk of 64 per SM are tiled in 32 (1, 2, T 500, N 64: 99 -> 66 us; 1, 8, T 1024: 109 -> 105).
-int64_t cuda_core_chunk(int64_t heads, int64_t T) {
-  return heads * ((T + 63) / 64) < at::cuda::getCurrentDeviceProperties()->multiProcessorCount ? 32 : 64;
+int64_t cuda_core_chunk(int64_t heads, int64_t T, const at::Device &dev) {
+  return heads * ((T + 63) / 64) < at::cuda::getDeviceProperties(dev.index())->multiProcessorCount ? 32 : 64;
 }
 
 // (U, M, K, B, C) -> [Y] or [Y, final, B_last, U_last] in the activation dtype, with autograd.  None: not the
@@ -348,7 +348,7 @@ std::optional<std::vector<Tensor>> v2x2ssd(const Tensor &U, const Tensor &M, con
   const bool tensor_cores = U.scalar_type() != at::kFloat && P == 64 && D % 64 == 0 && D <= 256;
   if (L > 0 && retile && tensor_cores) L = 128;
   if (L != 16 && L != 32 && L != 64 && L != 128) return std::nullopt;
-  if (retile && !tensor_cores) L = cuda_core_chunk(U.size(0) * U.size(1), U.size(2));
+  if (retile && !tensor_cores) L = cuda_core_chunk(U.size(0) * U.size(1), U.size(2), U.device());
   const at::ScalarType final_type = final_type_in.value_or(U.scalar_type());
   if (code_of(final_type) < 0) return std::nullopt;
   const ScanDims d = scan_dims(U, B, L);
