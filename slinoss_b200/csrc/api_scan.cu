@@ -189,10 +189,10 @@ static std::atomic<int> g_max_ctas{0};
 static int sm_count() {
   static std::atomic<int> cached[64];
   int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return kB200Sms;
   int n = cached[dev].load(std::memory_order_relaxed);
   if (n == 0) {
-    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = kB200Sms;
     cached[dev].store(n, std::memory_order_relaxed);
   }
   return n;

@@ -47,6 +47,10 @@ inline int check_launch(const char *what) {  // cudaGetLastError -> status
     if (!(cond)) return ::slx::fail(code, __VA_ARGS__); \
   } while (0)
 
+// SMs of a B200.  The tile rules size grids by it as a constant, since the workspace queries that follow the same rules
+// are answered without a device; another count makes a grid uneven, not wrong.
+constexpr int kB200Sms = 148;
+
 inline cudaStream_t as_stream(void *s) { return reinterpret_cast<cudaStream_t>(s); }
 
 // Per-kernel set-up that the driver keeps per device is done once per (kernel, device) and

@@ -790,7 +790,9 @@ static int check_conv(const slx_conv_shape *s, ConvDims *d) {
 // halo per tile and the backward's partial sums stop mattering.  (b2 T1000 C512: 63-token walks left 32 blocks for
 // 148 SMs, 0.038 ms.)
 constexpr int kConvTileFwd = 64, kConvTileBwd = 128;
-constexpr long long kConvResident = 148LL * 4 * kConvThreads;  // threads in flight with four rings to an SM
+// threads in flight with the forward's ring, of which four fit an SM; of the backward's (64 KB) three do, so its tiles
+// stop growing while the last shares still make a thin second wave
+constexpr long long kConvResident = kB200Sms * 4LL * kConvThreads;
 constexpr size_t kNoAllocFloats = 1u << 20;  // partial sums that slx_cconv1d_bwd_noalloc can hold
 
 static int conv_tile(const ConvDims &d, int vec, bool bwd) {

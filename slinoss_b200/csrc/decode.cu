@@ -9,9 +9,9 @@
 //   z'[p][n]        = rho z[p][n] + k^p u_prev[p] b_prev[n] + k^c u[p] b[n]
 //   y[p]            = sum_n Re(conj(c[n]) z'[p][n])
 //   out[p]          = (y[p] + skip[p] u[p]) * silu(gate[p])
-// One CTA per (batch, head).  The fp32 state (P x 2N) is the only large operand: every warp
-// streams whole rows with 16-byte accesses (a row is contiguous) and reduces its own y[p] by
-// shuffles, so there is no cross-warp reduction and no atomics.
+// The fp32 state (P x 2N) is the only large operand: a streaming warp owns four of every 32 rows, reads and
+// writes them with 16-byte accesses (a row is contiguous) and reduces their y[p] by shuffles, so there is no
+// cross-warp reduction and no atomics.
 // The step is bound by HBM: 2 * P * 2N * 4 bytes per (batch, head).  The CTAs that fit the GPU
 // walk over the heads: eight warps stream states, four others meanwhile prepare the operands of
 // the next head (a serial chain of norms and the coefficient map, as long as the streaming

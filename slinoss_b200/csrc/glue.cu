@@ -253,7 +253,7 @@ static int check_glue(const slx_glue_shape *s, GlueDims *d) {
 // 1024, the last third of it on half the SMs).  Backward: the walk also sums d_skip, one partial row per tile; it
 // grows from 4 to 16 tokens (where the partials are 2 % of the traffic) while the threads of the call overfill the GPU.
 static void glue_tile(GlueDims *d, bool bwd) {
-  const long long C8 = (long long)d->H * d->P / 8, resident = 148LL * 1024;
+  const long long C8 = (long long)d->H * d->P / 8, resident = (long long)kB200Sms * 1024;
   int tile = 4;
   while (bwd && tile < 16 && C8 * d->batch * ((d->T + tile - 1) / tile) > resident) tile *= 2;
   d->tile = tile;

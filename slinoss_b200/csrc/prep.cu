@@ -981,7 +981,7 @@ static int launch_prep_fwd_any(const slx_prep_shape *s, const PrepDims &d, const
   constexpr int G = prep_group<VEC>();
   long long n_rows = (long long)d.batch * d.H * d.T;
   long long blocks = (n_rows + 255) / 256;
-  if (blocks > 148LL * 32) blocks = 148LL * 32;
+  if (blocks > kB200Sms * 32LL) blocks = kB200Sms * 32LL;
   scanprep_fwd_any_kernel<T, VEC, G><<<(unsigned)blocks, 256, 0, st>>>(
       (const T *)value, (const T *)params, (const T *)bc, pp, (T *)U, M, K, (T *)B, (T *)C, d, hp);
   return check_launch("scanprep_fwd");
@@ -990,7 +990,7 @@ static int launch_prep_fwd_any(const slx_prep_shape *s, const PrepDims &d, const
 // Rows per CTA of the one-slice forward: as many as make the grid whole waves of three CTAs per SM, at most 256 (one
 // per thread in the coefficient map), at least 32.
 static int prep_rows_per_cta(long long n_rows) {
-  const long long slots = 148LL * 3, waves = (n_rows + slots * 256 - 1) / (slots * 256);
+  const long long slots = kB200Sms * 3LL, waves = (n_rows + slots * 256 - 1) / (slots * 256);
   long long r = (n_rows + slots * waves - 1) / (slots * waves);
   r = (r + 7) / 8 * 8;
   return (int)(r < 32 ? 32 : r);
@@ -1037,7 +1037,7 @@ static PrepBwdPlan prep_bwd_plan(const slx_prep_shape *s, int VEC) {
   p.kmax = (s->N + VEC * p.G - 1) / (VEC * p.G);
   // Tiles of at most 256 rows (one per thread in the coefficient part), as many as make whole waves of two CTAs per
   // SM, of 32 rows at least.
-  const long long slots = 148LL * 2, bh = (long long)s->batch * s->heads;
+  const long long slots = kB200Sms * 2LL, bh = (long long)s->batch * s->heads;
   const long long waves = (bh * ((s->T + 255) / 256) + slots - 1) / slots;
   long long n = waves * slots / bh;
   if (n < (s->T + 255) / 256) n = (s->T + 255) / 256;

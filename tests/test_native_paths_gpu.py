@@ -39,14 +39,14 @@ def test_cuda_core_chunks_as_requested(L, T, N, P, dtype, monkeypatch):
     monkeypatch.setattr(sb, "v2x2ssd_b200", lambda *a, **kw: op(*a, retile=False, **kw))
     inp = make_scan_inputs(1, 2, T, N, P, dtype, seed=L + T, streaming=True, with_init=True)
     errs = _scan_errors(inp, lambda: run_b200_fwd_bwd(inp, L))
-    assert max(errs.values()) < (2e-4 if dtype == F32 else 2e-2), errs
+    assert max(errs.values()) < (1e-5 if dtype == F32 else 2e-2), errs
 
 
 @pytest.mark.parametrize("b,h,T", [(1, 1, 40), (2, 80, 65)])   # tiled in 32 tokens; in 64
 def test_cuda_core_tiling_follows_the_work(b, h, T):
     inp = make_scan_inputs(b, h, T, 4, 8, F32, seed=h, streaming=True, with_init=True)
     errs = _scan_errors(inp, lambda: run_b200_fwd_bwd(inp, 128))
-    assert max(errs.values()) < 2e-4, errs
+    assert max(errs.values()) < 1e-5, errs
 
 
 @pytest.mark.parametrize("dtype,N,T", [(BF16, 64, 129), (F16, 128, 256)])
