@@ -2,6 +2,7 @@
 
 from __future__ import annotations
 
+import contextlib
 import ctypes
 
 import pytest
@@ -393,3 +394,31 @@ def test_scanprep_refuses_parameters_of_other_shapes():
     for kw in (dict(dt_bias=r(H, 1)), dict(b_scale=r(2 * H * N)), dict(c_scale=r(2, H, N)), dict(c_scale=r(H, 2, N + 1))):
         with pytest.raises((ValueError, RuntimeError)):
             call(**kw)
+
+
+@pytest.mark.gpu
+def test_saved_tensors_may_come_back_with_other_strides():
+    """Column slices that a saved-tensor hook moves away come back dense: the backward takes the distances it gets."""
+    import slinoss_b200 as sb
+
+    b, T, H, P, N = 2, 7, 2, 16, 8
+    g = torch.Generator().manual_seed(6)
+    r = lambda *s: torch.randn(*s, generator=g).to(BF16).cuda()
+    names = ("dt_bias", "gamma_bias", "omega_bias", "mix_r_bias", "mix_theta_bias", "mix_k_prev_bias",
+             "mix_k_curr_bias")
+    pars = dict({k: r(H) for k in names}, b_scale=r(H, 2, N), c_scale=r(H, 2, N))
+    value, params, gate = r(b, T, 48)[..., 8:40], r(b, T, 40)[..., 8:34], r(b, T, 48)[..., 16:]
+    bc, w, skip = r(b, T, 80)[..., 8:72].view(b, T, H, 4, N), r(H * P, 4), r(H * P)
+
+    def grads(hooks):
+        leaves = [t.detach().requires_grad_(True) for t in (value, params, bc, gate)]
+        with hooks:
+            x, _ = sb.cconv1d_b200(leaves[0], w, None, activation="silu")
+            o = sb.scanprep_b200(x, leaves[1], leaves[2], n_heads=H, d_state=N, d_head=P, normalize_bc=True, dt_min=1e-4,
+                                 dt_max=1e-1, r_min=0.9, r_max=1.0, theta_bound=3.0, k_max=0.5, eps=1e-8, **pars)
+            y = sb.v2x2ssd_b200(o.U, o.M, o.K, o.B, o.C, chunk_size=16)
+            out = sb.gate_skip_b200(y, o.U, leaves[3], skip)
+        return torch.autograd.grad(out, leaves, torch.ones_like(out))
+
+    moved = grads(torch.autograd.graph.saved_tensors_hooks(lambda t: t.contiguous().cpu(), lambda t: t.cuda()))
+    assert all(torch.equal(x, y) for x, y in zip(moved, grads(contextlib.nullcontext())))
