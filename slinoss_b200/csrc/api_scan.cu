@@ -135,12 +135,13 @@ static bool all_aligned16(std::initializer_list<const void *> ptrs) {
 // verified that the combination exists.
 static bool use_tc(const slx_scan_shape *s) { return s->starts_dtype != SLX_F32; }
 
-// Tensor map of a (BH, T, width) half tensor for boxes of [rows][64 columns], 128-byte swizzle.
-template <typename T>
+// Tensor map of a (BH, T, width) half tensor for boxes of [rows][64 columns], 128-byte swizzle, or [rows][32 columns],
+// 64-byte swizzle.
+template <typename T, int BOX_COLS = 64>
 static int make_tile_map(CUtensorMap *map, const void *base, int BH, int T_, int width, int box_rows, const char *what) {
   const cuuint64_t dims[3] = {(cuuint64_t)width, (cuuint64_t)T_, (cuuint64_t)BH};
   const cuuint64_t strides[2] = {(cuuint64_t)width * sizeof(T), (cuuint64_t)T_ * width * sizeof(T)};
-  const cuuint32_t box[3] = {64u, (cuuint32_t)box_rows, 1u};
+  const cuuint32_t box[3] = {(cuuint32_t)BOX_COLS, (cuuint32_t)box_rows, 1u};
   const cuuint32_t estr[3] = {1u, 1u, 1u};
   const CUtensorMapDataType dt =
       std::is_same<T, __half>::value ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
@@ -160,7 +161,8 @@ static int make_tile_map(CUtensorMap *map, const void *base, int BH, int T_, int
     encode_fn.store(encode, std::memory_order_release);
   }
   CUresult r = encode(map, dt, 3, const_cast<void *>(base), dims, strides, box, estr,
-                                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                                      CU_TENSOR_MAP_INTERLEAVE_NONE,
+                                      BOX_COLS == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
                                       CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return fail(SLX_E_UNSUPPORTED, "%s: tensor map could not be encoded (CUresult %d)", what, (int)r);
   return SLX_OK;
@@ -254,12 +256,8 @@ static int launch_scan_bwd_tc(const ScanDims &d, const ScanBwdArgs<T> &a, cudaSt
   int rc = set_smem(kern, smem);
   if (rc) return rc;
   ScanBwdMaps maps;
-  rc = make_tile_map<T>(&maps.C, a.C, d.BH, d.T, d.D, 128, "chunk_scan_bwd");
-  if (rc) return rc;
-  rc = make_tile_map<T>(&maps.B, a.B, d.BH, d.T, d.D, 128, "chunk_scan_bwd");
-  if (rc) return rc;
-  if ((rc = make_tile_map<T>(&maps.dC, a.dC, d.BH, d.T, d.D, 128, "chunk_scan_bwd"))) return rc;
-  if ((rc = make_tile_map<T>(&maps.dB, a.dB, d.BH, d.T, d.D, 128, "chunk_scan_bwd"))) return rc;
+  if ((rc = make_tile_map<T, 32>(&maps.C, a.C, d.BH, d.T, d.D, 128, "chunk_scan_bwd"))) return rc;
+  if ((rc = make_tile_map<T, 32>(&maps.B, a.B, d.BH, d.T, d.D, 128, "chunk_scan_bwd"))) return rc;
   kern<<<dim3(d.NC, d.BH), kTcBwdThreads, smem, st>>>(a, maps);
   return check_launch("chunk_scan_bwd_tc");
 }

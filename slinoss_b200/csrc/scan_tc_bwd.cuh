@@ -1,38 +1,40 @@
 // Tensor-core per-chunk backward of the v2x2ssd scan (chunk 128, P 64, half
 // inputs, fp32 state).  Same mathematics as chunk_scan_bwd_kernel in
 // scan_simt.cuh; every contraction runs on tcgen05 with fp32 accumulators in
-// tensor memory.  One CTA of 16 worker warps and an issuing warp per (chunk, batch*head), one CTA per SM.
+// tensor memory.  One CTA of 8 warps per (chunk, batch*head), two CTAs per SM.
 //
-// Operands per 64-column slab of the state (half precision, every one rounded once from fp32 or as it is stored):
-//   Qbar_t = c_t conj(phi_t),  kappa_s = gamma_s b_s conj(phi_{s+1}),  Bhat_s = w_s b_s,  Z0,  Lambda
-// with w_s = gamma_s p_{L-1}/p_{s+1} (k^c for the last token), and per chunk
-//   dS' = decay * (dY U^T),   Ye_t = exp(lp_t) dY_t,   U
+// Phases are taken relative to the end of the chunk, f_t = phi_t conj(phi_{L-1}), so that Lambda, Z0, U and dY enter
+// their products as they are stored.  Operands per 32-column slab of the state (half precision, every one rounded once
+// from fp32 or as it is stored):
+//   Q_t = c_t conj(f_t),  kappa_s = gamma_s b_s conj(f_{s+1}),  Z0,  Lambda
+// and per chunk  dS' = decay * (dY U^T),  dY,  U.  With es_s = p_{L-1}/p_{s+1} in magnitude, p_t = exp(lp_t) phi_t:
+//   dC_t = f_t (dS' kappa)_t + p_t (dY Z0)_t + (k^c_t G_tt) b_t
+//   xi_s = (dS'^T Q)_s + es_s (U Lambda)_s,   dB_s = conj(gamma_s) f_{s+1} xi_s + conj(k^c_s G_ss) c_s
+//   dU   = S'^T dY + es (kappa Lambda^T)
+// Scales and rotations of a row are applied to the fp32 accumulators, never to an operand that is rounded already.
 //
-// Tensor-memory map (fp32 columns):
-//   [  0,128)  S^T = kappa Qbar^T                    (accumulated over the slabs)
-//   [128,192)  dU, increment path:  Bhat Lambda^T    (accumulated over the slabs)
-//   [192,448)  two buffers, one per slab parity, of  dq = dS' kappa + Ye Z0  and  X = dS'^T Qbar
-//              (buffer 0 holds G = dY U^T first, and S'^T dY at the end)
-//   [448,512)  UL = U Lambda of one slab
+// Slot 127 of the source axis (U, kappa) holds the token in front of the chunk: the merged-tap column of token 127 is
+// empty (no query follows it), and that row of dS', dS'^T Q, U Lambda, kappa Lambda^T and S'^T dY is then what the carry
+// gradients need.  Token 127's own increment path, u_127 . Lambda and (k^c b_127) . Lambda, and its diagonal terms are
+// summed on the CUDA cores.
 //
-// The source token in front of the chunk (b_{-1}, u_{-1}) borrows key slot 127,
-// whose own merged-tap column is empty (no query follows the last token):
-//   dS'[t][127] = exp(lp_t - lp_0) dY_t.u_{-1},   kappa_127 = k^p_0 b_{-1} conj(phi_0)
-// so that row 127 of X is the column sum the carry gradient needs, the boundary term of dq comes out of the same
-// product, and row 127 of S'^T dY is the dU carried to the previous token.  What that token gets from the increment
-// path, u_{-1} . Lambda and (w_{-1} b_{-1}) . Lambda, is summed on the CUDA cores (carry helpers below).
+// Tensor-memory map (256 fp32 columns):
+//   [  0,128)  G = dY U^T, then S^T = kappa Q^T       (accumulated over the slabs)
+//   [128,192)  kappa Lambda^T                         (accumulated over the slabs)
+//   [192,224)  dS'^T Q of a slab, then dS' kappa      [224,256)  U Lambda, then dY Z0;  [192,256) at the end S'^T dY
 //
-// What bounds it: neither HBM (35 %) nor the tensor pipe (a slab's 32 products take about 2 K cycles) but the
-// rotations and the epilogue on the CUDA cores, so everything else has to run in their shadow.  The tiles of kappa,
-// Qbar, Lambda and Z0 and the accumulators dq and X are double-buffered: while the tensor core works on slab i+1, all
-// warps are in the epilogue of slab i and the staging of slab i+2.  Bhat and UL have one buffer, which is what shared
-// and tensor memory still hold: their two products are issued behind the epilogue of the slab before and run under
-// the staging of the next.  dY gives its tile to Ye and is fetched again (from L2) for the last product.  The raw
-// (C, B) slab travels by TMA one slab ahead; dC / dB leave by TMA from the operand tiles.
-// 8192 chunks of D 256: 1.207 ms (1.395 with single buffers, where staging, products and epilogue of a slab took
-// turns).  Scaling the increment path's operands to meet the score path's (X += round(es u) round(conj(phi_{L-1})
-// Lambda), dU from kappa and the same Lambda) needs neither Bhat nor UL and took 1.095 ms, but rounds two operands a
-// second time: with |m| in (0.99, 1) and a large gradient of the final state dK was 2.9 times as far from float64.
+// Columns of kappa, Q, Lambda and Z0 are stored (re, re, re, re, im, im, im, im) inside each group of four complex
+// values: sums over the state do not see the order, and the accumulators then hold real and imaginary parts of two
+// values side by side, which is what the packed fp32 arithmetic (two fmas per instruction) takes.
+//
+// What bounds it: neither HBM (46 %) nor the tensor pipe (12 %) but instruction issue and the latencies between a
+// chunk's phases (loads and prefix, slabs, tail).  8192 chunks of D 256: 1.044 ms.  One CTA of 16 worker warps per SM
+// with 64-column slabs and two buffers for every operand took 1.205 ms: its phases followed one another and nothing
+// filled their latencies.  Two CTAs of 8 warps run different phases at the same time.  They fit because the slabs are 32
+// columns wide with one buffer, dS'^T Q / U Lambda and dS' kappa / dY Z0 take turns in the same 64 accumulator columns,
+// and dC / dB leave from registers (whole 32-byte sectors).  Measured on the way: a ninth warp that issues the products
+// leaves 96 registers to a thread, and the spills cost more than the issuing (1.097 against 0.997 ms); one thread that
+// waits for the products and a CTA barrier behind it 1.198 against 1.070 ms.
 //
 // Thread mapping: thread = (row 32*(warp%4)+lane, 16-byte chunks 2*(warp/4) and +1 of the slab), the tensor-memory
 // lane mapping, for staging and epilogue alike, so that the raw b, c of a cell stay in registers from one to the other.
@@ -42,74 +44,88 @@
 
 namespace slx {
 
-// tensor maps of the raw C and B operands (loads) and of dC, dB (stores): (D, T, BH), boxes of 64 columns x 128 tokens
+// tensor maps of the raw C and B operands: (D, T, BH), boxes of 32 columns x 128 tokens, 64-byte swizzle
 struct alignas(64) ScanBwdMaps {
-  CUtensorMap C, B, dC, dB;
+  CUtensorMap C, B;
 };
 
-constexpr int kTcBwdWorkers = 512, kTcBwdThreads = kTcBwdWorkers + 32;  // the last warp issues products and loads
-constexpr uint32_t kBwdStage = 49152;  // [kappa 16 K][Qbar 16 K][Lambda 8 K][Z0 8 K], one per slab parity
-constexpr uint32_t kBwdScalars = 81920 + 2 * kBwdStage + 32768;
-constexpr size_t scan_bwd_tc_smem_bytes() { return 1024 + kBwdScalars + 17920; }
-constexpr int kTmR = 128, kTmSlab = 192, kTmUL = 448, kTmU = kTmSlab;  // accumulator columns (S^T at 0)
+constexpr int kTcBwdThreads = 256;
+constexpr uint32_t kBwdScalars = 106496;
+constexpr size_t scan_bwd_tc_smem_bytes() { return kBwdScalars + 8320; }
+constexpr int kTmR = 128, kTmX = 192, kTmUL = 224, kTmU = kTmX;  // accumulator columns (G / S^T at 0)
 
-// S^T -> S'^T of one 32-column block: row s, columns t = c0 + i.  lpb = lp_{s+1} (lp_0 for the boundary slot, whose
-// row takes every column).  FAST factors exp(lp_t - lpb) through the table e3[t] = exp(lp_t - lp_{32 (t / 32)}).
-template <bool FAST>
-__device__ __forceinline__ void decay_mask32_rows(float (&v)[32], int c0, int s, bool boundary, float lpb,
-                                                  const float *lp, const float *e3, float diag) {
-  const float rf = FAST ? __expf(lp[c0] - lpb) : 0.f;
+// (a + i b) * cell, packed as four real parts and four imaginary parts
+template <typename T>
+__device__ __forceinline__ uint4 rotate_cell_split(const CellF &c, float a, float b) {
+  uint4 out;
+  uint32_t *o = reinterpret_cast<uint32_t *>(&out);
 #pragma unroll
-  for (int i = 0; i < 32; ++i) {
-    const int t = c0 + i;
-    const float f = FAST ? rf * e3[t] : __expf(lp[t] - lpb);
-    v[i] = (t > s || boundary) ? v[i] * f : (t == s ? diag : 0.f);
+  for (int q = 0; q < 2; ++q) {
+    const float2 re = __ffma2_rn(both(a), c.re[q], __fmul2_rn(both(-b), c.im[q]));
+    const float2 im = __ffma2_rn(both(a), c.im[q], __fmul2_rn(both(b), c.re[q]));
+    o[q] = umma::pack2(re.x, re.y, T());
+    o[2 + q] = umma::pack2(im.x, im.y, T());
   }
+  return out;
+}
+__device__ __forceinline__ uint4 split_cell(uint4 v) {  // (re, im) pairs -> four real parts, four imaginary parts
+  return make_uint4(__byte_perm(v.x, v.y, 0x5410), __byte_perm(v.z, v.w, 0x5410), __byte_perm(v.x, v.y, 0x7632),
+                    __byte_perm(v.z, v.w, 0x7632));
+}
+template <typename T>
+__device__ __forceinline__ CellF unpack_cell_split(uint4 v) {  // of a cell packed by rotate_cell_split
+  return CellF{{umma::unpack2(v.x, T()), umma::unpack2(v.y, T())}, {umma::unpack2(v.z, T()), umma::unpack2(v.w, T())}};
+}
+__device__ __forceinline__ float2 tm_pair(const uint32_t *r) {
+  return make_float2(__uint_as_float(r[0]), __uint_as_float(r[1]));
 }
 
 template <typename T>
-__global__ void __launch_bounds__(kTcBwdThreads, 1) chunk_scan_bwd_tc_kernel(ScanBwdArgs<T> a,
+__global__ void __launch_bounds__(kTcBwdThreads, 2) chunk_scan_bwd_tc_kernel(ScanBwdArgs<T> a,
                                                                               const __grid_constant__ ScanBwdMaps maps) {
   constexpr int L = kTcL, P = kTcP;
-  extern __shared__ unsigned char smem_raw[];
-  unsigned char *base =
-      reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  unsigned char *tYe = base;                   // [t][p]  dY until G is done, then Ye
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  unsigned char *base = smem_raw;
+  unsigned char *tdY = base;                   // [t][p]
   unsigned char *tU = base + 16384;            // [s][p]
   unsigned char *tdS = base + 32768;           // 2 x [t][64 s]  dS', at the end 2 x [s][64 t]  S'^T
-  unsigned char *tBh = base + 65536;           // [s][d]  Bhat
-  unsigned char *tSt = base + 81920;           // two staging buffers
-  unsigned char *sC = tSt + 2 * kBwdStage;     // raw C slab (swizzled tile), by TMA; dY once more at the end
-  unsigned char *sB = sC + 16384;              // raw B slab
+  unsigned char *tK = base + 65536;            // [s][32 d]  kappa
+  unsigned char *tQ = base + 73728;            // [t][32 d]  Q
+  unsigned char *tLm = base + 81920;           // [p][32 d]  Lambda
+  unsigned char *tZ = base + 86016;            // [p][32 d]  Z0
+  unsigned char *sC = base + 90112;            // raw C slab, by TMA; scratch of the tail
+  unsigned char *sB = base + 98304;            // raw B slab
   float *lp = reinterpret_cast<float *>(base + kBwdScalars);
-  float *gd = lp + L;                          // G[t][t]
-  float *gm1 = gd + L;                         // dY_t . u_{-1}
-  float *um1 = gm1 + L;                        // 64   u_{-1}
-  float *duc = um1 + 64;                       // 64   (w_{-1} b_{-1}) . Lambda[p]
-  float *e2 = duc + 64;                        // 128  decay table of dS' (decay_mask32)
-  float *e3 = e2 + L;                          // 128  decay table of S'^T
-  float *xb = e3 + L;                          // 256  row 127 of X, all slabs
-  float *ulf = xb + 256;                       // 256  u_{-1} . Lambda, all slabs
-  float *ulw = ulf + 256;                      // [16][64] per-warp partials of u_{-1} . Lambda
-  float2 *gA = reinterpret_cast<float2 *>(ulw), *bX = gA + L;  // (after the slabs)
-  float2 *ph = reinterpret_cast<float2 *>(ulw + 16 * 64);
-  float2 *mraw = ph + L, *kc = mraw + L, *kp = kc + L, *bc = kp + L, *gsum = bc + L;
-  float2 *bm1 = gsum + L;                      // 128  b_{-1}
-  float2 *bh1 = bm1 + 128;                     // 128  w_{-1} b_{-1}
-  float2 *misc = bh1 + 128;                    // [0] conj(b_127) . (u_127 . Lambda)   [1..4] dk^p_0, by warp   [5] zdot
-  __shared__ uint64_t bars[4];  // [0], [1] products of a slab, by parity; [2] G, then S'^T dY; [3] raw slab by TMA
-  __shared__ uint32_t tmem_slot;
+  float *tab = lp + L;                         // decay table of dS' (decay_table_entry), then of S'^T
+  float *gd = tab + L;                         // G[t][t]
+  float *um = gd + L;                          // 64   u_127
+  float *duc = um + 64;                        // 64   (k^c b_127) . Lambda[p]
+  float *xb = duc + 64;                        // 256  xi of the token in front of the chunk
+  float *ulf = xb + 256;                       // 256  u_127 . Lambda
+  float *ulw = ulf + 256;                      // [8][32] per-warp partials of u_127 . Lambda
+  float2 *mraw = reinterpret_cast<float2 *>(xb), *kc = reinterpret_cast<float2 *>(ulf),
+         *kp = reinterpret_cast<float2 *>(ulw);  // until the rows' coefficients are formed
+  float2 *ph = reinterpret_cast<float2 *>(ulw + 256);
+  float2 *bm1 = ph + L;                        // 128  b_{-1}
+  float2 *bh1 = bm1 + 128;                     // 128  k^c b_127
+  float2 *misc = bh1 + 128;                    // [0..3] dk^p_0, [4..7] sum conj(b_127) (u_127 . Lambda), by warp
+  uint64_t *bars = reinterpret_cast<uint64_t *>(misc + 8);  // [0] first, [1] second products of a slab; [2] G, then
+                                                            // S'^T dY; [3] raw slab by TMA
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 4);
+  static_assert(kBwdScalars + 4 * (3 * 128 + 2 * 64 + 3 * 256) + 8 * 3 * 128 + 64 + 4 * 8 + 4 <=
+                    scan_bwd_tc_smem_bytes(), "shared-memory layout");
+  // scratch of the tail, over the raw slabs
+  float2 *pgs = reinterpret_cast<float2 *>(sC), *pbs = pgs + L, *pcs = pbs + L;  // second column half: gA, bX; bc
+  float2 *bXs = pcs + 2 * L, *sums = bXs + L;  // sums: [0..3] g by warp, [4], [5] conj(kappa) xi of slot 127
 
   const ScanDims d = a.d;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const bool issuer = warp == kTcBwdWorkers / 32;
-  auto workers_sync = [] { asm volatile("bar.sync 2, 512;" ::: "memory"); };
   const int c = blockIdx.x, bh = blockIdx.y;
   const int t0 = c * L;
   const int valid = min(L, d.T - t0);
   const size_t tok0 = (size_t)bh * d.T + t0;
-  const int NB = d.D / 64;
-  const uint32_t bar0 = umma::smem_u32(&bars[0]), gbar = bar0 + 16, tbar = bar0 + 24;
+  const int NB = d.D / 32;
+  const uint32_t bar0 = umma::smem_u32(bars), gbar = bar0 + 16, tbar = bar0 + 24;
   constexpr int fmt = umma::HalfFmt<T>::value;
 
 #define SLX_STAMP(i) SLX_DIAG_STAMP(i)
@@ -120,57 +136,62 @@ __global__ void __launch_bounds__(kTcBwdThreads, 1) chunk_scan_bwd_tc_kernel(Sca
   float2 mreg[4];  // the prefix warp's multipliers, requested ahead of the bulk copies
   if (warp == 2) chunk_prefix_load4(a.M + tok0 * 2, valid, mreg);
   // U and dY land in their tiles by asynchronous copy (rows past the chunk end are zero-filled)
-  auto fetch_rows = [&](unsigned char *tile, const T *src) {
-    const int j = tid & 7, r0 = tid >> 3;
+  const int j8 = tid & 7, r8 = tid >> 3;
+  uint4 ub = make_uint4(0, 0, 0, 0);  // the thread that copies a cell of row 127: that cell of u_{-1}
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const int r = r0 + 64 * i;
-      const int rr = r < valid ? r : 0;
-      const uint32_t nbytes = r < valid ? 16u : 0u;
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(umma::smem_u32(tile + umma::swz_off(r, j))),
-                   "l"(src + (tok0 + rr) * P + 8 * j), "r"(nbytes)
-                   : "memory");
+  for (int i = 0; i < 4; ++i) {
+    const int r = r8 + 32 * i;
+    const int rr = r < valid ? r : 0;
+    const uint32_t nbytes = r < valid ? 16u : 0u;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(umma::smem_u32(tU + umma::swz_off(r, j8))),
+                 "l"(a.U + (tok0 + rr) * P + 8 * j8), "r"(nbytes)
+                 : "memory");
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(umma::smem_u32(tdY + umma::swz_off(r, j8))),
+                 "l"(a.dY + (tok0 + rr) * P + 8 * j8), "r"(nbytes)
+                 : "memory");
+  }
+  if (r8 == 31) {
+    if (t0 > 0) {
+      ub = *reinterpret_cast<const uint4 *>(a.U + (tok0 - 1) * P + 8 * j8);
+    } else if (a.Uprev) {
+      float v[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) v[e] = load_as_f(a.Uprev, a.prev_dtype, (size_t)bh * P + 8 * j8 + e);
+      ub = pack8<T>(v);
     }
-  };
-  if (!issuer) {
-    fetch_rows(tU, a.U);
-    fetch_rows(tYe, a.dY);
   }
   asm volatile("cp.async.commit_group;" ::: "memory");
-  // One raw (C, B) slab = two TMA boxes of [128 tokens][64 columns] into the swizzled staging tiles,
+  // One raw (C, B) slab = two TMA boxes of [128 tokens][32 columns] into the swizzled staging tiles,
   // issued by one thread; tokens past the end of the sequence arrive as zeros.
   auto prefetch_cb = [&](int sl) {
     umma::fence_smem_to_async();  // the tiles' earlier (generic) readers are behind a barrier
-    umma::mbar_expect_tx(tbar, 2u * 16384u);
-    umma::tma_load_3d(umma::smem_u32(sC), &maps.C, sl * 64, t0, bh, tbar);
-    umma::tma_load_3d(umma::smem_u32(sB), &maps.B, sl * 64, t0, bh, tbar);
+    umma::mbar_expect_tx(tbar, 2u * 8192u);
+    umma::tma_load_3d(umma::smem_u32(sC), &maps.C, sl * 32, t0, bh, tbar);
+    umma::tma_load_3d(umma::smem_u32(sB), &maps.B, sl * 32, t0, bh, tbar);
   };
-  if (tid == kTcBwdWorkers) {
-#pragma unroll
-    for (int i = 0; i < 4; ++i) umma::mbar_init(bar0 + 8 * i, 1);
+  if (tid == 0) {
+    umma::mbar_init(bar0, 2);      // commits of issue_first
+    umma::mbar_init(bar0 + 8, 3);  // and of issue_second
+    umma::mbar_init(gbar, 1);
+    umma::mbar_init(tbar, 1);
     umma::fence_mbar_init();
     umma::tma_prefetch_map(&maps.C);
     umma::tma_prefetch_map(&maps.B);
-    umma::tma_prefetch_map(&maps.dC);
-    umma::tma_prefetch_map(&maps.dB);
     prefetch_cb(0);
   }
   // Z0 / Lambda slab: one 8-value (16-byte) item per thread, prefetched into registers
-  const int zp = tid >> 3, zj = tid & 7;
+  const int zp = tid >> 2, zj = tid & 3;
   uint4 zr, lr;
   auto prefetch_zl = [&](int sl) {
-    zr = *reinterpret_cast<const uint4 *>(z0 + (size_t)zp * d.D + sl * 64 + 8 * zj);
-    lr = *reinterpret_cast<const uint4 *>(lam + (size_t)zp * d.D + sl * 64 + 8 * zj);
+    zr = *reinterpret_cast<const uint4 *>(z0 + (size_t)zp * d.D + sl * 32 + 8 * zj);
+    lr = *reinterpret_cast<const uint4 *>(lam + (size_t)zp * d.D + sl * 32 + 8 * zj);
   };
-  if (!issuer) prefetch_zl(0);
+  prefetch_zl(0);
 
-  if (issuer) {
-    __syncwarp();
-    umma::tmem_alloc(&tmem_slot, 512);
-  }
+  if (warp == 1) umma::tmem_alloc(tmem_slot, 256);
   if (warp == 2) chunk_prefix_fast128(mreg, lp, ph, mraw, &g_scan_bad);
-  if (tid >= 128 && tid < 256) {
-    int t = tid - 128;
+  if (tid >= 128) {
+    const int t = tid - 128;
     float2 vp = make_float2(0.f, 0.f), vc = vp;
     if (t < valid) {
       float4 k4 = *reinterpret_cast<const float4 *>(a.K + (tok0 + t) * 4);
@@ -179,183 +200,172 @@ __global__ void __launch_bounds__(kTcBwdThreads, 1) chunk_scan_bwd_tc_kernel(Sca
     }
     kp[t] = vp;
     kc[t] = vc;
-  } else if (tid >= 256 && tid < 320) {
-    int p = tid - 256;
-    float v = 0.f;
-    if (t0 > 0) v = to_f(a.U[(tok0 - 1) * P + p]);
-    else if (a.Uprev) v = load_as_f(a.Uprev, a.prev_dtype, (size_t)bh * P + p);
-    um1[p] = v;
-    duc[p] = 0.f;
-  } else if (tid >= 320 && tid < 320 + d.N) {
-    int n = tid - 320;
-    float2 bv = make_float2(0.f, 0.f);
-    if (t0 > 0) bv = load_pair<T>(a.B + (tok0 - 1) * d.D + 2 * n);
-    else if (a.Bprev) bv = load_as_f2(a.Bprev, a.prev_dtype, (size_t)bh * d.D + 2 * n);
-    bm1[n] = bv;
-  } else if (tid == 448) {
-    misc[5] = *reinterpret_cast<const float2 *>(a.zdot + ((size_t)bh * d.NC + c) * 2);
+    if (t < d.N) {
+      float2 bv = make_float2(0.f, 0.f), bl = bv;
+      if (t0 > 0) bv = load_pair<T>(a.B + (tok0 - 1) * d.D + 2 * t);
+      else if (a.Bprev) bv = load_as_f2(a.Bprev, a.prev_dtype, (size_t)bh * d.D + 2 * t);
+      if (valid == L)
+        bl = cmul(*reinterpret_cast<const float2 *>(a.K + (tok0 + L - 1) * 4 + 2),
+                  load_pair<T>(a.B + (tok0 + L - 1) * d.D + 2 * t));
+      bm1[t] = bv;
+      bh1[t] = bl;
+    }
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");  // U, dY tiles
+  if (r8 == 31) {  // source slot 127 is the token in front of the chunk; u_127 is kept aside
+    uint4 *cell = reinterpret_cast<uint4 *>(tU + umma::swz_off(L - 1, j8));
+    const uint4 own = *cell;
+    const uint32_t *w = reinterpret_cast<const uint32_t *>(&own);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) *reinterpret_cast<float2 *>(um + 8 * j8 + 2 * e) = umma::unpack2(w[e], T());
+    *cell = ub;
+  }
   umma::fence_smem_to_async();
   umma::fence_before_sync();
   __syncthreads();
   umma::fence_after_sync();
-  const uint32_t tmem = tmem_slot;
-  const uint32_t sYe = umma::smem_u32(tYe), sU = umma::smem_u32(tU), sdS = umma::smem_u32(tdS),
-                 sBh = umma::smem_u32(tBh), sSt = umma::smem_u32(tSt);
+  const uint32_t tmem = *tmem_slot;
   SLX_STAMP(1);
-  // The products of slab sl, by one thread.  Issuing is slow (the queue in front of the tensor core is short): done by
-  // a worker it held that warp, and with it every barrier, for 3 K cycles a slab; hence a warp of its own.
-  constexpr uint32_t id_kk = umma::make_idesc(128, 64, false, false, fmt);
-  constexpr uint32_t id_km = umma::make_idesc(128, 64, false, true, fmt);
-  constexpr uint32_t id_mm = umma::make_idesc(128, 64, true, true, fmt);
+  // ---- the products --------------------------------------------------------------------------
+  // Issuing a product takes about as long as the product (90 cycles), so several warps share it: nobody is held longer
+  // than the products that every warp waits for take (8192 chunks: 1.059 ms, all by one thread 1.141).
+  constexpr uint32_t id_km = umma::make_idesc(128, 32, false, true, fmt);
   constexpr uint32_t id_sq = umma::make_idesc(128, 128, false, false, fmt);
-  auto issue = [&](int sl) {  // dq, X and S^T: operands and accumulators of the slab's parity
-    umma::fence_after_sync();
-    const uint32_t sK = sSt + kBwdStage * (sl & 1), sQ = sK + 16384, sZ = sK + 40960;
-    const uint32_t dq = tmem + kTmSlab + 128 * (sl & 1), X = dq + 64;
-    const uint64_t dSk = umma::desc_kmajor(sdS, 0), dSm = umma::desc_mnmajor(sdS, 0, 16384u);
-    const uint64_t dKm = umma::desc_mnmajor(sK, 0, 0), dKk = umma::desc_kmajor(sK, 0);
-    const uint64_t dQm = umma::desc_mnmajor(sQ, 0, 0), dQk = umma::desc_kmajor(sQ, 0);
-    const uint64_t dYk = umma::desc_kmajor(sYe, 0), dZm = umma::desc_mnmajor(sZ, 0, 0);
-#pragma unroll
-    for (int kk = 0; kk < 8; ++kk) {
-      umma::mma_ss(dq, umma::desc_advance(dSk, 16384u * (kk >> 2) + umma::kStepK * (kk & 3)),
-                   umma::desc_advance(dKm, umma::kStepMN * kk), id_km, kk != 0);
-      umma::mma_ss(X, umma::desc_advance(dSm, umma::kStepMN * kk), umma::desc_advance(dQm, umma::kStepMN * kk), id_mm,
-                   kk != 0);
-    }
-#pragma unroll
-    for (int kk = 0; kk < 4; ++kk) {
-      umma::mma_ss(dq, umma::desc_advance(dYk, umma::kStepK * kk), umma::desc_advance(dZm, umma::kStepMN * kk), id_km, 1);
-      umma::mma_ss(tmem, umma::desc_advance(dKk, umma::kStepK * kk), umma::desc_advance(dQk, umma::kStepK * kk), id_sq,
-                   (sl | kk) != 0);
-    }
-  };
-  auto issue_increment = [&](int sl) {  // UL and the dU of the increment path, whose buffers are single
-    umma::fence_after_sync();
-    const uint32_t sLm = sSt + kBwdStage * (sl & 1) + 32768;
-    const uint64_t dUk = umma::desc_kmajor(sU, 0), dBk = umma::desc_kmajor(sBh, 0);
-    const uint64_t dLm = umma::desc_mnmajor(sLm, 0, 0), dLk = umma::desc_kmajor(sLm, 0);
-#pragma unroll
-    for (int kk = 0; kk < 4; ++kk) {
-      umma::mma_ss(tmem + kTmUL, umma::desc_advance(dUk, umma::kStepK * kk), umma::desc_advance(dLm, umma::kStepMN * kk),
-                   id_km, kk != 0);
-      umma::mma_ss(tmem + kTmR, umma::desc_advance(dBk, umma::kStepK * kk), umma::desc_advance(dLk, umma::kStepK * kk),
-                   id_kk, (sl | kk) != 0);
-    }
-    umma::commit(bar0 + 8 * (sl & 1));  // completes with every product of the slab
-  };
-  if (issuer) {
-    if (lane == 0) {
-#pragma unroll
-      for (int kk = 0; kk < 4; ++kk)  // G = dY U^T, while the first slab is staged
-        umma::mma_ss(tmem + kTmSlab, umma::desc_kmajor(sYe, kk), umma::desc_kmajor(sU, kk), id_sq, kk != 0);
-      umma::commit(gbar);
-    }
-    __syncwarp();
-    __syncthreads_or(0);
-    // the raw tile of slab sl+1 is free once every worker has its cells of slab sl
-    if (NB > 1 && lane == 0) prefetch_cb(1);
-    for (int sl = 0; sl < NB; ++sl) {
-      __syncthreads();  // slab sl is staged
+  const uint32_t sb = umma::smem_u32(base);
+  auto issue_first = [&](int sl) {  // dS'^T Q (warp 0), U Lambda (warp 1)
+    if (warp == 0) {
       if (lane == 0) {
-        if (sl > 0 && sl + 1 < NB) prefetch_cb(sl + 1);
-        issue(sl);
+        umma::fence_after_sync();
+        constexpr uint32_t id_mm = umma::make_idesc(128, 32, true, true, fmt);
+        const uint64_t dSm = umma::desc_mnmajor(sb + 32768, 0, 16384u), dQ = umma::make_desc64(sb + 73728);
+#pragma unroll
+        for (int kk = 0; kk < 8; ++kk)
+          umma::mma_ss(tmem + kTmX, umma::desc_advance(dSm, umma::kStepMN * kk),
+                       umma::desc_advance(dQ, umma::kStepMN64 * kk), id_mm, kk != 0);
+        umma::commit(bar0);
       }
       __syncwarp();
-      if (sl > 0) __syncthreads();  // slab sl-1 has left its accumulators, Bhat of slab sl is staged
-      if (lane == 0) issue_increment(sl);
+    } else if (warp == 1) {
+      if (lane == 0) {
+        umma::fence_after_sync();
+        const uint64_t dUk = umma::desc_kmajor(sb + 16384, 0), dLm = umma::make_desc64(sb + 81920);
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk)
+          umma::mma_ss(tmem + kTmUL, umma::desc_advance(dUk, umma::kStepK * kk),
+                       umma::desc_advance(dLm, umma::kStepMN64 * kk), id_km, kk != 0);
+        umma::commit(bar0);
+        if (sl > 0 && sl + 1 < NB) prefetch_cb(sl + 1);
+      }
       __syncwarp();
     }
-    __syncthreads();  // the last slab has left its accumulators
-    __syncthreads();  // S'^T and dY are complete
-    if (lane == 0) {
-      umma::fence_after_sync();
-      const uint32_t sdY = umma::smem_u32(sC);
+  };
+  auto issue_second = [&](int sl) {  // dS' kappa (warp 5), dY Z0 (warp 6), S^T and kappa Lambda^T (warp 7)
+    if (warp == 5) {
+      if (lane == 0) {
+        umma::fence_after_sync();
+        const uint64_t dSk = umma::desc_kmajor(sb + 32768, 0), dK = umma::make_desc64(sb + 65536);
 #pragma unroll
-      for (int kk = 0; kk < 8; ++kk)
-        umma::mma_ss(tmem + kTmU, umma::desc_kmajor(sdS + 16384u * (kk >> 2), kk & 3), umma::desc_mnmajor(sdY, kk, 0),
-                     id_km, kk != 0);
+        for (int kk = 0; kk < 8; ++kk)
+          umma::mma_ss(tmem + kTmX, umma::desc_advance(dSk, 16384u * (kk >> 2) + umma::kStepK * (kk & 3)),
+                       umma::desc_advance(dK, umma::kStepMN64 * kk), id_km, kk != 0);
+        umma::commit(bar0 + 8);
+      }
+      __syncwarp();
+    } else if (warp == 6) {
+      if (lane == 0) {
+        umma::fence_after_sync();
+        const uint64_t dYk = umma::desc_kmajor(sb, 0), dZ = umma::make_desc64(sb + 86016);
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk)
+          umma::mma_ss(tmem + kTmUL, umma::desc_advance(dYk, umma::kStepK * kk),
+                       umma::desc_advance(dZ, umma::kStepMN64 * kk), id_km, kk != 0);
+        umma::commit(bar0 + 8);
+      }
+      __syncwarp();
+    } else if (warp == 7) {
+      if (lane == 0) {
+        umma::fence_after_sync();
+        constexpr uint32_t id_kk = umma::make_idesc(128, 64, false, false, fmt);
+        const uint64_t dK = umma::make_desc64(sb + 65536), dQ = umma::make_desc64(sb + 73728),
+                       dLm = umma::make_desc64(sb + 81920);
+#pragma unroll
+        for (int kk = 0; kk < 2; ++kk) {
+          umma::mma_ss(tmem, umma::desc_advance(dK, umma::kStepK * kk), umma::desc_advance(dQ, umma::kStepK * kk), id_sq,
+                       (sl | kk) != 0);
+          umma::mma_ss(tmem + kTmR, umma::desc_advance(dK, umma::kStepK * kk),
+                       umma::desc_advance(dLm, umma::kStepK * kk), id_kk, (sl | kk) != 0);
+        }
+        umma::commit(bar0 + 8);
+      }
+      __syncwarp();
+    }
+  };
+  if (warp == 0) {
+    if (lane == 0) {
+      const uint64_t dYk = umma::desc_kmajor(sb, 0), dUk = umma::desc_kmajor(sb + 16384, 0);
+#pragma unroll
+      for (int kk = 0; kk < 4; ++kk)  // G = dY U^T, while the first slab is staged
+        umma::mma_ss(tmem, umma::desc_advance(dYk, umma::kStepK * kk), umma::desc_advance(dUk, umma::kStepK * kk), id_sq,
+                     kk != 0);
       umma::commit(gbar);
     }
     __syncwarp();
-    __syncthreads();  // every worker has read its accumulators
-    umma::tmem_dealloc(tmem, 512);
-    return;
   }
-  const int q4 = warp & 3, qc = warp >> 2;  // lane quarter of tensor memory, column quarter
+  const int q4 = warp & 3, h = warp >> 2;  // lane quarter of tensor memory, column half
   const int row = 32 * q4 + lane;
   const bool last_row = row == L - 1;
-  const float2 ph_r = ph[row];
+  const float lp_r = lp[row];
+  const float es = __expf(lp[L - 1] - (last_row ? lp[0] : lp[row + 1]));
+  const float2 f_r = cmulc(ph[row], ph[L - 1]);                               // f_t
+  const float2 f_n = cmulc(last_row ? ph[0] : ph[row + 1], ph[L - 1]);        // f_{s+1}; f_0 for the boundary slot
+  const float2 p_r = cscale(ph[row], __expf(lp_r));
   const float2 kc_r = kc[row];
-  // gamma_s conj(phi_{s+1}), the boundary slot: k^p_0 conj(phi_0);  w_s, the last token: k^c
-  float2 gk_r = cmulc(kp[0], ph[0]), w_r = kc_r;
-  if (!last_row) {
-    const float2 gam = cadd(cmul(mraw[row + 1], kc_r), kp[row + 1]);
-    gk_r = cmulc(gam, ph[row + 1]);
-    w_r = cmul(cscale(cmulc(ph[L - 1], ph[row + 1]), __expf(lp[L - 1] - lp[row + 1])), gam);
-  }
-  const float lpb = last_row ? lp[0] : lp[row + 1];
-  uint32_t ph_bits = 0;  // phases of the barriers: bit 0, 1 slab products, 2 gbar, 3 tbar
-  bool ok = true;
+  const float2 gk = cmulc(last_row ? kp[0] : cadd(cmul(mraw[row + 1], kc_r), kp[row + 1]), f_n);
+  uint32_t ph_bits = 0;  // phases of the barriers
+  bool ok = (umma::smem_u32(smem_raw) & 1023u) == 0;
   auto wait = [&](int which) {
     ok = umma::mbar_wait(bar0 + 8 * which, (ph_bits >> which) & 1) && ok;
     ph_bits ^= 1u << which;
+    __syncwarp();
   };
-  float2 acc_bc = make_float2(0.f, 0.f);  // conj(b) c over this thread's cells
-  uint4 cr[2], br[2], cn[2], bn[2];       // raw cells: slab in its epilogue, slab being staged
+  const float2 zero2 = make_float2(0.f, 0.f);
+  // conj(b) c;  conj(dC) c, the part through kappa against the rounded Q instead;  conj(b) xi;  conj(kappa) xi
+  CDot2 d_bc{zero2, zero2}, d_g = d_bc, d_x = d_bc, d_k = d_bc;
+  uint4 cr[2], br[2];                                       // raw cells of the slab
 
-  // Operand tiles of slab sl from its raw cells, written to its staging buffer.  The bulk stores of dC / dB of
-  // slab sl-2 leave from the same tiles: the rotated cells wait in registers until those have read them.
+  // operand tiles of slab sl
   auto stage = [&](int sl) {
     wait(3);
-    uint4 qv[2], kv[2];
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
-      const uint32_t off = umma::swz_off(row, 2 * qc + k);
-      cn[k] = *reinterpret_cast<const uint4 *>(sC + off);
-      bn[k] = *reinterpret_cast<const uint4 *>(sB + off);
-      uint4 src = bn[k];
+      const uint32_t off = umma::swz64_off(row, 2 * h + k);
+      cr[k] = *reinterpret_cast<const uint4 *>(sC + off);
+      br[k] = *reinterpret_cast<const uint4 *>(sB + off);
+      const CellF cf = unpack_cell<T>(cr[k]);
+      CellF bf = unpack_cell<T>(br[k]);
+#pragma unroll
+      for (int q = 0; q < 2; ++q) cdot2(bf.re[q], bf.im[q], cf.re[q], cf.im[q], d_bc);
+      *reinterpret_cast<uint4 *>(tQ + off) = rotate_cell_split<T>(cf, f_r.x, -f_r.y);
       if (last_row) {
-        float tmp[8];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float2 v = bm1[sl * 32 + 8 * qc + 4 * k + e];
-          tmp[2 * e] = v.x;
-          tmp[2 * e + 1] = v.y;
-        }
-        src = pack8<T>(tmp);
+        const float4 *bm = reinterpret_cast<const float4 *>(bm1 + 16 * sl + 8 * h + 4 * k);
+        const float4 b0 = bm[0], b1 = bm[1];
+        bf.re[0] = make_float2(b0.x, b0.z);
+        bf.im[0] = make_float2(b0.y, b0.w);
+        bf.re[1] = make_float2(b1.x, b1.z);
+        bf.im[1] = make_float2(b1.y, b1.w);
       }
-      qv[k] = rotate_chunk<T>(cn[k], cconj(ph_r));
-      kv[k] = rotate_chunk<T>(src, gk_r);
-      cdot_chunk<T>(bn[k], cn[k], acc_bc);
+      *reinterpret_cast<uint4 *>(tK + off) = rotate_cell_split<T>(bf, gk.x, gk.y);
     }
-    unsigned char *buf = tSt + kBwdStage * (sl & 1);
-    if (sl >= 2) {
-      if (tid == 0) umma::tma_store_wait_read();
-      workers_sync();
-    }
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      const uint32_t off = umma::swz_off(row, 2 * qc + k);
-      *reinterpret_cast<uint4 *>(buf + off) = kv[k];
-      *reinterpret_cast<uint4 *>(buf + 16384 + off) = qv[k];
-    }
-    *reinterpret_cast<uint4 *>(buf + 32768 + umma::swz_off(zp, zj)) = lr;
-    *reinterpret_cast<uint4 *>(buf + 40960 + umma::swz_off(zp, zj)) = zr;
+    const uint32_t offz = umma::swz64_off(zp, zj);
+    *reinterpret_cast<uint4 *>(tLm + offz) = split_cell(lr);
+    *reinterpret_cast<uint4 *>(tZ + offz) = split_cell(zr);
     umma::fence_smem_to_async();
     umma::fence_before_sync();
   };
-  // Bhat of the slab just staged, from the raw cells in registers
-  auto stage_bhat = [&]() {
-#pragma unroll
-    for (int k = 0; k < 2; ++k)
-      *reinterpret_cast<uint4 *>(tBh + umma::swz_off(row, 2 * qc + k)) = rotate_chunk<T>(bn[k], w_r);
-  };
-  // The increment path of the token in front of the chunk, from this thread's Lambda values (still in registers):
-  // per-warp partials of (u_{-1} . Lambda)[d] (rows zp of this warp, summed over the 4 lanes that share zj) and
-  // duc[p] += sum_d bh1[d] Lambda[p][d] (summed over the 8 lanes that share zp).
+  // Token 127's increment path, from this thread's Lambda values (still in registers): per-warp partials of
+  // (u_127 . Lambda)[d] (the warp's eight rows zp, summed over the 8 lanes that share zj) and this thread's share of
+  // (k^c b_127) . Lambda[zp].
+  float du127 = 0.f;
   auto helper = [&](int sl) {
     float tl[8];
     {
@@ -367,386 +377,415 @@ __global__ void __launch_bounds__(kTcBwdThreads, 1) chunk_scan_bwd_tc_kernel(Sca
         tl[2 * e + 1] = v.y;
       }
     }
-    const float4 *kbv = reinterpret_cast<const float4 *>(reinterpret_cast<const float *>(bh1) + 64 * sl + 8 * zj);
+    const float4 *kbv = reinterpret_cast<const float4 *>(reinterpret_cast<const float *>(bh1) + 32 * sl + 8 * zj);
     const float4 h0 = kbv[0], h1 = kbv[1];
     const float hb[8] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
-    const float uz = um1[zp];
-    float ds = 0.f, up[8];
+    const float uz = um[zp];
+    float up[8];
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
-      ds = fmaf(hb[e], tl[e], ds);
+      du127 = fmaf(hb[e], tl[e], du127);
       up[e] = uz * tl[e];
     }
-    // sums over the four lanes that share zj: the lanes trade halves, so that each ends with two of the eight columns
-    const bool hi8 = lane & 8, hi16 = lane & 16;
+    // the lanes trade halves, so that each ends with one of the eight columns
+    const bool hi4 = lane & 4, hi8 = lane & 8, hi16 = lane & 16;
     float w4[4], w2[2];
 #pragma unroll
-    for (int e = 0; e < 4; ++e) w4[e] = (hi8 ? up[4 + e] : up[e]) + __shfl_xor_sync(0xffffffffu, hi8 ? up[e] : up[4 + e], 8);
+    for (int e = 0; e < 4; ++e)
+      w4[e] = (hi16 ? up[4 + e] : up[e]) + __shfl_xor_sync(0xffffffffu, hi16 ? up[e] : up[4 + e], 16);
 #pragma unroll
-    for (int e = 0; e < 2; ++e) w2[e] = (hi16 ? w4[2 + e] : w4[e]) + __shfl_xor_sync(0xffffffffu, hi16 ? w4[e] : w4[2 + e], 16);
-#pragma unroll
-    for (int off = 4; off > 0; off >>= 1) ds += __shfl_xor_sync(0xffffffffu, ds, off);
-    if (zj == 0) duc[zp] += ds;
-    *reinterpret_cast<float2 *>(ulw + 64 * warp + 8 * zj + (hi8 ? 4 : 0) + (hi16 ? 2 : 0)) = make_float2(w2[0], w2[1]);
+    for (int e = 0; e < 2; ++e)
+      w2[e] = (hi8 ? w4[2 + e] : w4[e]) + __shfl_xor_sync(0xffffffffu, hi8 ? w4[e] : w4[2 + e], 8);
+    const float w1 = (hi4 ? w2[1] : w2[0]) + __shfl_xor_sync(0xffffffffu, hi4 ? w2[0] : w2[1], 4);
+    ulw[32 * warp + 8 * zj + (hi16 ? 4 : 0) + (hi8 ? 2 : 0) + (hi4 ? 1 : 0)] = w1;
   };
 
-  // ---- the boundary dots, the decay tables; the first slab's operands ------------------
-  {
-    const int j = tid & 7, r0 = tid >> 3;
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const int r = r0 + 64 * i;
-      const uint4 dyr = *reinterpret_cast<const uint4 *>(tYe + umma::swz_off(r, j));
-      const uint32_t *w = reinterpret_cast<const uint32_t *>(&dyr);
-      float dot = 0.f;
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const float2 v = umma::unpack2(w[e], T());
-        dot = fmaf(v.x, um1[8 * j + 2 * e], fmaf(v.y, um1[8 * j + 2 * e + 1], dot));
-      }
-#pragma unroll
-      for (int o = 4; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
-      if (j == 0) gm1[r] = dot;
-    }
-  }
-  if (tid < L) {
-    e2[tid] = decay_table_entry(lp, tid, L);
-    e3[tid] = __expf(lp[tid] - lp[32 * (tid >> 5)]);
-  } else if (tid >= 256 && tid < 256 + d.N) {
-    const float2 s0 = cscale(cmulc(ph[L - 1], ph[0]), __expf(lp[L - 1] - lp[0]));  // p_{L-1}/p_0
-    bh1[tid - 256] = cmul(cmul(s0, kp[0]), bm1[tid - 256]);
-  }
+  // ---- the decay table; the first slab's operands ------------------
+  if (tid < L) tab[tid] = decay_table_entry(lp, tid, L);
   stage(0);
-  stage_bhat();
-  umma::fence_smem_to_async();
   const bool fast_decay = !__syncthreads_or(tid < L && decay_step_out_of_range(lp, tid));
+  if (warp == 1) {
+    if (lane == 0) prefetch_cb(1);  // every thread has its cells of slab 0 (NB >= 2)
+    __syncwarp();
+  }
   helper(0);
-  if (NB > 1) prefetch_zl(1);
+  prefetch_zl(1);
   SLX_STAMP(2);
 
-  // ---- G -> dS'; dY -> Ye in its place ----------------------------------------------------------
+  // ---- G -> dS' ----------------------------------------------------------
   wait(2);
   umma::fence_after_sync();
-  {
-    const int j = tid & 7, r0 = tid >> 3;
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const int r = r0 + 64 * i;
-      uint4 *cell = reinterpret_cast<uint4 *>(tYe + umma::swz_off(r, j));
-      const uint4 dyr = *cell;
-      const uint32_t *w = reinterpret_cast<const uint32_t *>(&dyr);
-      const float el = __expf(lp[r]);
-      float ty[8];
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const float2 v = umma::unpack2(w[e], T());
-        ty[2 * e] = el * v.x;
-        ty[2 * e + 1] = el * v.y;
-      }
-      *cell = pack8<T>(ty);
-    }
-  }
-  {
-    const float lpt = lp[row];
-    const int c0 = 32 * qc;
+#pragma unroll 1
+  for (int jj = 0; jj < 2; ++jj) {
+    const int blk = 2 * jj + h, c0 = 32 * blk;  // blocks alternate between the two warps of a row quarter
     float v[32];
-    if (qc <= q4) {
-      umma::tmem_ld32(umma::tmem_addr(tmem + kTmSlab, 32 * q4, c0), v);
-      if (qc == q4) {  // the diagonal lives in the block with qc == q4
+    if (blk <= q4 || blk == 3) {
+      umma::tmem_ld32(umma::tmem_addr(tmem, 32 * q4, c0), v);
+      const float g127 = v[31];
+      if (blk < q4) {
+        if (fast_decay) scale32(v, __expf(lp_r - lp[c0 + 1]), tab + c0);
+        else decay_mask32<false>(v, c0, row, lp_r, lp, tab, 0.f);
+      } else if (blk == q4) {
         float gdv = 0.f;
 #pragma unroll
         for (int i = 0; i < 32; ++i)
           if (i == lane) gdv = v[i];
-        gd[row] = gdv;
+        if (!last_row) gd[row] = gdv;
+        if (fast_decay) decay_mask32<true>(v, c0, row, lp_r, lp, tab, 0.f);
+        else decay_mask32<false>(v, c0, row, lp_r, lp, tab, 0.f);
+      } else {
+#pragma unroll
+        for (int i = 0; i < 32; ++i) v[i] = 0.f;
       }
-      if (fast_decay) decay_mask32<true>(v, c0, row, lpt, lp, e2, 0.f);
-      else decay_mask32<false>(v, c0, row, lpt, lp, e2, 0.f);
+      if (blk == 3) v[31] = __expf(lp_r - lp[0]) * g127;  // boundary slot (column 127)
     } else {  // block entirely above the diagonal
 #pragma unroll
       for (int i = 0; i < 32; ++i) v[i] = 0.f;
     }
-    if (qc == 3) v[31] = __expf(lpt - lp[0]) * gm1[row];  // boundary slot (column 127)
 #pragma unroll
     for (int k = 0; k < 4; ++k)
-      *reinterpret_cast<uint4 *>(tdS + 16384 * (qc >> 1) + umma::swz_off(row, 4 * (qc & 1) + k)) = pack8<T>(v + 8 * k);
+      *reinterpret_cast<uint4 *>(tdS + 16384 * (blk >> 1) + umma::swz_off(row, 4 * (blk & 1) + k)) = pack8<T>(v + 8 * k);
+  }
+  if (warp == 0) {  // G[127][127] = dY_127 . u_127 (slot 127 of U is another token)
+    const uint32_t w = *reinterpret_cast<const uint32_t *>(tdY + umma::swz_off(L - 1, lane >> 2) + 4 * (lane & 3));
+    const float2 y = umma::unpack2(w, T()), u = *reinterpret_cast<const float2 *>(um + 2 * lane);
+    float s = fmaf(y.x, u.x, y.y * u.y);
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
+    if (lane == 0) gd[L - 1] = s;
   }
   umma::fence_smem_to_async();
   umma::fence_before_sync();
   __syncthreads();
   SLX_STAMP(3);
   const float gd_r = gd[row];
-  const float2 cA_r = cscale(kc_r, gd_r);
+  const float2 cA = cscale(kc_r, gd_r);
+  if (tid < L) tab[tid] = __expf(lp[tid] - lp[32 * (tid >> 5)]);  // for the tail: every reader of the first table is done
+  const bool wide = ((reinterpret_cast<uintptr_t>(a.dB) | reinterpret_cast<uintptr_t>(a.dC)) & 31) == 0;
+  auto store_row = [&](T *dst, const uint4 (&o)[2]) {  // 16 values of this thread's row, a whole 32-byte sector
+    if (wide) {
+      asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "r"(o[0].x), "r"(o[0].y),
+                   "r"(o[0].z), "r"(o[0].w), "r"(o[1].x), "r"(o[1].y), "r"(o[1].z), "r"(o[1].w)
+                   : "memory");
+    } else {
+      reinterpret_cast<uint4 *>(dst)[0] = o[0];
+      reinterpret_cast<uint4 *>(dst)[1] = o[1];
+    }
+  };
+  const size_t out0 = (tok0 + row) * d.D + 16 * h;
 
-  float2 pgA = make_float2(0.f, 0.f), pX = pgA, pUL = pgA;
-#pragma unroll
-  for (int k = 0; k < 2; ++k) {
-    cr[k] = cn[k];
-    br[k] = bn[k];
-  }
   for (int sl = 0; sl < NB; ++sl) {
-    SLX_STAMP(8 + 8 * sl);
-    // u_{-1} . Lambda of this slab: sum of the 16 per-warp partials (two warps, one column per thread)
-    if (tid >= 32 && tid < 96) {
-      const int dcol = tid - 32;
+    SLX_STAMP(8 + 4 * sl);
+    issue_first(sl);  // slab sl is staged, the accumulators of slab sl-1 are read
+    if (sl > 0) {
+      helper(sl);
+      if (sl + 1 < NB) prefetch_zl(sl + 1);
+    }
+    // ---- xi = dS'^T Q + es U Lambda ------------------------------------------------------------
+    float2 xr[4], xi[4];  // pairs of complex values: cell 0, cell 1
+    wait(0);
+  umma::fence_after_sync();
+    SLX_STAMP(9 + 4 * sl);
+    {
+      uint32_t r1[16], r2[16];
+      umma::tmem_ld16_issue(umma::tmem_addr(tmem + kTmX, 32 * q4, 16 * h), r1);
+      umma::tmem_ld16_issue(umma::tmem_addr(tmem + kTmUL, 32 * q4, 16 * h), r2);
+      umma::tmem_ld16_wait(r1);
+      umma::tmem_ld16_wait(r2);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int o = 8 * (q >> 1) + 2 * (q & 1);
+        xr[q] = __ffma2_rn(both(es), tm_pair(r2 + o), tm_pair(r1 + o));
+        xi[q] = __ffma2_rn(both(es), tm_pair(r2 + o + 4), tm_pair(r1 + o + 4));
+      }
+    }
+    umma::fence_before_sync();
+    __syncthreads();  // dS'^T Q and U Lambda are in registers
+    issue_second(sl);
+    if (warp == 4) {  // u_127 . Lambda of this slab: sum of the per-warp partials
       float acc = 0.f;
 #pragma unroll
-      for (int w = 0; w < 16; ++w) acc += ulw[64 * w + dcol];
-      ulf[64 * sl + dcol] = acc;
+      for (int w = 0; w < 8; ++w) acc += ulw[32 * w + lane];
+      ulf[32 * sl + lane] = acc;
     }
-    if (sl + 1 < NB) {
+    if (last_row) {  // xi of the token in front of the chunk; token 127's own dB is formed in the tail
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        *reinterpret_cast<float4 *>(xb + 32 * sl + 16 * h + 4 * q) = make_float4(xr[q].x, xi[q].x, xr[q].y, xi[q].y);
+    }
+    // ---- dB_s = conj(gk_s) xi_s + conj(cA_s) c_s -------------------------------------------------
+    {
+      uint4 o[2];
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        const CellF cf = unpack_cell<T>(cr[k]), bf = unpack_cell<T>(br[k]);
+        const CellF kf = unpack_cell_split<T>(*reinterpret_cast<const uint4 *>(tK + umma::swz64_off(row, 2 * h + k)));
+        uint32_t *w = reinterpret_cast<uint32_t *>(&o[k]);
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          const float2 x = xr[2 * k + q], y = xi[2 * k + q];
+          float2 re = __fmul2_rn(both(cA.x), cf.re[q]), im = __fmul2_rn(both(cA.x), cf.im[q]);
+          re = __ffma2_rn(both(cA.y), cf.im[q], re);
+          im = __ffma2_rn(both(-cA.y), cf.re[q], im);
+          re = __ffma2_rn(both(gk.x), x, re);
+          im = __ffma2_rn(both(gk.x), y, im);
+          re = __ffma2_rn(both(gk.y), y, re);
+          im = __ffma2_rn(both(-gk.y), x, im);
+          cdot2(bf.re[q], bf.im[q], x, y, d_x);
+          cdot2(kf.re[q], kf.im[q], x, y, d_k);
+          w[2 * q] = umma::pack2(re.x, im.x, T());
+          w[2 * q + 1] = umma::pack2(re.y, im.y, T());
+        }
+      }
+      if (row < valid && !last_row) store_row(a.dB + out0 + 32 * sl, o);
+    }
+    SLX_STAMP(10 + 4 * sl);
+    // ---- dC_t = f_t (dS' kappa)_t + p_t (dY Z0)_t + cA_t b_t ------------------------------------------
+    wait(1);
+  umma::fence_after_sync();
+    SLX_STAMP(11 + 4 * sl);
+    {
+      uint4 o[2];
+      uint32_t t1[16], t2[16];
+      umma::tmem_ld16_issue(umma::tmem_addr(tmem + kTmX, 32 * q4, 16 * h), t1);
+      umma::tmem_ld16_issue(umma::tmem_addr(tmem + kTmUL, 32 * q4, 16 * h), t2);
+      umma::tmem_ld16_wait(t1);
+      umma::tmem_ld16_wait(t2);
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        const uint32_t *r1 = t1 + 8 * k, *r2 = t2 + 8 * k;
+        const CellF cf = unpack_cell<T>(cr[k]), bf = unpack_cell<T>(br[k]);
+        const CellF qf = unpack_cell_split<T>(*reinterpret_cast<const uint4 *>(tQ + umma::swz64_off(row, 2 * h + k)));
+        uint32_t *w = reinterpret_cast<uint32_t *>(&o[k]);
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          const float2 x = tm_pair(r1 + 2 * q), y = tm_pair(r1 + 4 + 2 * q);
+          const float2 u = tm_pair(r2 + 2 * q), v = tm_pair(r2 + 4 + 2 * q);
+          float2 re = __fmul2_rn(both(cA.x), bf.re[q]), im = __fmul2_rn(both(cA.x), bf.im[q]);
+          re = __ffma2_rn(both(-cA.y), bf.im[q], re);
+          im = __ffma2_rn(both(cA.y), bf.re[q], im);
+          re = __ffma2_rn(both(p_r.x), u, re);
+          im = __ffma2_rn(both(p_r.x), v, im);
+          re = __ffma2_rn(both(-p_r.y), v, re);
+          im = __ffma2_rn(both(p_r.y), u, im);
+          cdot2(re, im, cf.re[q], cf.im[q], d_g);
+          cdot2(x, y, qf.re[q], qf.im[q], d_g);
+          re = __ffma2_rn(both(f_r.x), x, re);
+          im = __ffma2_rn(both(f_r.x), y, im);
+          re = __ffma2_rn(both(-f_r.y), y, re);
+          im = __ffma2_rn(both(f_r.y), x, im);
+          w[2 * q] = umma::pack2(re.x, im.x, T());
+          w[2 * q + 1] = umma::pack2(re.y, im.y, T());
+        }
+      }
+      if (row < valid) store_row(a.dC + out0 + 32 * sl, o);
+    }
+    if (sl + 1 < NB) {  // every product of the slab is done: its tiles are free
       stage(sl + 1);
-      SLX_STAMP(9 + 8 * sl);
       __syncthreads();
-      SLX_STAMP(10 + 8 * sl);
-      helper(sl + 1);
-      if (sl + 2 < NB) prefetch_zl(sl + 2);
-    } else {
-      // the raw tiles are free: dY comes back for the last product
-      fetch_rows(sC, a.dY);
-      asm volatile("cp.async.commit_group;" ::: "memory");
-    }
-    SLX_STAMP(11 + 8 * sl);
-    wait(sl & 1);
-    umma::fence_after_sync();
-    SLX_STAMP(12 + 8 * sl);
-    // ---- slab epilogue: dC, dB, per-token dots --------------------------------------------------
-    //   dC_t = phi_t dq_t + (k^c_t G_tt) b_t,
-    //   dB_s = (conj(k^c_s) G_ss) c_s + conj(gk_s) X_s + conj(w_s) UL_s
-    //   dots: gA += c conj(dC),  conj(b) X,  conj(b) UL
-    // Row 127 of X belongs to the token in front of the chunk; the last token takes no part in X.
-    unsigned char *buf = tSt + kBwdStage * (sl & 1);
-    const uint32_t acc = tmem + kTmSlab + 128 * (sl & 1);
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      // eight accumulator columns (four complex lanes) of dq, X and UL at a time
-      uint32_t r0[8], r1[8], r2[8];
-      umma::tmem_ld8_issue(umma::tmem_addr(acc, 32 * q4, 16 * qc + 8 * k), r0);
-      umma::tmem_ld8_issue(umma::tmem_addr(acc, 32 * q4, 64 + 16 * qc + 8 * k), r1);
-      umma::tmem_ld8_issue(umma::tmem_addr(tmem + kTmUL, 32 * q4, 16 * qc + 8 * k), r2);
-      umma::tmem_ld8_wait(r0);
-      umma::tmem_ld8_wait(r1);
-      umma::tmem_ld8_wait(r2);
-      if (last_row) {
-        float4 *dst = reinterpret_cast<float4 *>(xb + 64 * sl + 16 * qc + 8 * k);
-#pragma unroll
-        for (int i = 0; i < 2; ++i)
-          dst[i] = make_float4(__uint_as_float(r1[4 * i]), __uint_as_float(r1[4 * i + 1]),
-                               __uint_as_float(r1[4 * i + 2]), __uint_as_float(r1[4 * i + 3]));
-#pragma unroll
-        for (int i = 0; i < 8; ++i) r1[i] = 0;
-      }
-      const uint32_t *wb = reinterpret_cast<const uint32_t *>(&br[k]);
-      const uint32_t *wc = reinterpret_cast<const uint32_t *>(&cr[k]);
-      float odc[8], odb[8];
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const float2 bv = umma::unpack2(wb[e], T()), cv = umma::unpack2(wc[e], T());
-        const float2 dqv = make_float2(__uint_as_float(r0[2 * e]), __uint_as_float(r0[2 * e + 1]));
-        const float2 Xv = make_float2(__uint_as_float(r1[2 * e]), __uint_as_float(r1[2 * e + 1]));
-        const float2 ULv = make_float2(__uint_as_float(r2[2 * e]), __uint_as_float(r2[2 * e + 1]));
-        const float2 dcv = cmadd(ph_r, dqv, cmul(cA_r, bv));
-        pgA = cmadd(cv, cconj(dcv), pgA);
-        const float2 dbv = cmadd(cconj(gk_r), Xv, cmadd(cconj(w_r), ULv, cmul(cconj(cA_r), cv)));
-        pX = cmadd(cconj(bv), Xv, pX);
-        pUL = cmadd(cconj(bv), ULv, pUL);
-        odc[2 * e] = dcv.x;
-        odc[2 * e + 1] = dcv.y;
-        odb[2 * e] = dbv.x;
-        odb[2 * e + 1] = dbv.y;
-      }
-      // the results take the place of the slab's (now idle) Qbar / kappa cells and leave from there
-      const uint32_t off = umma::swz_off(row, 2 * qc + k);
-      *reinterpret_cast<uint4 *>(buf + 16384 + off) = pack8<T>(odc);
-      *reinterpret_cast<uint4 *>(buf + off) = pack8<T>(odb);
-    }
-    if (sl + 1 < NB) stage_bhat();  // of slab sl+1: the product that read the last one is done
-    umma::fence_smem_to_async();  // Bhat, and the dC / dB cells, which leave through the async proxy
-    umma::fence_before_sync();
-    SLX_STAMP(13 + 8 * sl);
-    __syncthreads();
-    SLX_STAMP(14 + 8 * sl);
-    if (tid == 0) {  // one thread sends both tiles (rows past the end of the sequence are clipped by the copy)
-      umma::tma_store_3d(&maps.dC, 64 * sl, t0, bh, sSt + kBwdStage * (sl & 1) + 16384);
-      umma::tma_store_3d(&maps.dB, 64 * sl, t0, bh, sSt + kBwdStage * (sl & 1));
-      umma::tma_store_commit();
-    }
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      cr[k] = cn[k];
-      br[k] = bn[k];
     }
   }
   SLX_STAMP(4);
 
-  // ---- fold the column quarters of the per-token dots (scratch: the idle Lambda and Z0 tiles) -----
-  float2 *part = reinterpret_cast<float2 *>(tSt + 32768);  // 3 x [4][128]: gA, bX, bc
-  part[128 * qc + row] = pgA;
-  // conj(b_s) xi_s = phi_{s+1} conj(b) X + conj(p_{L-1}/p_{s+1}) conj(b) UL; row 127: conj(b_127) . (u_127 . Lambda)
-  if (!last_row) {
-    const float2 sg = cscale(cmulc(ph[L - 1], ph[row + 1]), __expf(lp[L - 1] - lp[row + 1]));
-    pUL = cmadd(ph[row + 1], pX, cmul(cconj(sg), pUL));
+  // ---- fold the column halves of the per-token dots -----
+  // what only the tail needs of the taps, multipliers and phases is read again, not held through the slabs
+  float4 k4 = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (row < valid) k4 = *reinterpret_cast<const float4 *>(a.K + (tok0 + row) * 4);
+  const float2 kc_t = make_float2(k4.z, k4.w), k_edge = tid < 128 ? *reinterpret_cast<const float2 *>(a.K + tok0 * 4)
+      : valid == L ? *reinterpret_cast<const float2 *>(a.K + (tok0 + L - 1) * 4 + 2) : zero2;  // k^p_0; k^c_127
+  const float2 f_next = cmulc(last_row ? ph[0] : ph[row + 1], ph[L - 1]);
+  const float lpb = last_row ? lp[0] : lp[row + 1], gd_t = gd[row];
+  float2 m_own = make_float2(1.f, 0.f), m_next = m_own, zd = zero2;
+  float2 c127 = zero2, b127 = zero2;  // second half: values n of token 127
+  if (h == 0) {
+    if (row < valid) m_own = *reinterpret_cast<const float2 *>(a.M + (tok0 + row) * 2);
+    if (row + 1 < valid) m_next = *reinterpret_cast<const float2 *>(a.M + (tok0 + row + 1) * 2);
+    if (last_row) zd = *reinterpret_cast<const float2 *>(a.zdot + ((size_t)bh * d.NC + c) * 2);
+  } else if (row < d.N && valid == L) {
+    c127 = load_pair<T>(a.C + (tok0 + L - 1) * d.D + 2 * row);
+    b127 = load_pair<T>(a.B + (tok0 + L - 1) * d.D + 2 * row);
   }
-  part[512 + 128 * qc + row] = pUL;
-  part[1024 + 128 * qc + row] = acc_bc;
-  workers_sync();
-  {
-    // every thread needs its row's bc (diagonal of S'^T); the first quarter keeps the sums for the token phase
-    const float2 s2 = cadd(cadd(part[1024 + row], part[1152 + row]), cadd(part[1280 + row], part[1408 + row]));
-    acc_bc = s2;
-    if (qc == 0) {
-      gA[row] = cadd(cadd(part[row], part[128 + row]), cadd(part[256 + row], part[384 + row]));
-      const float2 s1 = cadd(cadd(part[512 + row], part[640 + row]), cadd(part[768 + row], part[896 + row]));
-      bX[row] = s1;
-      if (last_row) misc[0] = s1;
-      bc[row] = s2;
-    }
+  float2 bc = cdot2_sum(d_bc), gA = cdot2_sum(d_g), bX = cdot2_sum(d_x);
+  // dM sums, over the pairs (t, s) of the chunk, differences of the same products seen from t (gA) and from s (k^c, k^p
+  // against bX).  Taken with the rounded kappa and Q on both sides they cancel as the exact ones do: the term of s is
+  // corrected by sum conj(kappa) xi - conj(gk) sum conj(b) xi, and at t = 0 the sum over the token in front of the chunk
+  // is that of conj(kappa) xi.  With the unrounded b and c in these sums dM was 2.5 times as far from float64 (relative
+  // error 5e-3 against 2e-3 for one chunk of N 128 in bf16; the kernel took 0.978 instead of 1.058 ms).
+  if (last_row) sums[4 + h] = cdot2_sum(d_k);
+  else gA = csub(gA, csub(cdot2_sum(d_k), cmul(cconj(gk), bX)));
+  bX = cmul(f_next, bX);
+  pcs[L * h + row] = bc;
+  if (h == 1) {
+    pgs[row] = gA;
+    pbs[row] = bX;
   }
-  // Gradient of the token before the chunk: xi_n = phi_0 X_127[n] + conj(p_{L-1}/p_0) (u_{-1} . Lambda)[n],
-  // dB_{-1}[n] = conj(k^p_0) xi_n, dk^p_0 = sum_n conj(b_{-1}[n]) xi_n
+  du127 += __shfl_xor_sync(0xffffffffu, du127, 1);
+  du127 += __shfl_xor_sync(0xffffffffu, du127, 2);
+  if (zj == 0) duc[zp] = du127;
+  __syncthreads();
+  bc = cadd(pcs[row], pcs[L + row]);
+  if (h == 0) {
+    gA = cadd(gA, pgs[row]);
+    bX = cadd(bX, pbs[row]);
+    bXs[row] = bX;
+  }
   float *cB = a.carryB + ((size_t)bh * d.NC + c) * d.D;
-  if (tid >= 256 && tid < 256 + L) {
-    const int n = tid - 256;
-    float2 contrib = make_float2(0.f, 0.f);
+  {
+    const int n = tid & 127;  // = row
+    float2 contrib = zero2;
     if (n < d.N) {
-      const float2 s0 = cscale(cmulc(ph[L - 1], ph[0]), __expf(lp[L - 1] - lp[0]));
-      const float2 xi = cmadd(ph[0], make_float2(xb[2 * n], xb[2 * n + 1]),
-                              cmul(cconj(s0), make_float2(ulf[2 * n], ulf[2 * n + 1])));
-      *reinterpret_cast<float2 *>(cB + 2 * n) = cmul(cconj(kp[0]), xi);
-      contrib = cmul(cconj(bm1[n]), xi);
+      if (tid < 128) {
+        // token in front of the chunk: dB_{-1}[n] = conj(k^p_0) f_0 xi[n], dk^p_0 = sum_n conj(b_{-1}[n]) f_0 xi[n]
+        const float2 x = cmul(cmulc(ph[0], ph[L - 1]), *reinterpret_cast<const float2 *>(xb + 2 * n));
+        *reinterpret_cast<float2 *>(cB + 2 * n) = cmul(cconj(k_edge), x);
+        contrib = cmul(cconj(bm1[n]), x);
+      } else if (valid == L) {
+        // token 127: dB[n] = conj(k^c) (u_127 . Lambda)[n] + conj(k^c G) c[n]
+        const float2 ul = *reinterpret_cast<const float2 *>(ulf + 2 * n);
+        store_pair<T>(a.dB + (tok0 + L - 1) * d.D + 2 * n, cmul(cconj(k_edge), cadd(ul, cscale(c127, gd[L - 1]))));
+        contrib = cmul(cconj(b127), ul);
+      }
     }
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) {
       contrib.x += __shfl_xor_sync(0xffffffffu, contrib.x, off);
       contrib.y += __shfl_xor_sync(0xffffffffu, contrib.y, off);
     }
-    if (lane == 0) misc[1 + warp - 8] = contrib;
+    if (lane == 0) misc[warp] = contrib;
   }
   SLX_STAMP(56);
   // ---- S^T -> S'^T (forward scores; row 127 = boundary) --------------------------------
-  const float dg_r = kc_r.x * acc_bc.x + kc_r.y * acc_bc.y;  // Re(k^c conj(bc))
-  {
-    const int c0 = 32 * qc;
+  const float dg_r = kc_t.x * bc.x + kc_t.y * bc.y;  // Re(k^c conj(bc))
+#pragma unroll 1
+  for (int jj = 0; jj < 2; ++jj) {
+    const int blk = 2 * jj + h, c0 = 32 * blk;
     float v[32];
-    if (qc >= q4 || q4 == 3) {  // (the last row quarter holds the boundary row, which takes every column)
+    if (blk >= q4 || q4 == 3) {  // (the last row quarter holds the boundary row, which takes every column)
       umma::tmem_ld32(umma::tmem_addr(tmem, 32 * q4, c0), v);
-      if (fast_decay) decay_mask32_rows<true>(v, c0, row, last_row, lpb, lp, e3, dg_r);
-      else decay_mask32_rows<false>(v, c0, row, last_row, lpb, lp, e3, dg_r);
+      if (fast_decay) {
+        scale32(v, __expf(lp[c0] - lpb), tab + c0);
+        if (blk == q4 || q4 == 3) {
+#pragma unroll
+          for (int i = 0; i < 32; ++i)
+            if (!last_row && c0 + i <= row) v[i] = c0 + i == row ? dg_r : 0.f;
+        }
+      } else {
+#pragma unroll
+        for (int i = 0; i < 32; ++i) {
+          const int t = c0 + i;
+          v[i] = (t > row || last_row) ? v[i] * __expf(lp[t] - lpb) : (t == row ? dg_r : 0.f);
+        }
+      }
     } else {
 #pragma unroll
       for (int i = 0; i < 32; ++i) v[i] = 0.f;
     }
 #pragma unroll
     for (int k = 0; k < 4; ++k)
-      *reinterpret_cast<uint4 *>(tdS + 16384 * (qc >> 1) + umma::swz_off(row, 4 * (qc & 1) + k)) = pack8<T>(v + 8 * k);
+      *reinterpret_cast<uint4 *>(tdS + 16384 * (blk >> 1) + umma::swz_off(row, 4 * (blk & 1) + k)) = pack8<T>(v + 8 * k);
   }
-  asm volatile("cp.async.wait_group 0;" ::: "memory");  // dY
   umma::fence_smem_to_async();
   umma::fence_before_sync();
   __syncthreads();
-  SLX_STAMP(57);
-  // ---- dK and the per-token terms of dM (overlaps the last product) -----------------------
-  if (tid < L) {
-    const int t = tid;
-    float2 dkc = cscale(bc[t], gd[t]);
-    if (t + 1 < L) dkc = cadd(dkc, cmul(cconj(mraw[t + 1]), bX[t]));
-    else dkc = cadd(dkc, misc[0]);
-    const float2 dkp = (t == 0) ? cadd(cadd(misc[1], misc[2]), cadd(misc[3], misc[4])) : bX[t - 1];
-    if (t < valid) *reinterpret_cast<float4 *>(a.dK + (tok0 + t) * 4) = make_float4(dkp.x, dkp.y, dkc.x, dkc.y);
-    float2 g = csub(gA[t], cadd(cmul(cconj(kc[t]), dkc), cmul(cconj(kp[t]), dkp)));
-    if (t == L - 1) {
-      g = cadd(g, misc[5]);
-    }
-    gsum[t] = g;
-    asm volatile("bar.sync 1, 128;" ::: "memory");  // gsum of the four token warps is complete
-  }
-  // reverse cumulative sum of g over the chunk (warp 0: 4 tokens per lane + shuffle scan)
-  if (warp == 0) {
-    float2 loc[4];
-    float2 run = make_float2(0.f, 0.f);
+  if (warp == 7) {
+    if (lane == 0) {
+      umma::fence_after_sync();
+      constexpr uint32_t id_u = umma::make_idesc(128, 64, false, true, fmt);
+      const uint64_t dSk = umma::desc_kmajor(sb + 32768, 0), dYm = umma::desc_mnmajor(sb, 0, 0);
 #pragma unroll
-    for (int i = 3; i >= 0; --i) {
-      run = cadd(run, gsum[4 * lane + i]);
-      loc[i] = run;
+      for (int kk = 0; kk < 8; ++kk)
+        umma::mma_ss(tmem + kTmU, umma::desc_advance(dSk, 16384u * (kk >> 2) + umma::kStepK * (kk & 3)),
+                     umma::desc_advance(dYm, umma::kStepMN * kk), id_u, kk != 0);
+      umma::commit(gbar);
     }
-    float2 incl = run;
+    __syncwarp();
+  }
+  SLX_STAMP(57);
+  // ---- dK and dM (under the last product): dM_t is a reverse cumulative sum over the chunk -----------------------
+  float2 g_sum = zero2;
+  if (h == 0) {
+    const int t = row;
+    float2 dkc = cscale(bc, gd_t);
+    if (!last_row) dkc = cadd(dkc, cmul(cconj(m_next), bX));
+    else dkc = cadd(dkc, cadd(cadd(misc[4], misc[5]), cadd(misc[6], misc[7])));
+    const float2 dkp = (t == 0) ? cadd(cadd(misc[0], misc[1]), cadd(misc[2], misc[3])) : bXs[t - 1];
+    if (t < valid) *reinterpret_cast<float4 *>(a.dK + (tok0 + t) * 4) = make_float4(dkp.x, dkp.y, dkc.x, dkc.y);
+    const float2 kp_term = (t == 0) ? cadd(sums[4], sums[5]) : cmul(make_float2(k4.x, -k4.y), dkp);
+    float2 g = csub(gA, cadd(cmul(make_float2(k4.z, -k4.w), dkc), kp_term));
+    if (last_row) g = cadd(g, zd);
 #pragma unroll
     for (int off = 1; off < 32; off <<= 1) {
-      float ox = __shfl_down_sync(0xffffffffu, incl.x, off), oy = __shfl_down_sync(0xffffffffu, incl.y, off);
-      if (lane + off < 32) incl = cadd(incl, make_float2(ox, oy));
+      const float ox = __shfl_down_sync(0xffffffffu, g.x, off), oy = __shfl_down_sync(0xffffffffu, g.y, off);
+      if (lane + off < 32) g = cadd(g, make_float2(ox, oy));
     }
-    const float2 excl = csub(incl, run);  // sum over the lanes above
-#pragma unroll
-    for (int i = 0; i < 4; ++i) gsum[4 * lane + i] = cadd(loc[i], excl);
+    if (lane == 0) sums[warp] = g;
+    g_sum = g;  // the sums of the warps above are added behind the last barrier
   }
   SLX_STAMP(58);
   wait(2);
   umma::fence_after_sync();
   SLX_STAMP(59);
   // ---- dU = increment path + score path; carry of dU ------------------------------------------
-  {
+#pragma unroll 1
+  for (int k2 = 0; k2 < 2; ++k2) {
+    const int p0 = 32 * h + 16 * k2;
     uint32_t r0[16], r1[16];
-    umma::tmem_ld16_issue(umma::tmem_addr(tmem + kTmR, 32 * q4, 16 * qc), r0);
-    umma::tmem_ld16_issue(umma::tmem_addr(tmem + kTmU, 32 * q4, 16 * qc), r1);
+    umma::tmem_ld16_issue(umma::tmem_addr(tmem + kTmR, 32 * q4, p0), r0);
+    umma::tmem_ld16_issue(umma::tmem_addr(tmem + kTmU, 32 * q4, p0), r1);
     umma::tmem_ld16_wait(r0);
     umma::tmem_ld16_wait(r1);
     float du[16];
 #pragma unroll
-    for (int i = 0; i < 16; ++i) du[i] = __uint_as_float(r0[i]);
-    if (last_row) {  // the score path's sum belongs to the token in front of the chunk
-      float *cU = a.carryU + ((size_t)bh * d.NC + c) * P + 16 * qc;
+    for (int i = 0; i < 16; ++i) du[i] = fmaf(es, __uint_as_float(r0[i]), __uint_as_float(r1[i]));
+    if (last_row) {  // these sums belong to the token in front of the chunk
+      float *cU = a.carryU + ((size_t)bh * d.NC + c) * P + p0;
 #pragma unroll
       for (int k = 0; k < 2; ++k) {
-        const uint4 dyr = *reinterpret_cast<const uint4 *>(sC + umma::swz_off(L - 1, 2 * qc + k));
+        const uint4 dyr = *reinterpret_cast<const uint4 *>(tdY + umma::swz_off(L - 1, 4 * h + 2 * k2 + k));
         const uint32_t *w = reinterpret_cast<const uint32_t *>(&dyr);
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
           const float2 dyv = umma::unpack2(w[e], T());
           const int i = 8 * k + 2 * e;
-          cU[i] = __uint_as_float(r1[i]) + duc[16 * qc + i];
-          cU[i + 1] = __uint_as_float(r1[i + 1]) + duc[16 * qc + i + 1];
-          du[i] = fmaf(dg_r, dyv.x, du[i]);
-          du[i + 1] = fmaf(dg_r, dyv.y, du[i + 1]);
+          *reinterpret_cast<float2 *>(cU + i) = make_float2(du[i], du[i + 1]);
+          du[i] = fmaf(dg_r, dyv.x, duc[p0 + i]);
+          du[i + 1] = fmaf(dg_r, dyv.y, duc[p0 + i + 1]);
         }
       }
-    } else {
-#pragma unroll
-      for (int i = 0; i < 16; ++i) du[i] += __uint_as_float(r1[i]);
     }
     if (row < valid) {
 #pragma unroll
       for (int k = 0; k < 2; ++k)
-        *reinterpret_cast<uint4 *>(a.dU + (tok0 + row) * P + 16 * qc + 8 * k) = pack8<T>(du + 8 * k);
+        *reinterpret_cast<uint4 *>(a.dU + (tok0 + row) * P + p0 + 8 * k) = pack8<T>(du + 8 * k);
     }
   }
   umma::fence_before_sync();
-  __syncthreads();
-  if (tid < valid) {
-    const float2 m = mraw[tid];
-    const float inv = 1.f / (m.x * m.x + m.y * m.y);
-    *reinterpret_cast<float2 *>(a.dM + (tok0 + tid) * 2) = cscale(cmul(gsum[tid], m), inv);
-  }
   SLX_STAMP(5);
-  if (tid == 0) umma::tma_store_wait_all();  // the bulk stores of dC / dB have completed
-  int bad;
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\tsetp.ne.s32 p, %1, 0;\n\tbar.red.or.pred q, 2, 512, p;\n\tselp.s32 %0, 1, 0, q;\n\t}"
-      : "=r"(bad)
-      : "r"(ok ? 0 : 1)
-      : "memory");
+  const int bad = __syncthreads_or(!ok);
+  __syncwarp();
+  if (warp == 1) {
+    umma::fence_after_sync();
+    umma::tmem_dealloc(tmem, 256);
+  }
+  if (!bad && h == 0 && row < valid) {
+    for (int w = warp + 1; w < 4; ++w) g_sum = cadd(g_sum, sums[w]);
+    const float inv = 1.f / (m_own.x * m_own.x + m_own.y * m_own.y);
+    *reinterpret_cast<float2 *>(a.dM + (tok0 + row) * 2) = cscale(cmul(g_sum, m_own), inv);
+  }
   if (bad) {
     // a bounded wait ran out: every gradient row of this chunk came from unfinished products or copies;
     // overwrite them (and the carries) with NaN so that the failure shows in the data as well as in the status word
     const float nanf_ = __int_as_float(0x7fc00000);
     const T nanv = from_f<T>(nanf_);
-    for (int e = tid; e < valid * P; e += kTcBwdWorkers) a.dU[tok0 * P + e] = nanv;
-    for (int e = tid; e < valid * d.D; e += kTcBwdWorkers) {
+    for (int e = tid; e < valid * P; e += kTcBwdThreads) a.dU[tok0 * P + e] = nanv;
+    for (int e = tid; e < valid * d.D; e += kTcBwdThreads) {
       a.dB[tok0 * d.D + e] = nanv;
       a.dC[tok0 * d.D + e] = nanv;
     }
-    for (int e = tid; e < valid * 2; e += kTcBwdWorkers) a.dM[tok0 * 2 + e] = nanf_;
-    for (int e = tid; e < valid * 4; e += kTcBwdWorkers) a.dK[tok0 * 4 + e] = nanf_;
-    for (int e = tid; e < d.D; e += kTcBwdWorkers) cB[e] = nanf_;
-    for (int e = tid; e < P; e += kTcBwdWorkers) a.carryU[((size_t)bh * d.NC + c) * P + e] = nanf_;
+    for (int e = tid; e < valid * 2; e += kTcBwdThreads) a.dM[tok0 * 2 + e] = nanf_;
+    for (int e = tid; e < valid * 4; e += kTcBwdThreads) a.dK[tok0 * 4 + e] = nanf_;
+    for (int e = tid; e < d.D; e += kTcBwdThreads) cB[e] = nanf_;
+    for (int e = tid; e < P; e += kTcBwdThreads) a.carryU[((size_t)bh * d.NC + c) * P + e] = nanf_;
     if (tid == 0) atomicExch(&g_tc_status, 1);
   }
 #undef SLX_STAMP

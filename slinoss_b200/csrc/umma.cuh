@@ -42,6 +42,13 @@ __device__ __forceinline__ uint64_t desc_mnmajor(uint32_t tile_saddr, int kk, ui
   return make_desc(tile_saddr + 2048u * kk, block_stride_bytes, 1024u);
 }
 
+// The same for tiles of 32 halfs per row (64-byte rows, 64-byte swizzle: 16-byte chunk index XOR (row / 2) % 4, rows of
+// a group of eight 512 bytes): K-major views have two K-steps, MN-major ones one block of 32 M/N indices.
+__device__ __forceinline__ uint64_t make_desc64(uint32_t saddr) {
+  return (make_desc(saddr, 16u, 512u) & ~(uint64_t(7) << 61)) | (uint64_t(4) << 61);  // SWIZZLE_64B
+}
+constexpr uint32_t kStepMN64 = 1024;  // MN-major: next K-step = 16 rows of 64 bytes (K-major: kStepK, as below)
+
 // Descriptor of the same tile view advanced by `bytes` (a multiple of 16): only the
 // 14-bit start-address field changes, so this is one 64-bit add.
 __device__ __forceinline__ uint64_t desc_advance(uint64_t desc, uint32_t bytes) { return desc + (bytes >> 4); }
@@ -298,6 +305,11 @@ __device__ __forceinline__ uint32_t tmem_addr(uint32_t base, int lane, int col) 
 // byte offset of 16-byte chunk j (0..7) of row r inside a [R][64] swizzled tile
 __device__ __forceinline__ uint32_t swz_off(int r, int j) {
   return static_cast<uint32_t>(r) * 128u + (static_cast<uint32_t>(j ^ (r & 7)) << 4);
+}
+
+// the same inside a [R][32] tile (make_desc64): chunk j (0..3)
+__device__ __forceinline__ uint32_t swz64_off(int r, int j) {
+  return static_cast<uint32_t>(r) * 64u + (static_cast<uint32_t>(j ^ ((r >> 1) & 3)) << 4);
 }
 
 __device__ __forceinline__ uint32_t pack2(float lo, float hi, __nv_bfloat16) {
