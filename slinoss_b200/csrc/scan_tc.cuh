@@ -37,42 +37,6 @@ constexpr int kTcL = 128;
 constexpr int kTcP = 64;
 constexpr int kTcThreads = 256;
 
-// coef * (4 packed complex values) -> 4 packed complex values in T.
-// fp32 rotation, one rounding to T: used wherever the gradient identities rely on
-// consistently rounded operands (the packed variant above costs ~1e-2 on dM)
-template <typename T>
-__device__ __forceinline__ uint4 rotate_chunk(uint4 raw, float2 coef) {
-  const uint32_t *w = reinterpret_cast<const uint32_t *>(&raw);
-  uint4 out;
-  uint32_t *o = reinterpret_cast<uint32_t *>(&out);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    float2 v = umma::unpack2(w[i], T());
-    float2 r = cmul(coef, v);
-    o[i] = umma::pack2(r.x, r.y, T());
-  }
-  return out;
-}
-// acc += sum_i conj(a_i) * b_i over the 4 packed complex values of two chunks
-template <typename T>
-__device__ __forceinline__ void cdot_chunk(uint4 a, uint4 b, float2 &acc) {
-  const uint32_t *wa = reinterpret_cast<const uint32_t *>(&a);
-  const uint32_t *wb = reinterpret_cast<const uint32_t *>(&b);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    float2 x = umma::unpack2(wa[i], T()), y = umma::unpack2(wb[i], T());
-    acc.x = fmaf(x.x, y.x, fmaf(x.y, y.y, acc.x));
-    acc.y = fmaf(x.x, y.y, fmaf(-x.y, y.x, acc.y));
-  }
-}
-__device__ __forceinline__ float2 octet_sum(float2 v) {  // sum over the 8 lanes that share a tile row
-#pragma unroll
-  for (int off = 4; off > 0; off >>= 1) {
-    v.x += __shfl_xor_sync(0xffffffffu, v.x, off);
-    v.y += __shfl_xor_sync(0xffffffffu, v.y, off);
-  }
-  return v;
-}
 // The four complex values of a 16-byte cell for packed fp32 arithmetic (fma.rn.f32x2: two fmas per instruction, each of
 // them the IEEE one): the real parts of two values side by side, and their imaginary parts.
 struct CellF {
@@ -91,6 +55,24 @@ __device__ __forceinline__ CellF unpack_cell(uint4 raw) {
   return c;
 }
 __device__ __forceinline__ float2 both(float v) { return make_float2(v, v); }
+// (a + i b) * cell in fp32, rounded to T once
+template <typename T>
+__device__ __forceinline__ uint4 rotate_cell(const CellF &c, float a, float b) {
+  uint4 out;
+  uint32_t *o = reinterpret_cast<uint32_t *>(&out);
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    const float2 re = __ffma2_rn(both(a), c.re[q], __fmul2_rn(both(-b), c.im[q]));
+    const float2 im = __ffma2_rn(both(a), c.im[q], __fmul2_rn(both(b), c.re[q]));
+    o[2 * q] = umma::pack2(re.x, im.x, T());
+    o[2 * q + 1] = umma::pack2(re.y, im.y, T());
+  }
+  return out;
+}
+template <typename T>
+__device__ __forceinline__ uint4 rotate_chunk(uint4 raw, float2 coef) {
+  return rotate_cell<T>(unpack_cell<T>(raw), coef.x, coef.y);
+}
 // sums of conj(a) b in pairs: x = re re + im im,  p = re im - im re  (one sum for the two halves of p: the negation costs
 // less than the two registers that a second sum takes in the backward, 1.044 against 1.058 ms)
 struct CDot2 {
@@ -103,6 +85,14 @@ __device__ __forceinline__ void cdot2(float2 ar, float2 ai, float2 br, float2 bi
   acc.x = __ffma2_rn(ai, bi, acc.x);
 }
 __device__ __forceinline__ float2 cdot2_sum(const CDot2 &a) { return make_float2(a.x.x + a.x.y, a.p.x + a.p.y); }
+__device__ __forceinline__ float2 octet_sum(float2 v) {  // sum over the 8 lanes that share a tile row
+#pragma unroll
+  for (int off = 4; off > 0; off >>= 1) {
+    v.x += __shfl_xor_sync(0xffffffffu, v.x, off);
+    v.y += __shfl_xor_sync(0xffffffffu, v.y, off);
+  }
+  return v;
+}
 template <typename T>
 __device__ __forceinline__ uint4 pack8(const float *v) {
   uint4 out;
@@ -153,6 +143,10 @@ __device__ __forceinline__ void scale32(float (&v)[32], float rf, const float *t
   }
 }
 
+// The forward sends a chunk's rows through L2 as a whole where the launch is several waves of CTAs long and bound by
+// DRAM (8192 CTAs: 0.361 against 0.381 ms).  In a launch of one or two waves all CTAs ask for their first slab at the
+// same time, and it waits behind everybody's rows (512 CTAs: a whole inference pass takes 62.4 us with, 60.2 without).
+constexpr unsigned kL2PrefetchCtas = 4 * 2 * kB200Sms;
 constexpr size_t scan_fwd_tc_smem_bytes() { return 1024 + 88 * 1024 + 12 * 1024; }
 
 // Forward chunk scan (replaces reference.py:1059 chunk_scan) on tensor cores.
@@ -161,6 +155,10 @@ constexpr size_t scan_fwd_tc_smem_bytes() { return 1024 + 88 * 1024 + 12 * 1024;
 //   Yd = S' U                  (128 x 64,  K = 128),  S' = masked/decayed S (+ diagonal)
 //   Y  = Yd + exp(lp_t) Yo;  the token in front of the chunk takes source slot 127 of S' / U, token 127's own
 //        diagonal term is added by hand
+// 8192 chunks of D 256: 0.346 ms, 72 % of the copy rate (0.361 before rotations and dots worked on two complex values per
+// instruction, 0.381 before the rows went through L2 as a whole).  Bound by the latencies of a slab (copies, rotations,
+// products) with two CTAs per SM.  Slabs of 32 columns with two buffers for every operand, so that no product is waited
+// for, and copies by TMA two slabs ahead: 0.374 ms.
 template <typename T>
 __global__ void __launch_bounds__(kTcThreads, 2) chunk_scan_fwd_tc_kernel(ScanFwdArgs<T> a) {
   constexpr int L = kTcL, P = kTcP;
@@ -234,6 +232,13 @@ __global__ void __launch_bounds__(kTcThreads, 2) chunk_scan_fwd_tc_kernel(ScanFw
   }
   prefetch_cb(0);
   prefetch_z(0);
+  if (tid == 0 && gridDim.x * gridDim.y > kL2PrefetchCtas) {
+    // The chunk's rows and its start state are contiguous in memory: whole into L2, from where the slabs take their
+    // columns.  Without it DRAM sees every row in four visits of 128 bytes, and a slab waits for it.
+    umma::l2_prefetch(a.C + tok0 * d.D, valid * d.D * 2);
+    umma::l2_prefetch(a.B + tok0 * d.D, valid * d.D * 2);
+    umma::l2_prefetch(z0, P * d.D * 2);
+  }
 
 #define SLX_FSTAMP(i) SLX_DIAG_STAMP(64 + (i))
   SLX_FSTAMP(0);
@@ -283,9 +288,9 @@ __global__ void __launch_bounds__(kTcThreads, 2) chunk_scan_fwd_tc_kernel(ScanFw
 
   const uint32_t sQ = umma::smem_u32(tQ), sK = umma::smem_u32(tK), sU = umma::smem_u32(tU), sS = umma::smem_u32(tS);
   constexpr int fmt = umma::HalfFmt<T>::value;
-  float2 acc_cb[4];
+  CDot2 acc_cb[4];
 #pragma unroll
-  for (int i = 0; i < 4; ++i) acc_cb[i] = make_float2(0.f, 0.f);
+  for (int i = 0; i < 4; ++i) acc_cb[i].x = acc_cb[i].p = make_float2(0.f, 0.f);
   uint32_t phase = 0;
   bool ok = true;
 
@@ -330,9 +335,13 @@ __global__ void __launch_bounds__(kTcThreads, 2) chunk_scan_fwd_tc_kernel(ScanFw
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       int r = r0 + 32 * i;
-      *reinterpret_cast<uint4 *>(tQ + umma::swz_off(r, j)) = rotate_chunk<T>(cr[i], cconj(ph[r]));
-      *reinterpret_cast<uint4 *>(tK + umma::swz_off(r, j)) = rotate_chunk<T>(r == L - 1 ? bm : br[i], gk[r]);
-      cdot_chunk<T>(cr[i], br[i], acc_cb[i]);
+      const CellF cf = unpack_cell<T>(cr[i]), bf = unpack_cell<T>(br[i]);
+      const float2 f = ph[r], g = gk[r];
+      *reinterpret_cast<uint4 *>(tQ + umma::swz_off(r, j)) = rotate_cell<T>(cf, f.x, -f.y);
+      *reinterpret_cast<uint4 *>(tK + umma::swz_off(r, j)) =
+          i < 3 || r != L - 1 ? rotate_cell<T>(bf, g.x, g.y) : rotate_chunk<T>(bm, g);
+#pragma unroll
+      for (int q = 0; q < 2; ++q) cdot2(cf.re[q], cf.im[q], bf.re[q], bf.im[q], acc_cb[i]);
     }
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
@@ -365,7 +374,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) chunk_scan_fwd_tc_kernel(ScanFw
   // per-row dots: cb_t = <c_t, b_t>
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    float2 s1 = octet_sum(acc_cb[i]);
+    float2 s1 = octet_sum(cdot2_sum(acc_cb[i]));
     if (j == 0) cbv[r0 + 32 * i] = s1;
   }
   ok = umma::mbar_wait(mbar_s, phase) && ok;
@@ -388,7 +397,9 @@ __global__ void __launch_bounds__(kTcThreads, 2) chunk_scan_fwd_tc_kernel(ScanFw
       if (c0 <= 32 * q4 + 31 || last) {
         umma::tmem_ld32(umma::tmem_addr(tmem, 32 * q4, c0), v);
         const float s127 = v[31];
-        if (c0 <= 32 * q4 + 31) {
+        if (c0 < 32 * q4 && fast_decay) {
+          scale32(v, __expf(lpt - lp[c0 + 1]), e2 + c0);
+        } else if (c0 <= 32 * q4 + 31) {
           if (fast_decay) decay_mask32<true>(v, c0, t, lpt, lp, e2, dg);
           else decay_mask32<false>(v, c0, t, lpt, lp, e2, dg);
         } else {

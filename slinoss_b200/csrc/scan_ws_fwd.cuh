@@ -29,6 +29,19 @@
 
 namespace slx {
 
+// acc += sum_i conj(a_i) * b_i over the 4 packed complex values of two chunks
+template <typename T>
+__device__ __forceinline__ void cdot_chunk(uint4 a, uint4 b, float2 &acc) {
+  const uint32_t *wa = reinterpret_cast<const uint32_t *>(&a);
+  const uint32_t *wb = reinterpret_cast<const uint32_t *>(&b);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    float2 x = umma::unpack2(wa[i], T()), y = umma::unpack2(wb[i], T());
+    acc.x = fmaf(x.x, y.x, fmaf(x.y, y.y, acc.x));
+    acc.y = fmaf(x.x, y.y, fmaf(-x.y, y.x, acc.y));
+  }
+}
+
 struct alignas(64) WsFwdMaps {
   CUtensorMap C, B, Z, U, Y;
 };

@@ -120,6 +120,11 @@ __device__ __forceinline__ void tma_prefetch_map(const void *tensor_map) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(tensor_map)) : "memory");
 }
 
+// Contiguous bytes (multiples of 16) on their way into L2.
+__device__ __forceinline__ void l2_prefetch(const void *p, uint32_t bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
+}
+
 // ---- pieces of the warp-specialised (producer / issuer / worker) kernels ---------------------------
 __device__ __forceinline__ void mbar_arrive(uint32_t mbar_saddr) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(mbar_saddr) : "memory");
