@@ -209,20 +209,11 @@ __device__ __forceinline__ uint4 jchunk(uint4 v) { return make_uint4(jword(v.x),
 // instead of spinning forever (each try_wait poll blocks for a short
 // hardware-defined time by itself).
 __device__ __forceinline__ bool mbar_wait(uint32_t mbar_saddr, uint32_t parity) {
+  if (mbar_test(mbar_saddr, parity)) return true;  // (reading the clock takes longer than the test)
   const long long t0 = clock64();
-  for (;;) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t"
-        ".reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.b32 %0, 1, 0, p;\n\t"
-        "}\n"
-        : "=r"(done)
-        : "r"(mbar_saddr), "r"(parity)
-        : "memory");
-    if (done) return true;
-    if (clock64() - t0 > 2000000000LL) return false;
+  for (int poll = 1;; ++poll) {
+    if (mbar_test(mbar_saddr, parity)) return true;
+    if ((poll & 7) == 0 && clock64() - t0 > 2000000000LL) return false;
   }
 }
 
