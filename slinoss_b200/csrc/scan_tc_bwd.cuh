@@ -28,13 +28,15 @@
 // values side by side, which is what the packed fp32 arithmetic (two fmas per instruction) takes.
 //
 // What bounds it: neither HBM (46 %) nor the tensor pipe (12 %) but instruction issue and the latencies between a
-// chunk's phases (loads and prefix, slabs, tail).  8192 chunks of D 256: 1.044 ms.  One CTA of 16 worker warps per SM
+// chunk's phases (loads and prefix, slabs, tail).  8192 chunks of D 256: 1.036 ms.  One CTA of 16 worker warps per SM
 // with 64-column slabs and two buffers for every operand took 1.205 ms: its phases followed one another and nothing
 // filled their latencies.  Two CTAs of 8 warps run different phases at the same time.  They fit because the slabs are 32
 // columns wide with one buffer, dS'^T Q / U Lambda and dS' kappa / dY Z0 take turns in the same 64 accumulator columns,
 // and dC / dB leave from registers (whole 32-byte sectors).  Measured on the way: a ninth warp that issues the products
 // leaves 96 registers to a thread, and the spills cost more than the issuing (1.097 against 0.997 ms); one thread that
-// waits for the products and a CTA barrier behind it 1.198 against 1.070 ms.
+// waits for the products and a CTA barrier behind it 1.198 against 1.070 ms.  8192 chunks of D 64: 0.668 -> 0.460 ms.  Where a
+// launch has no more chunks than SMs the second CTA is missing and eight warps take longer than sixteen did: 128 chunks of
+// D 256 0.035 -> 0.043 ms (passes of that size are bound by the host or nearly so).
 //
 // Thread mapping: thread = (row 32*(warp%4)+lane, 16-byte chunks 2*(warp/4) and +1 of the slab), the tensor-memory
 // lane mapping, for staging and epilogue alike, so that the raw b, c of a cell stay in registers from one to the other.
