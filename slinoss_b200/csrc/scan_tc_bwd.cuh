@@ -102,7 +102,7 @@ __global__ void __launch_bounds__(kTcBwdThreads, 2) chunk_scan_bwd_tc_kernel(Sca
   float *gd = tab + L;                         // G[t][t]
   float *um = gd + L;                          // 64   u_127
   float *duc = um + 64;                        // 64   (k^c b_127) . Lambda[p]
-  float *xb = duc + 64;                        // 256  xi of the token in front of the chunk
+  float *xb = duc + 64;                        // 256  dS'^T Q of the token in front of the chunk
   float *ulf = xb + 256;                       // 256  u_127 . Lambda
   float *ulw = ulf + 256;                      // [8][32] per-warp partials of u_127 . Lambda
   float2 *mraw = reinterpret_cast<float2 *>(xb), *kc = reinterpret_cast<float2 *>(ulf),
@@ -110,6 +110,7 @@ __global__ void __launch_bounds__(kTcBwdThreads, 2) chunk_scan_bwd_tc_kernel(Sca
   float2 *ph = reinterpret_cast<float2 *>(ulw + 256);
   float2 *bm1 = ph + L;                        // 128  b_{-1}
   float2 *bh1 = bm1 + 128;                     // 128  k^c b_127
+  float *ub = reinterpret_cast<float *>(bh1);  // 256  U Lambda of the token in front of the chunk, behind helper()'s reads
   float2 *misc = bh1 + 128;                    // [0..3] dk^p_0, [4..7] sum conj(b_127) (u_127 . Lambda), by warp
   uint64_t *bars = reinterpret_cast<uint64_t *>(misc + 8);  // [0] first, [1] second products of a slab; [2] G, then
                                                             // S'^T dY; [3] raw slab by TMA
@@ -118,7 +119,7 @@ __global__ void __launch_bounds__(kTcBwdThreads, 2) chunk_scan_bwd_tc_kernel(Sca
                     scan_bwd_tc_smem_bytes(), "shared-memory layout");
   // scratch of the tail, over the raw slabs
   float2 *pgs = reinterpret_cast<float2 *>(sC), *pbs = pgs + L, *pcs = pbs + L;  // second column half: gA, bX; bc
-  float2 *bXs = pcs + 2 * L, *sums = bXs + L;  // sums: [0..3] g by warp, [4], [5] conj(kappa) xi of slot 127
+  float2 *bXs = pcs + 2 * L, *sums = bXs + L;  // sums: [0..3] g by warp, [4..7] correction of slot 127 by warp
 
   const ScanDims d = a.d;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -139,7 +140,7 @@ __global__ void __launch_bounds__(kTcBwdThreads, 2) chunk_scan_bwd_tc_kernel(Sca
   if (warp == 2) chunk_prefix_load4(a.M + tok0 * 2, valid, mreg);
   // U and dY land in their tiles by asynchronous copy (rows past the chunk end are zero-filled)
   const int j8 = tid & 7, r8 = tid >> 3;
-  uint4 ub = make_uint4(0, 0, 0, 0);  // the thread that copies a cell of row 127: that cell of u_{-1}
+  uint4 ucell = make_uint4(0, 0, 0, 0);  // the thread that copies a cell of row 127: that cell of u_{-1}
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const int r = r8 + 32 * i;
@@ -154,12 +155,12 @@ __global__ void __launch_bounds__(kTcBwdThreads, 2) chunk_scan_bwd_tc_kernel(Sca
   }
   if (r8 == 31) {
     if (t0 > 0) {
-      ub = *reinterpret_cast<const uint4 *>(a.U + (tok0 - 1) * P + 8 * j8);
+      ucell = *reinterpret_cast<const uint4 *>(a.U + (tok0 - 1) * P + 8 * j8);
     } else if (a.Uprev) {
       float v[8];
 #pragma unroll
       for (int e = 0; e < 8; ++e) v[e] = load_as_f(a.Uprev, a.prev_dtype, (size_t)bh * P + 8 * j8 + e);
-      ub = pack8<T>(v);
+      ucell = pack8<T>(v);
     }
   }
   asm volatile("cp.async.commit_group;" ::: "memory");
@@ -220,7 +221,7 @@ __global__ void __launch_bounds__(kTcBwdThreads, 2) chunk_scan_bwd_tc_kernel(Sca
     const uint32_t *w = reinterpret_cast<const uint32_t *>(&own);
 #pragma unroll
     for (int e = 0; e < 4; ++e) *reinterpret_cast<float2 *>(um + 8 * j8 + 2 * e) = umma::unpack2(w[e], T());
-    *cell = ub;
+    *cell = ucell;
   }
   umma::fence_smem_to_async();
   umma::fence_before_sync();
@@ -331,8 +332,9 @@ __global__ void __launch_bounds__(kTcBwdThreads, 2) chunk_scan_bwd_tc_kernel(Sca
     __syncwarp();
   };
   const float2 zero2 = make_float2(0.f, 0.f);
-  // conj(b) c;  conj(dC) c, the part through kappa against the rounded Q instead;  conj(b) xi;  conj(kappa) xi
-  CDot2 d_bc{zero2, zero2}, d_g = d_bc, d_x = d_bc, d_k = d_bc;
+  // conj(b) c;  conj(dC) c, the part through kappa against the rounded Q instead;  conj(b) xi;  and of dS'^T Q alone the
+  // dots with kappa and with b
+  CDot2 d_bc{zero2, zero2}, d_g = d_bc, d_x = d_bc, d_k = d_bc, d_b = d_bc;
   uint4 cr[2], br[2];                                       // raw cells of the slab
 
   // operand tiles of slab sl
@@ -484,23 +486,14 @@ __global__ void __launch_bounds__(kTcBwdThreads, 2) chunk_scan_bwd_tc_kernel(Sca
       if (sl + 1 < NB) prefetch_zl(sl + 1);
     }
     // ---- xi = dS'^T Q + es U Lambda ------------------------------------------------------------
-    float2 xr[4], xi[4];  // pairs of complex values: cell 0, cell 1
     wait(0);
-  umma::fence_after_sync();
+    umma::fence_after_sync();
     SLX_STAMP(9 + 4 * sl);
-    {
-      uint32_t r1[16], r2[16];
-      umma::tmem_ld16_issue(umma::tmem_addr(tmem + kTmX, 32 * q4, 16 * h), r1);
-      umma::tmem_ld16_issue(umma::tmem_addr(tmem + kTmUL, 32 * q4, 16 * h), r2);
-      umma::tmem_ld16_wait(r1);
-      umma::tmem_ld16_wait(r2);
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int o = 8 * (q >> 1) + 2 * (q & 1);
-        xr[q] = __ffma2_rn(both(es), tm_pair(r2 + o), tm_pair(r1 + o));
-        xi[q] = __ffma2_rn(both(es), tm_pair(r2 + o + 4), tm_pair(r1 + o + 4));
-      }
-    }
+    uint32_t x1[16], x2[16];  // dS'^T Q, U Lambda
+    umma::tmem_ld16_issue(umma::tmem_addr(tmem + kTmX, 32 * q4, 16 * h), x1);
+    umma::tmem_ld16_issue(umma::tmem_addr(tmem + kTmUL, 32 * q4, 16 * h), x2);
+    umma::tmem_ld16_wait(x1);
+    umma::tmem_ld16_wait(x2);
     umma::fence_before_sync();
     __syncthreads();  // dS'^T Q and U Lambda are in registers
     issue_second(sl);
@@ -510,10 +503,13 @@ __global__ void __launch_bounds__(kTcBwdThreads, 2) chunk_scan_bwd_tc_kernel(Sca
       for (int w = 0; w < 8; ++w) acc += ulw[32 * w + lane];
       ulf[32 * sl + lane] = acc;
     }
-    if (last_row) {  // xi of the token in front of the chunk; token 127's own dB is formed in the tail
+    if (last_row) {  // of the token in front of the chunk: dS'^T Q and U Lambda; token 127's own dB is formed in the tail
 #pragma unroll
-      for (int q = 0; q < 4; ++q)
-        *reinterpret_cast<float4 *>(xb + 32 * sl + 16 * h + 4 * q) = make_float4(xr[q].x, xi[q].x, xr[q].y, xi[q].y);
+      for (int q = 0; q < 4; ++q) {
+        const int o = 8 * (q >> 1) + 2 * (q & 1), col = 32 * sl + 16 * h + 4 * q;
+        *reinterpret_cast<uint4 *>(xb + col) = make_uint4(x1[o], x1[o + 4], x1[o + 1], x1[o + 5]);
+        *reinterpret_cast<uint4 *>(ub + col) = make_uint4(x2[o], x2[o + 4], x2[o + 1], x2[o + 5]);
+      }
     }
     // ---- dB_s = conj(gk_s) xi_s + conj(cA_s) c_s -------------------------------------------------
     {
@@ -525,7 +521,9 @@ __global__ void __launch_bounds__(kTcBwdThreads, 2) chunk_scan_bwd_tc_kernel(Sca
         uint32_t *w = reinterpret_cast<uint32_t *>(&o[k]);
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
-          const float2 x = xr[2 * k + q], y = xi[2 * k + q];
+          const float2 x0 = tm_pair(x1 + 8 * k + 2 * q), y0 = tm_pair(x1 + 8 * k + 4 + 2 * q);
+          const float2 x = __ffma2_rn(both(es), tm_pair(x2 + 8 * k + 2 * q), x0);
+          const float2 y = __ffma2_rn(both(es), tm_pair(x2 + 8 * k + 4 + 2 * q), y0);
           float2 re = __fmul2_rn(both(cA.x), cf.re[q]), im = __fmul2_rn(both(cA.x), cf.im[q]);
           re = __ffma2_rn(both(cA.y), cf.im[q], re);
           im = __ffma2_rn(both(-cA.y), cf.re[q], im);
@@ -534,7 +532,8 @@ __global__ void __launch_bounds__(kTcBwdThreads, 2) chunk_scan_bwd_tc_kernel(Sca
           re = __ffma2_rn(both(gk.y), y, re);
           im = __ffma2_rn(both(-gk.y), x, im);
           cdot2(bf.re[q], bf.im[q], x, y, d_x);
-          cdot2(kf.re[q], kf.im[q], x, y, d_k);
+          cdot2(kf.re[q], kf.im[q], x0, y0, d_k);
+          cdot2(bf.re[q], bf.im[q], x0, y0, d_b);
           w[2 * q] = umma::pack2(re.x, im.x, T());
           w[2 * q + 1] = umma::pack2(re.y, im.y, T());
         }
@@ -544,7 +543,7 @@ __global__ void __launch_bounds__(kTcBwdThreads, 2) chunk_scan_bwd_tc_kernel(Sca
     SLX_STAMP(10 + 4 * sl);
     // ---- dC_t = f_t (dS' kappa)_t + p_t (dY Z0)_t + cA_t b_t ------------------------------------------
     wait(1);
-  umma::fence_after_sync();
+    umma::fence_after_sync();
     SLX_STAMP(11 + 4 * sl);
     {
       uint4 o[2];
@@ -610,11 +609,12 @@ __global__ void __launch_bounds__(kTcBwdThreads, 2) chunk_scan_bwd_tc_kernel(Sca
   float2 bc = cdot2_sum(d_bc), gA = cdot2_sum(d_g), bX = cdot2_sum(d_x);
   // dM sums, over the pairs (t, s) of the chunk, differences of the same products seen from t (gA) and from s (k^c, k^p
   // against bX).  Taken with the rounded kappa and Q on both sides they cancel as the exact ones do: the term of s is
-  // corrected by sum conj(kappa) xi - conj(gk) sum conj(b) xi, and at t = 0 the sum over the token in front of the chunk
-  // is that of conj(kappa) xi.  With the unrounded b and c in these sums dM was 2.5 times as far from float64 (relative
-  // error 5e-3 against 2e-3 for one chunk of N 128 in bf16; the kernel took 0.978 instead of 1.058 ms).
-  if (last_row) sums[4 + h] = cdot2_sum(d_k);
-  else gA = csub(gA, csub(cdot2_sum(d_k), cmul(cconj(gk), bX)));
+  // corrected by sum conj(kappa) X - conj(gk) sum conj(b) X, X = dS'^T Q (for the token in front of the chunk at t = 0).
+  // With the unrounded b and c in these sums dM was 2.5 times as far from float64 (relative error 5e-3 against 2e-3 for one
+  // chunk of N 128 in bf16).  The increment path stays with the unrounded b: its other side, <z_end, Lambda>, holds the
+  // increments as the forward rounded them, and a second rounding only adds to that (a state gradient a hundred times
+  // its usual size, N 64, bf16: 8.3e-3 with conj(kappa) xi, 6.8e-3 so; 1.030 and 1.050 ms for 8192 chunks of D 256).
+  if (!last_row) gA = csub(gA, csub(cdot2_sum(d_k), cmul(cconj(gk), cdot2_sum(d_b))));
   bX = cmul(f_next, bX);
   pcs[L * h + row] = bc;
   if (h == 1) {
@@ -634,13 +634,16 @@ __global__ void __launch_bounds__(kTcBwdThreads, 2) chunk_scan_bwd_tc_kernel(Sca
   float *cB = a.carryB + ((size_t)bh * d.NC + c) * d.D;
   {
     const int n = tid & 127;  // = row
-    float2 contrib = zero2;
+    float2 contrib = zero2, corr = zero2;
     if (n < d.N) {
       if (tid < 128) {
         // token in front of the chunk: dB_{-1}[n] = conj(k^p_0) f_0 xi[n], dk^p_0 = sum_n conj(b_{-1}[n]) f_0 xi[n]
-        const float2 x = cmul(cmulc(ph[0], ph[L - 1]), *reinterpret_cast<const float2 *>(xb + 2 * n));
+        const float2 f_0 = cmulc(ph[0], ph[L - 1]), X = *reinterpret_cast<const float2 *>(xb + 2 * n), b = bm1[n];
+        const float2 x = cmul(f_0, cadd(X, cscale(*reinterpret_cast<const float2 *>(ub + 2 * n), __expf(lp[L - 1] - lp[0]))));
         *reinterpret_cast<float2 *>(cB + 2 * n) = cmul(cconj(k_edge), x);
-        contrib = cmul(cconj(bm1[n]), x);
+        contrib = cmul(cconj(b), x);
+        const float2 kap = cmul(cmulc(k_edge, f_0), b);
+        corr = cmul(cconj(csub(umma::unpack2(umma::pack2(kap.x, kap.y, T()), T()), kap)), X);
       } else if (valid == L) {
         // token 127: dB[n] = conj(k^c) (u_127 . Lambda)[n] + conj(k^c G) c[n]
         const float2 ul = *reinterpret_cast<const float2 *>(ulf + 2 * n);
@@ -654,6 +657,14 @@ __global__ void __launch_bounds__(kTcBwdThreads, 2) chunk_scan_bwd_tc_kernel(Sca
       contrib.y += __shfl_xor_sync(0xffffffffu, contrib.y, off);
     }
     if (lane == 0) misc[warp] = contrib;
+    if (h == 0) {
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1) {
+        corr.x += __shfl_xor_sync(0xffffffffu, corr.x, off);
+        corr.y += __shfl_xor_sync(0xffffffffu, corr.y, off);
+      }
+      if (lane == 0) sums[4 + warp] = corr;
+    }
   }
   SLX_STAMP(56);
   // ---- S^T -> S'^T (forward scores; row 127 = boundary) --------------------------------
@@ -712,8 +723,8 @@ __global__ void __launch_bounds__(kTcBwdThreads, 2) chunk_scan_bwd_tc_kernel(Sca
     else dkc = cadd(dkc, cadd(cadd(misc[4], misc[5]), cadd(misc[6], misc[7])));
     const float2 dkp = (t == 0) ? cadd(cadd(misc[0], misc[1]), cadd(misc[2], misc[3])) : bXs[t - 1];
     if (t < valid) *reinterpret_cast<float4 *>(a.dK + (tok0 + t) * 4) = make_float4(dkp.x, dkp.y, dkc.x, dkc.y);
-    const float2 kp_term = (t == 0) ? cadd(sums[4], sums[5]) : cmul(make_float2(k4.x, -k4.y), dkp);
-    float2 g = csub(gA, cadd(cmul(make_float2(k4.z, -k4.w), dkc), kp_term));
+    float2 g = csub(gA, cadd(cmul(make_float2(k4.z, -k4.w), dkc), cmul(make_float2(k4.x, -k4.y), dkp)));
+    if (t == 0) g = csub(g, cadd(cadd(sums[4], sums[5]), cadd(sums[6], sums[7])));
     if (last_row) g = cadd(g, zd);
 #pragma unroll
     for (int off = 1; off < 32; off <<= 1) {

@@ -94,13 +94,18 @@ def test_operands_are_rounded_once(dtype, N, lo, scale):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
-@pytest.mark.parametrize("N,lo", [(64, 0.3), (128, 0.3), (32, 0.6)])
-def test_sums_of_dM_cancel(dtype, N, lo):
+@pytest.mark.parametrize("N,lo,scale,bound", [(64, 0.3, 1.0, 0.6), (128, 0.3, 1.0, 0.6), (32, 0.6, 1.0, 0.6),
+                                              (64, 0.9, 100.0, 1.08)])
+def test_sums_of_dM_cancel(dtype, N, lo, scale, bound):
     """dM is a suffix sum of differences between the same products seen from the query and from the source.  The model
     takes one side against rounded operands and the other against the stored ones; with the rounded ones on both sides
-    the model's error falls to 0.25 (N 64) ... 0.39 (N 128) of that in float64 arithmetic, 0.6 leaves room for the draw."""
-    inp = _inputs(dtype, N, lo, 1.0, "cuda")
+    the model's error falls to 0.25 (N 64) ... 0.39 (N 128) of that in float64 arithmetic, 0.6 leaves room for the draw.
+
+    Where the gradient of the state decides dM, the other side of the increment path is the end state as the forward
+    rounded it: rounded operands there add to the error instead, 1.18 of the model's against 0.97 with the stored ones
+    (float64 arithmetic, scale 100, either type); the bound lies between the two."""
+    inp = _inputs(dtype, N, lo, scale, "cuda")
     exact = oracle_fwd_bwd(inp)[2]["dM"]
     model = _model(inp, lambda x: torch.from_numpy(np.ascontiguousarray(x)).to(dtype).double().numpy())["dM"]
     got = run_b200_fwd_bwd(inp, 128)[2]["dM"]
-    assert rel_err(to_np(got), exact) < 0.6 * rel_err(model, exact)
+    assert rel_err(to_np(got), exact) < bound * rel_err(model, exact)
