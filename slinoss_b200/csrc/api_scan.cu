@@ -251,8 +251,9 @@ static int launch_outer_tc(const ScanDims &d, const void *A, const void *X, cons
 
 template <typename T>
 static int launch_scan_bwd_tc(const ScanDims &d, const ScanBwdArgs<T> &a, cudaStream_t st) {
-  auto kern = chunk_scan_bwd_tc_kernel<T>;
-  size_t smem = scan_bwd_tc_smem_bytes();
+  const bool prev32 = a.Uprev && a.prev_dtype == SLX_F32;
+  auto kern = prev32 ? chunk_scan_bwd_tc_kernel<T, true> : chunk_scan_bwd_tc_kernel<T, false>;
+  const size_t smem = scan_bwd_tc_smem_bytes(prev32);
   int rc = set_smem(kern, smem);
   if (rc) return rc;
   ScanBwdMaps maps;

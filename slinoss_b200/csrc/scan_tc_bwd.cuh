@@ -38,6 +38,10 @@
 // launch has no more chunks than SMs the second CTA is missing and eight warps take longer than sixteen did: 128 chunks of
 // D 256 0.035 -> 0.043 ms (passes of that size are bound by the host or nearly so).
 //
+// PREV32: the streaming rows are fp32.  The tile then holds u_{-1} rounded, and its products with dY and Lambda get what
+// that lost from the CUDA cores, as u_{-1} enters dB_prev, dK and dM in fp32.  An instantiation of its own: as a branch it
+// costs every launch (8192 chunks of D 256: 1.064 against 1.050 ms).
+//
 // Thread mapping: thread = (row 32*(warp%4)+lane, 16-byte chunks 2*(warp/4) and +1 of the slab), the tensor-memory
 // lane mapping, for staging and epilogue alike, so that the raw b, c of a cell stay in registers from one to the other.
 #pragma once
@@ -53,7 +57,7 @@ struct alignas(64) ScanBwdMaps {
 
 constexpr int kTcBwdThreads = 256;
 constexpr uint32_t kBwdScalars = 106496;
-constexpr size_t scan_bwd_tc_smem_bytes() { return kBwdScalars + 8320; }
+constexpr size_t scan_bwd_tc_smem_bytes(bool prev32) { return kBwdScalars + 8320 + (prev32 ? 256 : 0); }
 constexpr int kTmR = 128, kTmX = 192, kTmUL = 224, kTmU = kTmX;  // accumulator columns (G / S^T at 0)
 
 // (a + i b) * cell, packed as four real parts and four imaginary parts
@@ -82,7 +86,7 @@ __device__ __forceinline__ float2 tm_pair(const uint32_t *r) {
   return make_float2(__uint_as_float(r[0]), __uint_as_float(r[1]));
 }
 
-template <typename T>
+template <typename T, bool PREV32>
 __global__ void __launch_bounds__(kTcBwdThreads, 2) chunk_scan_bwd_tc_kernel(ScanBwdArgs<T> a,
                                                                               const __grid_constant__ ScanBwdMaps maps) {
   constexpr int L = kTcL, P = kTcP;
@@ -115,8 +119,9 @@ __global__ void __launch_bounds__(kTcBwdThreads, 2) chunk_scan_bwd_tc_kernel(Sca
   uint64_t *bars = reinterpret_cast<uint64_t *>(misc + 8);  // [0] first, [1] second products of a slab; [2] G, then
                                                             // S'^T dY; [3] raw slab by TMA
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 4);
-  static_assert(kBwdScalars + 4 * (3 * 128 + 2 * 64 + 3 * 256) + 8 * 3 * 128 + 64 + 4 * 8 + 4 <=
-                    scan_bwd_tc_smem_bytes(), "shared-memory layout");
+  float *ulo = reinterpret_cast<float *>(base + scan_bwd_tc_smem_bytes(false));  // PREV32: 64  what u_{-1} loses in its tile
+  static_assert(kBwdScalars + 4 * (3 * 128 + 2 * 64 + 3 * 256) + 8 * 3 * 128 + 64 + 4 * 8 + 8 <=
+                    scan_bwd_tc_smem_bytes(false), "shared-memory layout");
   // scratch of the tail, over the raw slabs
   float2 *pgs = reinterpret_cast<float2 *>(sC), *pbs = pgs + L, *pcs = pbs + L;  // second column half: gA, bX; bc
   float2 *bXs = pcs + 2 * L, *sums = bXs + L;  // sums: [0..3] g by warp, [4..7] correction of slot 127 by warp
@@ -161,6 +166,10 @@ __global__ void __launch_bounds__(kTcBwdThreads, 2) chunk_scan_bwd_tc_kernel(Sca
 #pragma unroll
       for (int e = 0; e < 8; ++e) v[e] = load_as_f(a.Uprev, a.prev_dtype, (size_t)bh * P + 8 * j8 + e);
       ucell = pack8<T>(v);
+      if constexpr (PREV32) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) ulo[8 * j8 + e] = v[e] - to_f(from_f<T>(v[e]));
+      }
     }
   }
   asm volatile("cp.async.commit_group;" ::: "memory");
@@ -425,7 +434,7 @@ __global__ void __launch_bounds__(kTcBwdThreads, 2) chunk_scan_bwd_tc_kernel(Sca
     float v[32];
     if (blk <= q4 || blk == 3) {
       umma::tmem_ld32(umma::tmem_addr(tmem, 32 * q4, c0), v);
-      const float g127 = v[31];
+      float g127 = v[31];
       if (blk < q4) {
         if (fast_decay) scale32(v, __expf(lp_r - lp[c0 + 1]), tab + c0);
         else decay_mask32<false>(v, c0, row, lp_r, lp, tab, 0.f);
@@ -441,7 +450,21 @@ __global__ void __launch_bounds__(kTcBwdThreads, 2) chunk_scan_bwd_tc_kernel(Sca
 #pragma unroll
         for (int i = 0; i < 32; ++i) v[i] = 0.f;
       }
-      if (blk == 3) v[31] = __expf(lp_r - lp[0]) * g127;  // boundary slot (column 127)
+      if (blk == 3) {  // boundary slot (column 127)
+        if (PREV32 && c == 0) {
+#pragma unroll 1
+          for (int j = 0; j < 8; ++j) {
+            const uint4 y = *reinterpret_cast<const uint4 *>(tdY + umma::swz_off(row, j));
+            const uint32_t *w = reinterpret_cast<const uint32_t *>(&y);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              const float2 yv = umma::unpack2(w[e], T());
+              g127 = fmaf(yv.x, ulo[8 * j + 2 * e], fmaf(yv.y, ulo[8 * j + 2 * e + 1], g127));
+            }
+          }
+        }
+        v[31] = __expf(lp_r - lp[0]) * g127;
+      }
     } else {  // block entirely above the diagonal
 #pragma unroll
       for (int i = 0; i < 32; ++i) v[i] = 0.f;
@@ -639,7 +662,12 @@ __global__ void __launch_bounds__(kTcBwdThreads, 2) chunk_scan_bwd_tc_kernel(Sca
       if (tid < 128) {
         // token in front of the chunk: dB_{-1}[n] = conj(k^p_0) f_0 xi[n], dk^p_0 = sum_n conj(b_{-1}[n]) f_0 xi[n]
         const float2 f_0 = cmulc(ph[0], ph[L - 1]), X = *reinterpret_cast<const float2 *>(xb + 2 * n), b = bm1[n];
-        const float2 x = cmul(f_0, cadd(X, cscale(*reinterpret_cast<const float2 *>(ub + 2 * n), __expf(lp[L - 1] - lp[0]))));
+        float2 ul = *reinterpret_cast<const float2 *>(ub + 2 * n);
+        if (PREV32 && c == 0) {
+#pragma unroll 4
+          for (int p = 0; p < P; ++p) ul = cadd(ul, cscale(load_pair<T>(lam + (size_t)p * d.D + 2 * n), ulo[p]));
+        }
+        const float2 x = cmul(f_0, cadd(X, cscale(ul, __expf(lp[L - 1] - lp[0]))));
         *reinterpret_cast<float2 *>(cB + 2 * n) = cmul(cconj(k_edge), x);
         contrib = cmul(cconj(b), x);
         const float2 kap = cmul(cmulc(k_edge, f_0), b);

@@ -109,3 +109,24 @@ def test_sums_of_dM_cancel(dtype, N, lo, scale, bound):
     model = _model(inp, lambda x: torch.from_numpy(np.ascontiguousarray(x)).to(dtype).double().numpy())["dM"]
     got = run_b200_fwd_bwd(inp, 128)[2]["dM"]
     assert rel_err(to_np(got), exact) < bound * rel_err(model, exact)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype,u", [(torch.bfloat16, 2.0 ** -8), (torch.float16, 2.0 ** -11)])
+@pytest.mark.parametrize("N,T", [(32, 128), (128, 77), (96, 300)])
+def test_fp32_streaming_rows_beside_half_ones(dtype, u, N, T):
+    """U_prev in fp32, half a step of the activation dtype (u of [1, 2)) above a value of that type everywhere: rounded to
+    that type all of it would be lost, u / 1.5 of dB_prev.  Through the state gradient (one chunk, values that the type
+    holds) dB_prev is made of fp32 products.  Through the scores each of the summed tokens is rounded to the type, to either
+    side: the mean over 16 heads and the few tokens that the decay leaves moves by u / 3 / sqrt(50) = 0.05 u."""
+    inp = make_scan_inputs(1, 16, T, N, 64, dtype, seed=N, with_init=True, dist="cfg2", device="cuda", streaming=True)
+    steps = torch.randint(0, int(0.25 / u), (1, 16, 64), generator=torch.Generator().manual_seed(1))
+    inp["U_prev"] = (1 + 4 * u * steps + 0.999 * u).cuda()  # (an even neighbour below: the nearest value of the type)
+    inp["B_prev"] = inp["B_prev"].float()
+    paths = [dict(d_final=0 * inp["d_final"])] + [dict(dY=0 * inp["dY"])] * (T <= 128)
+    for path, bound in zip(paths, (0.25 * u, 1e-5)):
+        case = {**inp, **path}
+        exact, got = oracle_fwd_bwd(case)[2]["dB_prev"], run_b200_fwd_bwd(case, 128)[2]["dB_prev"]
+        assert got.dtype == torch.float32
+        got = to_np(got)
+        assert abs((got * exact).sum() / (exact * exact).sum() - 1) < bound, path.keys()
