@@ -18,6 +18,14 @@ extern "C" {
  * cudaError_t like the main library. */
 int slx_umma_selftest(int mode, const void *A, const void *B, float *C,
                       int *status, void *stream);
+
+/* The bounded waits of the chunk kernels (mode 0 backward, 1 forward), made to
+ * run out: one warp passes
+ * n_waits (at most 64) waits of `limit` clocks (at most 4e8) on barriers that
+ * nothing arrives at.  out (3 device long longs): clocks of the waits, clocks of
+ * the drain behind them, 1 if no wait ran out. */
+int slx_wait_chain_selftest(int mode, int n_waits, long long limit,
+                            long long *out, void *stream);
 const char *slx_selftest_last_error_string(void);
 
 #ifdef __cplusplus

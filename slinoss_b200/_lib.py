@@ -123,6 +123,7 @@ def host():
 SELFTEST_LIB_PATH = LIB_PATH.with_name("libslinoss_b200_selftest.so")
 SELFTEST_SIGNATURES = {
     "slx_umma_selftest": (c_int32, [c_int32] + [_P] * 5),
+    "slx_wait_chain_selftest": (c_int32, [c_int32, c_int32, c_int64, _P, _P]),
     "slx_selftest_last_error_string": (c_char_p, []),
 }
 

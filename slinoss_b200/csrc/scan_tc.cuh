@@ -291,8 +291,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) chunk_scan_fwd_tc_kernel(ScanFw
   CDot2 acc_cb[4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) acc_cb[i].x = acc_cb[i].p = make_float2(0.f, 0.f);
-  uint32_t phase = 0;
-  bool ok = true;
+  umma::WaitChain products{mbar_s, 0};
 
   SLX_FSTAMP(1);
   for (int sl = 0; sl < NB; ++sl) {
@@ -300,8 +299,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) chunk_scan_fwd_tc_kernel(ScanFw
     // this slab's raw C, B arrived through cp.async (issued one slab ahead)
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     if (sl > 0) {
-      ok = umma::mbar_wait(mbar_s, phase) && ok;  // previous slab's products are done: tiles are free
-      phase ^= 1;
+      products.wait();  // previous slab's products are done: tiles are free
     } else if (r0 == 31) {
       // source slot 127 of S' is the token in front of the chunk: its row of the U tile (which this thread
       // copied in) becomes u_{-1}; token 127's own diagonal term is added by hand in the epilogue
@@ -359,7 +357,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) chunk_scan_fwd_tc_kernel(ScanFw
     SLX_FSTAMP(10 + 4 * sl);
     __syncthreads();
     SLX_FSTAMP(11 + 4 * sl);
-    if (tid == 0) {
+    if (tid == 0 && products.ok()) {
       umma::fence_after_sync();
       // [S | Yo] = Qbar [kappa ; Z0]^T as one product of N = 192 per K-step: Qbar is fetched once for both, and at
       // this width the fetches fit under the product's own time (two products of N = 128 and N = 64 do not)
@@ -377,8 +375,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) chunk_scan_fwd_tc_kernel(ScanFw
     float2 s1 = octet_sum(cdot2_sum(acc_cb[i]));
     if (j == 0) cbv[r0 + 32 * i] = s1;
   }
-  ok = umma::mbar_wait(mbar_s, phase) && ok;
-  phase ^= 1;
+  products.wait();
   umma::fence_after_sync();
   __syncthreads();
 
@@ -422,7 +419,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) chunk_scan_fwd_tc_kernel(ScanFw
   umma::fence_before_sync();
   SLX_FSTAMP(4);
   __syncthreads();
-  if (tid == 0) {
+  if (tid == 0 && products.ok()) {
     umma::fence_after_sync();
     const uint32_t id_y = umma::make_idesc(128, 64, false, true, fmt);
 #pragma unroll
@@ -431,8 +428,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) chunk_scan_fwd_tc_kernel(ScanFw
                    kk != 0);
     umma::commit(mbar_s);
   }
-  ok = umma::mbar_wait(mbar_s, phase) && ok;
-  phase ^= 1;
+  products.wait();
   umma::fence_after_sync();
 
   SLX_FSTAMP(5);
@@ -470,12 +466,16 @@ __global__ void __launch_bounds__(kTcThreads, 2) chunk_scan_fwd_tc_kernel(ScanFw
       *reinterpret_cast<uint4 *>(a.Y + (tok0 + r) * P + 8 * j) = *reinterpret_cast<const uint4 *>(tQ + umma::swz_off(r, j));
   }
   SLX_FSTAMP(6);
-  if (__syncthreads_or(!ok)) {
+  if (__syncthreads_or(!products.ok())) {
     // a bounded wait ran out: the rows just written came from unfinished products; overwrite them with NaN
     // so that the failure shows in the data as well as in the status word
     const T nanv = from_f<T>(__int_as_float(0x7fc00000));
     for (int e = tid; e < valid * P; e += kTcThreads) a.Y[tok0 * P + e] = nanv;
-    if (tid == 0) atomicExch(&g_tc_status, 1);
+    if (tid == 0) {
+      atomicExch(&g_tc_status, 1);
+      umma::drain_waits(mbar_s, 1);
+    }
+    __syncthreads();
   }
   if (warp == 0) umma::tmem_dealloc(tmem, 256);
 #undef SLX_FSTAMP
@@ -662,7 +662,11 @@ __global__ void __launch_bounds__(kTcThreads, 2) chunk_outer_tc_kernel(OuterArgs
   if (__syncthreads_or(!ok)) {  // a bounded wait ran out: NaN instead of values from an unfinished product
     const float nanf_ = __int_as_float(0x7fc00000);
     for (int e = tid; e < P * d.D; e += kTcThreads) outc[e] = from_f<OT>(nanf_);
-    if (tid == 0) atomicExch(&g_tc_status, 1);
+    if (tid == 0) {
+      atomicExch(&g_tc_status, 1);
+      umma::drain_waits(mbar_s, 1);
+    }
+    __syncthreads();
   }
   if (warp == 0) umma::tmem_dealloc(tmem, 128);
 }

@@ -336,7 +336,7 @@ __global__ void __launch_bounds__(kTcBwdThreads, 2) chunk_scan_bwd_tc_kernel(Sca
   uint32_t ph_bits = 0;  // phases of the barriers
   bool ok = (umma::smem_u32(smem_raw) & 1023u) == 0;
   auto wait = [&](int which) {
-    ok = umma::mbar_wait(bar0 + 8 * which, (ph_bits >> which) & 1) && ok;
+    ok = umma::mbar_wait(bar0 + 8 * which, (ph_bits >> which) & 1, ok) && ok;
     ph_bits ^= 1u << which;
     __syncwarp();
   };
@@ -418,7 +418,7 @@ __global__ void __launch_bounds__(kTcBwdThreads, 2) chunk_scan_bwd_tc_kernel(Sca
   stage(0);
   const bool fast_decay = !__syncthreads_or(tid < L && decay_step_out_of_range(lp, tid));
   if (warp == 1) {
-    if (lane == 0) prefetch_cb(1);  // every thread has its cells of slab 0 (NB >= 2)
+    if (lane == 0 && ok) prefetch_cb(1);  // every thread has its cells of slab 0 (NB >= 2)
     __syncwarp();
   }
   helper(0);
@@ -803,6 +803,10 @@ __global__ void __launch_bounds__(kTcBwdThreads, 2) chunk_scan_bwd_tc_kernel(Sca
   umma::fence_before_sync();
   SLX_STAMP(5);
   const int bad = __syncthreads_or(!ok);
+  if (bad) {
+    if (tid == 0) umma::drain_waits(bar0, 4);
+    __syncthreads();
+  }
   __syncwarp();
   if (warp == 1) {
     umma::fence_after_sync();

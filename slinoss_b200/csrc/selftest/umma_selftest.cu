@@ -83,7 +83,46 @@ __global__ void __launch_bounds__(128) umma_selftest_kernel(int mode, const __nv
   if (warp == 0) umma::tmem_dealloc(tmem, 128);
 }
 
+// One warp passes n_waits waits on four barriers that nothing arrives at, then the drain.
+// mode 0: mbar_wait with a flag, 1: WaitChain (on the first).
+__global__ void __launch_bounds__(32) wait_chain_selftest_kernel(int mode, int n_waits, long long limit, long long *out) {
+  __shared__ uint64_t bars[4];
+  const uint32_t bar0 = umma::smem_u32(bars);
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < 4; ++i) umma::mbar_init(bar0 + 8 * i, 1);
+    umma::fence_mbar_init();
+  }
+  __syncthreads();
+  bool ok = true;
+  umma::WaitChain chain{bar0, 0};
+  const long long t0 = clock64();
+  if (mode == 1) {
+    for (int w = 0; w < n_waits; ++w) {
+      chain.state &= ~1u;  // (the phase before the first counts as complete)
+      chain.wait(limit);
+    }
+    ok = chain.ok();
+  }
+  for (int w = 0; mode == 0 && w < n_waits; ++w) ok = umma::mbar_wait(bar0 + 8 * (w & 3), 0, ok, limit) && ok;
+  const long long t1 = clock64();
+  if (!ok) umma::drain_waits(bar0, 4, limit / 10);
+  if (threadIdx.x == 0) {
+    out[0] = t1 - t0;
+    out[1] = clock64() - t1;
+    out[2] = ok;
+  }
+}
+
 }  // namespace slx
+
+extern "C" int slx_wait_chain_selftest(int mode, int n_waits, long long limit, long long *out, void *stream) {
+  using namespace slx;
+  SLX_REQUIRE(out != nullptr, SLX_E_NULL, "wait_chain_selftest: NULL pointer");
+  SLX_REQUIRE((mode == 0 || mode == 1) && n_waits >= 0 && n_waits <= 64 && limit > 0 && limit <= 400000000LL, SLX_E_SHAPE,
+              "wait_chain_selftest: mode %d, %d waits of %lld clocks", mode, n_waits, limit);
+  wait_chain_selftest_kernel<<<1, 32, 0, as_stream(stream)>>>(mode, n_waits, limit, out);
+  return check_launch("wait_chain_selftest");
+}
 
 extern "C" int slx_umma_selftest(int mode, const void *A, const void *B, float *C, int *status, void *stream) {
   using namespace slx;

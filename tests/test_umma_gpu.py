@@ -29,3 +29,17 @@ def test_umma_selftest(mode):
     ref = {0: lambda: a @ b.T, 1: lambda: a @ b, 2: lambda: a.T @ b, 3: lambda: a @ b.T}[mode]()
     err = (C - ref).norm() / ref.norm()
     assert float(err) < 1e-5, f"mode {mode}: relative error {float(err):.3e}"
+
+
+@pytest.mark.parametrize("mode", [0, 1])
+def test_waits_that_run_out_share_one_limit(mode):
+    """A chunk of the backward has 26 waits: the first that runs out is the only one that takes its limit."""
+    from slinoss_b200 import _lib
+
+    limit, out = 200_000_000, torch.zeros(3, dtype=torch.int64, device="cuda")
+    lib = _lib.selftest_lib()
+    rc = lib.slx_wait_chain_selftest(mode, 26, limit, out.data_ptr(), _lib.stream_ptr(out.device))
+    assert rc == 0, lib.slx_selftest_last_error_string()
+    waits, drain, ok = out.tolist()
+    assert ok == 0
+    assert limit <= waits < 1.5 * limit and drain < limit  # (0.4 of a limit and the last polls)
