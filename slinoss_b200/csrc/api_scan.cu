@@ -341,10 +341,11 @@ static int launch_state_bwd_t(int BH, int NC, int P, int N, const IT *dZ0, const
   const int vec = state_bwd_vec(P, N, sizeof(ST) == 2 && sizeof(IT) == 2);
   const int nblk = (elems / vec + 255) / 256;
   if (vec == 8) {
-    if constexpr (sizeof(ST) == 2 && sizeof(IT) == 2)
-      state_passing_bwd_kernel<8, ST, IT><<<dim3(nblk, BH), 256, 0, st>>>(dZ0, m_chunk, starts, final_state, ge.d_final,
-                                                                         ge.d_final_dtype, d_inc, ge.d_initial,
-                                                                         ge.d_initial_dtype, partials, NC, elems / 8);
+    if constexpr (sizeof(ST) == 2 && sizeof(IT) == 2) {
+      auto kern = nblk * BH > 3 * kB200Sms ? state_passing_bwd_kernel<8, ST, IT, 4> : state_passing_bwd_kernel<8, ST, IT, 3>;
+      kern<<<dim3(nblk, BH), 256, 0, st>>>(dZ0, m_chunk, starts, final_state, ge.d_final, ge.d_final_dtype, d_inc,
+                                           ge.d_initial, ge.d_initial_dtype, partials, NC, elems / 8);
+    }
   } else if (vec == 4) {
     state_passing_bwd_kernel<4, ST, IT><<<dim3(nblk, BH), 256, 0, st>>>(dZ0, m_chunk, starts, final_state, ge.d_final,
                                                                        ge.d_final_dtype, d_inc, ge.d_initial,

@@ -201,16 +201,17 @@ __global__ void __launch_bounds__(256) state_passing_fwd_kernel(const IT *inc, c
 // it to the activation dtype for its products anyway); with ST = float it may alias dZ0.  With zdot_partials == NULL the dot products (and the reads
 // of starts / final_state) are skipped, with d_inc == NULL nothing but d_initial is written: that
 // is the reduce-only pass that gives a segment's d_initial for a zero d_final.
-// Bound by HBM and the round trips of a walk: four CTAs per SM (64 registers a thread) keep more walks in flight than the
-// three that 80 registers leave: 0.146 against 0.163 ms for 8192 chunk states of 64 x 256 in half precision; five 0.180.
-template <int VEC, typename ST, typename IT>
-__global__ void __launch_bounds__(256, VEC == 8 ? 4 : 2) state_passing_bwd_kernel(const IT *dZ0,
-                                                                const float *__restrict__ m_chunk,
-                                                                const ST *__restrict__ starts,
-                                                                const float *__restrict__ final_state,
-                                                                const void *d_final, int d_final_dtype, ST *d_inc,
-                                                                void *d_initial, int d_initial_dtype,
-                                                                float *__restrict__ zdot_partials, int NC, int n_vec) {
+// Bound by HBM and the round trips of a walk.  CTAS: the CTAs per SM that the registers are bounded for.  8 values per
+// thread (half states): the compiler's own choice is 80 registers in bf16 and 95 in fp16; bounded for four CTAs it is 64 and
+// a spilled word, for three 68 and 71.  Four where more than three per SM run, else three (launch_state_bwd_t); us, bf16, inputs
+// beyond L2, four / three / own choice: grid 1024 of 64 chunks 136 / 142 / 150, 512 of 16 21.3 / 25.9 / 28.0, 444 of 16
+// 19.3 / 19.0 / 19.5, 256 of 32 25.4 / 24.8 / 26.8, 64 of 8 6.0 / 5.75 / 5.6.  Narrower vectors: the compiler's choice (0; 60
+// registers in fp32) is the better one: grid 2048 of 64 chunks 258 against 272 with 80 registers, 512 of 32 37 against 50.
+template <int VEC, typename ST, typename IT, int CTAS = 0>
+__global__ void __launch_bounds__(256, CTAS) state_passing_bwd_kernel(
+    const IT *dZ0, const float *__restrict__ m_chunk, const ST *__restrict__ starts, const float *__restrict__ final_state,
+    const void *d_final, int d_final_dtype, ST *d_inc, void *d_initial, int d_initial_dtype,
+    float *__restrict__ zdot_partials, int NC, int n_vec) {
   using V = typename VecT<VEC>::type;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int bh = blockIdx.y;

@@ -45,3 +45,36 @@ def test_gradient_rows_off_a_32_byte_boundary(dtype, N, T):
         outs.append([dU, dM, dK, dB.clone(), dC.clone(), cB, cU])
     for x, y in zip(*outs):
         assert torch.equal(x, y)
+
+
+@pytest.mark.parametrize("dtype,u", [(torch.bfloat16, 2.0 ** -8), (torch.float16, 2.0 ** -11), (torch.float32, 0.0)])
+@pytest.mark.parametrize("BH,NC", [(222, 5), (223, 6), (2, 9)])
+def test_reverse_state_pass_on_either_side_of_three_ctas_per_sm(dtype, u, BH, NC):
+    """Half states of 64 x 64 are two CTAs per head; the kernel changes above 444.  d_inc is rounded to its dtype once (u:
+    the largest relative error of that, 8 and 11 significant bits), the recurrence and the dots are fp32."""
+    from slinoss_b200 import _lib
+
+    g = torch.Generator().manual_seed(BH)
+    P, N, code = 64, 32, _lib.dtype_code(dtype)
+    dz, st = (torch.randn((BH, NC, P, 2 * N), generator=g).to(dtype) for _ in range(2))
+    m = torch.view_as_real(torch.polar(0.5 + 0.5 * torch.rand((BH, NC), generator=g), torch.randn((BH, NC), generator=g)))
+    fin, dfin = (torch.randn((BH, P, 2 * N), generator=g) for _ in range(2))
+    z = lambda t: torch.view_as_complex(t.double().reshape(*t.shape[:-1], -1, 2))
+    grad, want_inc, want_dot = z(dfin), [None] * NC, [None] * NC
+    for c in reversed(range(NC)):
+        want_inc[c] = torch.view_as_real(grad).flatten(-2)
+        want_dot[c] = ((z(fin) if c + 1 == NC else z(st[:, c + 1])).conj() * grad).sum((1, 2))
+        grad = z(dz[:, c]) + z(m)[:, c].reshape(-1, 1, 1).conj() * grad
+    dev = [t.cuda() for t in (dz, m, st, fin, dfin)]
+    inc, init, dot = torch.empty_like(dev[0]), torch.empty_like(dev[3]), torch.empty((BH, NC, 2), device="cuda")
+    part = torch.empty(_lib.lib().slx_state_passing_bwd_partials_bytes(BH, NC, P, N) // 4, device="cuda")
+    rc = _lib.lib().slx_state_passing_bwd(
+        BH, NC, P, N, dev[0].data_ptr(), code, dev[1].data_ptr(), dev[2].data_ptr(), code, dev[3].data_ptr(),
+        dev[4].data_ptr(), inc.data_ptr(), init.data_ptr(), dot.data_ptr(), part.data_ptr(), _lib.stream_ptr(inc.device))
+    _lib.check(rc, "state_passing_bwd")
+    want = torch.stack(want_inc, 1)
+    err = (inc.double().cpu() - want).abs()
+    assert (err <= u * want.abs() + 1e-5).all()
+    assert (init.double().cpu() - torch.view_as_real(grad).flatten(-2)).abs().max() < 1e-5
+    want = torch.view_as_real(torch.stack(want_dot, 1))
+    assert (dot.double().cpu() - want).norm() < 1e-5 * want.norm()
