@@ -143,10 +143,13 @@ __device__ __forceinline__ void scale32(float (&v)[32], float rf, const float *t
   }
 }
 
-// The forward sends a chunk's rows through L2 as a whole where the launch is several waves of CTAs long and bound by
-// DRAM (8192 CTAs: 0.361 against 0.381 ms).  In a launch of one or two waves all CTAs ask for their first slab at the
-// same time, and it waits behind everybody's rows (512 CTAs: a whole inference pass takes 62.4 us with, 60.2 without).
-constexpr unsigned kL2PrefetchCtas = 4 * 2 * kB200Sms;
+// The forward sends a chunk's rows through L2 as a whole where there are slabs to come back for (D > 64) and the launch is
+// more than nine waves of two CTAs per SM.  In the first waves all CTAs ask for their first slab at the same time, and it
+// waits behind everybody's rows; with the waves out of step the rows are there when their slabs are.  us with / without,
+// inputs beyond L2: D 256: 1024 CTAs 58.9 / 53.9, 2048 99.8 / 95.5, 2560 119.1 / 118.8, 2816 129.1 / 129.8, 4096 180 / 183, 8192
+// 339 / 354, 16384 655 / 692; D 128: 1536 55.4 / 54.8, 2560 85.9 / 84.5, 3072 99.4 / 100.0, 3584 114.6 / 114.1, 6144
+// 185 / 188, 16384 464 / 477; D 64 (one slab): 2048 58.1 / 56.8, 8192 199 / 197, 16384 380 / 379.
+constexpr unsigned kL2PrefetchCtas = 9 * 2 * kB200Sms;
 constexpr size_t scan_fwd_tc_smem_bytes() { return 1024 + 88 * 1024 + 12 * 1024; }
 
 // Forward chunk scan (replaces reference.py:1059 chunk_scan) on tensor cores.
@@ -232,7 +235,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) chunk_scan_fwd_tc_kernel(ScanFw
   }
   prefetch_cb(0);
   prefetch_z(0);
-  if (tid == 0 && gridDim.x * gridDim.y > kL2PrefetchCtas) {
+  if (tid == 0 && NB > 1 && gridDim.x * gridDim.y > kL2PrefetchCtas) {
     // The chunk's rows and its start state are contiguous in memory: whole into L2, from where the slabs take their
     // columns.  Without it DRAM sees every row in four visits of 128 bytes, and a slab waits for it.
     umma::l2_prefetch(a.C + tok0 * d.D, valid * d.D * 2);

@@ -78,3 +78,23 @@ def test_reverse_state_pass_on_either_side_of_three_ctas_per_sm(dtype, u, BH, NC
     assert (init.double().cpu() - torch.view_as_real(grad).flatten(-2)).abs().max() < 1e-5
     want = torch.view_as_real(torch.stack(want_dot, 1))
     assert (dot.double().cpu() - want).norm() < 1e-5 * want.norm()
+
+
+@pytest.mark.parametrize("N,dtype", [(32, torch.bfloat16), (64, torch.bfloat16), (128, torch.float16)])
+def test_rows_through_l2_leave_the_outputs_alone(N, dtype):
+    """Forwards of more than 2664 chunks fetch whole rows into L2 (N > 32), the ragged last chunk's among them: same bits as
+    the same heads in launches of half the size, which do not."""
+    import slinoss_b200 as sb
+
+    inp = make_scan_inputs(1, 1340, 128 + 71, N, 64, dtype, seed=N, dist="cfg2", with_init=True, streaming=True)
+    names = ("U", "M", "K", "B", "C")
+    carried = ("initial_states", "B_prev", "U_prev")
+
+    def run(h):
+        with torch.no_grad():
+            return sb.v2x2ssd_b200(*(inp[k][:, h] for k in names), chunk_size=128, return_state=True,
+                                   **{k: inp[k][:, h] for k in carried})
+
+    whole, halves = run(slice(None)), [run(slice(i, i + 670)) for i in (0, 670)]
+    for w, *h in zip(whole, *halves):
+        assert torch.equal(w, torch.cat(h, 1))
