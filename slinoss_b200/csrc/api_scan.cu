@@ -252,14 +252,17 @@ static int launch_outer_tc(const ScanDims &d, const void *A, const void *X, cons
 template <typename T>
 static int launch_scan_bwd_tc(const ScanDims &d, const ScanBwdArgs<T> &a, cudaStream_t st) {
   const bool prev32 = a.Uprev && a.prev_dtype == SLX_F32;
-  auto kern = prev32 ? chunk_scan_bwd_tc_kernel<T, true> : chunk_scan_bwd_tc_kernel<T, false>;
-  const size_t smem = scan_bwd_tc_smem_bytes(prev32);
+  const bool lone = (long long)d.NC * d.BH <= kB200Sms;  // no second CTA on an SM: one of twice the threads
+  auto kern = lone ? (prev32 ? chunk_scan_bwd_tc_kernel<T, true, 512> : chunk_scan_bwd_tc_kernel<T, false, 512>)
+                   : (prev32 ? chunk_scan_bwd_tc_kernel<T, true, 256> : chunk_scan_bwd_tc_kernel<T, false, 256>);
+  const size_t smem = scan_bwd_tc_smem_bytes(lone, prev32);
   int rc = set_smem(kern, smem);
   if (rc) return rc;
   ScanBwdMaps maps;
-  if ((rc = make_tile_map<T, 32>(&maps.C, a.C, d.BH, d.T, d.D, 128, "chunk_scan_bwd"))) return rc;
-  if ((rc = make_tile_map<T, 32>(&maps.B, a.B, d.BH, d.T, d.D, 128, "chunk_scan_bwd"))) return rc;
-  kern<<<dim3(d.NC, d.BH), kTcBwdThreads, smem, st>>>(a, maps);
+  auto make = lone ? make_tile_map<T, 64> : make_tile_map<T, 32>;  // the kernel's slab width
+  if ((rc = make(&maps.C, a.C, d.BH, d.T, d.D, 128, "chunk_scan_bwd"))) return rc;
+  if ((rc = make(&maps.B, a.B, d.BH, d.T, d.D, 128, "chunk_scan_bwd"))) return rc;
+  kern<<<dim3(d.NC, d.BH), lone ? 512 : 256, smem, st>>>(a, maps);
   return check_launch("chunk_scan_bwd_tc");
 }
 

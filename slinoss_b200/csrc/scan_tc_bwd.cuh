@@ -1,11 +1,12 @@
 // Tensor-core per-chunk backward of the v2x2ssd scan (chunk 128, P 64, half
 // inputs, fp32 state).  Same mathematics as chunk_scan_bwd_kernel in
 // scan_simt.cuh; every contraction runs on tcgen05 with fp32 accumulators in
-// tensor memory.  One CTA of 8 warps per (chunk, batch*head), two CTAs per SM.
+// tensor memory.  One CTA per (chunk, batch*head): 8 warps, two CTAs per SM, or, in launches of at most one CTA per SM
+// (LONE), 16 warps.
 //
 // Phases are taken relative to the end of the chunk, f_t = phi_t conj(phi_{L-1}), so that Lambda, Z0, U and dY enter
-// their products as they are stored.  Operands per 32-column slab of the state (half precision, every one rounded once
-// from fp32 or as it is stored):
+// their products as they are stored.  Operands per slab of the state, 32 columns or LONE 64 (half precision, every one
+// rounded once from fp32 or as it is stored):
 //   Q_t = c_t conj(f_t),  kappa_s = gamma_s b_s conj(f_{s+1}),  Z0,  Lambda
 // and per chunk  dS' = decay * (dY U^T),  dY,  U.  With es_s = p_{L-1}/p_{s+1} in magnitude, p_t = exp(lp_t) phi_t:
 //   dC_t = f_t (dS' kappa)_t + p_t (dY Z0)_t + (k^c_t G_tt) b_t
@@ -22,27 +23,32 @@
 //   [  0,128)  G = dY U^T, then S^T = kappa Q^T       (accumulated over the slabs)
 //   [128,192)  kappa Lambda^T                         (accumulated over the slabs)
 //   [192,224)  dS'^T Q of a slab, then dS' kappa      [224,256)  U Lambda, then dY Z0;  [192,256) at the end S'^T dY
+// LONE: 512 columns, [192,256) dS'^T Q, [256,320) U Lambda, [320,384) dS' kappa, [384,448) dY Z0.
 //
 // Columns of kappa, Q, Lambda and Z0 are stored (re, re, re, re, im, im, im, im) inside each group of four complex
 // values: sums over the state do not see the order, and the accumulators then hold real and imaginary parts of two
 // values side by side, which is what the packed fp32 arithmetic (two fmas per instruction) takes.
 //
 // What bounds it: neither HBM (46 %) nor the tensor pipe (12 %) but instruction issue and the latencies between a
-// chunk's phases (loads and prefix, slabs, tail).  8192 chunks of D 256: 1.036 ms.  One CTA of 16 worker warps per SM
+// chunk's phases (loads and prefix, slabs, tail).  8192 chunks of D 256: 1.052 ms.  One CTA of 16 worker warps per SM
 // with 64-column slabs and two buffers for every operand took 1.205 ms: its phases followed one another and nothing
 // filled their latencies.  Two CTAs of 8 warps run different phases at the same time.  They fit because the slabs are 32
 // columns wide with one buffer, dS'^T Q / U Lambda and dS' kappa / dY Z0 take turns in the same 64 accumulator columns,
 // and dC / dB leave from registers (whole 32-byte sectors).  Measured on the way: a ninth warp that issues the products
 // leaves 96 registers to a thread, and the spills cost more than the issuing (1.097 against 0.997 ms); one thread that
-// waits for the products and a CTA barrier behind it 1.198 against 1.070 ms.  8192 chunks of D 64: 0.668 -> 0.460 ms.  Where a
-// launch has no more chunks than SMs the second CTA is missing and eight warps take longer than sixteen did: 128 chunks of
-// D 256 0.035 -> 0.043 ms (passes of that size are bound by the host or nearly so).
+// waits for the products and a CTA barrier behind it 1.198 against 1.070 ms.
+//
+// LONE: where a launch has no more chunks than SMs the second CTA is missing, and the latencies of one chain show.  Twice
+// the threads and slabs of 64 columns halve the steps of that chain, and accumulators of their own for all four products of
+// a slab let them be issued together, with one CTA barrier per slab.  us, 8 warps and 32 columns / LONE: 148 chunks of D 256
+// 33.4 / 26.2, of D 128 23.3 / 18.7, 64 of D 64 17.6 / 14.3, 16 of D 256 27.3 / 22.5 (one CTA of 16 warps per SM with double
+// buffers: 23.6, 16.8, 13.6, 21.1).  16 warps with 32 columns 29.9, the same with accumulators of their own 29.7 (148 of D 256).
 //
 // PREV32: the streaming rows are fp32.  The tile then holds u_{-1} rounded, and its products with dY and Lambda get what
 // that lost from the CUDA cores, as u_{-1} enters dB_prev, dK and dM in fp32.  An instantiation of its own: as a branch it
 // costs every launch (8192 chunks of D 256: 1.064 against 1.050 ms).
 //
-// Thread mapping: thread = (row 32*(warp%4)+lane, 16-byte chunks 2*(warp/4) and +1 of the slab), the tensor-memory
+// Thread mapping: thread = (row 32*(warp%4)+lane, 16-byte cells 2*(warp/4) and +1 of the slab), the tensor-memory
 // lane mapping, for staging and epilogue alike, so that the raw b, c of a cell stay in registers from one to the other.
 #pragma once
 
@@ -50,15 +56,16 @@
 
 namespace slx {
 
-// tensor maps of the raw C and B operands: (D, T, BH), boxes of 32 columns x 128 tokens, 64-byte swizzle
+// tensor maps of the raw C and B operands: (D, T, BH), boxes of a slab x 128 tokens, 64-byte swizzle (LONE: 128-byte)
 struct alignas(64) ScanBwdMaps {
   CUtensorMap C, B;
 };
 
-constexpr int kTcBwdThreads = 256;
-constexpr uint32_t kBwdScalars = 106496;
-constexpr size_t scan_bwd_tc_smem_bytes(bool prev32) { return kBwdScalars + 8320 + (prev32 ? 256 : 0); }
-constexpr int kTmR = 128, kTmX = 192, kTmUL = 224, kTmU = kTmX;  // accumulator columns (G / S^T at 0)
+constexpr uint32_t bwd_scalars(bool lone) { return lone ? 147456 : 106496; }
+constexpr size_t scan_bwd_tc_smem_bytes(bool lone, bool prev32) {
+  return bwd_scalars(lone) + 8320 + (lone ? 9216 : 0) + (prev32 ? 256 : 0);
+}
+constexpr int kTmR = 128, kTmX = 192, kTmU = kTmX;  // accumulator columns (G / S^T at 0)
 
 // (a + i b) * cell, packed as four real parts and four imaginary parts
 template <typename T>
@@ -86,22 +93,30 @@ __device__ __forceinline__ float2 tm_pair(const uint32_t *r) {
   return make_float2(__uint_as_float(r[0]), __uint_as_float(r[1]));
 }
 
-template <typename T, bool PREV32>
-__global__ void __launch_bounds__(kTcBwdThreads, 2) chunk_scan_bwd_tc_kernel(ScanBwdArgs<T> a,
+template <typename T, bool PREV32, int THREADS>
+__global__ void __launch_bounds__(THREADS, 512 / THREADS) chunk_scan_bwd_tc_kernel(ScanBwdArgs<T> a,
                                                                               const __grid_constant__ ScanBwdMaps maps) {
   constexpr int L = kTcL, P = kTcP;
+  constexpr bool LONE = THREADS == 512;
+  constexpr int COLS = THREADS / 128, PARTS = 4 / COLS;  // threads per row; passes over the 128 columns of a score tile
+  constexpr int SW = 16 * COLS;                          // columns of a slab: two 16-byte cells per thread and row
+  constexpr uint32_t kTmUL = kTmX + SW, kTmX2 = LONE ? kTmX + 2 * SW : kTmX, kTmUL2 = LONE ? kTmX + 3 * SW : kTmUL;
+  // shared memory from 65536 on: kappa, Q, Lambda, Z0, raw C, raw B, scalars
+  constexpr uint32_t oK = 65536, oQ = oK + 256 * SW, oLm = oQ + 256 * SW, oZ = oLm + 128 * SW, oC = oZ + 128 * SW,
+                     oB = oC + 256 * SW, oS = oB + 256 * SW;
+  static_assert(oS == bwd_scalars(LONE), "shared-memory layout");
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char *base = smem_raw;
   unsigned char *tdY = base;                   // [t][p]
   unsigned char *tU = base + 16384;            // [s][p]
   unsigned char *tdS = base + 32768;           // 2 x [t][64 s]  dS', at the end 2 x [s][64 t]  S'^T
-  unsigned char *tK = base + 65536;            // [s][32 d]  kappa
-  unsigned char *tQ = base + 73728;            // [t][32 d]  Q
-  unsigned char *tLm = base + 81920;           // [p][32 d]  Lambda
-  unsigned char *tZ = base + 86016;            // [p][32 d]  Z0
-  unsigned char *sC = base + 90112;            // raw C slab, by TMA; scratch of the tail
-  unsigned char *sB = base + 98304;            // raw B slab
-  float *lp = reinterpret_cast<float *>(base + kBwdScalars);
+  unsigned char *tK = base + oK;               // [s][SW d]  kappa
+  unsigned char *tQ = base + oQ;               // [t][SW d]  Q
+  unsigned char *tLm = base + oLm;             // [p][SW d]  Lambda
+  unsigned char *tZ = base + oZ;               // [p][SW d]  Z0
+  unsigned char *sC = base + oC;               // raw C slab, by TMA; scratch of the tail
+  unsigned char *sB = base + oB;               // raw B slab
+  float *lp = reinterpret_cast<float *>(base + oS);
   float *tab = lp + L;                         // decay table of dS' (decay_table_entry), then of S'^T
   float *gd = tab + L;                         // G[t][t]
   float *um = gd + L;                          // 64   u_127
@@ -114,17 +129,19 @@ __global__ void __launch_bounds__(kTcBwdThreads, 2) chunk_scan_bwd_tc_kernel(Sca
   float2 *ph = reinterpret_cast<float2 *>(ulw + 256);
   float2 *bm1 = ph + L;                        // 128  b_{-1}
   float2 *bh1 = bm1 + 128;                     // 128  k^c b_127
-  float *ub = reinterpret_cast<float *>(bh1);  // 256  U Lambda of the token in front of the chunk, behind helper()'s reads
+  float *more = reinterpret_cast<float *>(base + oS + 8320);  // LONE: 256, 2 x [16][64] partials of u_127 . Lambda
+  // 256  U Lambda of the token in front of the chunk; without LONE over bh1, behind helper()'s reads
+  float *ub = LONE ? more : reinterpret_cast<float *>(bh1);
   float2 *misc = bh1 + 128;                    // [0..3] dk^p_0, [4..7] sum conj(b_127) (u_127 . Lambda), by warp
   uint64_t *bars = reinterpret_cast<uint64_t *>(misc + 8);  // [0] first, [1] second products of a slab; [2] G, then
                                                             // S'^T dY; [3] raw slab by TMA
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 4);
-  float *ulo = reinterpret_cast<float *>(base + scan_bwd_tc_smem_bytes(false));  // PREV32: 64  what u_{-1} loses in its tile
-  static_assert(kBwdScalars + 4 * (3 * 128 + 2 * 64 + 3 * 256) + 8 * 3 * 128 + 64 + 4 * 8 + 8 <=
-                    scan_bwd_tc_smem_bytes(false), "shared-memory layout");
+  float *ulo = more + (LONE ? 2304 : 0);       // PREV32: 64  what u_{-1} loses in its tile
+  static_assert(4 * (3 * 128 + 2 * 64 + 3 * 256) + 8 * 3 * 128 + 64 + 4 * 8 + 8 <= 8320, "shared-memory layout");
   // scratch of the tail, over the raw slabs
-  float2 *pgs = reinterpret_cast<float2 *>(sC), *pbs = pgs + L, *pcs = pbs + L;  // second column half: gA, bX; bc
-  float2 *bXs = pcs + 2 * L, *sums = bXs + L;  // sums: [0..3] g by warp, [4..7] correction of slot 127 by warp
+  float2 *pgs = reinterpret_cast<float2 *>(sC), *pbs = pgs + (COLS - 1) * L;  // gA, bX of the column parts behind the first
+  float2 *pcs = pbs + (COLS - 1) * L, *bXs = pcs + COLS * L;                   // bc by column part; bX
+  float2 *sums = bXs + L;  // [0..3] g by warp, [4..7] correction of slot 127 by warp
 
   const ScanDims d = a.d;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -132,7 +149,7 @@ __global__ void __launch_bounds__(kTcBwdThreads, 2) chunk_scan_bwd_tc_kernel(Sca
   const int t0 = c * L;
   const int valid = min(L, d.T - t0);
   const size_t tok0 = (size_t)bh * d.T + t0;
-  const int NB = d.D / 32;
+  const int NB = d.D / SW;
   const uint32_t bar0 = umma::smem_u32(bars), gbar = bar0 + 16, tbar = bar0 + 24;
   constexpr int fmt = umma::HalfFmt<T>::value;
 
@@ -144,11 +161,12 @@ __global__ void __launch_bounds__(kTcBwdThreads, 2) chunk_scan_bwd_tc_kernel(Sca
   float2 mreg[4];  // the prefix warp's multipliers, requested ahead of the bulk copies
   if (warp == 2) chunk_prefix_load4(a.M + tok0 * 2, valid, mreg);
   // U and dY land in their tiles by asynchronous copy (rows past the chunk end are zero-filled)
+  constexpr int ROWS = THREADS / 8;
   const int j8 = tid & 7, r8 = tid >> 3;
   uint4 ucell = make_uint4(0, 0, 0, 0);  // the thread that copies a cell of row 127: that cell of u_{-1}
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int r = r8 + 32 * i;
+  for (int i = 0; i < L / ROWS; ++i) {
+    const int r = r8 + ROWS * i;
     const int rr = r < valid ? r : 0;
     const uint32_t nbytes = r < valid ? 16u : 0u;
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(umma::smem_u32(tU + umma::swz_off(r, j8))),
@@ -158,7 +176,7 @@ __global__ void __launch_bounds__(kTcBwdThreads, 2) chunk_scan_bwd_tc_kernel(Sca
                  "l"(a.dY + (tok0 + rr) * P + 8 * j8), "r"(nbytes)
                  : "memory");
   }
-  if (r8 == 31) {
+  if (r8 == ROWS - 1) {
     if (t0 > 0) {
       ucell = *reinterpret_cast<const uint4 *>(a.U + (tok0 - 1) * P + 8 * j8);
     } else if (a.Uprev) {
@@ -173,13 +191,13 @@ __global__ void __launch_bounds__(kTcBwdThreads, 2) chunk_scan_bwd_tc_kernel(Sca
     }
   }
   asm volatile("cp.async.commit_group;" ::: "memory");
-  // One raw (C, B) slab = two TMA boxes of [128 tokens][32 columns] into the swizzled staging tiles,
+  // One raw (C, B) slab = two TMA boxes of [128 tokens][SW columns] into the swizzled staging tiles,
   // issued by one thread; tokens past the end of the sequence arrive as zeros.
   auto prefetch_cb = [&](int sl) {
     umma::fence_smem_to_async();  // the tiles' earlier (generic) readers are behind a barrier
-    umma::mbar_expect_tx(tbar, 2u * 8192u);
-    umma::tma_load_3d(umma::smem_u32(sC), &maps.C, sl * 32, t0, bh, tbar);
-    umma::tma_load_3d(umma::smem_u32(sB), &maps.B, sl * 32, t0, bh, tbar);
+    umma::mbar_expect_tx(tbar, 2u * 256u * SW);
+    umma::tma_load_3d(umma::smem_u32(sC), &maps.C, sl * SW, t0, bh, tbar);
+    umma::tma_load_3d(umma::smem_u32(sB), &maps.B, sl * SW, t0, bh, tbar);
   };
   if (tid == 0) {
     umma::mbar_init(bar0, 2);      // commits of issue_first
@@ -192,17 +210,17 @@ __global__ void __launch_bounds__(kTcBwdThreads, 2) chunk_scan_bwd_tc_kernel(Sca
     prefetch_cb(0);
   }
   // Z0 / Lambda slab: one 8-value (16-byte) item per thread, prefetched into registers
-  const int zp = tid >> 2, zj = tid & 3;
+  const int zp = tid / (SW / 8), zj = tid % (SW / 8);
   uint4 zr, lr;
   auto prefetch_zl = [&](int sl) {
-    zr = *reinterpret_cast<const uint4 *>(z0 + (size_t)zp * d.D + sl * 32 + 8 * zj);
-    lr = *reinterpret_cast<const uint4 *>(lam + (size_t)zp * d.D + sl * 32 + 8 * zj);
+    zr = *reinterpret_cast<const uint4 *>(z0 + (size_t)zp * d.D + sl * SW + 8 * zj);
+    lr = *reinterpret_cast<const uint4 *>(lam + (size_t)zp * d.D + sl * SW + 8 * zj);
   };
   prefetch_zl(0);
 
-  if (warp == 1) umma::tmem_alloc(tmem_slot, 256);
+  if (warp == 1) umma::tmem_alloc(tmem_slot, LONE ? 512 : 256);
   if (warp == 2) chunk_prefix_fast128(mreg, lp, ph, mraw, &g_scan_bad);
-  if (tid >= 128) {
+  if ((tid >> 7) == 1) {
     const int t = tid - 128;
     float2 vp = make_float2(0.f, 0.f), vc = vp;
     if (t < valid) {
@@ -224,7 +242,7 @@ __global__ void __launch_bounds__(kTcBwdThreads, 2) chunk_scan_bwd_tc_kernel(Sca
     }
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");  // U, dY tiles
-  if (r8 == 31) {  // source slot 127 is the token in front of the chunk; u_127 is kept aside
+  if (r8 == ROWS - 1) {  // source slot 127 is the token in front of the chunk; u_127 is kept aside
     uint4 *cell = reinterpret_cast<uint4 *>(tU + umma::swz_off(L - 1, j8));
     const uint4 own = *cell;
     const uint32_t *w = reinterpret_cast<const uint32_t *>(&own);
@@ -241,30 +259,35 @@ __global__ void __launch_bounds__(kTcBwdThreads, 2) chunk_scan_bwd_tc_kernel(Sca
   // ---- the products --------------------------------------------------------------------------
   // Issuing a product takes about as long as the product (90 cycles), so several warps share it: nobody is held longer
   // than the products that every warp waits for take (8192 chunks: 1.059 ms, all by one thread 1.141).
-  constexpr uint32_t id_km = umma::make_idesc(128, 32, false, true, fmt);
+  constexpr uint32_t id_km = umma::make_idesc(128, SW, false, true, fmt);
   constexpr uint32_t id_sq = umma::make_idesc(128, 128, false, false, fmt);
   const uint32_t sb = umma::smem_u32(base);
+  // a slab tile as an operand: 64-byte rows (SW 32, one descriptor for both views) or 128-byte rows
+  constexpr uint32_t kMN = LONE ? umma::kStepMN : umma::kStepMN64;
+  auto mn_view = [&](uint32_t off) { return LONE ? umma::desc_mnmajor(sb + off, 0, 0) : umma::make_desc64(sb + off); };
+  auto k_view = [&](uint32_t off) { return LONE ? umma::desc_kmajor(sb + off, 0) : umma::make_desc64(sb + off); };
+  // (LONE: all five of a slab at its start, by warps that have no helper())
   auto issue_first = [&](int sl) {  // dS'^T Q (warp 0), U Lambda (warp 1)
-    if (warp == 0) {
+    if (warp == (LONE ? 8 : 0)) {
       if (lane == 0) {
         umma::fence_after_sync();
-        constexpr uint32_t id_mm = umma::make_idesc(128, 32, true, true, fmt);
-        const uint64_t dSm = umma::desc_mnmajor(sb + 32768, 0, 16384u), dQ = umma::make_desc64(sb + 73728);
+        constexpr uint32_t id_mm = umma::make_idesc(128, SW, true, true, fmt);
+        const uint64_t dSm = umma::desc_mnmajor(sb + 32768, 0, 16384u), dQ = mn_view(oQ);
 #pragma unroll
         for (int kk = 0; kk < 8; ++kk)
           umma::mma_ss(tmem + kTmX, umma::desc_advance(dSm, umma::kStepMN * kk),
-                       umma::desc_advance(dQ, umma::kStepMN64 * kk), id_mm, kk != 0);
+                       umma::desc_advance(dQ, kMN * kk), id_mm, kk != 0);
         umma::commit(bar0);
       }
       __syncwarp();
-    } else if (warp == 1) {
+    } else if (warp == (LONE ? 9 : 1)) {
       if (lane == 0) {
         umma::fence_after_sync();
-        const uint64_t dUk = umma::desc_kmajor(sb + 16384, 0), dLm = umma::make_desc64(sb + 81920);
+        const uint64_t dUk = umma::desc_kmajor(sb + 16384, 0), dLm = mn_view(oLm);
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk)
           umma::mma_ss(tmem + kTmUL, umma::desc_advance(dUk, umma::kStepK * kk),
-                       umma::desc_advance(dLm, umma::kStepMN64 * kk), id_km, kk != 0);
+                       umma::desc_advance(dLm, kMN * kk), id_km, kk != 0);
         umma::commit(bar0);
         if (sl > 0 && sl + 1 < NB) prefetch_cb(sl + 1);
       }
@@ -272,36 +295,35 @@ __global__ void __launch_bounds__(kTcBwdThreads, 2) chunk_scan_bwd_tc_kernel(Sca
     }
   };
   auto issue_second = [&](int sl) {  // dS' kappa (warp 5), dY Z0 (warp 6), S^T and kappa Lambda^T (warp 7)
-    if (warp == 5) {
+    if (warp == (LONE ? 10 : 5)) {
       if (lane == 0) {
         umma::fence_after_sync();
-        const uint64_t dSk = umma::desc_kmajor(sb + 32768, 0), dK = umma::make_desc64(sb + 65536);
+        const uint64_t dSk = umma::desc_kmajor(sb + 32768, 0), dK = mn_view(oK);
 #pragma unroll
         for (int kk = 0; kk < 8; ++kk)
-          umma::mma_ss(tmem + kTmX, umma::desc_advance(dSk, 16384u * (kk >> 2) + umma::kStepK * (kk & 3)),
-                       umma::desc_advance(dK, umma::kStepMN64 * kk), id_km, kk != 0);
+          umma::mma_ss(tmem + kTmX2, umma::desc_advance(dSk, 16384u * (kk >> 2) + umma::kStepK * (kk & 3)),
+                       umma::desc_advance(dK, kMN * kk), id_km, kk != 0);
         umma::commit(bar0 + 8);
       }
       __syncwarp();
-    } else if (warp == 6) {
+    } else if (warp == (LONE ? 11 : 6)) {
       if (lane == 0) {
         umma::fence_after_sync();
-        const uint64_t dYk = umma::desc_kmajor(sb, 0), dZ = umma::make_desc64(sb + 86016);
+        const uint64_t dYk = umma::desc_kmajor(sb, 0), dZ = mn_view(oZ);
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk)
-          umma::mma_ss(tmem + kTmUL, umma::desc_advance(dYk, umma::kStepK * kk),
-                       umma::desc_advance(dZ, umma::kStepMN64 * kk), id_km, kk != 0);
+          umma::mma_ss(tmem + kTmUL2, umma::desc_advance(dYk, umma::kStepK * kk),
+                       umma::desc_advance(dZ, kMN * kk), id_km, kk != 0);
         umma::commit(bar0 + 8);
       }
       __syncwarp();
-    } else if (warp == 7) {
+    } else if (warp == (LONE ? 12 : 7)) {
       if (lane == 0) {
         umma::fence_after_sync();
         constexpr uint32_t id_kk = umma::make_idesc(128, 64, false, false, fmt);
-        const uint64_t dK = umma::make_desc64(sb + 65536), dQ = umma::make_desc64(sb + 73728),
-                       dLm = umma::make_desc64(sb + 81920);
+        const uint64_t dK = k_view(oK), dQ = k_view(oQ), dLm = k_view(oLm);
 #pragma unroll
-        for (int kk = 0; kk < 2; ++kk) {
+        for (int kk = 0; kk < SW / 16; ++kk) {
           umma::mma_ss(tmem, umma::desc_advance(dK, umma::kStepK * kk), umma::desc_advance(dQ, umma::kStepK * kk), id_sq,
                        (sl | kk) != 0);
           umma::mma_ss(tmem + kTmR, umma::desc_advance(dK, umma::kStepK * kk),
@@ -323,7 +345,7 @@ __global__ void __launch_bounds__(kTcBwdThreads, 2) chunk_scan_bwd_tc_kernel(Sca
     }
     __syncwarp();
   }
-  const int q4 = warp & 3, h = warp >> 2;  // lane quarter of tensor memory, column half
+  const int q4 = warp & 3, h = warp >> 2;  // lane quarter of tensor memory, column part
   const int row = 32 * q4 + lane;
   const bool last_row = row == L - 1;
   const float lp_r = lp[row];
@@ -346,12 +368,13 @@ __global__ void __launch_bounds__(kTcBwdThreads, 2) chunk_scan_bwd_tc_kernel(Sca
   CDot2 d_bc{zero2, zero2}, d_g = d_bc, d_x = d_bc, d_k = d_bc, d_b = d_bc;
   uint4 cr[2], br[2];                                       // raw cells of the slab
 
+  auto slab_off = [](int r, int j) { return LONE ? umma::swz_off(r, j) : umma::swz64_off(r, j); };
   // operand tiles of slab sl
   auto stage = [&](int sl) {
     wait(3);
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
-      const uint32_t off = umma::swz64_off(row, 2 * h + k);
+      const uint32_t off = slab_off(row, 2 * h + k);
       cr[k] = *reinterpret_cast<const uint4 *>(sC + off);
       br[k] = *reinterpret_cast<const uint4 *>(sB + off);
       const CellF cf = unpack_cell<T>(cr[k]);
@@ -360,7 +383,7 @@ __global__ void __launch_bounds__(kTcBwdThreads, 2) chunk_scan_bwd_tc_kernel(Sca
       for (int q = 0; q < 2; ++q) cdot2(bf.re[q], bf.im[q], cf.re[q], cf.im[q], d_bc);
       *reinterpret_cast<uint4 *>(tQ + off) = rotate_cell_split<T>(cf, f_r.x, -f_r.y);
       if (last_row) {
-        const float4 *bm = reinterpret_cast<const float4 *>(bm1 + 16 * sl + 8 * h + 4 * k);
+        const float4 *bm = reinterpret_cast<const float4 *>(bm1 + SW / 2 * sl + 8 * h + 4 * k);
         const float4 b0 = bm[0], b1 = bm[1];
         bf.re[0] = make_float2(b0.x, b0.z);
         bf.im[0] = make_float2(b0.y, b0.w);
@@ -369,7 +392,7 @@ __global__ void __launch_bounds__(kTcBwdThreads, 2) chunk_scan_bwd_tc_kernel(Sca
       }
       *reinterpret_cast<uint4 *>(tK + off) = rotate_cell_split<T>(bf, gk.x, gk.y);
     }
-    const uint32_t offz = umma::swz64_off(zp, zj);
+    const uint32_t offz = slab_off(zp, zj);
     *reinterpret_cast<uint4 *>(tLm + offz) = split_cell(lr);
     *reinterpret_cast<uint4 *>(tZ + offz) = split_cell(zr);
     umma::fence_smem_to_async();
@@ -390,7 +413,7 @@ __global__ void __launch_bounds__(kTcBwdThreads, 2) chunk_scan_bwd_tc_kernel(Sca
         tl[2 * e + 1] = v.y;
       }
     }
-    const float4 *kbv = reinterpret_cast<const float4 *>(reinterpret_cast<const float *>(bh1) + 32 * sl + 8 * zj);
+    const float4 *kbv = reinterpret_cast<const float4 *>(reinterpret_cast<const float *>(bh1) + SW * sl + 8 * zj);
     const float4 h0 = kbv[0], h1 = kbv[1];
     const float hb[8] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
     const float uz = um[zp];
@@ -400,7 +423,7 @@ __global__ void __launch_bounds__(kTcBwdThreads, 2) chunk_scan_bwd_tc_kernel(Sca
       du127 = fmaf(hb[e], tl[e], du127);
       up[e] = uz * tl[e];
     }
-    // the lanes trade halves, so that each ends with one of the eight columns
+    // the lanes that share zj trade halves, so that each ends with one of the eight columns (LONE: four lanes, two columns)
     const bool hi4 = lane & 4, hi8 = lane & 8, hi16 = lane & 16;
     float w4[4], w2[2];
 #pragma unroll
@@ -409,8 +432,13 @@ __global__ void __launch_bounds__(kTcBwdThreads, 2) chunk_scan_bwd_tc_kernel(Sca
 #pragma unroll
     for (int e = 0; e < 2; ++e)
       w2[e] = (hi8 ? w4[2 + e] : w4[e]) + __shfl_xor_sync(0xffffffffu, hi8 ? w4[e] : w4[2 + e], 8);
-    const float w1 = (hi4 ? w2[1] : w2[0]) + __shfl_xor_sync(0xffffffffu, hi4 ? w2[0] : w2[1], 4);
-    ulw[32 * warp + 8 * zj + (hi16 ? 4 : 0) + (hi8 ? 2 : 0) + (hi4 ? 1 : 0)] = w1;
+    const int col = 8 * zj + (hi16 ? 4 : 0) + (hi8 ? 2 : 0);
+    if constexpr (LONE) {
+      *reinterpret_cast<float2 *>(more + 256 + 1024 * (sl & 1) + 64 * warp + col) = make_float2(w2[0], w2[1]);
+    } else {
+      const float w1 = (hi4 ? w2[1] : w2[0]) + __shfl_xor_sync(0xffffffffu, hi4 ? w2[0] : w2[1], 4);
+      ulw[32 * warp + col + (hi4 ? 1 : 0)] = w1;
+    }
   };
 
   // ---- the decay table; the first slab's operands ------------------
@@ -418,19 +446,19 @@ __global__ void __launch_bounds__(kTcBwdThreads, 2) chunk_scan_bwd_tc_kernel(Sca
   stage(0);
   const bool fast_decay = !__syncthreads_or(tid < L && decay_step_out_of_range(lp, tid));
   if (warp == 1) {
-    if (lane == 0 && ok) prefetch_cb(1);  // every thread has its cells of slab 0 (NB >= 2)
+    if (lane == 0 && ok && (!LONE || NB > 1)) prefetch_cb(1);  // every thread has its cells of slab 0
     __syncwarp();
   }
   helper(0);
-  prefetch_zl(1);
+  if (!LONE || NB > 1) prefetch_zl(1);  // (32-column slabs: at least two)
   SLX_STAMP(2);
 
   // ---- G -> dS' ----------------------------------------------------------
   wait(2);
   umma::fence_after_sync();
 #pragma unroll 1
-  for (int jj = 0; jj < 2; ++jj) {
-    const int blk = 2 * jj + h, c0 = 32 * blk;  // blocks alternate between the two warps of a row quarter
+  for (int jj = 0; jj < PARTS; ++jj) {
+    const int blk = COLS * jj + h, c0 = 32 * blk;  // blocks alternate between the warps of a row quarter
     float v[32];
     if (blk <= q4 || blk == 3) {
       umma::tmem_ld32(umma::tmem_addr(tmem, 32 * q4, c0), v);
@@ -501,9 +529,28 @@ __global__ void __launch_bounds__(kTcBwdThreads, 2) chunk_scan_bwd_tc_kernel(Sca
   };
   const size_t out0 = (tok0 + row) * d.D + 16 * h;
 
+  auto sum_ulw = [&](int sl) {  // u_127 . Lambda of a slab: sum of the per-warp partials
+    if constexpr (LONE) {
+      float2 acc = zero2;
+#pragma unroll
+      for (int w = 0; w < 16; ++w)
+        acc = cadd(acc, *reinterpret_cast<const float2 *>(more + 256 + 1024 * (sl & 1) + 64 * w + 2 * lane));
+      *reinterpret_cast<float2 *>(ulf + 64 * sl + 2 * lane) = acc;
+    } else {
+      float acc = 0.f;
+#pragma unroll
+      for (int w = 0; w < 8; ++w) acc += ulw[32 * w + lane];
+      ulf[32 * sl + lane] = acc;
+    }
+  };
+
   for (int sl = 0; sl < NB; ++sl) {
     SLX_STAMP(8 + 4 * sl);
     issue_first(sl);  // slab sl is staged, the accumulators of slab sl-1 are read
+    if (LONE) {
+      issue_second(sl);
+      if (warp == 13 && sl > 0) sum_ulw(sl - 1);
+    }
     if (sl > 0) {
       helper(sl);
       if (sl + 1 < NB) prefetch_zl(sl + 1);
@@ -517,19 +564,16 @@ __global__ void __launch_bounds__(kTcBwdThreads, 2) chunk_scan_bwd_tc_kernel(Sca
     umma::tmem_ld16_issue(umma::tmem_addr(tmem + kTmUL, 32 * q4, 16 * h), x2);
     umma::tmem_ld16_wait(x1);
     umma::tmem_ld16_wait(x2);
-    umma::fence_before_sync();
-    __syncthreads();  // dS'^T Q and U Lambda are in registers
-    issue_second(sl);
-    if (warp == 4) {  // u_127 . Lambda of this slab: sum of the per-warp partials
-      float acc = 0.f;
-#pragma unroll
-      for (int w = 0; w < 8; ++w) acc += ulw[32 * w + lane];
-      ulf[32 * sl + lane] = acc;
+    if (!LONE) {
+      umma::fence_before_sync();
+      __syncthreads();  // dS'^T Q and U Lambda are in registers
+      issue_second(sl);
+      if (warp == 4) sum_ulw(sl);
     }
     if (last_row) {  // of the token in front of the chunk: dS'^T Q and U Lambda; token 127's own dB is formed in the tail
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
-        const int o = 8 * (q >> 1) + 2 * (q & 1), col = 32 * sl + 16 * h + 4 * q;
+        const int o = 8 * (q >> 1) + 2 * (q & 1), col = SW * sl + 16 * h + 4 * q;
         *reinterpret_cast<uint4 *>(xb + col) = make_uint4(x1[o], x1[o + 4], x1[o + 1], x1[o + 5]);
         *reinterpret_cast<uint4 *>(ub + col) = make_uint4(x2[o], x2[o + 4], x2[o + 1], x2[o + 5]);
       }
@@ -540,7 +584,7 @@ __global__ void __launch_bounds__(kTcBwdThreads, 2) chunk_scan_bwd_tc_kernel(Sca
 #pragma unroll
       for (int k = 0; k < 2; ++k) {
         const CellF cf = unpack_cell<T>(cr[k]), bf = unpack_cell<T>(br[k]);
-        const CellF kf = unpack_cell_split<T>(*reinterpret_cast<const uint4 *>(tK + umma::swz64_off(row, 2 * h + k)));
+        const CellF kf = unpack_cell_split<T>(*reinterpret_cast<const uint4 *>(tK + slab_off(row, 2 * h + k)));
         uint32_t *w = reinterpret_cast<uint32_t *>(&o[k]);
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
@@ -561,7 +605,7 @@ __global__ void __launch_bounds__(kTcBwdThreads, 2) chunk_scan_bwd_tc_kernel(Sca
           w[2 * q + 1] = umma::pack2(re.y, im.y, T());
         }
       }
-      if (row < valid && !last_row) store_row(a.dB + out0 + 32 * sl, o);
+      if (row < valid && !last_row) store_row(a.dB + out0 + SW * sl, o);
     }
     SLX_STAMP(10 + 4 * sl);
     // ---- dC_t = f_t (dS' kappa)_t + p_t (dY Z0)_t + cA_t b_t ------------------------------------------
@@ -571,15 +615,15 @@ __global__ void __launch_bounds__(kTcBwdThreads, 2) chunk_scan_bwd_tc_kernel(Sca
     {
       uint4 o[2];
       uint32_t t1[16], t2[16];
-      umma::tmem_ld16_issue(umma::tmem_addr(tmem + kTmX, 32 * q4, 16 * h), t1);
-      umma::tmem_ld16_issue(umma::tmem_addr(tmem + kTmUL, 32 * q4, 16 * h), t2);
+      umma::tmem_ld16_issue(umma::tmem_addr(tmem + kTmX2, 32 * q4, 16 * h), t1);
+      umma::tmem_ld16_issue(umma::tmem_addr(tmem + kTmUL2, 32 * q4, 16 * h), t2);
       umma::tmem_ld16_wait(t1);
       umma::tmem_ld16_wait(t2);
 #pragma unroll
       for (int k = 0; k < 2; ++k) {
         const uint32_t *r1 = t1 + 8 * k, *r2 = t2 + 8 * k;
         const CellF cf = unpack_cell<T>(cr[k]), bf = unpack_cell<T>(br[k]);
-        const CellF qf = unpack_cell_split<T>(*reinterpret_cast<const uint4 *>(tQ + umma::swz64_off(row, 2 * h + k)));
+        const CellF qf = unpack_cell_split<T>(*reinterpret_cast<const uint4 *>(tQ + slab_off(row, 2 * h + k)));
         uint32_t *w = reinterpret_cast<uint32_t *>(&o[k]);
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
@@ -602,12 +646,16 @@ __global__ void __launch_bounds__(kTcBwdThreads, 2) chunk_scan_bwd_tc_kernel(Sca
           w[2 * q + 1] = umma::pack2(re.y, im.y, T());
         }
       }
-      if (row < valid) store_row(a.dC + out0 + 32 * sl, o);
+      if (row < valid) store_row(a.dC + out0 + SW * sl, o);
     }
     if (sl + 1 < NB) {  // every product of the slab is done: its tiles are free
       stage(sl + 1);
       __syncthreads();
     }
+  }
+  if (LONE) {
+    __syncthreads();
+    if (warp == 13) sum_ulw(NB - 1);
   }
   SLX_STAMP(4);
 
@@ -625,7 +673,7 @@ __global__ void __launch_bounds__(kTcBwdThreads, 2) chunk_scan_bwd_tc_kernel(Sca
     if (row < valid) m_own = *reinterpret_cast<const float2 *>(a.M + (tok0 + row) * 2);
     if (row + 1 < valid) m_next = *reinterpret_cast<const float2 *>(a.M + (tok0 + row + 1) * 2);
     if (last_row) zd = *reinterpret_cast<const float2 *>(a.zdot + ((size_t)bh * d.NC + c) * 2);
-  } else if (row < d.N && valid == L) {
+  } else if (h == 1 && row < d.N && valid == L) {
     c127 = load_pair<T>(a.C + (tok0 + L - 1) * d.D + 2 * row);
     b127 = load_pair<T>(a.B + (tok0 + L - 1) * d.D + 2 * row);
   }
@@ -640,18 +688,23 @@ __global__ void __launch_bounds__(kTcBwdThreads, 2) chunk_scan_bwd_tc_kernel(Sca
   if (!last_row) gA = csub(gA, csub(cdot2_sum(d_k), cmul(cconj(gk), cdot2_sum(d_b))));
   bX = cmul(f_next, bX);
   pcs[L * h + row] = bc;
-  if (h == 1) {
-    pgs[row] = gA;
-    pbs[row] = bX;
+  if (h > 0) {
+    pgs[L * (h - 1) + row] = gA;
+    pbs[L * (h - 1) + row] = bX;
   }
   du127 += __shfl_xor_sync(0xffffffffu, du127, 1);
   du127 += __shfl_xor_sync(0xffffffffu, du127, 2);
+  if constexpr (LONE) du127 += __shfl_xor_sync(0xffffffffu, du127, 4);
   if (zj == 0) duc[zp] = du127;
   __syncthreads();
   bc = cadd(pcs[row], pcs[L + row]);
+  if constexpr (COLS == 4) bc = cadd(bc, cadd(pcs[2 * L + row], pcs[3 * L + row]));
   if (h == 0) {
-    gA = cadd(gA, pgs[row]);
-    bX = cadd(bX, pbs[row]);
+#pragma unroll
+    for (int k = 0; k < COLS - 1; ++k) {
+      gA = cadd(gA, pgs[L * k + row]);
+      bX = cadd(bX, pbs[L * k + row]);
+    }
     bXs[row] = bX;
   }
   float *cB = a.carryB + ((size_t)bh * d.NC + c) * d.D;
@@ -672,7 +725,7 @@ __global__ void __launch_bounds__(kTcBwdThreads, 2) chunk_scan_bwd_tc_kernel(Sca
         contrib = cmul(cconj(b), x);
         const float2 kap = cmul(cmulc(k_edge, f_0), b);
         corr = cmul(cconj(csub(umma::unpack2(umma::pack2(kap.x, kap.y, T()), T()), kap)), X);
-      } else if (valid == L) {
+      } else if ((tid >> 7) == 1 && valid == L) {
         // token 127: dB[n] = conj(k^c) (u_127 . Lambda)[n] + conj(k^c G) c[n]
         const float2 ul = *reinterpret_cast<const float2 *>(ulf + 2 * n);
         store_pair<T>(a.dB + (tok0 + L - 1) * d.D + 2 * n, cmul(cconj(k_edge), cadd(ul, cscale(c127, gd[L - 1]))));
@@ -684,7 +737,7 @@ __global__ void __launch_bounds__(kTcBwdThreads, 2) chunk_scan_bwd_tc_kernel(Sca
       contrib.x += __shfl_xor_sync(0xffffffffu, contrib.x, off);
       contrib.y += __shfl_xor_sync(0xffffffffu, contrib.y, off);
     }
-    if (lane == 0) misc[warp] = contrib;
+    if (lane == 0 && warp < 8) misc[warp] = contrib;
     if (h == 0) {
 #pragma unroll
       for (int off = 16; off > 0; off >>= 1) {
@@ -698,8 +751,8 @@ __global__ void __launch_bounds__(kTcBwdThreads, 2) chunk_scan_bwd_tc_kernel(Sca
   // ---- S^T -> S'^T (forward scores; row 127 = boundary) --------------------------------
   const float dg_r = kc_t.x * bc.x + kc_t.y * bc.y;  // Re(k^c conj(bc))
 #pragma unroll 1
-  for (int jj = 0; jj < 2; ++jj) {
-    const int blk = 2 * jj + h, c0 = 32 * blk;
+  for (int jj = 0; jj < PARTS; ++jj) {
+    const int blk = COLS * jj + h, c0 = 32 * blk;
     float v[32];
     if (blk >= q4 || q4 == 3) {  // (the last row quarter holds the boundary row, which takes every column)
       umma::tmem_ld32(umma::tmem_addr(tmem, 32 * q4, c0), v);
@@ -768,8 +821,8 @@ __global__ void __launch_bounds__(kTcBwdThreads, 2) chunk_scan_bwd_tc_kernel(Sca
   SLX_STAMP(59);
   // ---- dU = increment path + score path; carry of dU ------------------------------------------
 #pragma unroll 1
-  for (int k2 = 0; k2 < 2; ++k2) {
-    const int p0 = 32 * h + 16 * k2;
+  for (int k2 = 0; k2 < PARTS; ++k2) {
+    const int p0 = 16 * (PARTS * h + k2);
     uint32_t r0[16], r1[16];
     umma::tmem_ld16_issue(umma::tmem_addr(tmem + kTmR, 32 * q4, p0), r0);
     umma::tmem_ld16_issue(umma::tmem_addr(tmem + kTmU, 32 * q4, p0), r1);
@@ -782,7 +835,7 @@ __global__ void __launch_bounds__(kTcBwdThreads, 2) chunk_scan_bwd_tc_kernel(Sca
       float *cU = a.carryU + ((size_t)bh * d.NC + c) * P + p0;
 #pragma unroll
       for (int k = 0; k < 2; ++k) {
-        const uint4 dyr = *reinterpret_cast<const uint4 *>(tdY + umma::swz_off(L - 1, 4 * h + 2 * k2 + k));
+        const uint4 dyr = *reinterpret_cast<const uint4 *>(tdY + umma::swz_off(L - 1, (p0 >> 3) + k));
         const uint32_t *w = reinterpret_cast<const uint32_t *>(&dyr);
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
@@ -810,7 +863,7 @@ __global__ void __launch_bounds__(kTcBwdThreads, 2) chunk_scan_bwd_tc_kernel(Sca
   __syncwarp();
   if (warp == 1) {
     umma::fence_after_sync();
-    umma::tmem_dealloc(tmem, 256);
+    umma::tmem_dealloc(tmem, LONE ? 512 : 256);
   }
   if (!bad && h == 0 && row < valid) {
     for (int w = warp + 1; w < 4; ++w) g_sum = cadd(g_sum, sums[w]);
@@ -822,15 +875,15 @@ __global__ void __launch_bounds__(kTcBwdThreads, 2) chunk_scan_bwd_tc_kernel(Sca
     // overwrite them (and the carries) with NaN so that the failure shows in the data as well as in the status word
     const float nanf_ = __int_as_float(0x7fc00000);
     const T nanv = from_f<T>(nanf_);
-    for (int e = tid; e < valid * P; e += kTcBwdThreads) a.dU[tok0 * P + e] = nanv;
-    for (int e = tid; e < valid * d.D; e += kTcBwdThreads) {
+    for (int e = tid; e < valid * P; e += THREADS) a.dU[tok0 * P + e] = nanv;
+    for (int e = tid; e < valid * d.D; e += THREADS) {
       a.dB[tok0 * d.D + e] = nanv;
       a.dC[tok0 * d.D + e] = nanv;
     }
-    for (int e = tid; e < valid * 2; e += kTcBwdThreads) a.dM[tok0 * 2 + e] = nanf_;
-    for (int e = tid; e < valid * 4; e += kTcBwdThreads) a.dK[tok0 * 4 + e] = nanf_;
-    for (int e = tid; e < d.D; e += kTcBwdThreads) cB[e] = nanf_;
-    for (int e = tid; e < P; e += kTcBwdThreads) a.carryU[((size_t)bh * d.NC + c) * P + e] = nanf_;
+    for (int e = tid; e < valid * 2; e += THREADS) a.dM[tok0 * 2 + e] = nanf_;
+    for (int e = tid; e < valid * 4; e += THREADS) a.dK[tok0 * 4 + e] = nanf_;
+    for (int e = tid; e < d.D; e += THREADS) cB[e] = nanf_;
+    for (int e = tid; e < P; e += THREADS) a.carryU[((size_t)bh * d.NC + c) * P + e] = nanf_;
     if (tid == 0) atomicExch(&g_tc_status, 1);
   }
 #undef SLX_STAMP

@@ -7,44 +7,70 @@ from ctypes import byref
 import pytest
 import torch
 
-from gpu_util import make_scan_inputs
+from gpu_util import make_scan_inputs, oracle_fwd_bwd, run_b200_fwd_bwd, to_np
+from util import rel_err
 
 pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
-@pytest.mark.parametrize("N,T", [(32, 128), (96, 300), (128, 129)])
-def test_gradient_rows_off_a_32_byte_boundary(dtype, N, T):
+@pytest.mark.parametrize("N,T,BH", [(32, 128, 2), (96, 300, 2), (128, 129, 2), (32, 128, 150), (96, 300, 50), (128, 129, 76)])
+def test_gradient_rows_off_a_32_byte_boundary(dtype, N, T, BH):
     """dB and dC leave as whole 32-byte sectors where their base allows it, else as two 16-byte stores: same bits."""
     import slinoss_b200 as sb
     from slinoss_b200 import _lib
 
-    inp = make_scan_inputs(1, 2, T, N, 64, dtype, seed=N, dist="cfg2", with_init=True)
+    inp = make_scan_inputs(1, BH, T, N, 64, dtype, seed=N, dist="cfg2", with_init=True)
     U, M, K, B, C, dY = (inp[k] for k in ("U", "M", "K", "B", "C", "dY"))
-    s = _lib.scan_shape(2, T, 64, N, 128, dtype, _lib.starts_dtype(_lib.scan_shape(2, T, 64, N, 128, dtype)))
+    s = _lib.scan_shape(BH, T, 64, N, 128, dtype, _lib.starts_dtype(_lib.scan_shape(BH, T, 64, N, 128, dtype)))
     NC = (T + 127) // 128
     inc, mch = sb.chunk_increment_b200(U, M, K, B, chunk_size=128)
     starts, _ = sb.state_passing_b200(inc, mch, initial_states=inp["initial_states"])
     starts = starts.to(dtype).contiguous()
     d_inc = torch.randn_like(starts)
-    zdot = torch.randn(2, NC, 2, device="cuda")
+    zdot = torch.randn(BH, NC, 2, device="cuda")
     outs = []
     for off in (0, 8):
-        flat = [torch.zeros(2 * T * 2 * N + 16, device="cuda", dtype=dtype) for _ in range(2)]
-        dB, dC = (f[off:off + 2 * T * 2 * N] for f in flat)
+        flat = [torch.zeros(BH * T * 2 * N + 16, device="cuda", dtype=dtype) for _ in range(2)]
+        dB, dC = (f[off:off + BH * T * 2 * N] for f in flat)
         assert dB.data_ptr() % 32 == 2 * off and dC.data_ptr() % 32 == 2 * off
         dU, dM, dK = torch.empty_like(U), torch.empty_like(M), torch.empty_like(K)
-        cB, cU = torch.empty(2, NC, 2 * N, device="cuda"), torch.empty(2, NC, 64, device="cuda")
+        cB, cU = torch.empty(BH, NC, 2 * N, device="cuda"), torch.empty(BH, NC, 64, device="cuda")
         rc = _lib.lib().slx_chunk_scan_bwd(
             byref(s), U.data_ptr(), M.data_ptr(), K.data_ptr(), B.data_ptr(), C.data_ptr(), None, None,
             starts.data_ptr(), d_inc.data_ptr(), zdot.data_ptr(), dY.data_ptr(), dU.data_ptr(), dM.data_ptr(),
             dK.data_ptr(), dB.data_ptr(), dC.data_ptr(), cB.data_ptr(), cU.data_ptr(), _lib.stream_ptr(U.device))
         _lib.check(rc, "chunk_scan_bwd")
         for f in flat:  # nothing outside the rows
-            assert not f[:off].any() and not f[off + 2 * T * 2 * N:].any()
+            assert not f[:off].any() and not f[off + BH * T * 2 * N:].any()
         outs.append([dU, dM, dK, dB.clone(), dC.clone(), cB, cU])
     for x, y in zip(*outs):
         assert torch.equal(x, y)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("N,T", [(32, 77), (64, 300), (96, 128), (128, 257)])
+@pytest.mark.parametrize("prev", ["none", "half", "fp32"])
+def test_backward_on_either_side_of_one_cta_per_sm(dtype, N, T, prev):
+    """Launches of up to 148 chunks run CTAs of 512 threads over 64-column slabs, larger ones CTAs of 256 over 32: the same
+    operands and products, fp32 sums in another order.  Outputs in half precision may round to the other neighbour (half a
+    step at most differs from one step by the sums' 1e-5); both sides are as far from the oracle as the operands' rounding."""
+    heads = 150 // ((T + 127) // 128) + 1
+    inp = make_scan_inputs(1, heads, T, N, 64, dtype, seed=N, dist="cfg2", with_init=True, streaming=prev != "none")
+    if prev == "fp32":
+        inp["B_prev"], inp["U_prev"] = inp["B_prev"].float() * 1.001, inp["U_prev"].float() * 1.001
+    few = {k: None if v is None else v[:, :3].contiguous() for k, v in inp.items()}
+    large, small = run_b200_fwd_bwd(inp, 128)[2], run_b200_fwd_bwd(few, 128)[2]
+    exact = oracle_fwd_bwd(few)[2]
+    tol = 2e-2 if dtype == torch.bfloat16 else 3e-3
+    for k, x in small.items():
+        if x is None:
+            continue
+        y = large[k][:, :3]
+        assert rel_err(to_np(x), exact[k]) < tol, k
+        assert rel_err(to_np(y), exact[k]) < tol, k
+        assert rel_err(to_np(x), to_np(y)) < (2.0 ** -9 if x.dtype == dtype == torch.bfloat16 else
+                                              2.0 ** -12 if x.dtype == dtype else 1e-4), k
 
 
 @pytest.mark.parametrize("dtype,u", [(torch.bfloat16, 2.0 ** -8), (torch.float16, 2.0 ** -11), (torch.float32, 0.0)])
