@@ -15,11 +15,6 @@
 
 namespace slx {
 
-// tensor maps of the raw C and B operands: (D, T, BH), boxes of 64 columns x 128 tokens, 128-byte swizzle
-struct alignas(64) ScanTileMaps {
-  CUtensorMap C, B;
-};
-
 __device__ int g_tc_status = 0;  // becomes non-zero when a bounded wait ran out
 // Phase-clock stamps (clock64() of the CTA in the middle of the grid, i.e. of a steady-state wave, at the
 // phase boundaries) exist only in builds with
