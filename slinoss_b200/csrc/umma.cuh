@@ -221,9 +221,9 @@ __device__ __forceinline__ bool mbar_wait(uint32_t mbar_saddr, uint32_t parity, 
   }
 }
 // The same for a thread that waits on one barrier, phase after phase, in one word of state: bit 0 = parity of the next
-// wait, bit 31 = a wait ran out.  In the forward chunk kernel launches of up to one CTA per SM take 9.6 us with it and 10.0
-// with mbar_wait and a flag (148 chunks of D 128; 8192 of D 256 0.339 and 0.341 ms); the backward, whose registers are all
-// taken, 1.078 and 1.052 ms.
+// wait, bit 31 = a wait ran out.  With it and with mbar_wait and a flag: the forward chunk kernel 9.85 and 10.25 us for 148
+// chunks of D 128 (one CTA per SM), 0.339 and 0.341 ms for 8192 of D 256; the backward, whose registers are all taken, 1.078
+// and 1.052 ms.
 struct WaitChain {
   uint32_t mbar_saddr, state;
   __device__ __forceinline__ bool ok() const { return static_cast<int>(state) >= 0; }

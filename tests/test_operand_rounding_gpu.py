@@ -86,10 +86,11 @@ def test_operands_are_rounded_once(dtype, N, lo, scale):
     got = run_b200_fwd_bwd(inp, 128)[2]
     for k in NAMES:
         e, want = rel_err(to_np(got[k]), exact[k]), rel_err(model[k], exact[k])
-        # The same number of roundings, drawn once more: norms over >= 1e5 values repeat to a few per cent; dM is a
-        # suffix sum along the chunk, 16 nearly independent errors, so its norm spreads by about 1/sqrt(2 * 16).
+        # The same number of roundings, drawn once more: norms over >= 1e5 values repeat to a few per cent.  dM is a suffix
+        # sum along the chunk, 16 nearly independent errors (a spread of 1/sqrt(2 * 16)), but its sums cancel better than
+        # the model's: 0.48 to 0.91 of the model's error here in float64 arithmetic.
         # A second rounding of both operands of the increment path gives dK 1.3 to 2.9 times the model's error here.
-        assert e < (1.35 if k == "dM" else 1.12) * want, (k, e, want)
+        assert e < 1.12 * want, (k, e, want)
 
 
 @pytest.mark.gpu
